@@ -48,6 +48,29 @@ def test_predictions_match_cpu():
     np.testing.assert_allclose(got, want, rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 32, 33, 296 * 32, 296 * 32 + 1, 20011])
+def test_passes_at_group_and_tile_edges(rows):
+    # 8 rows a warp, 32-row gradient tiles, one more tile a CTA past 296 of
+    # them. A 64-term fp32 sum is off by at most 64 * 2^-24 = 4e-6 of its
+    # terms' magnitudes; three such layers each way stay well below 1e-4 of
+    # the largest value.
+    x, y = _data(max(rows, 4), seed=rows)
+    norm = _norm(x, y)
+    x, y = x[:rows], y[:rows]
+    with tb.Counter() as c:
+        c.model_init(norm, seed=11)
+        p = c.model_params(effective=True)
+        pred = c.model_predict(x)
+        g, loss = c.model_gradients(x, y)
+        again, _ = c.model_gradients(x, y)
+    _, want_loss, want = mlp.forward_backward(p, norm, x, y)
+    want_pred = mlp.predict(p, norm, x)
+    assert np.abs(pred - want_pred).max() <= 1e-4 * np.abs(want_pred).max()
+    assert abs(loss - want_loss) <= 1e-4 * want_loss
+    assert np.abs(g - want).max() <= 1e-4 * np.abs(want).max()
+    np.testing.assert_array_equal(g, again)  # summed in a fixed order
+
+
 def test_training_reduces_loss_and_save_load_roundtrip(tmp_path):
     x, y = _data(20000, seed=2)
     with tb.Counter() as c:

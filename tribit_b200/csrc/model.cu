@@ -14,7 +14,6 @@
 namespace tb {
 namespace {
 
-constexpr uint32_t kFull = 0xffffffffu;
 constexpr int kNorm = 2 * kIn + 2 * kOut;  // in_mean, in_std, out_mean, out_std
 constexpr int kModelThreads = 256;
 constexpr char kMagic[8] = {'T', 'B', 'M', 'L', 'P', '0', '0', '1'};
@@ -23,21 +22,34 @@ __host__ __device__ __forceinline__ bool is_weight(int p) {
   return p < kB1 || (p >= kW2 && p < kB2) || (p >= kW3 && p < kB3);
 }
 
-// Shared-memory image of a model: parameters, W2 transposed (so the backward
-// reads of W2 run across lanes without bank conflicts) and normalisation.
-struct SmemModel {
-  float p[kNumParams];
-  float w2t[kH1 * kH2];
-  float norm[kNorm];
-};
+// Rows a warp carries through the network together (one float4 of a row's
+// features a lane: kRows * kIn / 4 lanes). A weight read from shared memory
+// then serves kRows rows, and a unit's activations are read back four at a time
+// as one broadcast. One row a warp, its activations passed by shuffles, was
+// bound by the shuffles and weight reads: 65,521 rows predicted in 110 us, now
+// 36; forward and backward 161, now 71.
+constexpr int kRows = 8;
+static_assert(kRows * kIn == 4 * 32, "a warp loads kRows rows of features as one float4 a lane");
+constexpr int kW2tStride = kH1 + 1;  // padded: transposing W2 writes 32 different banks
 
-__device__ void load_model(SmemModel& s, const float* __restrict__ eff, const float* __restrict__ norm) {
+// Shared-memory image of a model: parameters, normalisation and, for the
+// backward pass, W2 transposed; and each warp's activations.
+struct SmemModel {
+  float p[kNumParams + 1];
+  float norm[kNorm + 2];
+  float act[kModelThreads / 32][kRows * kH1];
+};
+struct SmemTrain {
+  SmemModel m;
+  float w2t[kH2 * kW2tStride];
+};
+static_assert((kNumParams + 1) % 4 == 0 && (kNorm + 2) % 4 == 0, "activations are read as float4");
+
+__device__ void load_model(SmemModel& s, const float* __restrict__ eff, const float* __restrict__ norm, float* w2t) {
   for (int i = threadIdx.x; i < kNumParams; i += blockDim.x) s.p[i] = eff[i];
-  for (int i = threadIdx.x; i < kH1 * kH2; i += blockDim.x) {
-    const int k = i / kH2, j = i % kH2;
-    s.w2t[j * kH1 + k] = eff[kW2 + i];
-  }
   for (int i = threadIdx.x; i < kNorm; i += blockDim.x) s.norm[i] = norm[i];
+  if (w2t)
+    for (int i = threadIdx.x; i < kH1 * kH2; i += blockDim.x) w2t[(i % kH2) * kW2tStride + i / kH2] = eff[kW2 + i];
   __syncthreads();
 }
 
@@ -50,85 +62,131 @@ struct Acts {  // per-row activations kept for the weight gradients
   float* dy;   // B x kOut
 };
 
-// One warp per row; lane l owns hidden units l and l + 32 of both layers.
-// Computes the normalised prediction; with Train also the backward pass for
-// the MSE loss on normalised targets (scaled by inv_count), storing what the
-// weight-gradient kernel needs.
-template <bool Train>
-__device__ __forceinline__ void row_pass(const SmemModel& s, const float* __restrict__ x, const float* __restrict__ y,
-                                         float inv_count, float out[kOut], const Acts* acts, uint32_t slot,
-                                         float* loss) {
+// a[r], b[r] += sum over the K inputs of row r (at h + r * K, ascending) times
+// columns lane and lane + 32 of w (rows of `stride` floats).
+template <int K>
+__device__ __forceinline__ void dense(const float* __restrict__ w, int stride, const float* __restrict__ h,
+                                      float (&a)[kRows], float (&b)[kRows]) {
   const int lane = threadIdx.x & 31;
-  float xn[kIn];
+#pragma unroll 4
+  for (int k = 0; k < K; k += 4) {
+    float4 x[kRows];
 #pragma unroll
-  for (int q = 0; q < kIn; ++q) xn[q] = (x[q] - s.norm[q]) / s.norm[kIn + q];
-  float z1a = s.p[kB1 + lane], z1b = s.p[kB1 + lane + 32];
+    for (int r = 0; r < kRows; ++r) x[r] = *reinterpret_cast<const float4*>(h + r * K + k);
 #pragma unroll
-  for (int q = 0; q < kIn; ++q) {
-    z1a = fmaf(xn[q], s.p[kW1 + q * kH1 + lane], z1a);
-    z1b = fmaf(xn[q], s.p[kW1 + q * kH1 + lane + 32], z1b);
-  }
-  const float h1a = fmaxf(z1a, 0.f), h1b = fmaxf(z1b, 0.f);
-  float z2a = s.p[kB2 + lane], z2b = s.p[kB2 + lane + 32];
-#pragma unroll 8
-  for (int k = 0; k < 32; ++k) {
-    const float hk = __shfl_sync(kFull, h1a, k);
-    z2a = fmaf(hk, s.p[kW2 + k * kH2 + lane], z2a);
-    z2b = fmaf(hk, s.p[kW2 + k * kH2 + lane + 32], z2b);
-  }
-#pragma unroll 8
-  for (int k = 0; k < 32; ++k) {
-    const float hk = __shfl_sync(kFull, h1b, k);
-    z2a = fmaf(hk, s.p[kW2 + (k + 32) * kH2 + lane], z2a);
-    z2b = fmaf(hk, s.p[kW2 + (k + 32) * kH2 + lane + 32], z2b);
-  }
-  const float h2a = fmaxf(z2a, 0.f), h2b = fmaxf(z2b, 0.f);
+    for (int q = 0; q < 4; ++q) {
+      const float wa = w[(k + q) * stride + lane], wb = w[(k + q) * stride + lane + 32];
 #pragma unroll
-  for (int o = 0; o < kOut; ++o)
-    out[o] = s.p[kB3 + o] + warp_sum(h2a * s.p[kW3 + lane * kOut + o] + h2b * s.p[kW3 + (lane + 32) * kOut + o]);
-  if (!Train) return;
-  float dy[kOut];
+      for (int r = 0; r < kRows; ++r) {
+        const float v = q == 0 ? x[r].x : q == 1 ? x[r].y : q == 2 ? x[r].z : x[r].w;
+        a[r] = fmaf(v, wa, a[r]);
+        b[r] = fmaf(v, wb, b[r]);
+      }
+    }
+  }
+}
+
+// Lane l's two units of every row into the warp's activations.
+__device__ __forceinline__ void put_units(float* act, const float (&a)[kRows], const float (&b)[kRows]) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    act[r * kH1 + lane] = a[r];
+    act[r * kH1 + lane + 32] = b[r];
+  }
+  __syncwarp();
+}
+
+// kRows rows a warp; lane l owns hidden units l and l + 32 of both layers.
+// Computes the normalised predictions of the rows x(r), r < rows (the others
+// repeat row 0 and are not stored); with Train also the backward pass for the
+// MSE loss on normalised targets y(r) (scaled by inv_count), storing what the
+// weight-gradient kernel needs in slots slot .. slot + rows and returning the
+// rows' summed squared error.
+template <bool Train, class RowOf>
+__device__ __forceinline__ float rows_pass(const SmemModel& s, const float* w2t, float* act, const float* __restrict__ X,
+                                           const float* __restrict__ Y, const RowOf& row_of, int rows, float inv_count,
+                                           float (&out)[kRows][kOut], const Acts* acts, uint32_t slot) {
+  const int lane = threadIdx.x & 31;
+  {
+    const int r = lane / (kIn / 4), q = (lane % (kIn / 4)) * 4;
+    const float4 x = *reinterpret_cast<const float4*>(X + (size_t)row_of(r < rows ? r : 0) * kIn + q);
+    const float4 v = make_float4((x.x - s.norm[q]) / s.norm[kIn + q], (x.y - s.norm[q + 1]) / s.norm[kIn + q + 1],
+                                 (x.z - s.norm[q + 2]) / s.norm[kIn + q + 2],
+                                 (x.w - s.norm[q + 3]) / s.norm[kIn + q + 3]);
+    __syncwarp();
+    *reinterpret_cast<float4*>(act + r * kIn + q) = v;
+    if (Train && r < rows) *reinterpret_cast<float4*>(acts->xn + (size_t)(slot + r) * kIn + q) = v;
+    __syncwarp();
+  }
+  float a[kRows], b[kRows];  // the layer's pre-activations
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) a[r] = s.p[kB1 + lane], b[r] = s.p[kB1 + lane + 32];
+  dense<kIn>(s.p + kW1, kH1, act, a, b);
+  uint32_t on1 = 0;  // bits 2r, 2r + 1: row r's two units are active
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    if (Train) on1 |= (a[r] > 0.f ? 1u << (2 * r) : 0u) | (b[r] > 0.f ? 2u << (2 * r) : 0u);
+    a[r] = fmaxf(a[r], 0.f), b[r] = fmaxf(b[r], 0.f);
+    if (Train && r < rows) {
+      acts->h1[(size_t)(slot + r) * kH1 + lane] = a[r];
+      acts->h1[(size_t)(slot + r) * kH1 + lane + 32] = b[r];
+    }
+  }
+  put_units(act, a, b);
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) a[r] = s.p[kB2 + lane], b[r] = s.p[kB2 + lane + 32];
+  dense<kH1>(s.p + kW2, kH2, act, a, b);
+  uint32_t on2 = 0;
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    if (Train) on2 |= (a[r] > 0.f ? 1u << (2 * r) : 0u) | (b[r] > 0.f ? 2u << (2 * r) : 0u);
+    const float h2a = fmaxf(a[r], 0.f), h2b = fmaxf(b[r], 0.f);
+#pragma unroll
+    for (int o = 0; o < kOut; ++o)
+      out[r][o] = s.p[kB3 + o] + warp_sum(h2a * s.p[kW3 + lane * kOut + o] + h2b * s.p[kW3 + (lane + 32) * kOut + o]);
+    if (Train && r < rows) {
+      acts->h2[(size_t)(slot + r) * kH2 + lane] = h2a;
+      acts->h2[(size_t)(slot + r) * kH2 + lane + 32] = h2b;
+    }
+  }
+  if constexpr (!Train) return 0.f;
   float sq = 0.f;
 #pragma unroll
-  for (int o = 0; o < kOut; ++o) {
-    const float t = (y[o] - s.norm[2 * kIn + o]) / s.norm[2 * kIn + kOut + o];
-    const float e = out[o] - t;
-    sq += e * e;
-    dy[o] = 2.f * e * inv_count;
-  }
-  float dh2a = 0.f, dh2b = 0.f;
+  for (int r = 0; r < kRows; ++r) {
+    float dh2a = 0.f, dh2b = 0.f;
+    const size_t yr = (size_t)row_of(r < rows ? r : 0) * kOut;
 #pragma unroll
-  for (int o = 0; o < kOut; ++o) {
-    dh2a = fmaf(s.p[kW3 + lane * kOut + o], dy[o], dh2a);
-    dh2b = fmaf(s.p[kW3 + (lane + 32) * kOut + o], dy[o], dh2b);
+    for (int o = 0; o < kOut; ++o) {
+      const float t = (Y[yr + o] - s.norm[2 * kIn + o]) / s.norm[2 * kIn + kOut + o];
+      const float e = out[r][o] - t;
+      const float dy = 2.f * e * inv_count;
+      dh2a = fmaf(s.p[kW3 + lane * kOut + o], dy, dh2a);
+      dh2b = fmaf(s.p[kW3 + (lane + 32) * kOut + o], dy, dh2b);
+      if (r < rows) {
+        sq += e * e;
+        if (lane == o) acts->dy[(size_t)(slot + r) * kOut + o] = dy;
+      }
+    }
+    a[r] = (on2 >> (2 * r)) & 1u ? dh2a : 0.f;
+    b[r] = (on2 >> (2 * r)) & 2u ? dh2b : 0.f;
+    if (r < rows) {
+      acts->dz2[(size_t)(slot + r) * kH2 + lane] = a[r];
+      acts->dz2[(size_t)(slot + r) * kH2 + lane + 32] = b[r];
+    }
   }
-  const float dz2a = z2a > 0.f ? dh2a : 0.f, dz2b = z2b > 0.f ? dh2b : 0.f;
-  float dh1a = 0.f, dh1b = 0.f;
-#pragma unroll 8
-  for (int j = 0; j < 32; ++j) {
-    const float dj = __shfl_sync(kFull, dz2a, j);
-    dh1a = fmaf(s.w2t[j * kH1 + lane], dj, dh1a);
-    dh1b = fmaf(s.w2t[j * kH1 + lane + 32], dj, dh1b);
-  }
-#pragma unroll 8
-  for (int j = 0; j < 32; ++j) {
-    const float dj = __shfl_sync(kFull, dz2b, j);
-    dh1a = fmaf(s.w2t[(j + 32) * kH1 + lane], dj, dh1a);
-    dh1b = fmaf(s.w2t[(j + 32) * kH1 + lane + 32], dj, dh1b);
-  }
-  const float dz1a = z1a > 0.f ? dh1a : 0.f, dz1b = z1b > 0.f ? dh1b : 0.f;
-  const size_t r64 = (size_t)slot * 64;
-  if (lane < kIn) acts->xn[(size_t)slot * kIn + lane] = (x[lane] - s.norm[lane]) / s.norm[kIn + lane];
-  acts->h1[r64 + lane] = h1a;
-  acts->h1[r64 + lane + 32] = h1b;
-  acts->dz1[r64 + lane] = dz1a;
-  acts->dz1[r64 + lane + 32] = dz1b;
-  acts->h2[r64 + lane] = h2a;
-  acts->h2[r64 + lane + 32] = h2b;
-  acts->dz2[r64 + lane] = dz2a;
-  acts->dz2[r64 + lane + 32] = dz2b;
-  if (lane < kOut) acts->dy[(size_t)slot * kOut + lane] = dy[lane];
-  if (lane == 0) atomicAdd(loss, sq);
+  put_units(act, a, b);
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) a[r] = 0.f, b[r] = 0.f;
+  dense<kH2>(w2t, kW2tStride, act, a, b);
+#pragma unroll
+  for (int r = 0; r < kRows; ++r)
+    if (r < rows) {
+      acts->dz1[(size_t)(slot + r) * kH1 + lane] = (on1 >> (2 * r)) & 1u ? a[r] : 0.f;
+      acts->dz1[(size_t)(slot + r) * kH1 + lane + 32] = (on1 >> (2 * r)) & 2u ? b[r] : 0.f;
+    }
+  return sq;
 }
 
 // Forward + backward over rows idx[r0 .. r0 + B) (idx null: identity).
@@ -138,41 +196,109 @@ __global__ void __launch_bounds__(kModelThreads) k_fwd_bwd(const float* __restri
                                                             const float* __restrict__ norm, float inv_count, Acts acts,
                                                             float* loss) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmemModel& s = *reinterpret_cast<SmemModel*>(smem_raw);
-  load_model(s, eff, norm);
+  SmemTrain& st = *reinterpret_cast<SmemTrain*>(smem_raw);
+  load_model(st.m, eff, norm, st.w2t);
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = warp; i < B; i += nw) {
-    const uint32_t row = idx ? idx[r0 + i] : r0 + i;
-    float out[kOut];
-    row_pass<true>(s, X + (size_t)row * kIn, Y + (size_t)row * kOut, inv_count, out, &acts, i, loss);
+  float* act = st.m.act[threadIdx.x >> 5];
+  float sq = 0.f;
+  for (uint64_t i = (uint64_t)warp * kRows; i < B; i += (uint64_t)nw * kRows) {
+    const uint32_t base = r0 + (uint32_t)i;
+    float out[kRows][kOut];
+    sq += rows_pass<true>(st.m, st.w2t, act, X, Y, [&](int r) { return idx ? idx[base + r] : base + r; },
+                          (int)min((uint64_t)kRows, B - i), inv_count, out, &acts, (uint32_t)i);
   }
+  if ((threadIdx.x & 31) == 0 && sq != 0.f) atomicAdd(loss, sq);
 }
 
-// grad[p] = sum over the B rows of the batch, in row order (deterministic).
-__global__ void k_wgrad(Acts a, uint32_t B, float* __restrict__ grad) {
+// The weight gradients in two steps: CTA c sums rows [c R, c R + R) of the
+// batch into part[c] (every parameter's sum in registers, rows staged kGradTile
+// at a time), and k_wgrad_sum adds the CTAs' sums in order, so the result depends on the
+// batch size alone. The 64 x 64 block is 4 x 4 sums a thread (two 16-byte
+// shared reads for 16 products). One thread a parameter walking all rows left
+// all but 22 CTAs of the chip idle, each step a pair of dependent L2 reads:
+// 65,521 rows in 4,656 us, now 99.
+constexpr uint32_t kGradTile = 32;    // rows staged at a time
+constexpr uint32_t kGradCtas = 296;   // two a multiprocessor
+__host__ __device__ inline uint32_t wgrad_rows(uint32_t B) {  // rows a CTA sums: whole tiles
+  const uint32_t per = (uint32_t)(((uint64_t)B + kGradCtas - 1) / kGradCtas);
+  return (per + kGradTile - 1) / kGradTile * kGradTile;
+}
+__host__ __device__ inline uint32_t wgrad_ctas(uint32_t B) {
+  const uint32_t R = wgrad_rows(B);
+  return (uint32_t)(((uint64_t)B + R - 1) / R);
+}
+
+__global__ void __launch_bounds__(256) k_wgrad(Acts a, uint32_t B, float* __restrict__ part) {
+  __shared__ __align__(16) float xn[kGradTile][kIn], h1[kGradTile][kH1], z1[kGradTile][kH1], h2[kGradTile][kH2],
+      z2[kGradTile][kH2], dy[kGradTile][kOut];
+  const int t = threadIdx.x, ti = t >> 4, tj = (t & 15) * 4;
+  const uint32_t R = wgrad_rows(B);
+  const uint32_t c0 = blockIdx.x * R;
+  const uint32_t c1 = (uint32_t)min((uint64_t)B, (uint64_t)c0 + R);
+  float g1[4] = {0.f, 0.f, 0.f, 0.f}, g2[4][4] = {}, g3 = 0.f, gb = 0.f;
+  auto stage = [&](float* dst, const float* src, uint32_t words) {  // words: a multiple of 4, but for dy
+    if (words % 4 == 0)
+      for (uint32_t i = t; i < words / 4; i += 256)
+        reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(src)[i];
+    else
+      for (uint32_t i = t; i < words; i += 256) dst[i] = src[i];
+  };
+  for (uint32_t r0 = c0; r0 < c1; r0 += kGradTile) {
+    const uint32_t n = min(kGradTile, c1 - r0);
+    __syncthreads();
+    stage(&xn[0][0], a.xn + (size_t)r0 * kIn, n * kIn);
+    stage(&h1[0][0], a.h1 + (size_t)r0 * kH1, n * kH1);
+    stage(&z1[0][0], a.dz1 + (size_t)r0 * kH1, n * kH1);
+    stage(&h2[0][0], a.h2 + (size_t)r0 * kH2, n * kH2);
+    stage(&z2[0][0], a.dz2 + (size_t)r0 * kH2, n * kH2);
+    stage(&dy[0][0], a.dy + (size_t)r0 * kOut, n * kOut);
+    __syncthreads();
+    for (uint32_t r = 0; r < n; ++r) {
+      const float4 h = *reinterpret_cast<const float4*>(&h1[r][ti * 4]);
+      const float4 z = *reinterpret_cast<const float4*>(&z2[r][tj]);
+      const float4 d = *reinterpret_cast<const float4*>(&z1[r][tj]);
+      const float x = xn[r][ti];
+      const float hv[4] = {h.x, h.y, h.z, h.w}, zv[4] = {z.x, z.y, z.z, z.w}, dv[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        g1[i] = fmaf(x, dv[i], g1[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) g2[i][j] = fmaf(hv[i], zv[j], g2[i][j]);
+      }
+      if (t < kH2 * kOut) g3 = fmaf(h2[r][t / kOut], dy[r][t % kOut], g3);
+      if (t < kH1)
+        gb += z1[r][t];
+      else if (t < kH1 + kH2)
+        gb += z2[r][t - kH1];
+      else if (t < kH1 + kH2 + kOut)
+        gb += dy[r][t - kH1 - kH2];
+    }
+  }
+  float* out = part + (size_t)blockIdx.x * kNumParams;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    out[kW1 + ti * kH1 + tj + i] = g1[i];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[kW2 + (ti * 4 + i) * kH2 + tj + j] = g2[i][j];
+  }
+  if (t < kH2 * kOut) out[kW3 + t] = g3;
+  if (t < kH1)
+    out[kB1 + t] = gb;
+  else if (t < kH1 + kH2)
+    out[kB2 + t - kH1] = gb;
+  else if (t < kH1 + kH2 + kOut)
+    out[kB3 + t - kH1 - kH2] = gb;
+}
+static_assert(kIn == 16 && kH1 == 64 && kH2 == 64 && kH2 * kOut <= 256 && kH1 + kH2 + kOut <= 256,
+              "k_wgrad's thread layout");
+
+__global__ void k_wgrad_sum(const float* __restrict__ part, uint32_t ctas, float* __restrict__ grad) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kNumParams) return;
   float g = 0.f;
-  if (p < kB1) {
-    const int i = p / kH1, j = p % kH1;
-    for (uint32_t r = 0; r < B; ++r) g = fmaf(a.xn[(size_t)r * kIn + i], a.dz1[(size_t)r * kH1 + j], g);
-  } else if (p < kW2) {
-    const int j = p - kB1;
-    for (uint32_t r = 0; r < B; ++r) g += a.dz1[(size_t)r * kH1 + j];
-  } else if (p < kB2) {
-    const int k = (p - kW2) / kH2, j = (p - kW2) % kH2;
-    for (uint32_t r = 0; r < B; ++r) g = fmaf(a.h1[(size_t)r * kH1 + k], a.dz2[(size_t)r * kH2 + j], g);
-  } else if (p < kW3) {
-    const int j = p - kB2;
-    for (uint32_t r = 0; r < B; ++r) g += a.dz2[(size_t)r * kH2 + j];
-  } else if (p < kB3) {
-    const int k = (p - kW3) / kOut, o = (p - kW3) % kOut;
-    for (uint32_t r = 0; r < B; ++r) g = fmaf(a.h2[(size_t)r * kH2 + k], a.dy[(size_t)r * kOut + o], g);
-  } else {
-    const int o = p - kB3;
-    for (uint32_t r = 0; r < B; ++r) g += a.dy[(size_t)r * kOut + o];
-  }
+#pragma unroll 8
+  for (uint32_t c = 0; c < ctas; ++c) g += part[(size_t)c * kNumParams + p];
   grad[p] = g;
 }
 
@@ -205,16 +331,22 @@ __global__ void __launch_bounds__(kModelThreads) k_predict(const float* __restri
                                                             const float* __restrict__ norm, float* __restrict__ Y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmemModel& s = *reinterpret_cast<SmemModel*>(smem_raw);
-  load_model(s, eff, norm);
+  load_model(s, eff, norm, nullptr);
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t r = warp; r < rows; r += nw) {
-    float out[kOut];
-    row_pass<false>(s, X + (size_t)r * kIn, nullptr, 0.f, out, nullptr, 0, nullptr);
-    if ((threadIdx.x & 31) < kOut) {
-      const int o = threadIdx.x & 31;
-      Y[(size_t)r * kOut + o] = out[o] * s.norm[2 * kIn + kOut + o] + s.norm[2 * kIn + o];
-    }
+  const int lane = threadIdx.x & 31;
+  for (uint64_t i = (uint64_t)warp * kRows; i < rows; i += (uint64_t)nw * kRows) {
+    const uint32_t base = (uint32_t)i, n = (uint32_t)min((uint64_t)kRows, rows - i);
+    float out[kRows][kOut];
+    rows_pass<false>(s, nullptr, s.act[threadIdx.x >> 5], X, nullptr, [&](int r) { return base + r; }, (int)n, 0.f, out,
+                     nullptr, 0);
+    float v = 0.f;  // lane r * kOut + o: output o of row r
+#pragma unroll
+    for (int q = 0; q < kRows * kOut; ++q)
+      if (lane == q) v = out[q / kOut][q % kOut];
+    const int o = lane % kOut;
+    if (lane < (int)n * kOut)
+      Y[(size_t)base * kOut + lane] = v * s.norm[2 * kIn + kOut + o] + s.norm[2 * kIn + o];
   }
 }
 
@@ -225,43 +357,52 @@ __global__ void __launch_bounds__(kModelThreads) k_dispatch(const float* __restr
                                                              uint8_t* __restrict__ variant_of) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmemModel& s = *reinterpret_cast<SmemModel*>(smem_raw);
-  load_model(s, eff, norm);
+  load_model(s, eff, norm, nullptr);
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t rb = warp; rb < nrb; rb += nw) {
-    float out[kOut];
-    row_pass<false>(s, feat + (size_t)rb * kIn, nullptr, 0.f, out, nullptr, 0, nullptr);
-    if ((threadIdx.x & 31) == 0) {
+  const int lane = threadIdx.x & 31;
+  for (uint64_t i = (uint64_t)warp * kRows; i < nrb; i += (uint64_t)nw * kRows) {
+    const uint32_t base = (uint32_t)i, n = (uint32_t)min((uint64_t)kRows, nrb - i);
+    float out[kRows][kOut];
+    rows_pass<false>(s, nullptr, s.act[threadIdx.x >> 5], feat, nullptr, [&](int r) { return base + r; }, (int)n, 0.f,
+                     out, nullptr, 0);
+    float y[kOut] = {};  // lane r: the outputs of row r
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int o = 0; o < kOut; ++o)
+        if (lane == r) y[o] = out[r][o];
+    if (lane < (int)n) {
       // Bit tiles only where the block fits one tile (span of 1..kTileMaxK
       // column blocks); elsewhere the tile kernel would sweep the block's rows
       // one at a time on a single warp.
-      const float span = feat[(size_t)rb * kIn + kFeatSpan];
+      const float span = feat[(size_t)(base + lane) * kIn + kFeatSpan];
       const bool tile_ok = span > 0.f && span <= log2f(1.f + (float)kTileMaxK) + 1e-4f;
       int best = -1;
       float bt = 0.f;
+#pragma unroll
       for (int o = 0; o < kOut; ++o) {
         if (o == TRIBIT_VARIANT_MMA && !tile_ok) continue;
-        const float t = out[o] * s.norm[2 * kIn + kOut + o] + s.norm[2 * kIn + o];
+        const float t = y[o] * s.norm[2 * kIn + kOut + o] + s.norm[2 * kIn + o];
         if (best < 0 || t < bt) bt = t, best = o;
       }
-      variant_of[rb] = (uint8_t)best;
+      variant_of[base + lane] = (uint8_t)best;
     }
   }
 }
 
-constexpr size_t kModelSmem = sizeof(SmemModel);
-
 void set_smem_attrs() {
   once_per_device<1>([] {
-    TB_CUDA(cudaFuncSetAttribute(k_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kModelSmem));
-    TB_CUDA(cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kModelSmem));
-    TB_CUDA(cudaFuncSetAttribute(k_dispatch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kModelSmem));
+    TB_CUDA(cudaFuncSetAttribute(k_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemTrain)));
+    TB_CUDA(cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemModel)));
+    TB_CUDA(cudaFuncSetAttribute(k_dispatch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemModel)));
   });
 }
 
+// CTAs for `rows` rows, kRows a warp at a time.
 unsigned grid_warps(uint64_t rows) {
-  const uint64_t g = ceil_div<uint64_t>(rows, kModelThreads / 32);
-  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g, 148ull * 8));
+  const uint64_t g = ceil_div<uint64_t>(rows, kModelThreads / 32 * kRows);
+  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g, 148ull * 3));
 }
 
 struct TrainBuffers {
@@ -269,6 +410,7 @@ struct TrainBuffers {
   float* Y = nullptr;
   uint32_t* idx = nullptr;
   float* loss = nullptr;
+  float* part = nullptr;  // wgrad_ctas(B) x kNumParams: the gradient's partial sums
   Acts acts{};
 };
 
@@ -284,6 +426,7 @@ TrainBuffers layout_train(Arena& ar, uint64_t rows, uint32_t B) {
   t.acts.h2 = ar.take<float>((uint64_t)B * kH2);
   t.acts.dz2 = ar.take<float>((uint64_t)B * kH2);
   t.acts.dy = ar.take<float>((uint64_t)B * kOut);
+  t.part = ar.take<float>((uint64_t)wgrad_ctas(B) * kNumParams);
   return t;
 }
 
@@ -297,6 +440,15 @@ TrainBuffers stage_training(tribit_context* c, const float* X, const float* Y, u
   TB_CUDA(cudaMemcpyAsync(t.X, X, rows * kIn * sizeof(float), cudaMemcpyHostToDevice, c->st));
   if (Y) TB_CUDA(cudaMemcpyAsync(t.Y, Y, rows * kOut * sizeof(float), cudaMemcpyHostToDevice, c->st));
   return t;
+}
+
+// The gradient of the batch of B rows in t.acts (B at most the batch t was laid out for).
+void weight_gradients(const TrainBuffers& t, uint32_t B, float* grad, cudaStream_t st) {
+  const uint32_t ctas = wgrad_ctas(B);
+  k_wgrad<<<ctas, 256, 0, st>>>(t.acts, B, t.part);
+  TB_LAUNCH_CHECK();
+  k_wgrad_sum<<<(kNumParams + 63) / 64, 64, 0, st>>>(t.part, ctas, grad);
+  TB_LAUNCH_CHECK();
 }
 
 void require_model(tribit_context* c) {
@@ -333,7 +485,7 @@ void model_refresh_eff(DeviceModel& m, cudaStream_t st) {
 void model_dispatch(const DeviceModel& m, const float* features, uint32_t nrb, uint8_t* variant_of, cudaStream_t st) {
   if (nrb == 0) return;
   set_smem_attrs();
-  k_dispatch<<<grid_warps(nrb), kModelThreads, kModelSmem, st>>>(features, nrb, m.eff, m.norm, variant_of);
+  k_dispatch<<<grid_warps(nrb), kModelThreads, sizeof(SmemModel), st>>>(features, nrb, m.eff, m.norm, variant_of);
   TB_LAUNCH_CHECK();
 }
 
@@ -426,8 +578,8 @@ tribit_status tribit_model_predict(tribit_context* c, const float* x, uint64_t r
     if (rows == 0) return;
     tb::set_smem_attrs();
     tb::TrainBuffers t = tb::stage_training(c, x, nullptr, rows, 1);
-    tb::k_predict<<<tb::grid_warps(rows), tb::kModelThreads, tb::kModelSmem, c->st>>>(t.X, (uint32_t)rows,
-                                                                                     c->model.eff, c->model.norm, t.Y);
+    tb::k_predict<<<tb::grid_warps(rows), tb::kModelThreads, sizeof(tb::SmemModel), c->st>>>(
+        t.X, (uint32_t)rows, c->model.eff, c->model.norm, t.Y);
     TB_LAUNCH_CHECK();
     TB_CUDA(cudaMemcpyAsync(y, t.Y, rows * tb::kOut * sizeof(float), cudaMemcpyDeviceToHost, c->st));
     TB_CUDA(cudaStreamSynchronize(c->st));
@@ -444,11 +596,10 @@ tribit_status tribit_model_gradients(tribit_context* c, const float* x, const fl
     tb::TrainBuffers t = tb::stage_training(c, x, y, rows, (uint32_t)rows);
     TB_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(float), c->st));
     const float inv = 1.f / (float)(tb::kOut * rows);
-    tb::k_fwd_bwd<<<tb::grid_warps(rows), tb::kModelThreads, tb::kModelSmem, c->st>>>(
+    tb::k_fwd_bwd<<<tb::grid_warps(rows), tb::kModelThreads, sizeof(tb::SmemTrain), c->st>>>(
         t.X, t.Y, nullptr, 0, (uint32_t)rows, c->model.eff, c->model.norm, inv, t.acts, t.loss);
     TB_LAUNCH_CHECK();
-    tb::k_wgrad<<<(tb::kNumParams + 255) / 256, 256, 0, c->st>>>(t.acts, (uint32_t)rows, c->model.grad);
-    TB_LAUNCH_CHECK();
+    tb::weight_gradients(t, (uint32_t)rows, c->model.grad, c->st);
     float loss = 0.f;
     TB_CUDA(cudaMemcpyAsync(grad, c->model.grad, tb::kNumParams * sizeof(float), cudaMemcpyDeviceToHost, c->st));
     TB_CUDA(cudaMemcpyAsync(&loss, t.loss, sizeof(float), cudaMemcpyDeviceToHost, c->st));
@@ -477,11 +628,10 @@ tribit_status tribit_model_train(tribit_context* c, const float* x, const float*
       for (uint64_t r0 = 0; r0 < rows; r0 += B) {
         const uint32_t nb = (uint32_t)std::min<uint64_t>(B, rows - r0);
         const float inv = 1.f / (float)(tb::kOut * nb);
-        tb::k_fwd_bwd<<<tb::grid_warps(nb), tb::kModelThreads, tb::kModelSmem, c->st>>>(
+        tb::k_fwd_bwd<<<tb::grid_warps(nb), tb::kModelThreads, sizeof(tb::SmemTrain), c->st>>>(
             t.X, t.Y, t.idx, (uint32_t)r0, nb, c->model.eff, c->model.norm, inv, t.acts, t.loss);
         TB_LAUNCH_CHECK();
-        tb::k_wgrad<<<(tb::kNumParams + 255) / 256, 256, 0, c->st>>>(t.acts, nb, c->model.grad);
-        TB_LAUNCH_CHECK();
+        tb::weight_gradients(t, nb, c->model.grad, c->st);
         const int step = ++c->model.steps;
         tb::k_adam<<<(tb::kNumParams + 255) / 256, 256, 0, c->st>>>(
             c->model.master, c->model.eff, c->model.m, c->model.v, c->model.grad, lr, b1, b2, eps,
