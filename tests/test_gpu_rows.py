@@ -1,8 +1,8 @@
 """Row construction of the preprocessing (a counting sort of the oriented
-entries by their lower endpoint, then a sort + dedup of each row): rows of
-every sorting class -- the warp's register sorts (up to 1,024 entries), a
-CTA's shared-memory sort (up to 8,192) and its global-scratch sort (longer) --
-with duplicated and reversed entries, against the oracle."""
+entries by their lower endpoint, then a sort + dedup of each row): rows of every
+sorting class -- lane groups and the warp's register sorts (up to 1,024
+entries), a CTA's column bitmaps and its bitonic sorts in shared memory and in
+global scratch (longer) -- with duplicated and reversed entries, against the oracle."""
 import numpy as np
 import pytest
 
@@ -61,3 +61,45 @@ def test_self_loops_and_empty_rows():
     with tb.Counter() as c:
         r = c.count_edges(e, 1000)
         assert (r.triangles, r.edges) == (comb(40), 40 * 39 // 2)
+
+
+def fans(rows, n):
+    """In id order, vertex 2 i owns a row of rows[i] = (length, first, stride)
+    columns, and the columns of each row are joined in a path."""
+    parts = []
+    for i, (length, first, stride) in enumerate(rows):
+        cols = first + stride * np.arange(length, dtype=np.uint64)
+        assert cols[-1] < n and first > 2 * len(rows)
+        parts.append((np.uint64(2 * i) << np.uint64(32)) | cols)
+        parts.append((cols[:-1] << np.uint64(32)) | cols[1:])
+    return np.concatenate(parts)
+
+
+@pytest.mark.parametrize("name, n, rows", [
+    # each class of the warp and lane-group sorts and the first CTA row, one block to many
+    ("classes", 40000, [(k, 2000 + 7 * k, 1 + k % 37) for k in (1, 2, 8, 9, 16, 17, 31, 32, 33, 64, 65, 128, 129, 256,
+                                                               257, 512, 513, 1023, 1024, 1025)]),
+    # a column window exactly, one block past it (then bitonic), and rows of several windows
+    ("windows", 3_000_000, [(1025, 32, 360), (1440, 32, 256), (1441, 32, 256), (2048, 32, 190), (2049, 64, 1000),
+                            (8192, 64, 300), (8193, 96, 299)]),
+    # rows of too few entries for their windows: bitonic in shared memory and in global scratch
+    ("bitonic", 9_000_000, [(1100, 1000, 8000), (2047, 1000, 4000), (8192, 1001, 1000), (9000, 1002, 999)]),
+])
+def test_rows_of_every_length_and_span(name, n, rows):
+    e = noisy(fans(rows, n), seed=len(rows), copies=1 if name == "classes" else 2)
+    want, m = oracle.count(e, n)
+    with tb.Counter(order="id") as c:
+        r = c.count_edges(e, n)
+        assert (r.triangles, r.edges) == (want, m)
+
+
+def test_rows_between_long_runs_of_empty_rows():
+    # 2^20 ids between one clique and the next, a long row among short ones,
+    # and rows that end at and cross the emitting warps' shares.
+    n = 5 << 20
+    e = np.concatenate([clique(70, base=k << 20) for k in range(5)] + [fans([(3000, 1 << 19, 5), (64, 1 << 19, 64)], n)])
+    want, m = oracle.count(e, n)
+    for order in ("id", "degree"):
+        with tb.Counter(order=order) as c:
+            r = c.count_edges(noisy(e, seed=3, copies=2), n)
+            assert (r.triangles, r.edges) == (want, m)

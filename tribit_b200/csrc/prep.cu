@@ -206,9 +206,22 @@ __global__ void __launch_bounds__(kSortThreads) k_row_keys_hist(PrepInput in, co
 // (measured: RMAT-22 13.3 ms without, 13.6-14.1 with; RMAT-24 50.8 -> 48.6).
 constexpr uint64_t kPresortMinEntries = TB_PRESORT_MIN;
 constexpr uint32_t kPad = 0xFFFFFFFFu;  // sorts last; no vertex has this rank (n < 2^32)
+constexpr uint32_t kShortRow = 32;       // longer rows go to the lists of k_sort_long
 constexpr uint32_t kWarpSortMax = 1024;  // longer rows are sorted by a CTA
-constexpr uint32_t kCtaSortThreads = 1024;
-constexpr uint32_t kCtaSortSmem = 8192;  // longer rows are sorted in global scratch
+constexpr uint32_t kLongThreads = 256;
+static_assert(kLongThreads == kScanThreads, "window_sort scans its CTA's threads");
+constexpr uint32_t kBitWords = 11520;    // 45 KiB: a bitmap of 368,640 columns (four CTAs an SM)
+constexpr uint32_t kCtaSortSmem = 8192;  // bitonic rows longer than this are sorted in global scratch
+
+// Rows of more than kShortRow entries, listed by k_sort_rows: CTA rows (over
+// kWarpSortMax) from the front of rows[], warp rows from its end (index n - i).
+// The lists spread the long rows over the whole grid: under degree order the
+// top row blocks hold 32 rows of hundreds of entries each, and one warp a
+// block left them to a few warps (RMAT-20: the row sort 607 us, the emit 487).
+struct LongRows {
+  uint32_t* rows;   // n + 1
+  uint32_t* count;  // [0] CTA rows, [1] warp rows
+};
 
 // Bitonic sort of the warp's 32 K values, value r * 32 + lane in x[r] of
 // lane lane, ascending.
@@ -317,199 +330,388 @@ __device__ __forceinline__ void sort_short_rows(uint32_t pending, uint32_t s_l, 
   }
 }
 
-// One warp per 32-row block: rows of up to 8 and 16 entries are sorted four
-// and two at a time in lane groups, rows of up to kWarpSortMax one at a time
-// in registers; longer rows go to big[] for k_sort_big_rows. Row u holds
-// nbr[start[u], end[u]). rows[u] = (distinct << 32) | blocks, rows[n] = 0.
-// (Four CTAs of 256 per SM: 64 registers, no spills.)
-__global__ void __launch_bounds__(256, 4)
-    k_sort_rows(const uint32_t* __restrict__ start, const uint32_t* __restrict__ end, uint32_t n,
-                uint32_t* __restrict__ nbr, uint64_t* __restrict__ rows, uint32_t* __restrict__ big,
-                uint32_t* __restrict__ nbig) {
+// One warp per `per` rows (at most 32): rows of up to 8 and 16 entries are
+// sorted four and two at a time in lane groups, up to kShortRow one at a time;
+// longer rows are listed for k_sort_long. Row u holds nbr[start[u], end[u]).
+// rows[u] = (distinct << 32) | blocks, rows[n] = 0.
+__global__ void __launch_bounds__(256)
+    k_sort_rows(const uint32_t* __restrict__ start, const uint32_t* __restrict__ end, uint32_t n, uint32_t per,
+                uint32_t* __restrict__ nbr, uint64_t* __restrict__ rows, LongRows lng) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   if (warp == 0 && lane == 0) rows[n] = 0;
-  for (uint32_t ubase = warp * 32; ubase < n; ubase += nwarps * 32) {
-    const uint32_t u = ubase + lane;
-    const bool here = u < n;
+  for (uint64_t ub = (uint64_t)warp * per; ub < n; ub += (uint64_t)nwarps * per) {
+    const uint32_t ubase = (uint32_t)ub, u = ubase + lane;
+    const bool here = lane < per && ub + lane < n;
     const uint32_t s_l = here ? start[u] : 0u, L_l = here ? end[u] - s_l : 0u;
     if (here && L_l == 0) rows[u] = 0;
+    const uint32_t cta = __ballot_sync(kFull, L_l > kWarpSortMax);
+    const uint32_t mid = __ballot_sync(kFull, L_l > kShortRow && L_l <= kWarpSortMax);
+    if (cta | mid) {
+      const uint32_t lt = (1u << lane) - 1u;
+      uint32_t at = 0;
+      if (lane == 0 && cta) at = atomicAdd(&lng.count[0], (uint32_t)__popc(cta));
+      if (lane == 1 && mid) at = atomicAdd(&lng.count[1], (uint32_t)__popc(mid));
+      const uint32_t c0 = __shfl_sync(kFull, at, 0), m0 = __shfl_sync(kFull, at, 1);
+      if ((cta >> lane) & 1u) lng.rows[c0 + __popc(cta & lt)] = u;
+      if ((mid >> lane) & 1u) lng.rows[n - (m0 + __popc(mid & lt))] = u;
+    }
     sort_short_rows<8>(__ballot_sync(kFull, L_l >= 1 && L_l <= 8), s_l, L_l, ubase, nbr, rows);
     sort_short_rows<16>(__ballot_sync(kFull, L_l > 8 && L_l <= 16), s_l, L_l, ubase, nbr, rows);
-    sort_short_rows<32>(__ballot_sync(kFull, L_l > 16 && L_l <= 32), s_l, L_l, ubase, nbr, rows);
-    uint32_t longer = __ballot_sync(kFull, L_l > 32);
-    while (longer) {
-      const uint32_t r = __ffs(longer) - 1;
-      longer &= longer - 1;
-      const uint32_t s = __shfl_sync(kFull, s_l, r), L = __shfl_sync(kFull, L_l, r);
-      uint32_t* a = nbr + s;
-      uint64_t res;
-      if (L <= 64) {
-        res = warp_sort_row<2>(a, L);
-      } else if (L <= 128) {
-        res = warp_sort_row<4>(a, L);
-      } else if (L <= 256) {
-        res = warp_sort_row<8>(a, L);
-      } else if (L <= 512) {
-        res = warp_sort_row<16>(a, L);
-      } else if (L <= kWarpSortMax) {
-        res = warp_sort_row<32>(a, L);
-      } else {
-        if (lane == 0) big[atomicAdd(nbig, 1u)] = ubase + r;
-        continue;
-      }
-      if (lane == 0) rows[ubase + r] = res;
-    }
+    sort_short_rows<32>(__ballot_sync(kFull, L_l > 16 && L_l <= kShortRow), s_l, L_l, ubase, nbr, rows);
   }
 }
 
-// Rows longer than kWarpSortMax, one CTA per row: a bitonic sort of the row
-// padded to a power of two P, in shared memory (P <= kCtaSortSmem) or in the
-// row's slice [2 s, 2 s + P) of scratch (P <= 2 L; scratch holds twice the
-// entries nbr's row slots hold), then the distinct values written back to the
-// front of the row.
-__global__ void __launch_bounds__(kCtaSortThreads) k_sort_big_rows(const uint32_t* __restrict__ start,
-                                                                   const uint32_t* __restrict__ end,
-                                                                   uint32_t* __restrict__ nbr,
-                                                                   uint32_t* __restrict__ scratch,
-                                                                   uint64_t* __restrict__ rows,
-                                                                   const uint32_t* __restrict__ big,
-                                                                   const uint32_t* __restrict__ nbig) {
-  __shared__ uint32_t sm[kCtaSortSmem];
-  __shared__ uint32_t wsum[2][kCtaSortThreads / 32];
+// Sorts and deduplicates a CTA row through bitmaps of its columns: the window
+// of kBitWords words from block w0 on gets a bit per entry in it, and its set
+// bits, in order, are the row's distinct values (to out[nu...)). Returns
+// (values << 32) | blocks of the window. A bit set costs one shared atomic an
+// entry and a window kBitWords / 256 words a thread, where a bitonic sort of P
+// values takes log2(P) (log2(P) + 1) / 2 barriers.
+__device__ __forceinline__ uint64_t window_sort(const uint32_t* a, uint32_t L, uint32_t w0, uint32_t words, uint32_t* sm,
+                                                uint32_t* out, uint32_t nu) {
+  const uint32_t tid = threadIdx.x;
+  for (uint32_t i = tid; i < words; i += kLongThreads) sm[i] = 0u;
+  __syncthreads();
+  for (uint32_t i = tid; i < L; i += kLongThreads) {
+    const uint32_t x = a[i], d = (x >> 5) - w0;
+    if (d < words) atomicOr(&sm[d], 1u << (x & 31));
+  }
+  __syncthreads();
+  // Each thread takes an odd number of words in a row (odd: its neighbours'
+  // words lie in other banks).
+  const uint32_t per = ((words + kLongThreads - 1) / kLongThreads) | 1u;
+  const uint32_t i0 = min(tid * per, words), i1 = min(i0 + per, words);
+  uint32_t c = 0, nb = 0;
+  for (uint32_t i = i0; i < i1; ++i) {
+    const uint32_t m = sm[i];
+    c += __popc(m);
+    nb += m != 0u;
+  }
+  uint64_t tot;
+  const uint64_t ex = block_exclusive_scan<uint64_t>(((uint64_t)c << 32) | nb, OpSum{}, 0ull, &tot);
+  uint32_t at = nu + (uint32_t)(ex >> 32);
+  for (uint32_t i = i0; i < i1; ++i)
+    for (uint32_t m = sm[i]; m; m &= m - 1) out[at++] = ((w0 + i) << 5) + (uint32_t)__ffs(m) - 1u;
+  __syncthreads();  // sm is cleared for the next window or row
+  return tot;
+}
+
+// The listed long rows: a CTA per row of more than kWarpSortMax entries, then
+// a warp per row in registers (bitonic). A CTA row is sorted through column
+// bitmaps when its block span takes at most L / 1024 windows (one window for
+// rows under 2,048), else bitonically, padded to a power of two P, in shared
+// memory (P <= kCtaSortSmem) or in the row's slice [2 s, 2 s + P) of scratch
+// (P <= 2 L; scratch holds twice the entries nbr's row slots hold). Rows are
+// taken in strides over the grid (the lists run roughly by rank, so every warp
+// gets the same mix), the longest first.
+__global__ void __launch_bounds__(kLongThreads, 4)
+    k_sort_long(const uint32_t* __restrict__ start, const uint32_t* __restrict__ end, uint32_t n,
+                uint32_t* __restrict__ nbr, uint32_t* __restrict__ scratch, uint64_t* __restrict__ rows, LongRows lng) {
+  __shared__ uint32_t sm[kBitWords];
+  __shared__ uint32_t wsum[2][kLongThreads / 32];
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const uint32_t count = *nbig;
-  for (uint32_t bi = blockIdx.x; bi < count; bi += gridDim.x) {
-    const uint32_t u = big[bi];
+  const uint32_t ncta = lng.count[0], nmid = lng.count[1];
+  for (uint32_t bi = blockIdx.x; bi < ncta; bi += gridDim.x) {
+    const uint32_t u = lng.rows[ncta - 1 - bi];
     const uint32_t s = start[u], L = end[u] - s;
-    uint32_t P = 1;
-    while (P < L) P <<= 1;
-    uint32_t* a = P <= kCtaSortSmem ? sm : scratch + 2ull * s;
-    for (uint32_t i = tid; i < P; i += blockDim.x) a[i] = i < L ? nbr[s + i] : kPad;
+    uint32_t lo = kFull, hi = 0;
+    for (uint32_t i = tid; i < L; i += kLongThreads) {
+      const uint32_t b = nbr[s + i] >> 5;
+      lo = min(lo, b);
+      hi = max(hi, b);
+    }
+    lo = __reduce_min_sync(kFull, lo);
+    hi = __reduce_max_sync(kFull, hi);
+    if (lane == 0) {
+      wsum[0][w] = lo;
+      wsum[1][w] = hi;
+    }
     __syncthreads();
-    for (uint32_t k = 2; k <= P; k <<= 1) {
-      for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-        for (uint32_t t = tid; t < P / 2; t += blockDim.x) {
-          const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1));  // pairs (i, i + j); j is a power of 2
-          const bool up = (i & k) == 0;
-          const uint32_t x = a[i], y = a[i + j];
-          if (up ? x > y : x < y) {
-            a[i] = y;
-            a[i + j] = x;
+#pragma unroll
+    for (uint32_t q = 0; q < kLongThreads / 32; ++q) {
+      lo = min(lo, wsum[0][q]);
+      hi = max(hi, wsum[1][q]);
+    }
+    __syncthreads();
+    const uint32_t span = hi - lo + 1, windows = (span + kBitWords - 1) / kBitWords;
+    uint64_t res = 0;
+    if (windows == 1) {  // every entry is read before the first is overwritten
+      res = window_sort(nbr + s, L, lo, span, sm, nbr + s, 0);
+    } else if ((uint64_t)windows * 1024 <= L) {
+      uint32_t* out = scratch + 2ull * s;
+      for (uint32_t k = 0; k < windows; ++k) {
+        const uint32_t w0 = k * kBitWords;
+        res += window_sort(nbr + s, L, lo + w0, min(kBitWords, span - w0), sm, out, (uint32_t)(res >> 32));
+      }
+      for (uint32_t i = tid; i < (uint32_t)(res >> 32); i += kLongThreads) nbr[s + i] = out[i];
+    } else {
+      uint32_t P = 1;
+      while (P < L) P <<= 1;
+      uint32_t* a = P <= kCtaSortSmem ? sm : scratch + 2ull * s;
+      for (uint32_t i = tid; i < P; i += kLongThreads) a[i] = i < L ? nbr[s + i] : kPad;
+      __syncthreads();
+      for (uint32_t k = 2; k <= P; k <<= 1) {
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+          for (uint32_t t = tid; t < P / 2; t += kLongThreads) {
+            const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1));  // pairs (i, i + j); j is a power of 2
+            const bool up = (i & k) == 0;
+            const uint32_t x = a[i], y = a[i + j];
+            if (up ? x > y : x < y) {
+              a[i] = y;
+              a[i + j] = x;
+            }
           }
+          __syncthreads();
+        }
+      }
+      // Distinct values in order: per tile of kLongThreads values, a
+      // block-wide count of the new ones places them.
+      uint32_t nu = 0, nbk = 0;
+      for (uint32_t base = 0; base < L; base += kLongThreads) {
+        const uint32_t i = base + tid;
+        const uint32_t x = i < L ? a[i] : kPad;
+        const uint32_t p = i > 0 && i < L ? a[i - 1] : kPad;
+        const bool is_new = x != kPad && (i == 0 || x != p);
+        const bool new_blk = is_new && (i == 0 || (x >> 5) != (p >> 5));
+        const uint32_t bn = __ballot_sync(kFull, is_new), bb = __ballot_sync(kFull, new_blk);
+        if (lane == 0) {
+          wsum[0][w] = __popc(bn);
+          wsum[1][w] = __popc(bb);
         }
         __syncthreads();
+        uint32_t before = 0, tile_u = 0, tile_b = 0;
+        for (uint32_t q = 0; q < kLongThreads / 32; ++q) {
+          if (q < w) before += wsum[0][q];
+          tile_u += wsum[0][q];
+          tile_b += wsum[1][q];
+        }
+        if (is_new) nbr[s + nu + before + __popc(bn & ((1u << lane) - 1u))] = x;
+        nu += tile_u;
+        nbk += tile_b;
+        __syncthreads();  // a[] reads of this tile and wsum before the next tile
       }
+      res = ((uint64_t)nu << 32) | nbk;
     }
-    // Distinct values in order: per tile of blockDim values, a block-wide
-    // count of the new ones places them.
-    uint32_t nu = 0, nbk = 0;
-    for (uint32_t base = 0; base < L; base += blockDim.x) {
-      const uint32_t i = base + tid;
-      const uint32_t x = i < L ? a[i] : kPad;
-      const uint32_t p = i > 0 && i < L ? a[i - 1] : kPad;
-      const bool is_new = x != kPad && (i == 0 || x != p);
-      const bool new_blk = is_new && (i == 0 || (x >> 5) != (p >> 5));
-      const uint32_t bn = __ballot_sync(kFull, is_new), bb = __ballot_sync(kFull, new_blk);
-      if (lane == 0) {
-        wsum[0][w] = __popc(bn);
-        wsum[1][w] = __popc(bb);
-      }
-      __syncthreads();
-      uint32_t before = 0, tile_u = 0, tile_b = 0;
-      for (uint32_t q = 0; q < blockDim.x / 32; ++q) {
-        if (q < w) before += wsum[0][q];
-        tile_u += wsum[0][q];
-        tile_b += wsum[1][q];
-      }
-      if (is_new) nbr[s + nu + before + __popc(bn & ((1u << lane) - 1u))] = x;
-      nu += tile_u;
-      nbk += tile_b;
-      __syncthreads();  // a[] reads of this tile and wsum before the next tile
-    }
-    if (tid == 0) rows[u] = ((uint64_t)nu << 32) | nbk;
-    __syncthreads();
+    if (tid == 0) rows[u] = res;
+  }
+  const uint32_t warp = blockIdx.x * (kLongThreads / 32) + w, nwarps = gridDim.x * (kLongThreads / 32);
+  for (uint32_t i = warp; i < nmid; i += nwarps) {
+    const uint32_t u = lng.rows[n - (nmid - 1 - i)];
+    const uint32_t s = start[u], L = end[u] - s;
+    uint32_t* a = nbr + s;
+    uint64_t res;
+    if (L <= 64)
+      res = warp_sort_row<2>(a, L);
+    else if (L <= 128)
+      res = warp_sort_row<4>(a, L);
+    else if (L <= 256)
+      res = warp_sort_row<8>(a, L);
+    else if (L <= 512)
+      res = warp_sort_row<16>(a, L);
+    else
+      res = warp_sort_row<32>(a, L);
+    if (lane == 0) rows[u] = res;
   }
 }
 
-// The row's distinct sorted values (front of its nbr slice, from off[u]) to col, and its
-// bit-row entries (block << 32 | mask) to bent, each written once. One warp
-// per 32 rows: a row of at most kLaneEmit values is written by its own lane;
-// a longer one by the whole warp, where the mask of a block is a segmented OR
-// over the lanes holding its values (a block cut by a chunk boundary carries
-// its partial mask over). Most rows of a power-law graph hold 0 or 1 values.
-constexpr uint32_t kLaneEmit = 8;
-__global__ void k_emit_rows(const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr,
-                            const uint64_t* __restrict__ rp, uint32_t n, uint32_t* __restrict__ col,
-                            uint64_t* __restrict__ bent) {
+// The first u in [0, n] with rp_row(rp[u]) - begin + u >= t: rows and positions
+// counted together, so that a run of empty rows is work like any other. The
+// whole warp searches, 32 probes a step.
+__device__ __forceinline__ uint64_t first_row_at(const uint64_t* __restrict__ rp, uint32_t n, uint32_t begin,
+                                                 uint64_t t) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t ubase = warp * 32; ubase < n; ubase += nwarps * 32) {
-    const uint32_t mu = ubase + lane;
-    const bool here = mu < n;
-    uint32_t mslot = 0, mnu = 0, mb0 = 0, moff = 0;
-    if (here) {
-      const uint64_t r0 = rp[mu], r1 = rp[mu + 1];
-      mslot = (uint32_t)(r0 >> 32);
-      mnu = (uint32_t)(r1 >> 32) - mslot;
-      mb0 = (uint32_t)r0;
-      moff = mnu ? off[mu] : 0u;
+  uint64_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint64_t step = (hi - lo + 31) / 32, u = lo + (lane + 1) * step - 1;
+    const uint32_t below = __popc(__ballot_sync(kFull, u < hi && rp_row(rp[u]) - begin + u < t));
+    const uint64_t next = lo + (below + 1) * step - 1;
+    lo = min(hi, lo + below * step);
+    if (below < 32) hi = min(hi, next);
+  }
+  return lo;
+}
+
+// Emits CSR positions [ps, pe): col[p] and the positions' bit-row entries from
+// bent[b] on, one warp, 32 positions a step with the values of the next
+// kEmitAhead steps loaded before they are used. starts(c): bit l set iff a row
+// starts at position c + l (one does at ps); source(p, i): the index in nbr of
+// position p, in the i-th row that starts in the range. A bit-row entry is
+// written by the lane of its block's last value: the mask is a segmented OR,
+// and a block cut by a step carries its partial mask over.
+constexpr int kEmitAhead = 3;
+template <class Starts, class Source>
+__device__ __forceinline__ void emit_span(uint32_t ps, uint32_t pe, uint32_t b, const Starts& starts,
+                                          const Source& source, const uint32_t* __restrict__ nbr,
+                                          uint32_t* __restrict__ col, uint64_t* __restrict__ bent) {
+  const uint32_t lane = threadIdx.x & 31, le = kFull >> (31 - lane);
+  uint32_t m[kEmitAhead + 1], x[kEmitAhead + 1];  // row starts and values of this step and the next ones
+  uint32_t at = 0, row = kFull;                   // positions loaded; rows started in them, less one
+  const uint32_t len = pe - ps;
+  auto load = [&](int k) {
+    m[k] = 0;
+    x[k] = kPad;
+    if (at < len) {
+      m[k] = starts(ps + at);
+      const uint32_t i = row + __popc(m[k] & le);
+      if (lane < len - at) x[k] = nbr[source(ps + at + lane, i)];
+      row += __popc(m[k]);
+      at += min(32u, len - at);
     }
-    if (here && mnu <= kLaneEmit && mnu > 0) {
-      const uint32_t* a = nbr + moff;
-      uint32_t nblk = 0, cur = a[0] >> 5, m = 0;
-      for (uint32_t i = 0; i < mnu; ++i) {
-        const uint32_t x = a[i];
-        col[mslot + i] = x;
-        if ((x >> 5) != cur) {
-          bent[mb0 + nblk++] = ((uint64_t)cur << 32) | m;
-          cur = x >> 5;
-          m = 0;
-        }
-        m |= 1u << (x & 31);
+  };
+#pragma unroll
+  for (int k = 0; k <= kEmitAhead; ++k) load(k);
+  uint32_t last = kPad >> 5, carry = 0;
+  for (uint32_t left = len, c = ps;; left -= 32, c += 32) {
+    const bool in = lane < left, more = left > 32;
+    const uint32_t blk = x[0] >> 5;
+    uint32_t prev = __shfl_up_sync(kFull, blk, 1);
+    if (lane == 0) prev = last;
+    const uint32_t heads = __ballot_sync(kFull, in && (((m[0] >> lane) & 1u) || blk != prev));
+    last = __shfl_sync(kFull, blk, 31);
+    const bool next_head = !more || (m[1] & 1u) || (__shfl_sync(kFull, x[1], 0) >> 5) != last;
+    const uint32_t own = heads & le, first = own ? 31 - __clz(own) : 0u;  // first lane of the block here
+    uint32_t bits = in ? 1u << (x[0] & 31) : 0u;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, bits, o);
+      if (lane >= first + o) bits |= y;
+    }
+    if (!own) bits |= carry;
+    const bool end = in && (lane == 31 ? next_head : (lane + 1 >= left || ((heads >> (lane + 1)) & 1u)));
+    if (in) col[c + lane] = x[0];
+    if (end) bent[b + __popc(own) - 1] = ((uint64_t)blk << 32) | bits;
+    if (!more) break;
+    carry = __shfl_sync(kFull, bits, 31);
+    b += __popc(heads);
+#pragma unroll
+    for (int k = 0; k < kEmitAhead; ++k) {
+      m[k] = m[k + 1];
+      x[k] = x[k + 1];
+    }
+    load(kEmitAhead);
+  }
+}
+
+// The rows' distinct sorted values (the front of each row's nbr slice, from
+// off[u]) to col, and their bit-row entries (block << 32 | mask) to bent, each
+// written once. Listed CTA rows of more than kWarpSortMax values are emitted
+// by a CTA, each warp an eighth of the row from the first block that starts in
+// it. All others are shared out by rows and CSR positions together (`chunk` of
+// them a warp): a warp takes the rows that start in its share, 32 at a time, and
+// walks their positions flat, so its work is the values it writes, whatever the
+// rows' lengths. One warp per 32
+// rows, a row at a time, left the top ranks to a few warps (RMAT-20: 487 us, now
+// 139; RMAT-17 by id: 1,881, now 157; planted partition, even rows: 257, now 280).
+__global__ void __launch_bounds__(256) k_emit_rows(const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr,
+                                                   const uint64_t* __restrict__ rp, uint32_t n, uint32_t chunk,
+                                                   LongRows lng, uint32_t* __restrict__ col,
+                                                   uint64_t* __restrict__ bent) {
+  __shared__ uint32_t s_delta[8][32];
+  __shared__ uint32_t s_head[9], s_cnt[8];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (uint32_t bi = blockIdx.x, ncta = lng.count[0]; bi < ncta; bi += gridDim.x) {
+    const uint32_t u = lng.rows[ncta - 1 - bi];
+    const uint64_t r0 = rp[u], r1 = rp[u + 1];
+    const uint32_t p0 = rp_row(r0), nu = rp_row(r1) - p0;
+    if (nu <= kWarpSortMax) continue;  // duplicates: walked flat below
+    const uint32_t* a = nbr + off[u];
+    auto new_block = [&](uint32_t i) { return i < nu && (i == 0 || (a[i] >> 5) != (a[i - 1] >> 5)); };
+    // The warp's first block head at or after its share (a block has at most 32 values).
+    const uint32_t s0 = (uint32_t)((uint64_t)nu * w / 8);
+    const uint32_t hm = __ballot_sync(kFull, new_block(s0 + lane));
+    if (lane == 0) {
+      s_head[w] = hm ? s0 + (uint32_t)__ffs(hm) - 1u : nu;
+      if (w == 0) s_head[8] = nu;
+    }
+    __syncthreads();
+    const uint32_t i0 = s_head[w], i1 = s_head[w + 1];
+    uint32_t c = 0;
+    for (uint32_t i = i0; i < i1; i += 32) c += __popc(__ballot_sync(kFull, i + lane < i1 && new_block(i + lane)));
+    if (lane == 0) s_cnt[w] = c;
+    __syncthreads();
+    uint32_t b = rp_blk(r0);
+    for (uint32_t q = 0; q < w; ++q) b += s_cnt[q];
+    if (i0 < i1)
+      emit_span(p0 + i0, p0 + i1, b, [&](uint32_t p) { return p == p0 + i0 ? 1u : 0u; },
+                [&](uint32_t p, uint32_t) { return off[u] + (p - p0); }, nbr, col, bent);
+    __syncthreads();  // s_head and s_cnt are rewritten for the next row
+  }
+  const uint32_t begin = rp_row(rp[0]);
+  const uint64_t total = (uint64_t)(rp_row(rp[n]) - begin) + n;
+  const uint32_t warp = blockIdx.x * 8 + w, nwarps = gridDim.x * 8;
+  for (uint64_t t = (uint64_t)warp * chunk; t < total; t += (uint64_t)nwarps * chunk) {
+    for (uint64_t ub = first_row_at(rp, n, begin, t);; ub += 32) {
+      const uint64_t ul = ub + lane;
+      const uint32_t u = (uint32_t)ul;
+      uint64_t r0 = 0, r1 = 0;
+      bool here = ul < n;
+      if (here) {
+        r0 = rp[u];
+        r1 = rp[u + 1];
+        here = rp_row(r0) - begin + ul < t + chunk;
       }
-      bent[mb0 + nblk] = ((uint64_t)cur << 32) | m;
-    }
-    uint32_t longer = __ballot_sync(kFull, here && mnu > kLaneEmit);
-    while (longer) {
-      const uint32_t r = __ffs(longer) - 1;
-      longer &= longer - 1;
-      const uint32_t slot = __shfl_sync(kFull, mslot, r), nu = __shfl_sync(kFull, mnu, r),
-                     b0 = __shfl_sync(kFull, mb0, r);
-      const uint32_t* a = nbr + __shfl_sync(kFull, moff, r);
-      // Blocks written so far; the previous chunk's last value and the partial
-      // mask of its last block.
-      uint32_t nblk = 0, last = kPad, carry = 0;
-      for (uint32_t c = 0; c < nu; c += 32) {
-        const uint32_t i = c + lane;
-        const bool in = i < nu;
-        const uint32_t x = in ? a[i] : kPad;
-        const uint32_t blk = x >> 5;
-        uint32_t prev = __shfl_up_sync(kFull, x, 1);
-        if (lane == 0) prev = last;
-        uint32_t next = __shfl_down_sync(kFull, x, 1);
-        if (lane == 31) next = c + 32 < nu ? a[c + 32] : kPad;
-        const bool new_blk = in && (i == 0 || blk != (prev >> 5));
-        const bool end_blk = in && (i + 1 == nu || blk != (next >> 5));
-        // Segmented OR of the block's bits from its first lane in this chunk.
-        uint32_t m = in ? 1u << (x & 31) : 0u;
-  #pragma unroll
-        for (uint32_t o = 1; o < 32; o <<= 1) {
-          const uint32_t y = __shfl_up_sync(kFull, m, o);
-          const uint32_t yb = __shfl_up_sync(kFull, blk, o);
-          if (lane >= o && yb == blk) m |= y;
-        }
-        if (i > 0 && c > 0 && blk == (last >> 5)) m |= carry;  // the block began in the previous chunk
-        const uint32_t incl = warp_inclusive_sum(new_blk ? 1u : 0u);
-        if (in) col[slot + i] = x;
-        if (end_blk) bent[b0 + nblk + incl - 1] = ((uint64_t)blk << 32) | m;
-        carry = __shfl_sync(kFull, m, 31);
-        last = __shfl_sync(kFull, x, 31);
-        nblk += __shfl_sync(kFull, incl, 31);
+      const uint32_t hm = __ballot_sync(kFull, here);
+      if (!hm) break;
+      const uint32_t p = rp_row(r0), nu = here ? rp_row(r1) - p : 0u;
+      const uint32_t bigs = __ballot_sync(kFull, nu > kWarpSortMax);
+      // Runs of rows between CTA rows.
+      for (uint32_t todo = hm; todo;) {
+        const uint32_t first = (uint32_t)__ffs(todo) - 1u;
+        const uint32_t stop = bigs & todo;
+        const uint32_t run = stop ? todo & ((stop & (0u - stop)) - 1u) : todo;
+        todo = stop ? todo & ~((stop & (0u - stop)) | run) : 0u;
+        if (!run) continue;
+        const bool mine = ((run >> lane) & 1u) && nu > 0;
+        const uint32_t rows = __ballot_sync(kFull, mine);
+        if (!rows) continue;
+        __syncwarp();
+        if (mine) s_delta[w][__popc(rows & ((1u << lane) - 1u))] = off[u] - p;
+        __syncwarp();
+        const uint32_t ps = __shfl_sync(kFull, p, first), tail = 31u - (uint32_t)__clz(run);
+        const uint32_t pe = __shfl_sync(kFull, rp_row(r1), tail), b = __shfl_sync(kFull, rp_blk(r0), first);
+        emit_span(ps, pe, b,
+                  [&](uint32_t c) { return __reduce_or_sync(kFull, mine && p - c < 32u ? 1u << (p - c) : 0u); },
+                  [&](uint32_t q, uint32_t i) { return q + s_delta[w][i]; }, nbr, col, bent);
       }
+      if (hm != kFull) break;
     }
+  }
+}
+
+// Rows and CSR positions a warp of k_emit_rows takes, for at most E of them:
+// enough warps to fill the chip several times over, up to 1,024 a search.
+uint32_t emit_chunk(uint64_t E) {
+  const uint64_t c = ceil_div<uint64_t>(E, 148ull * 64);
+  return (uint32_t)std::min<uint64_t>(1024, std::max<uint64_t>(64, (c + 31) & ~31ull));
+}
+
+unsigned emit_grid(uint64_t E) {
+  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div<uint64_t>(E, 8ull * emit_chunk(E)), 148ull * 32));
+}
+
+// Rows a warp of k_sort_rows takes: 32 once that fills the chip, fewer below.
+uint32_t sort_rows_per_warp(uint64_t n) {
+  return (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(4, ceil_div<uint64_t>(n, 148ull * 64)));
+}
+
+unsigned sort_grid(uint64_t n) {
+  return (unsigned)std::max<uint64_t>(
+      1, std::min<uint64_t>(ceil_div<uint64_t>(n, 8ull * sort_rows_per_warp(n)), 148ull * 32));
+}
+
+// Row u = nbr[start[u], end[u]) sorted and deduplicated in place for u < n,
+// rows[u] = (distinct << 32) | blocks; E bounds the entries of all rows.
+void sort_rows(const uint32_t* start, const uint32_t* end, uint32_t n, uint64_t E, uint32_t* nbr, uint32_t* scratch,
+               uint64_t* rows, const LongRows& lng, cudaStream_t st) {
+  TB_CUDA(cudaMemsetAsync(lng.count, 0, 2 * sizeof(uint32_t), st));
+  k_sort_rows<<<sort_grid(n), kThreads, 0, st>>>(start, end, n, sort_rows_per_warp(n), nbr, rows, lng);
+  TB_LAUNCH_CHECK();
+  if (E > kShortRow) {
+    k_sort_long<<<(unsigned)std::min<uint64_t>(148 * 4, ceil_div<uint64_t>(E, kShortRow)), kLongThreads, 0, st>>>(
+        start, end, n, nbr, scratch, rows, lng);
+    TB_LAUNCH_CHECK();
   }
 }
 
@@ -583,7 +785,7 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
   uint32_t* otmp = take_scan_temp<uint32_t>(ar, n + 1);
   uint64_t* rtmp = take_scan_temp<uint64_t>(ar, n + 1);
   uint32_t* big = ar.take<uint32_t>(n + 1);
-  uint32_t* nbig = ar.take<uint32_t>(1);
+  uint32_t* nbig = ar.take<uint32_t>(2);
   uint32_t* nbr = ar.take<uint32_t>(cap ? cap : 1);
   // The oriented keys (on the slot path both presort buffers), then long
   // rows' sort space (twice nbr).
@@ -601,10 +803,9 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
   out->view.bent = bent;
   if (ar.measuring()) return;
 
-  const unsigned wgrid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div<uint64_t>(n, 8), 148ull * 32));
+  const LongRows lng{big, nbig};
   uint64_t* keys = reinterpret_cast<uint64_t*>(scratch);
   const int top = 32 + bits_for(n) - 8;  // the presort digit: the top 8 bits of lo
-  TB_CUDA(cudaMemsetAsync(nbig, 0, sizeof(uint32_t), st));
   if (slots) {
     k_slot_sizes<<<grid_for(n + 1), kThreads, 0, st>>>(deg, rank, n, cnt);
     TB_LAUNCH_CHECK();
@@ -634,14 +835,9 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
     TB_LAUNCH_CHECK();
   }
   // Row u: nbr[off[u], cnt[u]) (with no entries every row is empty: 0, 0).
-  k_sort_rows<<<wgrid, kThreads, 0, st>>>(off, cnt, (uint32_t)n, nbr, rp, big, nbig);
-  TB_LAUNCH_CHECK();
-  if (E > kWarpSortMax) {
-    k_sort_big_rows<<<148 * 2, kCtaSortThreads, 0, st>>>(off, cnt, nbr, scratch, rp, big, nbig);
-    TB_LAUNCH_CHECK();
-  }
+  sort_rows(off, cnt, (uint32_t)n, E, nbr, scratch, rp, lng, st);
   device_scan<uint64_t, OpSum>(rp, rp, n + 1, true, OpSum{}, 0ull, rtmp, st);
-  k_emit_rows<<<wgrid, kThreads, 0, st>>>(off, nbr, rp, (uint32_t)n, col, bent);
+  k_emit_rows<<<emit_grid(E + n), kThreads, 0, st>>>(off, nbr, rp, (uint32_t)n, emit_chunk(E + n), lng, col, bent);
   TB_LAUNCH_CHECK();
   k_finalize<<<1, 1, 0, st>>>(rp, n, stats);
   TB_LAUNCH_CHECK();
@@ -657,7 +853,7 @@ RowRangeBuffers take_row_range_buffers(Arena& ar, uint64_t n, uint64_t cap) {
   b.off = ar.take<uint32_t>(n + 1);
   b.cursor = ar.take<uint32_t>(n + 1);
   b.big = ar.take<uint32_t>(n + 1);
-  b.nbig = ar.take<uint32_t>(1);
+  b.nbig = ar.take<uint32_t>(2);
   b.carry = ar.take<uint64_t>(1);
   b.scan_tmp = take_scan_temp<uint64_t>(ar, n + 1);
   return b;
@@ -672,7 +868,6 @@ void begin_row_range(const RowRangeBuffers& b, const uint64_t* row_start, uint32
     TB_CUDA(cudaMemsetAsync(b.carry, 0, sizeof(uint64_t), st));
   else
     TB_CUDA(cudaMemcpyAsync(b.carry, rp + s, sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
-  TB_CUDA(cudaMemsetAsync(b.nbig, 0, sizeof(uint32_t), st));
   k_range_starts<<<grid_for((uint64_t)z + 1), kThreads, 0, st>>>(row_start, s, z, b.off, b.cursor);
   TB_LAUNCH_CHECK();
 }
@@ -682,18 +877,12 @@ void finish_row_range(const RowRangeBuffers& b, uint32_t s, uint32_t z, uint64_t
   if (z == 0) return;
   k_range_check<<<grid_for(z), kThreads, 0, st>>>(b.off, b.cursor, z, err);
   TB_LAUNCH_CHECK();
-  const unsigned wgrid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div<uint64_t>(z, 8), 148ull * 32));
-  k_sort_rows<<<wgrid, kThreads, 0, st>>>(b.off, b.off + 1, z, b.nbr, rp + s, b.big, b.nbig);
-  TB_LAUNCH_CHECK();
-  if (cnt > kWarpSortMax) {
-    k_sort_big_rows<<<148 * 2, kCtaSortThreads, 0, st>>>(b.off, b.off + 1, b.nbr, b.scratch, rp + s, b.big,
-                                                         b.nbig);
-    TB_LAUNCH_CHECK();
-  }
+  const LongRows lng{b.big, b.nbig};
+  sort_rows(b.off, b.off + 1, z, cnt, b.nbr, b.scratch, rp + s, lng, st);
   device_scan<uint64_t, OpSum>(rp + s, rp + s, (uint64_t)z + 1, true, OpSum{}, 0ull, b.scan_tmp, st);
   k_range_carry<<<grid_for((uint64_t)z + 1), kThreads, 0, st>>>(rp + s, z + 1, b.carry);
   TB_LAUNCH_CHECK();
-  k_emit_rows<<<wgrid, kThreads, 0, st>>>(b.off, b.nbr, rp + s, z, col, bent);
+  k_emit_rows<<<emit_grid(cnt + z), kThreads, 0, st>>>(b.off, b.nbr, rp + s, z, emit_chunk(cnt + z), lng, col, bent);
   TB_LAUNCH_CHECK();
 }
 

@@ -110,8 +110,8 @@ struct RowRangeBuffers {
   uint32_t* nbr = nullptr;      // cap: the range's rows
   uint32_t* off = nullptr;      // n + 1: range-relative row starts
   uint32_t* cursor = nullptr;   // n + 1: fill cursors
-  uint32_t* big = nullptr;      // n + 1: rows for the CTA sort
-  uint32_t* nbig = nullptr;
+  uint32_t* big = nullptr;      // n + 1: the long rows' lists
+  uint32_t* nbig = nullptr;     // 2: their lengths
   uint64_t* carry = nullptr;    // rp of the range's first row before the range is built
   uint64_t* scan_tmp = nullptr;
 };
