@@ -1785,25 +1785,168 @@ __global__ void __launch_bounds__(kHubWarps * 32, TB_HUB_MIN_CTAS) k_queue(
 
 // ---- schedule ----------------------------------------------------------------
 
+// Neighbour-side work of a row block: what the sweeps of its rows will read.
+struct BlockWork {
+  uint64_t wb = 0, wm = 0;      // the neighbours' bit blocks and ids
+  uint32_t vmax = 0, top = 0;   // longest neighbour row, neighbours among the top 4,096 ranks
+};
+
+// Adds the neighbours at CSR positions p0 + lane, p0 + lane + step, ... below
+// pe, kFeatDepth of them in flight a lane; start / d: lane r's row of the
+// block, whose single neighbour (d == 1) is left out, as the sweeps leave it.
+constexpr int kFeatDepth = 4;
+__device__ __forceinline__ void add_work(const GraphView& g, uint32_t p0, uint32_t pe, uint32_t step, uint32_t start,
+                                         uint32_t d, BlockWork& x) {
+  const uint32_t lane = threadIdx.x & 31;
+  const bool singles = __any_sync(kFull, d == 1);
+  for (uint64_t c = p0; c < pe; c += (uint64_t)step * kFeatDepth) {
+    uint32_t v[kFeatDepth];
+#pragma unroll
+    for (int r = 0; r < kFeatDepth; ++r) {
+      const uint64_t q = c + (uint64_t)step * r;
+      uint32_t skip = 0;
+      if (singles) skip = __reduce_or_sync(kFull, d == 1 && start - (uint32_t)q < 32u ? 1u << (start - (uint32_t)q) : 0u);
+      v[r] = q + lane < pe && !((skip >> lane) & 1u) ? g.col[q + lane] : kNoRow;
+    }
+    uint64_t a[kFeatDepth], b[kFeatDepth];
+#pragma unroll
+    for (int r = 0; r < kFeatDepth; ++r) {
+      const bool in = v[r] != kNoRow;
+      a[r] = in ? g.rp[v[r]] : 0ull;
+      b[r] = in ? g.rp[v[r] + 1] : 0ull;
+    }
+#pragma unroll
+    for (int r = 0; r < kFeatDepth; ++r) {
+      const uint32_t dv = rp_row(b[r]) - rp_row(a[r]);
+      x.wb += rp_blk(b[r]) - rp_blk(a[r]);
+      x.wm += dv;
+      x.vmax = max(x.vmax, dv);
+      x.top += v[r] != kNoRow && (uint64_t)v[r] + 4096u >= g.n ? 1u : 0u;
+    }
+  }
+}
+
+// A row block of more than kFeatWarp edges is walked by the whole CTA; under
+// id order, where one block can hold a quarter of the edges, a block of more
+// than kFeatGrid by kFeatParts warps of a launch before (k_wide_work).
+constexpr uint32_t kFeatWarp = 1024;
+constexpr uint32_t kFeatGrid = 8192;
+constexpr uint32_t kFeatParts = 32;
+
+// Id order: the neighbour-side work of the blocks of more than kFeatGrid
+// edges, added to the block's first feature words (zeroed before), which
+// k_features reads and then overwrites. A warp takes one part of every wide
+// block among 32.
+__global__ void __launch_bounds__(256) k_wide_work(GraphView g, uint32_t nrb, float* __restrict__ feat) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t part = (uint32_t)(warp % kFeatParts);
+  const uint64_t rb = warp / kFeatParts * 32 + lane;
+  uint32_t s = 0, e = 0;
+  if (rb < nrb) {
+    s = rp_row(g.rp[rb * 32]);
+    e = rp_row(g.rp[min((uint64_t)g.n, rb * 32 + 32)]);
+  }
+  for (uint32_t wide = __ballot_sync(kFull, e - s > kFeatGrid); wide; wide &= wide - 1) {
+    const int k = __ffs(wide) - 1;
+    const uint32_t bs = __shfl_sync(kFull, s, k), len = __shfl_sync(kFull, e, k) - bs;
+    const uint64_t b = __shfl_sync(kFull, rb, k), u = b * 32 + lane;
+    uint32_t start = 0, d = 0;
+    if (u < g.n) {
+      start = rp_row(g.rp[u]);
+      d = rp_row(g.rp[u + 1]) - start;
+    }
+    const uint32_t chunks = (len + 31) / 32;  // whole 32-position chunks a part
+    const uint32_t c0 = (uint32_t)((uint64_t)chunks * part / kFeatParts) * 32;
+    const uint32_t c1 = min(len, (uint32_t)((uint64_t)chunks * (part + 1) / kFeatParts) * 32);
+    BlockWork x;
+    add_work(g, bs + c0, bs + c1, 32, start, d, x);
+    const uint64_t wb = warp_sum(x.wb), wm = warp_sum(x.wm);
+    const uint32_t vmax = __reduce_max_sync(kFull, x.vmax), top = __reduce_add_sync(kFull, x.top);
+    if (lane == 0) {
+      unsigned long long* acc = reinterpret_cast<unsigned long long*>(feat + b * kNumFeatures);
+      atomicAdd(&acc[0], (unsigned long long)wb);
+      atomicAdd(&acc[1], (unsigned long long)wm);
+      atomicMax(reinterpret_cast<unsigned int*>(&acc[2]), vmax);
+      atomicAdd(reinterpret_cast<unsigned int*>(&acc[2]) + 1, top);
+    }
+  }
+}
+
 // Row-block features (one warp per row block) and the plain dispatcher's
 // choice. Features are log-scaled so the learned dispatcher sees O(1) inputs.
-__global__ void k_features(GraphView g, uint32_t nrb, int mode, float* __restrict__ feat,
-                           uint8_t* __restrict__ variant_of, int full, float tile_min_nnz, float merge_ratio) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t rb = warp; rb < nrb; rb += nwarps) {
+// A block's neighbours are walked flat, CSR position by position with four
+// loads in flight a lane, and a wide block's by all warps of the CTA: walked
+// row by row on one warp, the top ranks' blocks (32 long rows each) ran long
+// after the rest (RMAT-20: 341 us, now 192; RMAT-17 by id: 1,459, now 206).
+__global__ void __launch_bounds__(256) k_features(GraphView g, uint32_t nrb, int mode, float* __restrict__ feat,
+                                                  uint8_t* __restrict__ variant_of, int full, float tile_min_nnz,
+                                                  float merge_ratio) {
+  __shared__ uint64_t s_wb[8], s_wm[8];
+  __shared__ uint32_t s_vmax[8], s_top[8], s_wide[8];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (uint32_t rb0 = blockIdx.x * 8; rb0 < nrb; rb0 += gridDim.x * 8) {
+    const uint32_t rb = rb0 + w;
     const uint32_t u = rb * 32 + lane;
-    uint32_t d = 0, nbu = 0, lo = 0xFFFFFFFFu, hi = 0;
-    if (u < g.n) {
+    uint32_t d = 0, nbu = 0, lo = 0xFFFFFFFFu, hi = 0, start = 0;
+    if (rb < nrb && u < g.n) {
       const uint64_t a = g.rp[u], b = g.rp[u + 1];
-      d = rp_row(b) - rp_row(a);
+      start = rp_row(a);
+      d = rp_row(b) - start;
       nbu = rp_blk(b) - rp_blk(a);
       if (d >= 2 && nbu <= kWarpMaxBlocks) {
         lo = (uint32_t)(g.bent[rp_blk(a)] >> 32);
         hi = (uint32_t)(g.bent[rp_blk(b) - 1] >> 32);
       }
     }
+    const uint32_t all = __reduce_add_sync(kFull, d);
+    BlockWork x;
+    if (full) {
+      const uint32_t ps = __shfl_sync(kFull, start, 0);  // lane 0's row exists (or all is 0)
+      const bool grid = g.by_id && all > kFeatGrid, wide = !grid && all > kFeatWarp;
+      if (!grid && !wide) add_work(g, ps, ps + all, 32, start, d, x);
+      if (grid && lane == 0) {
+        const unsigned long long* acc = reinterpret_cast<const unsigned long long*>(feat + (size_t)rb * kNumFeatures);
+        x.wb = acc[0];
+        x.wm = acc[1];
+        x.vmax = (uint32_t)acc[2];
+        x.top = (uint32_t)(acc[2] >> 32);
+      }
+      if (lane == 0) s_wide[w] = wide ? 1u : 0u;
+      if (__syncthreads_or(wide ? 1 : 0)) {
+        uint32_t wides = 0;  // read before the barriers below: s_wide is rewritten after them
+        for (uint32_t k = 0; k < 8; ++k) wides |= s_wide[k] << k;
+        for (uint32_t k = 0; k < 8; ++k) {
+          if (!((wides >> k) & 1u)) continue;
+          const uint32_t uk = (rb0 + k) * 32 + lane;
+          uint32_t sk = 0, dk = 0;
+          if (uk < g.n) {
+            sk = rp_row(g.rp[uk]);
+            dk = rp_row(g.rp[uk + 1]) - sk;
+          }
+          const uint32_t p = __shfl_sync(kFull, sk, 0), len = __reduce_add_sync(kFull, dk);
+          BlockWork y;
+          add_work(g, p + 32 * w, p + len, 256, sk, dk, y);
+          const uint64_t wb = warp_sum(y.wb), wm = warp_sum(y.wm);
+          const uint32_t vmax = __reduce_max_sync(kFull, y.vmax), top = __reduce_add_sync(kFull, y.top);
+          if (lane == 0) {
+            s_wb[w] = wb;
+            s_wm[w] = wm;
+            s_vmax[w] = vmax;
+            s_top[w] = top;
+          }
+          __syncthreads();
+          if (w == k && lane < 8) {
+            x.wb = s_wb[lane];
+            x.wm = s_wm[lane];
+            x.vmax = s_vmax[lane];
+            x.top = s_top[lane];
+          }
+          __syncthreads();
+        }
+      }
+    }
+    if (rb >= nrb) continue;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       lo = min(lo, __shfl_xor_sync(kFull, lo, o));
@@ -1811,38 +1954,13 @@ __global__ void k_features(GraphView g, uint32_t nrb, int mode, float* __restric
     }
     const float span = hi >= lo ? (float)(hi - lo + 1) : 0.f;  // column blocks the tile would cover
     const float fd = (float)d;
-    const float rows = (float)warp_sum(d >= 2 ? 1u : 0u);
-    const float nnz = (float)warp_sum(d);
-    const float nb = (float)warp_sum(nbu);
+    const float rows = (float)__popc(__ballot_sync(kFull, d >= 2));
+    const float nnz = (float)all;
+    const float nb = (float)__reduce_add_sync(kFull, nbu);
     const float sq = warp_sum(fd * fd);
-    uint32_t dmax = d;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dmax = max(dmax, __shfl_xor_sync(kFull, dmax, o));
-    // Neighbour-side work: the bit blocks and ids the sweeps will read.
-    float wb = 0.f, wm = 0.f, vmax = 0.f, top = 0.f;
-    if (full) {
-      for (uint32_t r = 0; r < 32; ++r) {
-        const uint32_t ur = rb * 32 + r;
-        if (ur >= g.n) break;
-        const uint64_t a = g.rp[ur], b = g.rp[ur + 1];
-        const uint32_t rs = rp_row(a), re = rp_row(b);
-        if (re - rs < 2) continue;
-        for (uint32_t k = rs + lane; k < re; k += 32) {
-          const uint32_t v = g.col[k];
-          const uint64_t va = g.rp[v], vb = g.rp[v + 1];
-          const float dv = (float)(rp_row(vb) - rp_row(va));
-          wb += (float)(rp_blk(vb) - rp_blk(va));
-          wm += dv;
-          vmax = fmaxf(vmax, dv);
-          top += v + 4096u >= g.n ? 1.f : 0.f;
-        }
-      }
-      wb = warp_sum(wb);
-      wm = warp_sum(wm);
-      top = warp_sum(top);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(kFull, vmax, o));
-    }
+    const uint32_t dmax = __reduce_max_sync(kFull, d);
+    const float wb = (float)warp_sum(x.wb), wm = (float)warp_sum(x.wm);
+    const float vmax = (float)__reduce_max_sync(kFull, x.vmax), top = (float)__reduce_add_sync(kFull, x.top);
     if (lane == 0) {
       float* f = feat + (size_t)rb * kNumFeatures;
       const float mean = rows > 0 ? nnz / fmaxf(rows, 1.f) : 0.f;
@@ -2486,6 +2604,12 @@ void compute_features(const GraphView& g, Schedule& s, int mode, bool full_featu
   const uint32_t nrb = s.num_row_blocks;
   if (nrb == 0) return;
   const unsigned blocks = (unsigned)std::min<uint64_t>(ceil_div<uint64_t>(nrb, 8), 148ull * 16);
+  if (g.by_id && full_features) {
+    TB_CUDA(cudaMemsetAsync(s.features, 0, (size_t)nrb * kNumFeatures * sizeof(float), st));
+    k_wide_work<<<(unsigned)ceil_div<uint64_t>(ceil_div<uint64_t>(nrb, 32) * kFeatParts, 8), 256, 0, st>>>(g, nrb,
+                                                                                                          s.features);
+    TB_LAUNCH_CHECK();
+  }
   k_features<<<blocks, 256, 0, st>>>(g, nrb, mode, s.features, s.variant_of, full_features ? 1 : 0,
                                      s.tile_min_nnz, s.merge_ratio);
   TB_LAUNCH_CHECK();

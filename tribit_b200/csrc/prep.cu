@@ -952,6 +952,7 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
   out->view.rp = rp;
   out->view.graph_of_rank = graph_of_rank;
   out->view.eflag = nullptr;
+  out->view.by_id = !by_degree;
 
   // Phase 1 (launch only when not measuring): the upload of host entries,
   // degrees and the rank order.

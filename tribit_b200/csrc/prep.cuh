@@ -28,6 +28,7 @@ struct GraphView {
   const uint32_t* graph_of_rank;  // batch mode: graph id of each rank, else null
   const uint32_t* eflag;          // per CSR position, bit set: the edge is counted by the
                                   // hub pass, not by its row (set by the schedule), or null
+  bool by_id = false;             // id order: rows as long as their vertices' degrees
 };
 
 __device__ __forceinline__ uint32_t rp_row(uint64_t w) { return (uint32_t)(w >> 32); }
