@@ -151,12 +151,11 @@ void count_device_input(tribit_context* c, const uint64_t* d_entries, uint64_t E
 }
 
 void fill_schedule_stats(tribit_context* c, tribit_result* res) {
-  uint32_t lens[TRIBIT_NUM_VARIANTS], hub_edges = 0;
-  TB_CUDA(cudaMemcpyAsync(lens, c->sched.list_len, sizeof lens, cudaMemcpyDeviceToHost, c->st));
-  TB_CUDA(cudaMemcpyAsync(&hub_edges, c->sched.piece_off + TRIBIT_NUM_VARIANTS + 4, sizeof hub_edges,
-                          cudaMemcpyDeviceToHost, c->st));
+  uint32_t words[tb::kScheduleWords];
+  TB_CUDA(cudaMemcpyAsync(words, c->sched.piece_off, sizeof words, cudaMemcpyDeviceToHost, c->st));
   TB_CUDA(cudaStreamSynchronize(c->st));
-  res->hub_edges = hub_edges;
+  const uint32_t* lens = words + tb::kOffRowBlocks;
+  res->hub_edges = words[tb::kOffHubEdges];
   res->row_blocks = 0;
   for (int v = 0; v < TRIBIT_NUM_VARIANTS; ++v) {
     res->row_blocks_by_variant[v] = lens[v];

@@ -7,9 +7,10 @@
 // same row, then visits every item of every neighbour v of the piece: v's bit
 // blocks (bitmap) or v's neighbours (merge), each looked up in u's structure.
 // Neighbours with long lists are swept by all 32 lanes; short lists are
-// flattened across lanes. Rows whose structure does not fit a warp's slice go
-// whole to a CTA-wide pass, and rows too large for that to a global-memory
-// pass, so every piece of every list is counted exactly once.
+// flattened across lanes. Rows whose structure does not fit a warp's slice are
+// cut into pieces of their own for a CTA each (heavy), and rows too large for
+// that for a CTA with a larger table or a search in global memory (wide), so
+// every piece of every list is counted exactly once.
 #include <cstddef>
 
 #include "count.cuh"
@@ -25,18 +26,21 @@ constexpr uint32_t kWarpMaxBlocks = kWarpSlots / 2;  // bitmap rows up to this m
 constexpr int kCtaThreads = 512;
 constexpr int kCtaLogSlots = 14;                     // 16384 slots = 128 KiB
 constexpr uint32_t kCtaMaxBlocks = (1u << kCtaLogSlots) / 2;
+constexpr uint32_t kCtaMaxSpan = 2u << kCtaLogSlots;  // masks in the same 128 KiB
 constexpr uint32_t kLong = 24;                       // lists at least this long are swept by the whole warp
 constexpr uint32_t kGrab = 4;                        // pieces taken per cursor update
 constexpr uint64_t kEmptySlot = 0xFFFFFFFF00000000ull;
 
-enum { kCurVariant0 = 0, kCurHubWarp = 3, kCurCta = 4, kCurGlobal = 5, kCurHeavy = 6, kCurHub = 7 };
-// Heavy phase: CTA-shared table in the first 16 KiB of the kernel's shared
-// memory, the row's per-neighbour item prefix in the second 16 KiB.
-constexpr uint32_t kHeavyMaxBlocks = kWarpsPerCta * kWarpSlots / 4;
-constexpr uint32_t kHeavyMaxDeg = kWarpsPerCta * kWarpSlots - 1;
-constexpr uint32_t kHeavyMaxSpan = kWarpsPerCta * kWarpSlots;  // direct-mapped row: 16 KiB of masks
+enum { kCurVariant0 = 0, kCurHubWarp = 3, kCurWide = 4, kCurHeavy = 6, kCurHub = 7 };
+// Heavy phase, in the kernel's 32 KiB of shared memory: the row as masks over
+// its block span (or, wider, as a hash), then the piece's per-neighbour item
+// prefix. A heavy row's neighbours are cut into pieces so that a hub's row
+// (tens of thousands of neighbours under id order) occupies many CTAs.
+constexpr uint32_t kHeavyPiece = 512;
+constexpr uint32_t kHeavyMaxSpan = 2 * kWarpsPerCta * kWarpSlots - (kHeavyPiece + 4);  // words of masks
+constexpr uint32_t kHeavyMaxBlocks = kWarpsPerCta * kWarpSlots / 4;                    // blocks: 16 KiB of hash
+constexpr uint32_t kWidePiece = 2048;
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;
-enum { kOvfCta = 0, kOvfGlobal = 1 };
 
 __device__ __forceinline__ int log2_ceil(uint32_t x) { return x <= 1 ? 0 : 32 - __clz(x - 1); }
 
@@ -375,11 +379,6 @@ __device__ __forceinline__ uint64_t sweep_merge(const GraphView& g, const uint64
   return acc;
 }
 
-__device__ __forceinline__ void push_row(DeviceStats* stats, int which, uint32_t* list, uint32_t u) {
-  const uint32_t i = atomicAdd(&stats->overflow[which], 1u);
-  list[i] = u;
-}
-
 // SM cycle counter; a piece runs on one SM, so differences are meaningful.
 __device__ __forceinline__ unsigned long long cycles() { return (unsigned long long)clock64(); }
 
@@ -406,12 +405,11 @@ struct PiecesShared {
 };
 
 // The row-piece variant V over its pieces (and, with `heavy`, first the heavy
-// rows, one CTA per row); returns this thread's partial count.
+// pieces, one CTA per piece); returns this thread's partial count.
 template <int V>
 __device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64_t* __restrict__ pieces,
                                                 const uint32_t* __restrict__ piece_off, DeviceStats* stats,
-                                                uint32_t* __restrict__ ovf_cta, unsigned long long* per_graph,
-                                                unsigned long long* block_ns, const uint32_t* __restrict__ heavy,
+                                                unsigned long long* per_graph, unsigned long long* block_ns, bool heavy,
                                                 uint32_t width, const PiecesShared& sh) {
   constexpr bool kSorted = V == TRIBIT_VARIANT_MERGE && !TB_MERGE_BITS;  // u staged as a sorted row
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -421,37 +419,31 @@ __device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64
 
   const uint32_t p0 = piece_off[V], len = piece_off[V + 1] - p0;
   uint64_t acc = 0;
-  // Phase 1 (first kernel only): rows too wide for a warp's slice, one at a
-  // time per CTA, with a CTA-shared table in the same shared memory and all
-  // warps sweeping the row's neighbour chunks.
+  // Phase 1 (first kernel only): pieces of the rows too wide for a warp's
+  // slice, one at a time per CTA, with a CTA-shared table in the same shared
+  // memory and all warps sweeping the piece's neighbour chunks.
   if (heavy) {
     uint64_t* ctbl = sh.smem;
-    uint32_t* pre = reinterpret_cast<uint32_t*>(sh.smem + (kWarpsPerCta / 2) * kWarpSlots);
-    const uint32_t hlen = piece_off[TRIBIT_NUM_VARIANTS + 1];
+    uint32_t* pre = reinterpret_cast<uint32_t*>(sh.smem) + kHeavyMaxSpan;
+    const uint32_t h0 = piece_off[kListHeavy], hlen = piece_off[kListHeavy + 1] - h0;
     for (;;) {
-      if (threadIdx.x == 0) {
-        const uint32_t t = atomicAdd(&stats->cursor[kCurHeavy], 1u);
-        s_row = t < hlen ? heavy[hlen - 1 - t] : kNoRow;
-      }
+      if (threadIdx.x == 0) s_row = atomicAdd(&stats->cursor[kCurHeavy], 1u);
       __syncthreads();
-      const uint32_t u = s_row;
-      if (u == kNoRow) break;
+      const uint32_t t = s_row;
+      if (t >= hlen) break;
+      const uint64_t pc = pieces[h0 + (hlen - 1 - t)];
+      const uint32_t u = (uint32_t)(pc >> 32);
       const unsigned long long h_start = (block_ns && threadIdx.x == 0) ? cycles() : 0ull;
       const uint64_t a = g.rp[u], b = g.rp[u + 1];
-      const uint32_t rs = rp_row(a), re = rp_row(b), bs = rp_blk(a), be = rp_blk(b), nb = be - bs;
-      const uint32_t d = re - rs;
-      if (nb > kHeavyMaxBlocks || d > kHeavyMaxDeg) {
-        if (threadIdx.x == 0) push_row(stats, kOvfCta, ovf_cta, u);
-        __syncthreads();
-        continue;
-      }
+      const uint32_t rs = rp_row(a) + (uint32_t)pc, bs = rp_blk(a), be = rp_blk(b);
+      const uint32_t d = min(rp_row(b) - rs, kHeavyPiece);
       // u's row: a direct-mapped mask array over its block span when that
-      // fits the table's 16 KiB (the top-ranked rows), else the bucketed hash.
+      // fits, else the bucketed hash.
       const uint32_t bmin = (uint32_t)(g.bent[bs] >> 32), bmax = (uint32_t)(g.bent[be - 1] >> 32);
       const uint32_t span = bmax - bmin + 1;
       const bool direct = span <= kHeavyMaxSpan;
       uint32_t* cmap = reinterpret_cast<uint32_t*>(ctbl);
-      const int logb = table_logb(nb);
+      const int logb = table_logb(be - bs);
       if (direct) {
         for (uint32_t i = threadIdx.x; i < span; i += blockDim.x) cmap[i] = 0u;
       } else {
@@ -486,7 +478,7 @@ __device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64
       }
       __syncthreads();
       // Warp w takes the neighbours whose first item falls in the w-th equal
-      // share of the row's items, so the warps finish together.
+      // share of the piece's items, so the warps finish together.
       const uint32_t tot = pre[d];
       auto first_at = [&](uint32_t x) -> uint32_t {  // first j with pre[j] >= x
         uint32_t lo = 0, hi = d;
@@ -516,14 +508,14 @@ __device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64
         if (lane == 0 && s) atomicAdd(&per_graph[g.graph_of_rank[u]], (unsigned long long)s);
       }
       acc += racc;
-      __syncthreads();  // the table and s_row are rewritten for the next row
-      // Timing: the row's CTA cycles in warp-cycles, like the warp pieces'.
+      __syncthreads();  // the table and s_row are rewritten for the next piece
+      // Timing: the piece's CTA cycles in warp-cycles, like the warp pieces'.
       if (block_ns && threadIdx.x == 0) atomicAdd(&block_ns[u >> 5], (cycles() - h_start) * kWarpsPerCta);
     }
     __syncthreads();
   }
   uint32_t cur = 0xFFFFFFFFu;  // row whose structure is loaded
-  bool cur_ok = false, cur_direct = false;
+  bool cur_direct = false;
   int logb = 0;
   uint32_t bmin = 0, bmax = 0, d = 0;
   uint32_t* wmap = reinterpret_cast<uint32_t*>(tbl);  // the slice as a direct-mapped row
@@ -545,40 +537,30 @@ __device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64
         cur = u;
         if (kSorted) {
           const uint32_t bs = rp_blk(a), be = rp_blk(b);
-          d = be - bs;  // u's bit-row length
-          cur_ok = d <= kWarpMaxBlocks;
-          if (cur_ok)
-            for (uint32_t k = lane; k < d; k += 32) tbl[k] = g.bent[bs + k];
+          d = be - bs;  // u's bit-row length, at most kWarpMaxBlocks
+          for (uint32_t k = lane; k < d; k += 32) tbl[k] = g.bent[bs + k];
         } else {
-          const uint32_t bs = rp_blk(a), be = rp_blk(b), nb = be - bs;
-          cur_ok = nb <= kWarpMaxBlocks;
-          if (cur_ok) {
-            bmin = (uint32_t)(g.bent[bs] >> 32);
-            bmax = (uint32_t)(g.bent[be - 1] >> 32);
-            // A row whose blocks span at most the slice's 1,024 words is
-            // direct-mapped (one load per probe); others are hashed.
-            cur_direct = bmax - bmin < kWarpSlots * 2;
-            if (cur_direct) {
-              for (uint32_t i = lane; i <= bmax - bmin; i += 32) wmap[i] = 0u;
-              __syncwarp();
-              for (uint32_t k = bs + lane; k < be; k += 32) {
-                const uint64_t e = g.bent[k];
-                wmap[(uint32_t)(e >> 32) - bmin] = (uint32_t)e;
-              }
-            } else {
-              logb = table_logb(nb);
-              table_clear(tbl, logb, lane, 32);
-              __syncwarp();
-              table_insert(tbl, logb, g.bent, bs, be, lane, 32);
+          const uint32_t bs = rp_blk(a), be = rp_blk(b);
+          bmin = (uint32_t)(g.bent[bs] >> 32);
+          bmax = (uint32_t)(g.bent[be - 1] >> 32);
+          // A row whose blocks span at most the slice's 1,024 words is
+          // direct-mapped (one load per probe); others are hashed.
+          cur_direct = bmax - bmin < kWarpSlots * 2;
+          if (cur_direct) {
+            for (uint32_t i = lane; i <= bmax - bmin; i += 32) wmap[i] = 0u;
+            __syncwarp();
+            for (uint32_t k = bs + lane; k < be; k += 32) {
+              const uint64_t e = g.bent[k];
+              wmap[(uint32_t)(e >> 32) - bmin] = (uint32_t)e;
             }
+          } else {
+            logb = table_logb(be - bs);
+            table_clear(tbl, logb, lane, 32);
+            __syncwarp();
+            table_insert(tbl, logb, g.bent, bs, be, lane, 32);
           }
         }
         __syncwarp();
-      }
-      if (!cur_ok) {
-        // The whole row goes to the CTA pass once, from its first piece.
-        if (first == 0 && lane == 0) push_row(stats, kOvfCta, ovf_cta, u);
-        continue;
       }
       const uint32_t cs = rs + first, ce = min(cs + width, re);
       uint64_t racc;
@@ -611,16 +593,14 @@ __device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64
 template <int V>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) k_pieces_warp(GraphView g, const uint64_t* __restrict__ pieces,
                                                                     const uint32_t* __restrict__ piece_off,
-                                                                    DeviceStats* stats, uint32_t* __restrict__ ovf_cta,
-                                                                    unsigned long long* per_graph,
-                                                                    unsigned long long* block_ns,
-                                                                    const uint32_t* __restrict__ heavy,
+                                                                    DeviceStats* stats, unsigned long long* per_graph,
+                                                                    unsigned long long* block_ns, bool heavy,
                                                                     uint32_t width) {
   __shared__ __align__(16) uint64_t smem[kWarpsPerCta][kWarpSlots];
   __shared__ uint32_t runs[kWarpsPerCta][64];
   __shared__ uint32_t s_row;
   const PiecesShared sh{&smem[0][0], kWarpSlots, &runs[0][0], 64, &s_row};
-  uint64_t acc = pieces_body<V>(g, pieces, piece_off, stats, ovf_cta, per_graph, block_ns, heavy, width, sh);
+  uint64_t acc = pieces_body<V>(g, pieces, piece_off, stats, per_graph, block_ns, heavy, width, sh);
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(&stats->triangles, (unsigned long long)acc);
 }
@@ -1165,101 +1145,81 @@ __global__ void __launch_bounds__(kTcThreads) k_tiles_tc(GraphView g, const uint
   if (lane == 0 && acc) atomicAdd(&stats->triangles, (unsigned long long)acc);
 }
 
-// ---- CTA-per-row pass for rows deferred by the warp kernels ---------------
+// ---- wide rows: a CTA per piece, any row size --------------------------------
+// u's row as masks over its block span (up to 32,768 blocks), as a hash (up to
+// kCtaMaxBlocks), or, larger still, left in global memory and binary-searched.
 
-__device__ __forceinline__ uint64_t block_sum_u64(uint64_t v) {
-  __shared__ unsigned long long part[kCtaThreads / 32];
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
-  __syncthreads();
-  uint64_t s = 0;
-  if (threadIdx.x < 32) {
-    s = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0ull;
-    s = warp_sum(s);
-  }
-  __syncthreads();
-  return s;  // valid in thread 0
-}
-
-__global__ void __launch_bounds__(kCtaThreads) k_rows_cta(GraphView g, const uint32_t* __restrict__ rows,
-                                                           DeviceStats* stats, uint32_t* __restrict__ ovf_global,
-                                                           unsigned long long* per_graph,
-                                                           unsigned long long* block_ns) {
+__global__ void __launch_bounds__(kCtaThreads) k_rows_wide(GraphView g, const uint64_t* __restrict__ pieces,
+                                                            const uint32_t* __restrict__ piece_off, DeviceStats* stats,
+                                                            unsigned long long* per_graph,
+                                                            unsigned long long* block_ns) {
   extern __shared__ __align__(16) uint64_t tbl[];
   __shared__ uint32_t runs[kCtaThreads / 32][64];
   __shared__ uint32_t s_t;
-  const uint32_t w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t len = stats->overflow[kOvfCta];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint32_t p0 = piece_off[kListWide], len = piece_off[kListWide + 1] - p0;
   uint64_t acc = 0;
   for (;;) {
-    if (threadIdx.x == 0) s_t = atomicAdd(&stats->cursor[kCurCta], 1u);
+    if (threadIdx.x == 0) s_t = atomicAdd(&stats->cursor[kCurWide], 1u);
     __syncthreads();
     const uint32_t t = s_t;
-    __syncthreads();
     if (t >= len) break;
-    const uint32_t u = rows[t];
+    const uint64_t pc = pieces[p0 + (len - 1 - t)];
+    const uint32_t u = (uint32_t)(pc >> 32);
     const uint64_t a = g.rp[u], b = g.rp[u + 1];
-    const uint32_t rs = rp_row(a), re = rp_row(b), bs = rp_blk(a), be = rp_blk(b), nb = be - bs;
-    if (nb > kCtaMaxBlocks) {
-      if (threadIdx.x == 0) push_row(stats, kOvfGlobal, ovf_global, u);
-      continue;
-    }
+    const uint32_t cs = rp_row(a) + (uint32_t)pc, re = rp_row(b), ce = cs + min(re - cs, kWidePiece);
+    const uint32_t bs = rp_blk(a), be = rp_blk(b), nb = be - bs;
     const unsigned long long t_start = block_ns ? cycles() : 0ull;
-    const int logb = table_logb(nb);
-    table_clear(tbl, logb, threadIdx.x, blockDim.x);
-    __syncthreads();
-    table_insert(tbl, logb, g.bent, bs, be, threadIdx.x, blockDim.x);
-    __syncthreads();
-    const BitmapProbe probe{tbl, logb, (uint32_t)(g.bent[bs] >> 32), (uint32_t)(g.bent[be - 1] >> 32)};
-    const uint64_t racc =
-        sweep_bits(g, rs, re, w, nw, probe, runs[w]);
-    const uint64_t s = block_sum_u64(racc);  // also the barrier before the table is rebuilt
-    if (threadIdx.x == 0) {
-      if (per_graph && s) atomicAdd(&per_graph[g.graph_of_rank[u]], (unsigned long long)s);
-      if (block_ns) atomicAdd(&block_ns[u >> 5], (cycles() - t_start) * (blockDim.x >> 5));
+    const uint32_t bmin = (uint32_t)(g.bent[bs] >> 32), bmax = (uint32_t)(g.bent[be - 1] >> 32);
+    const uint32_t span = bmax - bmin + 1;
+    uint64_t racc;
+    if (span <= kCtaMaxSpan) {
+      uint32_t* cmap = reinterpret_cast<uint32_t*>(tbl);
+      for (uint32_t i = threadIdx.x; i < span; i += blockDim.x) cmap[i] = 0u;
+      __syncthreads();
+      for (uint32_t k = bs + threadIdx.x; k < be; k += blockDim.x) {
+        const uint64_t e = g.bent[k];
+        cmap[(uint32_t)(e >> 32) - bmin] = (uint32_t)e;
+      }
+      __syncthreads();
+      racc = sweep_bits(g, cs, ce, w, nw, [&](uint64_t e) -> uint32_t {
+        const uint32_t o = (uint32_t)(e >> 32) - bmin;
+        return o < span ? (uint32_t)__popc((uint32_t)e & cmap[o]) : 0u;
+      }, runs[w]);
+    } else if (nb <= kCtaMaxBlocks) {
+      const int logb = table_logb(nb);
+      table_clear(tbl, logb, threadIdx.x, blockDim.x);
+      __syncthreads();
+      table_insert(tbl, logb, g.bent, bs, be, threadIdx.x, blockDim.x);
+      __syncthreads();
+      const BitmapProbe probe{tbl, logb, bmin, bmax};
+      racc = sweep_bits(g, cs, ce, w, nw, probe, runs[w]);
+    } else {
+      const uint32_t last = g.col[re - 1];
+      racc = sweep<false>(g, cs, ce, w, nw, [&](uint32_t k, uint32_t c) -> uint32_t {
+        const uint32_t x = g.col[k];
+        if (x > last) return 0u;
+        uint32_t lo = c + 1, hi = re;
+        while (lo < hi) {
+          const uint32_t mid = lo + ((hi - lo) >> 1);
+          if (g.col[mid] < x)
+            lo = mid + 1;
+          else
+            hi = mid;
+        }
+        return (lo < re && g.col[lo] == x) ? 1u : 0u;
+      });
+    }
+    if (per_graph) {
+      const uint64_t s = warp_sum(racc);
+      if (lane == 0 && s) atomicAdd(&per_graph[g.graph_of_rank[u]], (unsigned long long)s);
     }
     acc += racc;
+    __syncthreads();  // the table and s_t are rewritten for the next piece
+    if (block_ns && threadIdx.x == 0) atomicAdd(&block_ns[u >> 5], (cycles() - t_start) * (blockDim.x >> 5));
   }
   acc = warp_sum(acc);
-  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(&stats->triangles, (unsigned long long)acc);
-}
-
-// ---- global-memory pass: any row size, binary search in global memory -----
-
-__global__ void __launch_bounds__(kCtaThreads) k_rows_global(GraphView g, const uint32_t* __restrict__ rows,
-                                                              DeviceStats* stats, unsigned long long* per_graph) {
-  __shared__ uint32_t s_t;
-  const uint32_t w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t len = stats->overflow[kOvfGlobal];
-  uint64_t acc = 0;
-  for (;;) {
-    if (threadIdx.x == 0) s_t = atomicAdd(&stats->cursor[kCurGlobal], 1u);
-    __syncthreads();
-    const uint32_t t = s_t;
-    __syncthreads();
-    if (t >= len) break;
-    const uint32_t u = rows[t];
-    const uint32_t rs = rp_row(g.rp[u]), re = rp_row(g.rp[u + 1]);
-    const uint32_t last = g.col[re - 1];
-    const uint64_t racc = sweep<false>(g, rs, re, w, nw, [&](uint32_t k, uint32_t c) -> uint32_t {
-      const uint32_t x = g.col[k];
-      if (x > last) return 0u;
-      uint32_t lo = c + 1, hi = re;
-      while (lo < hi) {
-        const uint32_t mid = lo + ((hi - lo) >> 1);
-        if (g.col[mid] < x)
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-      return (lo < re && g.col[lo] == x) ? 1u : 0u;
-    });
-    const uint64_t s = block_sum_u64(racc);
-    if (threadIdx.x == 0 && per_graph && s) atomicAdd(&per_graph[g.graph_of_rank[u]], (unsigned long long)s);
-    acc += racc;
-  }
-  acc = warp_sum(acc);
-  if ((threadIdx.x & 31) == 0 && acc) atomicAdd(&stats->triangles, (unsigned long long)acc);
+  if (lane == 0 && acc) atomicAdd(&stats->triangles, (unsigned long long)acc);
 }
 
 // ---- hub pass: the merge variant's walks of u's tail ------------------------
@@ -1579,8 +1539,8 @@ __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t*
   unsigned long long& s_dt = *sh.s_dt;
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t* wruns = sh.runs + w * sh.run_stride;
-  const uint32_t len = piece_off[TRIBIT_NUM_VARIANTS + 2];  // CTA pieces; warp pieces follow them
-  const uint32_t wlen = piece_off[TRIBIT_NUM_VARIANTS + 3] - len;
+  const uint32_t len = piece_off[kOffHubCta];  // CTA pieces; warp pieces follow them
+  const uint32_t wlen = piece_off[kOffHubAll] - len;
   uint64_t acc = 0;
   // Phase 1: hubs with wide rows, one CTA per piece.
   for (;;) {
@@ -1759,8 +1719,7 @@ static_assert(kHubWarpStride % 4 == 0 && kHubWarpStride * 4 >= kWarpSlots * 8, "
 static_assert(kHubMapWords * 4 >= kWarpsPerCta * kWarpSlots * 8, "the map holds the CTA row table and prefix");
 __global__ void __launch_bounds__(kHubWarps * 32, TB_HUB_MIN_CTAS) k_queue(
     GraphView g, const uint64_t* __restrict__ pieces, const uint32_t* __restrict__ piece_off, DeviceStats* stats,
-    uint32_t* __restrict__ ovf_cta, unsigned long long* per_graph, const uint32_t* __restrict__ heavy, uint32_t width,
-    const uint64_t* __restrict__ hub_pieces, const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ in_bits,
+    unsigned long long* per_graph, uint32_t width, const uint64_t* __restrict__ hub_pieces, const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ in_bits,
     const uint64_t* __restrict__ inl) {
   __shared__ __align__(16) uint32_t map[kHubMapWords];
   __shared__ uint32_t pre[kHubPiece + 1];
@@ -1774,9 +1733,8 @@ __global__ void __launch_bounds__(kHubWarps * 32, TB_HUB_MIN_CTAS) k_queue(
   // (warps), then, once the CTA's warps meet, the hub's CTA pieces and its
   // warp pieces. (Hub CTA pieces right after the heavy rows, before the warp
   // pieces, measured 0.5-3% slower on RMAT-18 to 24.)
-  acc += pieces_body<TRIBIT_VARIANT_BITMAP>(g, pieces, piece_off, stats, ovf_cta, per_graph, nullptr, heavy, width, ps);
-  acc += pieces_body<TRIBIT_VARIANT_MERGE>(g, pieces, piece_off, stats, ovf_cta, per_graph, nullptr, nullptr, width,
-                                           ps);
+  acc += pieces_body<TRIBIT_VARIANT_BITMAP>(g, pieces, piece_off, stats, per_graph, nullptr, true, width, ps);
+  acc += pieces_body<TRIBIT_VARIANT_MERGE>(g, pieces, piece_off, stats, per_graph, nullptr, false, width, ps);
   __syncthreads();  // the hub's CTA pieces take the whole map
   acc += hub_body(g, hub_pieces, piece_off, in_off, in_bits, inl, nullptr, stats, per_graph, nullptr, hs);
   acc = warp_sum(acc);
@@ -2003,32 +1961,27 @@ __global__ void __launch_bounds__(256) k_features(GraphView g, uint32_t nrb, int
   }
 }
 
-// Pieces of row u; rows wider than a warp's table are counted whole in the
-// heavy phase instead and get none.
-__device__ __forceinline__ uint32_t row_pieces(const GraphView& g, uint32_t u, uint32_t width) {
+// The list a row's pieces go to: its block's variant's, or, for a row with more
+// bit blocks than a warp's table holds, the heavy or the wide list.
+__device__ __forceinline__ int row_list(const GraphView& g, uint32_t bs, uint32_t be, int variant) {
+  if (be - bs <= kWarpMaxBlocks) return variant;
+  const uint32_t span = (uint32_t)(g.bent[be - 1] >> 32) - (uint32_t)(g.bent[bs] >> 32) + 1;
+  return span <= kHeavyMaxSpan || be - bs <= kHeavyMaxBlocks ? kListHeavy : kListWide;
+}
+
+// Row u's list (of its variant's, the heavy and the wide one) and its pieces
+// there. Rows of fewer than two neighbours, and the rows a bit tile takes with
+// its block, have none.
+__device__ __forceinline__ uint32_t row_pieces(const GraphView& g, uint32_t u, int variant, uint32_t width, int& list) {
+  list = variant;
   if (u >= g.n) return 0u;
   const uint64_t a = g.rp[u], b = g.rp[u + 1];
   const uint32_t d = rp_row(b) - rp_row(a);
-  if (d < 2 || rp_blk(b) - rp_blk(a) > kWarpMaxBlocks) return 0u;
-  return (d + width - 1) / width;
-}
-
-__global__ void k_heavy_flags(GraphView g, uint32_t* __restrict__ flags) {
-  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u > g.n) return;
-  uint32_t f = 0;
-  if (u < g.n) {
-    const uint64_t a = g.rp[u], b = g.rp[u + 1];
-    f = (rp_row(b) - rp_row(a) >= 2 && rp_blk(b) - rp_blk(a) > kWarpMaxBlocks) ? 1u : 0u;
-  }
-  flags[u] = f;
-}
-
-__global__ void k_heavy_scatter(GraphView g, const uint32_t* __restrict__ pos, uint32_t* __restrict__ heavy,
-                                uint32_t* __restrict__ piece_off) {
-  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u < g.n && pos[u + 1] != pos[u]) heavy[pos[u]] = u;
-  if (u == g.n) piece_off[TRIBIT_NUM_VARIANTS + 1] = pos[g.n];
+  if (d < 2) return 0u;
+  list = row_list(g, rp_blk(a), rp_blk(b), variant);
+  if (list == TRIBIT_VARIANT_MMA) return 0u;
+  const uint32_t w = list == kListHeavy ? kHeavyPiece : list == kListWide ? kWidePiece : width;
+  return (d + w - 1) / w;
 }
 
 // Pieces of a bit-tile row block: its neighbour set V (the OR of the active
@@ -2076,54 +2029,75 @@ __device__ uint32_t tile_pieces(const GraphView& g, uint32_t rb, uint32_t* vm) {
   return (c + kTileNbrPiece - 1) / kTileNbrPiece;
 }
 
-// Pieces of each row block (one warp per row block): bit-tile blocks by
-// tile_pieces, the others one per piece_width neighbours of each row.
+// Pieces of each row block (one warp per row block) in every list:
+// counts[l * nrb + rb] = pieces, and 1 << 32 for a block with pieces in its
+// variant's list (the scan then counts those blocks too). Bit-tile blocks have
+// tile_pieces, the others one per `width` neighbours of each row.
 __global__ void __launch_bounds__(256) k_block_pieces(GraphView g, uint32_t nrb, const uint8_t* __restrict__ variant_of,
-                                                      uint32_t* __restrict__ cnt, uint32_t width) {
+                                                      uint64_t* __restrict__ counts, uint32_t width) {
   __shared__ uint32_t vm[8][kTileMaxK];
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  if (warp == 0 && lane == 0) counts[(uint64_t)kPieceLists * nrb] = 0;
   for (uint32_t rb = warp; rb < nrb; rb += nwarps) {
-    const uint32_t s = variant_of[rb] == TRIBIT_VARIANT_MMA ? tile_pieces(g, rb, vm[threadIdx.x >> 5])
-                                                            : warp_sum(row_pieces(g, rb * 32 + lane, width));
-    if (lane == 0) cnt[rb] = s;
+    const int v = variant_of[rb];
+    int list;
+    const uint32_t np = row_pieces(g, rb * 32 + lane, v, width, list);
+    uint32_t own = __reduce_add_sync(kFull, list == v ? np : 0u), heavy = 0, wide = 0;
+    if (__any_sync(kFull, list != v)) {
+      heavy = __reduce_add_sync(kFull, list == kListHeavy ? np : 0u);
+      wide = __reduce_add_sync(kFull, list == kListWide ? np : 0u);
+    }
+    if (v == TRIBIT_VARIANT_MMA) own = tile_pieces(g, rb, vm[threadIdx.x >> 5]);
+    const uint32_t c = (int)lane == v ? own : lane == kListHeavy ? heavy : lane == kListWide ? wide : 0u;
+    if (lane < kPieceLists)
+      counts[(uint64_t)lane * nrb + rb] = c | (lane < TRIBIT_NUM_VARIANTS && c ? 1ull << 32 : 0ull);
   }
 }
 
-__global__ void k_piece_flags(const uint8_t* __restrict__ variant_of, const uint32_t* __restrict__ cnt, uint32_t nrb,
-                              int v, uint32_t* __restrict__ flags, uint32_t* __restrict__ list_len) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nrb) flags[i] = variant_of[i] == v ? cnt[i] : 0u;
-  if (i == nrb) flags[i] = 0u;
-  // row blocks per variant, for reporting
-  if (i < nrb && variant_of[i] == v && cnt[i]) atomicAdd(&list_len[v], 1u);
-}
-
-__global__ void k_piece_segment(const uint32_t* __restrict__ off, uint32_t nrb, int v, uint32_t* piece_off) {
-  if (v == 0) piece_off[0] = 0u;
-  piece_off[v + 1] = piece_off[v] + off[nrb];
-}
-
-__global__ void k_piece_scatter(GraphView g, uint32_t nrb, const uint8_t* __restrict__ variant_of, int v,
-                                const uint32_t* __restrict__ off, const uint32_t* __restrict__ piece_off,
-                                uint64_t* __restrict__ pieces, uint32_t width) {
+// After the scan of counts: every list's pieces, in (list, row) order, and
+// piece_off. The hub words of piece_off start at 0.
+__global__ void __launch_bounds__(256) k_piece_scatter(GraphView g, uint32_t nrb,
+                                                       const uint8_t* __restrict__ variant_of,
+                                                       const uint64_t* __restrict__ counts,
+                                                       uint32_t* __restrict__ piece_off, uint64_t* __restrict__ pieces,
+                                                       uint32_t width) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t seg = piece_off[v];
+  if (warp == 0) {
+    if (lane <= kPieceLists) piece_off[lane] = (uint32_t)counts[(uint64_t)lane * nrb];
+    if (lane >= kOffHubCta && lane <= kOffHubEdges) piece_off[lane] = 0;
+    if (lane < TRIBIT_NUM_VARIANTS)
+      piece_off[kOffRowBlocks + lane] =
+          (uint32_t)(counts[(uint64_t)(lane + 1) * nrb] >> 32) - (uint32_t)(counts[(uint64_t)lane * nrb] >> 32);
+  }
   for (uint32_t rb = warp; rb < nrb; rb += nwarps) {
-    if (variant_of[rb] != v) continue;
-    if (v == TRIBIT_VARIANT_MMA) {
-      const uint32_t base = seg + off[rb], np = off[rb + 1] - off[rb];
+    const int v = variant_of[rb];
+    // Lane l < kPieceLists: where the block's pieces of list l start and end.
+    uint32_t at = 0, end = 0;
+    if (lane < kPieceLists) {
+      at = (uint32_t)counts[(uint64_t)lane * nrb + rb];
+      end = (uint32_t)counts[(uint64_t)lane * nrb + rb + 1];
+    }
+    const uint32_t some = __ballot_sync(kFull, end != at);
+    if (!some) continue;
+    if (v == TRIBIT_VARIANT_MMA && (some & (1u << TRIBIT_VARIANT_MMA))) {
+      const uint32_t base = __shfl_sync(kFull, at, TRIBIT_VARIANT_MMA);
+      const uint32_t np = __shfl_sync(kFull, end, TRIBIT_VARIANT_MMA) - base;
       for (uint32_t k = lane; k < np; k += 32) pieces[base + k] = ((uint64_t)(rb * 32) << 32) | (k * kTileNbrPiece);
-      continue;
     }
     const uint32_t u = rb * 32 + lane;
-    const uint32_t np = row_pieces(g, u, width);
-    const uint32_t incl = warp_inclusive_sum(np);
-    const uint32_t base = seg + off[rb] + incl - np;
-    for (uint32_t k = 0; k < np; ++k) pieces[base + k] = ((uint64_t)u << 32) | (k * width);
+    int list;
+    const uint32_t np = row_pieces(g, u, v, width, list);
+    for (uint32_t todo = some & ~(1u << TRIBIT_VARIANT_MMA); todo; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const uint32_t mine = list == l ? np : 0u;
+      const uint32_t incl = warp_inclusive_sum(mine), base = __shfl_sync(kFull, at, l) + incl - mine;
+      const uint32_t w = l == kListHeavy ? kHeavyPiece : l == kListWide ? kWidePiece : width;
+      for (uint32_t k = 0; k < mine; ++k) pieces[base + k] = ((uint64_t)u << 32) | (k * w);
+    }
   }
 }
 
@@ -2389,13 +2363,13 @@ __global__ void k_hub_piece_scatter(const uint32_t* __restrict__ pos, uint32_t n
       pieces[wpos[v] + k] = ((uint64_t)v << 32) | (k * kHubWarpPiece);
   }
   if (v == n) {
-    piece_off[TRIBIT_NUM_VARIANTS + 2] = pos[n];          // CTA pieces
-    piece_off[TRIBIT_NUM_VARIANTS + 3] = pos[2 * n + 1];  // all pieces
+    piece_off[kOffHubCta] = pos[n];          // CTA pieces
+    piece_off[kOffHubAll] = pos[2 * n + 1];  // all pieces
   }
 }
 
 __global__ void k_hub_total(const uint32_t* __restrict__ in_off, uint32_t n, uint32_t* __restrict__ piece_off) {
-  piece_off[TRIBIT_NUM_VARIANTS + 4] = in_off[n];
+  piece_off[kOffHubEdges] = in_off[n];
 }
 
 // Waves: kHubWaves ranges of rows with equal shares of the bit-row array.
@@ -2442,7 +2416,7 @@ __global__ void k_piece_waves(const uint64_t* __restrict__ pieces, const uint32_
                               const uint64_t* __restrict__ inl, const uint32_t* __restrict__ wave_bk,
                               const uint32_t* __restrict__ wave_cp, uint32_t* __restrict__ cnt,
                               uint8_t* __restrict__ wave) {
-  const uint32_t pc_n = piece_off[TRIBIT_NUM_VARIANTS + 2], all = piece_off[TRIBIT_NUM_VARIANTS + 3];
+  const uint32_t pc_n = piece_off[kOffHubCta], all = piece_off[kOffHubAll];
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < all; p += gridDim.x * blockDim.x) {
     const uint64_t pc = pieces[p];
     const uint32_t v = (uint32_t)(pc >> 32), k = (uint32_t)pc;  // the piece's first entry: k of v's list
@@ -2456,7 +2430,7 @@ __global__ void k_piece_waves(const uint64_t* __restrict__ pieces, const uint32_
 __global__ void k_wave_scan(uint32_t* __restrict__ cnt, const uint32_t* __restrict__ piece_off) {
   uint32_t run = 0;
   for (uint32_t i = 0; i < 2 * kHubWaves; ++i) {
-    if (i == kHubWaves) run = piece_off[TRIBIT_NUM_VARIANTS + 2];  // warp pieces follow the CTA pieces
+    if (i == kHubWaves) run = piece_off[kOffHubCta];  // warp pieces follow the CTA pieces
     const uint32_t c = cnt[i];
     cnt[i] = run;
     run += c;
@@ -2466,7 +2440,7 @@ __global__ void k_wave_scan(uint32_t* __restrict__ cnt, const uint32_t* __restri
 __global__ void k_piece_wave_scatter(const uint64_t* __restrict__ pieces, const uint32_t* __restrict__ piece_off,
                                      const uint8_t* __restrict__ wave, uint32_t* __restrict__ pos,
                                      uint64_t* __restrict__ out) {
-  const uint32_t pc_n = piece_off[TRIBIT_NUM_VARIANTS + 2], all = piece_off[TRIBIT_NUM_VARIANTS + 3];
+  const uint32_t pc_n = piece_off[kOffHubCta], all = piece_off[kOffHubAll];
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < all; p += gridDim.x * blockDim.x)
     out[atomicAdd(&pos[(p < pc_n ? 0 : kHubWaves) + wave[p]], 1u)] = pieces[p];
 }
@@ -2480,16 +2454,10 @@ Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, bool hubs) {
   s.variant_of = ar.take<uint8_t>(nrb + 1);
   s.piece_cap = 2 * n + E / kMinPieceWidth + 64;  // row pieces, plus up to 16 per bit-tile block
   s.pieces = ar.take<uint64_t>(s.piece_cap);
-  s.piece_off = ar.take<uint32_t>(TRIBIT_NUM_VARIANTS + 5);
-  s.heavy = ar.take<uint32_t>(n + 1);
-  s.row_flags = ar.take<uint32_t>(n + 1);
+  s.piece_off = ar.take<uint32_t>(kScheduleWords);
+  s.counts = ar.take<uint64_t>((uint64_t)kPieceLists * nrb + 1);
+  s.scan_tmp = take_scan_temp<uint64_t>(ar, (uint64_t)kPieceLists * nrb + 1);
   s.row_scan_tmp = take_scan_temp<uint32_t>(ar, n + 1);
-  s.list_len = ar.take<uint32_t>(TRIBIT_NUM_VARIANTS);
-  s.block_pieces = ar.take<uint32_t>(nrb + 1);
-  s.flags = ar.take<uint32_t>(nrb + 1);
-  s.scan_tmp = take_scan_temp<uint32_t>(ar, nrb + 1);
-  s.overflow_cap = (uint32_t)(n + 1);
-  s.overflow = ar.take<uint32_t>(2 * (n + 1));
   s.features = ar.take<float>((uint64_t)nrb * kNumFeatures + 1);
   if (hubs) {
     s.eflag_words = E / 32 + 2;
@@ -2513,12 +2481,11 @@ Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, bool hubs) {
   return s;
 }
 
-// Hub in-lists and pieces of the merge row blocks (after the heavy-row list:
-// its scan space is reused for the in-list offsets). Without hub arrays, or
-// with hubs off, the hub pass gets no pieces and no edge is flagged.
+// Hub in-lists and pieces of the merge row blocks (after k_piece_scatter, which
+// clears the hub words of piece_off). Without hub arrays, or with hubs off, the
+// hub pass gets no pieces and no edge is flagged.
 static void build_hubs(const GraphView& g, Schedule& s, cudaStream_t st) {
   s.hubs_active = false;
-  TB_CUDA(cudaMemsetAsync(s.piece_off + TRIBIT_NUM_VARIANTS + 2, 0, 3 * sizeof(uint32_t), st));
   if (!s.eflag || !s.hubs || g.n == 0) return;
   const uint64_t n = g.n;
   const unsigned vblocks = (unsigned)ceil_div<uint64_t>(n + 1, 256);
@@ -2573,29 +2540,11 @@ static void build_hubs(const GraphView& g, Schedule& s, cudaStream_t st) {
 void build_pieces(const GraphView& g, Schedule& s, cudaStream_t st) {
   const uint32_t nrb = s.num_row_blocks;
   const unsigned wblocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div<uint64_t>(nrb, 8), 148ull * 16));
-  const unsigned fblocks = (unsigned)ceil_div<uint64_t>(nrb + 1, 256);
-  TB_CUDA(cudaMemsetAsync(s.list_len, 0, TRIBIT_NUM_VARIANTS * sizeof(uint32_t), st));
-  if (nrb) {
-    k_block_pieces<<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.block_pieces, s.piece_width);
-    TB_LAUNCH_CHECK();
-  }
-  for (int v = 0; v < TRIBIT_NUM_VARIANTS; ++v) {
-    k_piece_flags<<<fblocks, 256, 0, st>>>(s.variant_of, s.block_pieces, nrb, v, s.flags, s.list_len);
-    TB_LAUNCH_CHECK();
-    device_scan<uint32_t, OpSum>(s.flags, s.flags, nrb + 1, true, OpSum{}, 0u, s.scan_tmp, st);
-    k_piece_segment<<<1, 1, 0, st>>>(s.flags, nrb, v, s.piece_off);
-    TB_LAUNCH_CHECK();
-    if (nrb) {
-      k_piece_scatter<<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, v, s.flags, s.piece_off, s.pieces,
-                                               s.piece_width);
-      TB_LAUNCH_CHECK();
-    }
-  }
-  const unsigned rblocks = (unsigned)ceil_div<uint64_t>((uint64_t)g.n + 1, 256);
-  k_heavy_flags<<<rblocks, 256, 0, st>>>(g, s.row_flags);
+  k_block_pieces<<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.counts, s.piece_width);
   TB_LAUNCH_CHECK();
-  device_scan<uint32_t, OpSum>(s.row_flags, s.row_flags, (uint64_t)g.n + 1, true, OpSum{}, 0u, s.row_scan_tmp, st);
-  k_heavy_scatter<<<rblocks, 256, 0, st>>>(g, s.row_flags, s.heavy, s.piece_off);
+  device_scan<uint64_t, OpSum>(s.counts, s.counts, (uint64_t)kPieceLists * nrb + 1, true, OpSum{}, 0ull, s.scan_tmp,
+                               st);
+  k_piece_scatter<<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.counts, s.piece_off, s.pieces, s.piece_width);
   TB_LAUNCH_CHECK();
   build_hubs(g, s, st);
 }
@@ -2639,7 +2588,7 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
   GraphView g = graph;
   g.eflag = s.hubs_active ? s.eflag : nullptr;
   once_per_device<0>([] {
-    TB_CUDA(cudaFuncSetAttribute(k_rows_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    TB_CUDA(cudaFuncSetAttribute(k_rows_wide, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(uint64_t) << kCtaLogSlots)));
     TB_CUDA(cudaFuncSetAttribute(k_tiles_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(kTileWarps * sizeof(TileSmem))));
@@ -2649,20 +2598,22 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
   const int per_sm = cfg.ctas_per_sm > 0 ? cfg.ctas_per_sm : 6;
   const unsigned warp_grid = (unsigned)(sms * per_sm);
   LaunchInfo info;
-  static_assert(offsetof(DeviceStats, cursor) == offsetof(DeviceStats, count_err) + sizeof(unsigned int) &&
-                    offsetof(DeviceStats, overflow) == offsetof(DeviceStats, cursor) + sizeof(DeviceStats::cursor),
-                "count_err, cursor and overflow are cleared by one memset");
-  TB_CUDA(cudaMemsetAsync(&stats->count_err, 0,
-                          sizeof(stats->count_err) + sizeof(stats->cursor) + sizeof(stats->overflow), st));
-  TB_CUDA(cudaMemsetAsync(&stats->triangles, 0, sizeof(stats->triangles), st));
-  uint32_t* ovf_cta = s.overflow;
-  uint32_t* ovf_global = s.overflow + s.overflow_cap;
+  TB_CUDA(cudaMemsetAsync(&stats->triangles, 0, sizeof(DeviceStats) - offsetof(DeviceStats, triangles), st));
+  // Wide rows span more blocks than the heavy phase's masks, so smaller graphs have none.
+  const bool wide = ceil_div<uint64_t>(g.n, 32) > kHeavyMaxSpan;
+  auto rows_wide = [&] {
+    if (!wide) return;
+    k_rows_wide<<<(unsigned)sms, kCtaThreads, sizeof(uint64_t) << kCtaLogSlots, st>>>(g, s.pieces, s.piece_off, stats,
+                                                                                      per_graph, cfg.block_ns);
+    TB_LAUNCH_CHECK();
+    info.ctas += sms;
+    ++info.kernels;
+  };
   if (cfg.queue && !cfg.block_ns && !cfg.variant_start) {
     // One persistent kernel for the row pieces and the hub pass; the tiles and
     // the fallback rows (whose list k_queue fills) after it.
     k_queue<<<(unsigned)(sms * kHubCtasPerSm), kHubWarps * 32, 0, st>>>(
-        g, s.pieces, s.piece_off, stats, ovf_cta, per_graph, s.heavy, s.piece_width, s.hub_pieces, s.in_off,
-        s.in_cnt, s.inl);
+        g, s.pieces, s.piece_off, stats, per_graph, s.piece_width, s.hub_pieces, s.in_off, s.in_cnt, s.inl);
     TB_LAUNCH_CHECK();
     if (s.tile_engine == TRIBIT_TILES_TCGEN05)
       k_tiles_tc<<<(unsigned)(sms * kTcCtasPerSm), kTcThreads, sizeof(TcSmem), st>>>(
@@ -2671,20 +2622,16 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
       k_tiles_mma<<<(unsigned)(sms * 5), kTileWarps * 32, kTileWarps * sizeof(TileSmem), st>>>(
           g, s.pieces, s.piece_off, stats, per_graph, nullptr);
     TB_LAUNCH_CHECK();
-    k_rows_cta<<<(unsigned)sms, kCtaThreads, sizeof(uint64_t) << kCtaLogSlots, st>>>(g, ovf_cta, stats, ovf_global,
-                                                                                     per_graph, nullptr);
-    TB_LAUNCH_CHECK();
-    k_rows_global<<<(unsigned)sms, kCtaThreads, 0, st>>>(g, ovf_global, stats, per_graph);
-    TB_LAUNCH_CHECK();
-    info.ctas = (uint64_t)(kHubCtasPerSm + (s.tile_engine == TRIBIT_TILES_TCGEN05 ? kTcCtasPerSm : 5) + 2) * sms;
-    info.kernels = 4;
+    info.ctas = (uint64_t)(kHubCtasPerSm + (s.tile_engine == TRIBIT_TILES_TCGEN05 ? kTcCtasPerSm : 5)) * sms;
+    info.kernels = 2;
+    rows_wide();
     return info;
   }
   // Timing mode: the events bracket every counting kernel, and every piece,
   // heavy row, tile block and hub piece adds its warp-cycles to its row block.
   if (cfg.variant_start) TB_CUDA(cudaEventRecord(cfg.variant_start, st));
   k_pieces_warp<TRIBIT_VARIANT_BITMAP><<<warp_grid, kWarpsPerCta * 32, 0, st>>>(
-      g, s.pieces, s.piece_off, stats, ovf_cta, per_graph, cfg.block_ns, s.heavy, s.piece_width);
+      g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, true, s.piece_width);
   TB_LAUNCH_CHECK();
   if (s.tile_engine == TRIBIT_TILES_TCGEN05)
     k_tiles_tc<<<(unsigned)(sms * kTcCtasPerSm), kTcThreads, sizeof(TcSmem), st>>>(
@@ -2693,22 +2640,17 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
     k_tiles_mma<<<(unsigned)(sms * 5), kTileWarps * 32, kTileWarps * sizeof(TileSmem), st>>>(
         g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns);
   TB_LAUNCH_CHECK();
-  k_pieces_warp<TRIBIT_VARIANT_MERGE><<<warp_grid, kWarpsPerCta * 32, 0, st>>>(g, s.pieces, s.piece_off, stats, ovf_cta,
-                                                                               per_graph, cfg.block_ns, nullptr,
-                                                                               s.piece_width);
+  k_pieces_warp<TRIBIT_VARIANT_MERGE><<<warp_grid, kWarpsPerCta * 32, 0, st>>>(
+      g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, false, s.piece_width);
   TB_LAUNCH_CHECK();
-  k_rows_cta<<<(unsigned)sms, kCtaThreads, sizeof(uint64_t) << kCtaLogSlots, st>>>(g, ovf_cta, stats, ovf_global,
-                                                                                   per_graph, cfg.block_ns);
-  TB_LAUNCH_CHECK();
-  k_rows_global<<<(unsigned)sms, kCtaThreads, 0, st>>>(g, ovf_global, stats, per_graph);
-  TB_LAUNCH_CHECK();
+  rows_wide();
   k_hub<<<(unsigned)(sms * kHubCtasPerSm), kHubWarps * 32, 0, st>>>(g, s.hub_pieces, s.piece_off, s.in_off, s.in_cnt,
                                                                      s.inl, s.inrow, stats, per_graph, cfg.block_ns);
   TB_LAUNCH_CHECK();
   if (cfg.variant_stop) TB_CUDA(cudaEventRecord(cfg.variant_stop, st));
-  info.ctas = 2ull * warp_grid +
-              (2ull + (s.tile_engine == TRIBIT_TILES_TCGEN05 ? (uint64_t)kTcCtasPerSm : 5ull) + kHubCtasPerSm) * sms;
-  info.kernels = 6;
+  info.ctas += 2ull * warp_grid +
+               ((s.tile_engine == TRIBIT_TILES_TCGEN05 ? (uint64_t)kTcCtasPerSm : 5ull) + kHubCtasPerSm) * sms;
+  info.kernels += 4;
   return info;
 }
 

@@ -32,22 +32,24 @@ constexpr uint32_t kMinPieceWidth = 32;  // piece_width is a multiple of 32, at 
 // RMAT-22/24 but loses 48% on planted and Erdos-Renyi, 2.0 loses 96% on RMAT-24).
 constexpr float kDefaultMergeRatio = 0.75f;
 
+// Piece lists: one per variant, the heavy rows' (too many bit blocks for a
+// warp's table: a CTA per piece) and the wide rows' (too many for the heavy
+// phase's 32 KiB as well: kernel k_rows_wide).
+enum { kListHeavy = TRIBIT_NUM_VARIANTS, kListWide, kPieceLists };
+// piece_off: where each list starts in `pieces` (and where the last ends), the
+// hub pass's CTA pieces, all its pieces and its edges, then the row blocks with
+// pieces of each variant.
+enum { kOffHubCta = kPieceLists + 1, kOffHubAll, kOffHubEdges, kOffRowBlocks, kScheduleWords = kOffRowBlocks + TRIBIT_NUM_VARIANTS };
+
 struct Schedule {
   uint32_t num_row_blocks = 0;
   uint8_t* variant_of = nullptr;   // device, per row block
-  uint64_t* pieces = nullptr;      // device, (row << 32) | first neighbour, grouped by variant
+  uint64_t* pieces = nullptr;      // device, (row << 32) | first neighbour, one segment per piece list
   uint64_t piece_cap = 0;
-  uint32_t* piece_off = nullptr;   // device, TRIBIT_NUM_VARIANTS + 1 segment starts, the heavy-row count,
-                                   // the CTA hub-piece count, all hub pieces, the hub-edge count
-  uint32_t* heavy = nullptr;       // device, rows too wide for one warp, counted CTA-cooperatively first
-  uint32_t* row_flags = nullptr;   // device, n + 1 scratch for the heavy-row scan
+  uint32_t* piece_off = nullptr;   // device, kScheduleWords words (see there)
+  uint64_t* counts = nullptr;      // device, kPieceLists * nrb + 1: pieces per (list, row block), scanned
+  uint64_t* scan_tmp = nullptr;
   uint32_t* row_scan_tmp = nullptr;
-  uint32_t* list_len = nullptr;    // device, row blocks per variant
-  uint32_t* block_pieces = nullptr;// device, pieces per row block
-  uint32_t* flags = nullptr;       // device, nrb + 1 scratch for the scans
-  uint32_t* scan_tmp = nullptr;
-  uint32_t* overflow = nullptr;    // device, rows deferred to the CTA / global passes
-  uint32_t overflow_cap = 0;
   float* features = nullptr;       // device, nrb x kNumFeatures
   // Hub pass of the merge variant (absent when taken without hubs).
   uint32_t* eflag = nullptr;       // device, bit per CSR position: edge counted by the hub pass

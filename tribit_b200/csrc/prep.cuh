@@ -36,13 +36,14 @@ __device__ __forceinline__ uint32_t rp_blk(uint64_t w) { return (uint32_t)w; }
 
 // Counters the device writes and the host reads back once per call.
 struct DeviceStats {
-  unsigned long long triangles;
   unsigned long long edges;        // undirected edges after dedup (m)
   unsigned long long blocks;       // bit-row entries (nb)
   unsigned int err;                // kErr* flags of the preprocessing
-  unsigned int count_err;          // kErr* flags of the latest counting launch (cleared by each launch)
+  unsigned int pad;
+  // From here on cleared by each counting launch.
+  unsigned long long triangles;
+  unsigned int count_err;          // kErr* flags of the latest counting launch
   unsigned int cursor[8];          // work cursors of the counting kernels
-  unsigned int overflow[8];        // overflow-list lengths
 };
 
 // Upload of host entries overlapped with the degree pass: the entries are
