@@ -1273,13 +1273,20 @@ constexpr uint32_t kHubPiece = TB_HUB_PIECE;    // in-edges per CTA piece
 #define TB_HUB_WARP_PIECE 128
 #endif
 constexpr uint32_t kHubWarpPiece = TB_HUB_WARP_PIECE;  // in-edges per warp piece
+#ifndef TB_HUB_WAVE_SHIFT
+#define TB_HUB_WAVE_SHIFT 22
+#endif
 #ifndef TB_HUB_WAVES
 #define TB_HUB_WAVES 32
 #endif
 constexpr uint32_t kHubWaves = TB_HUB_WAVES;    // row ranges the hub pieces are ordered by (power of 2)
-// Up to this many entries (bit rows of at most 64 MiB) the in-lists are filled
-// in one launch instead of one per wave.
-constexpr uint64_t kHubOneWaveEntries = 1ull << 23;
+// Waves of a graph of E entries: one up to 2^23 (bit rows of at most 64 MiB, which
+// the L2 holds whatever the order), then one per 2^22 entries: each wave is a
+// launch with a tail of its own (one per 2^21: RMAT-20 0.4%, cliques 2% slower; 2^20: 2%).
+inline uint32_t hub_waves(uint64_t E) {
+  if (E <= (1ull << 23)) return 1;
+  return (uint32_t)std::min<uint64_t>(kHubWaves, E >> TB_HUB_WAVE_SHIFT);
+}
 // Five CTAs per SM (48 registers), the occupancy the 41 KiB of shared memory
 // allows; with four the pair loads' extra registers cost more than they save.
 #ifndef TB_HUB_MIN_CTAS
@@ -2032,10 +2039,23 @@ __device__ uint32_t tile_pieces(const GraphView& g, uint32_t rb, uint32_t* vm) {
 // Pieces of each row block (one warp per row block) in every list:
 // counts[l * nrb + rb] = pieces, and 1 << 32 for a block with pieces in its
 // variant's list (the scan then counts those blocks too). Bit-tile blocks have
-// tile_pieces, the others one per `width` neighbours of each row.
+// tile_pieces, the others one per `width` neighbours of each row. With hub
+// arrays it also starts the hub builder: vinfo[v] = (span << 32) | nb, v's
+// bit-row length and the blocks it spans, and its counters and flags at 0.
+struct HubInit {
+  uint64_t* vinfo;  // null: no hub pass
+  unsigned long long* save;
+  uint32_t* in_cnt;
+  uint32_t* eflag;
+  uint64_t eflag_words;
+};
 __global__ void __launch_bounds__(256) k_block_pieces(GraphView g, uint32_t nrb, const uint8_t* __restrict__ variant_of,
-                                                      uint64_t* __restrict__ counts, uint32_t width) {
+                                                      uint64_t* __restrict__ counts, uint32_t width, HubInit hub) {
   __shared__ uint32_t vm[8][kTileMaxK];
+  if (hub.vinfo)
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < hub.eflag_words;
+         i += (uint64_t)gridDim.x * blockDim.x)
+      hub.eflag[i] = 0;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -2043,7 +2063,16 @@ __global__ void __launch_bounds__(256) k_block_pieces(GraphView g, uint32_t nrb,
   for (uint32_t rb = warp; rb < nrb; rb += nwarps) {
     const int v = variant_of[rb];
     int list;
-    const uint32_t np = row_pieces(g, rb * 32 + lane, v, width, list);
+    const uint32_t u = rb * 32 + lane;
+    if (hub.vinfo && u < g.n) {
+      const uint32_t bs = rp_blk(g.rp[u]), be = rp_blk(g.rp[u + 1]);
+      uint64_t x = 0;
+      if (be > bs) x = ((uint64_t)((uint32_t)(g.bent[be - 1] >> 32) - (uint32_t)(g.bent[bs] >> 32) + 1) << 32) | (be - bs);
+      hub.vinfo[u] = x;
+      hub.save[u] = 0;
+      hub.in_cnt[u] = 0;
+    }
+    const uint32_t np = row_pieces(g, u, v, width, list);
     uint32_t own = __reduce_add_sync(kFull, list == v ? np : 0u), heavy = 0, wide = 0;
     if (__any_sync(kFull, list != v)) {
       heavy = __reduce_add_sync(kFull, list == kListHeavy ? np : 0u);
@@ -2103,20 +2132,6 @@ __global__ void __launch_bounds__(256) k_piece_scatter(GraphView g, uint32_t nrb
 
 // ---- hub schedule -----------------------------------------------------------
 
-// vinfo[v] = (span << 32) | nb: v's bit-row length and the blocks it spans.
-__global__ void k_hub_vinfo(GraphView g, uint64_t* __restrict__ vinfo) {
-  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= g.n) return;
-  const uint64_t a = g.rp[v], b = g.rp[v + 1];
-  const uint32_t bs = rp_blk(a), be = rp_blk(b);
-  uint64_t x = 0;
-  if (be > bs) {
-    const uint32_t span = (uint32_t)(g.bent[be - 1] >> 32) - (uint32_t)(g.bent[bs] >> 32) + 1;
-    x = ((uint64_t)span << 32) | (be - bs);
-  }
-  vinfo[v] = x;
-}
-
 // Hub candidate: the edge at CSR position j (u -> v; v's block at index pos of
 // u's bit row, u's tail `tail` blocks from it) whose tail is shorter than v's
 // row, with v stageable. cost: what staging v's row costs (the direct map's
@@ -2137,8 +2152,10 @@ __device__ __forceinline__ bool hub_candidate(const uint64_t* __restrict__ vinfo
 
 // One pass over the edges of the merge row blocks; rows of at most
 // kHubLaneRow neighbours are walked by their own lane, longer rows by the
-// whole warp (mode 1 on a small wave: one warp per row). For the edge at CSR
-// position j, u's tail is u's bit blocks from v's block on.
+// whole warp (mode 1 on a small wave: one warp per row), rows of more than
+// kHubCtaRow, left to the end, by the whole CTA. For the edge at CSR position
+// j, u's tail is u's bit blocks from v's block on. Neighbouring row blocks go to
+// different CTAs, so the top ranks' long rows spread over the chip.
 // Mode 0: counts each hub's candidate in-edges (in_cnt) and adds to save[v]
 // the blocks a hub walk saves (v's row length - tail), but only while save[v]
 // is below the staging cost: the decision save[v] >= cost (k_hub_accept) is
@@ -2151,6 +2168,8 @@ __device__ __forceinline__ bool hub_candidate(const uint64_t* __restrict__ vinfo
 // save[v] counts them). rows (may be null): the pass covers rows
 // [rows[0], rows[1]).
 constexpr uint32_t kHubLaneRow = 64;
+constexpr uint32_t kHubCtaRow = 2048;
+constexpr uint32_t kHubCtaRows = 256;  // a CTA's list of them; rows past it are walked by their warp
 #ifndef TB_HUB_TOP
 #define TB_HUB_TOP 1024
 #endif
@@ -2166,9 +2185,11 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
                             uint32_t* __restrict__ in_cnt, const uint32_t* __restrict__ in_off,
                             uint64_t* __restrict__ inl, uint32_t* __restrict__ inrow,
                             const uint32_t* __restrict__ rows) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  __shared__ uint32_t s_long[kHubCtaRows], s_nlong, s_heads[8];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t warp = w * gridDim.x + blockIdx.x, nwarps = 8 * gridDim.x;  // 8 warps a CTA
+  if (threadIdx.x == 0) s_nlong = 0;
+  __syncthreads();
   const uint32_t u0 = rows ? rows[0] : 0u, u1 = rows ? rows[1] : g.n;  // rows [u0, u1)
   // Mode 0: candidate counts and savings of the vertices ranked top_lo and
   // above, per CTA. A CTA adds to a saving only while it is below the cost,
@@ -2214,12 +2235,13 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
       if (inrow) inrow[at] = u;  // timing mode only
     }
   };
-  // Walks row u (CSR [rs, re), nb bit blocks from bs) with the whole warp.
-  auto warp_row = [&](uint32_t u, uint32_t rs, uint32_t re, uint32_t bs, uint32_t nb) {
-    uint32_t carry = 0, prev_last = 0xFFFFFFFFu;
-    for (uint32_t c = rs; c < re; c += 32) {
+  // Walks positions [c0, c1) of row u (CSR up to re, nb bit blocks from bs)
+  // with the whole warp; carry: blocks begun before c0, prev_last: the last of them.
+  auto warp_span = [&](uint32_t u, uint32_t c0, uint32_t c1, uint32_t re, uint32_t bs, uint32_t nb, uint32_t carry,
+                       uint32_t prev_last) {
+    for (uint32_t c = c0; c < c1; c += 32) {
       const uint32_t j = c + lane;
-      const bool in = j < re;
+      const bool in = j < c1;
       const uint32_t v = in ? g.col[j] : 0u;
       const uint32_t blk = in ? v >> 5 : 0xFFFFFFFFu;
       uint32_t prev = __shfl_up_sync(kFull, blk, 1);
@@ -2243,7 +2265,19 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
       if (hub) edge(u, bs, j, re, v, pos, tail, nbv, cost);
     }
   };
-  if (Mode == 1 && u1 - u0 < 32u * nwarps) {
+  auto warp_row = [&](uint32_t u, uint32_t rs, uint32_t re, uint32_t bs, uint32_t nb) {
+    if (re - rs > kHubCtaRow) {
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&s_nlong, 1u);
+      at = __shfl_sync(kFull, at, 0);
+      if (at < kHubCtaRows) {
+        if (lane == 0) s_long[at] = u;
+        return;
+      }
+    }
+    warp_span(u, rs, re, re, bs, nb, 0, 0xFFFFFFFFu);
+  };
+  if (u1 - u0 < (Mode == 1 ? 32u : 8u) * nwarps) {
     // The in-list fill runs once per row wave; a wave of fewer rows than the
     // grid has lanes keeps every warp busy with one warp per row. Larger waves
     // (the first ones: millions of short rows) take the row-block loop below.
@@ -2304,6 +2338,27 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
       }
     }
   }
+  // The CTA's longest rows, an eighth a warp: the block heads of the shares
+  // before a warp's give the index of its first block.
+  __syncthreads();
+  for (uint32_t k = 0, cnt = min(s_nlong, kHubCtaRows); k < cnt; ++k) {
+    const uint32_t u = s_long[k];
+    const uint64_t a = g.rp[u], b = g.rp[u + 1];
+    const uint32_t rs = rp_row(a), d = rp_row(b) - rs;
+    const uint32_t c0 = rs + (uint32_t)((uint64_t)d * w / 8), c1 = rs + (uint32_t)((uint64_t)d * (w + 1) / 8);
+    uint32_t heads = 0;
+    for (uint32_t c = c0; c < c1; c += 32) {
+      const uint32_t j = c + lane;
+      heads += __popc(__ballot_sync(kFull, j < c1 && (j == rs || (g.col[j] >> 5) != (g.col[j - 1] >> 5))));
+    }
+    __syncthreads();  // s_heads of the row before has been read
+    if (lane == 0) s_heads[w] = heads;
+    __syncthreads();
+    uint32_t before = 0;
+    for (uint32_t q = 0; q < w; ++q) before += s_heads[q];
+    warp_span(u, c0, c1, rs + d, rp_blk(a), rp_blk(b) - rp_blk(a), before,
+              c0 == rs ? 0xFFFFFFFFu : g.col[c0 - 1] >> 5);
+  }
   if constexpr (kTop != 0) {
     __syncthreads();
     for (uint32_t t = threadIdx.x; t < kTop && top_lo + t < g.n; t += blockDim.x) {
@@ -2318,63 +2373,58 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
 // its candidate count (the length of its in-list) and is marked in save[v]
 // (1 << 32: the low word then counts its column tails in mode 1); any other
 // vertex gets no in-list, and its vinfo is cleared so that mode 1 takes none
-// of its edges.
+// of its edges. cnt: the in-list lengths, then the pieces of each hub for a
+// CTA and for a warp, n + 1 of each (0 at the ends), to be scanned as one array.
 __global__ void k_hub_accept(uint64_t* __restrict__ vinfo, uint32_t n, unsigned long long* __restrict__ save,
-                             uint32_t* __restrict__ in_cnt) {
-  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  const uint64_t vi = vinfo[v];
-  const bool acc = in_cnt[v] > 0 && save[v] >= hub_cost((uint32_t)(vi >> 32), (uint32_t)vi);
-  if (!acc) {
-    in_cnt[v] = 0;
-    vinfo[v] = 0;  // no candidate in mode 1, no pieces
-  }
-  save[v] = acc ? (1ull << 32) : 0ull;
-}
-
-__global__ void k_hub_piece_count(const uint32_t* __restrict__ in_off, const uint64_t* __restrict__ vinfo,
-                                  uint32_t n, uint32_t* __restrict__ cnt) {
+                             uint32_t* __restrict__ in_cnt, uint32_t* __restrict__ cnt) {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v > n) return;
-  uint32_t c = 0, wc = 0;
+  uint32_t k = 0, c = 0, wc = 0;
   if (v < n) {
-    const uint32_t k = in_off[v + 1] - in_off[v];
-    const uint32_t span = (uint32_t)(vinfo[v] >> 32), nb = (uint32_t)vinfo[v];
+    const uint64_t vi = vinfo[v];
+    const uint32_t span = (uint32_t)(vi >> 32), nb = (uint32_t)vi;
+    k = in_cnt[v];
+    in_cnt[v] = 0;
+    if (k > 0 && save[v] < hub_cost(span, nb)) k = 0;
+    if (k == 0) vinfo[v] = 0;  // no candidate in mode 1
+    save[v] = k ? (1ull << 32) : 0ull;
     // The warp stages the row when its direct map fits the warp's slice, or,
     // for a row too wide for the CTA's direct map, when its hash does.
-    const bool warp = span <= kHubWarpSpan || (span > kHubMaxSpan && nb <= kHubWarpHash);
-    if (warp)
+    if (span <= kHubWarpSpan || (span > kHubMaxSpan && nb <= kHubWarpHash))
       wc = (k + kHubWarpPiece - 1) / kHubWarpPiece;
     else
       c = (k + kHubPiece - 1) / kHubPiece;
   }
-  cnt[v] = c;
-  cnt[n + 1 + v] = wc;
+  cnt[v] = k;
+  cnt[(uint64_t)n + 1 + v] = c;
+  cnt[2 * ((uint64_t)n + 1) + v] = wc;
 }
 
+// After the scan: the pieces of every hub and the hub words of piece_off;
+// wave_cnt (2 kHubWaves words, may be null) at 0. Positions count from pos[0],
+// where the in-list entries end.
 __global__ void k_hub_piece_scatter(const uint32_t* __restrict__ pos, uint32_t n, uint64_t* __restrict__ pieces,
-                                    uint32_t* __restrict__ piece_off) {
+                                    uint32_t* __restrict__ piece_off, uint32_t* __restrict__ wave_cnt) {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t* wpos = pos + (uint64_t)n + 1;
+  const uint32_t base = pos[0];
   if (v < n) {
-    for (uint32_t k = 0, np = pos[v + 1] - pos[v]; k < np; ++k)
-      pieces[pos[v] + k] = ((uint64_t)v << 32) | (k * kHubPiece);
-    const uint32_t* wpos = pos + n + 1;
-    for (uint32_t k = 0, np = wpos[v + 1] - wpos[v]; k < np; ++k)
-      pieces[wpos[v] + k] = ((uint64_t)v << 32) | (k * kHubWarpPiece);
+    for (uint32_t k = 0, at = pos[v] - base, np = pos[v + 1] - pos[v]; k < np; ++k)
+      pieces[at + k] = ((uint64_t)v << 32) | (k * kHubPiece);
+    for (uint32_t k = 0, at = wpos[v] - base, np = wpos[v + 1] - wpos[v]; k < np; ++k)
+      pieces[at + k] = ((uint64_t)v << 32) | (k * kHubWarpPiece);
   }
   if (v == n) {
-    piece_off[kOffHubCta] = pos[n];          // CTA pieces
-    piece_off[kOffHubAll] = pos[2 * n + 1];  // all pieces
+    piece_off[kOffHubCta] = pos[n] - base;    // CTA pieces
+    piece_off[kOffHubAll] = wpos[n] - base;   // all pieces
+    piece_off[kOffHubEdges] = base;           // in-list entries
   }
+  if (wave_cnt && v < 2 * kHubWaves) wave_cnt[v] = 0;
 }
 
-__global__ void k_hub_total(const uint32_t* __restrict__ in_off, uint32_t n, uint32_t* __restrict__ piece_off) {
-  piece_off[kOffHubEdges] = in_off[n];
-}
-
-// Waves: kHubWaves ranges of rows with equal shares of the bit-row array.
-// wave_lo[w] = first row whose bit row starts at or after w / kHubWaves of
-// it (wave_lo[kHubWaves] = n). The in-lists are filled one wave of rows at a
+// Waves: up to kHubWaves ranges of rows with equal shares of the bit-row array.
+// wave_lo[w] = first row whose bit row starts at or after w / waves of
+// it (wave_lo[waves] = n). The in-lists are filled one wave of rows at a
 // time, so each hub's in-list is ordered by wave, and the hub pieces are then
 // ordered by the wave of their first tail: the CTAs working at one time walk
 // the tails of rows of one wave, whose bit rows fit the L2.
@@ -2382,12 +2432,12 @@ __global__ void k_hub_total(const uint32_t* __restrict__ in_off, uint32_t n, uin
 // the last w with wave_bk[w] <= k for any bit-row index k of u's row (a tail
 // start), so a piece's wave follows from its first tail without its row.
 // wave_cp[w]: the same in CSR positions, for column tails.
-__global__ void k_wave_bounds(GraphView g, uint32_t* __restrict__ wave_lo, uint32_t* __restrict__ wave_bk,
-                              uint32_t* __restrict__ wave_cp) {
+__global__ void k_wave_bounds(GraphView g, uint32_t waves, uint32_t* __restrict__ wave_lo,
+                              uint32_t* __restrict__ wave_bk, uint32_t* __restrict__ wave_cp) {
   const uint32_t w = threadIdx.x;
   if (w > kHubWaves) return;
   const uint64_t nb = rp_blk(g.rp[g.n]);
-  const uint64_t target = nb * w / kHubWaves;
+  const uint64_t target = nb * w / waves;
   uint32_t lo = 0, hi = g.n;  // first u with brow_ptr[u] >= target
   while (lo < hi) {
     const uint32_t mid = lo + ((hi - lo) >> 1);
@@ -2396,9 +2446,9 @@ __global__ void k_wave_bounds(GraphView g, uint32_t* __restrict__ wave_lo, uint3
     else
       hi = mid;
   }
-  wave_lo[w] = w == kHubWaves ? g.n : lo;
-  wave_bk[w] = w == kHubWaves ? 0xFFFFFFFFu : rp_blk(g.rp[lo]);
-  wave_cp[w] = w == kHubWaves ? 0xFFFFFFFFu : rp_row(g.rp[lo]);
+  wave_lo[w] = w >= waves ? g.n : lo;
+  wave_bk[w] = w >= waves ? 0xFFFFFFFFu : rp_blk(g.rp[lo]);
+  wave_cp[w] = w >= waves ? 0xFFFFFFFFu : rp_row(g.rp[lo]);
 }
 
 __device__ __forceinline__ uint32_t wave_of_block(const uint32_t* __restrict__ wave_bk, uint32_t k) {
@@ -2457,7 +2507,6 @@ Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, bool hubs) {
   s.piece_off = ar.take<uint32_t>(kScheduleWords);
   s.counts = ar.take<uint64_t>((uint64_t)kPieceLists * nrb + 1);
   s.scan_tmp = take_scan_temp<uint64_t>(ar, (uint64_t)kPieceLists * nrb + 1);
-  s.row_scan_tmp = take_scan_temp<uint32_t>(ar, n + 1);
   s.features = ar.take<float>((uint64_t)nrb * kNumFeatures + 1);
   if (hubs) {
     s.eflag_words = E / 32 + 2;
@@ -2465,7 +2514,7 @@ Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, bool hubs) {
     s.vinfo = ar.take<uint64_t>(n + 1);
     s.save = ar.take<unsigned long long>(n + 1);
     s.in_cnt = ar.take<uint32_t>(n + 1);
-    s.in_off = ar.take<uint32_t>(n + 1);
+    s.in_off = ar.take<uint32_t>(3 * (n + 1));
     s.inl_cap = E + 1;
     s.inl = ar.take<uint64_t>(s.inl_cap);
     s.hub_pieces = ar.take<uint64_t>(2 * n + E / kHubWarpPiece + 64);
@@ -2475,8 +2524,7 @@ Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, bool hubs) {
     s.wave_bk = ar.take<uint32_t>(kHubWaves + 1);
     s.wave_cp = ar.take<uint32_t>(kHubWaves + 1);
     s.wave_cnt = ar.take<uint32_t>(2 * kHubWaves);
-    s.hub_pos = ar.take<uint32_t>(2 * (n + 1));
-    s.hub_scan_tmp = take_scan_temp<uint32_t>(ar, 2 * (n + 1));
+    s.hub_scan_tmp = take_scan_temp<uint32_t>(ar, 3 * (n + 1));
   }
   return s;
 }
@@ -2490,57 +2538,47 @@ static void build_hubs(const GraphView& g, Schedule& s, cudaStream_t st) {
   const uint64_t n = g.n;
   const unsigned vblocks = (unsigned)ceil_div<uint64_t>(n + 1, 256);
   const unsigned eblocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div<uint64_t>(n, 8), 148ull * 16));
-  k_hub_vinfo<<<vblocks, 256, 0, st>>>(g, s.vinfo);
-  TB_LAUNCH_CHECK();
-  TB_CUDA(cudaMemsetAsync(s.save, 0, n * sizeof(unsigned long long), st));
-  TB_CUDA(cudaMemsetAsync(s.eflag, 0, (s.eflag_words) * sizeof(uint32_t), st));
-  TB_CUDA(cudaMemsetAsync(s.in_cnt, 0, (n + 1) * sizeof(uint32_t), st));
-  // Candidates counted and savings summed in one pass; each hub accepted or
-  // not as a whole; its in-list sized by its candidates, then filled.
+  // Candidates counted and savings summed in one pass (k_block_pieces zeroed
+  // the counters); each hub accepted or not as a whole; its in-list sized by
+  // its candidates, then filled.
   k_hub_edges<0><<<eblocks, 256, 0, st>>>(g, s.variant_of, s.vinfo, s.save, s.eflag, s.in_cnt, s.in_off, s.inl,
                                            nullptr, nullptr);
   TB_LAUNCH_CHECK();
-  k_hub_accept<<<vblocks, 256, 0, st>>>(s.vinfo, (uint32_t)n, s.save, s.in_cnt);
+  k_hub_accept<<<vblocks, 256, 0, st>>>(s.vinfo, (uint32_t)n, s.save, s.in_cnt, s.in_off);
   TB_LAUNCH_CHECK();
-  device_scan<uint32_t, OpSum>(s.in_cnt, s.in_off, n + 1, true, OpSum{}, 0u, s.row_scan_tmp, st);
-  TB_CUDA(cudaMemsetAsync(s.in_cnt, 0, (n + 1) * sizeof(uint32_t), st));
-  k_wave_bounds<<<1, kHubWaves + 1, 0, st>>>(g, s.wave_lo, s.wave_bk, s.wave_cp);
-  TB_LAUNCH_CHECK();
-  if (s.inl_cap <= kHubOneWaveEntries) {
-    // A graph whose bit rows fit the L2 many times over gains nothing from
-    // the wave order: one launch fills every in-list.
-    k_hub_edges<1><<<eblocks, 256, 0, st>>>(g, s.variant_of, s.vinfo, s.save, s.eflag, s.in_cnt, s.in_off, s.inl,
-                                             s.hub_rows ? s.inrow : nullptr, nullptr);
+  device_scan<uint32_t, OpSum>(s.in_off, s.in_off, 3 * (n + 1), true, OpSum{}, 0u, s.hub_scan_tmp, st);
+  const uint32_t waves = hub_waves(s.inl_cap - 1);
+  uint64_t* pieces = waves == 1 ? s.hub_pieces : s.hub_pieces2;
+  if (waves > 1) {
+    k_wave_bounds<<<1, kHubWaves + 1, 0, st>>>(g, waves, s.wave_lo, s.wave_bk, s.wave_cp);
     TB_LAUNCH_CHECK();
-  } else {
-    for (uint32_t w = 0; w < kHubWaves; ++w) {  // in-lists filled wave by wave: ordered by wave
-      k_hub_edges<1><<<eblocks, 256, 0, st>>>(g, s.variant_of, s.vinfo, s.save, s.eflag, s.in_cnt, s.in_off, s.inl,
-                                               s.hub_rows ? s.inrow : nullptr, s.wave_lo + w);
-      TB_LAUNCH_CHECK();
-    }
   }
-  k_hub_piece_count<<<vblocks, 256, 0, st>>>(s.in_off, s.vinfo, (uint32_t)n, s.hub_pos);
+  for (uint32_t w = 0; w < waves; ++w) {  // in-lists filled wave by wave: ordered by wave
+    k_hub_edges<1><<<eblocks, 256, 0, st>>>(g, s.variant_of, s.vinfo, s.save, s.eflag, s.in_cnt, s.in_off, s.inl,
+                                             s.hub_rows ? s.inrow : nullptr, waves == 1 ? nullptr : s.wave_lo + w);
+    TB_LAUNCH_CHECK();
+  }
+  k_hub_piece_scatter<<<std::max(vblocks, 1u), 256, 0, st>>>(s.in_off + n + 1, (uint32_t)n, pieces, s.piece_off,
+                                                             waves == 1 ? nullptr : s.wave_cnt);
   TB_LAUNCH_CHECK();
-  device_scan<uint32_t, OpSum>(s.hub_pos, s.hub_pos, 2 * (n + 1), true, OpSum{}, 0u, s.hub_scan_tmp, st);
-  k_hub_piece_scatter<<<vblocks, 256, 0, st>>>(s.hub_pos, (uint32_t)n, s.hub_pieces2, s.piece_off);
-  TB_LAUNCH_CHECK();
-  k_hub_total<<<1, 1, 0, st>>>(s.in_off, (uint32_t)n, s.piece_off);
-  TB_LAUNCH_CHECK();
-  TB_CUDA(cudaMemsetAsync(s.wave_cnt, 0, 2 * kHubWaves * sizeof(uint32_t), st));
-  k_piece_waves<<<148 * 8, 256, 0, st>>>(s.hub_pieces2, s.piece_off, s.in_off, s.in_cnt, s.inl, s.wave_bk,
-                                          s.wave_cp, s.wave_cnt, s.piece_wave);
-  TB_LAUNCH_CHECK();
-  k_wave_scan<<<1, 1, 0, st>>>(s.wave_cnt, s.piece_off);
-  TB_LAUNCH_CHECK();
-  k_piece_wave_scatter<<<148 * 8, 256, 0, st>>>(s.hub_pieces2, s.piece_off, s.piece_wave, s.wave_cnt, s.hub_pieces);
-  TB_LAUNCH_CHECK();
+  if (waves > 1) {
+    k_piece_waves<<<148 * 8, 256, 0, st>>>(s.hub_pieces2, s.piece_off, s.in_off, s.in_cnt, s.inl, s.wave_bk,
+                                            s.wave_cp, s.wave_cnt, s.piece_wave);
+    TB_LAUNCH_CHECK();
+    k_wave_scan<<<1, 1, 0, st>>>(s.wave_cnt, s.piece_off);
+    TB_LAUNCH_CHECK();
+    k_piece_wave_scatter<<<148 * 8, 256, 0, st>>>(s.hub_pieces2, s.piece_off, s.piece_wave, s.wave_cnt, s.hub_pieces);
+    TB_LAUNCH_CHECK();
+  }
   s.hubs_active = true;
 }
 
 void build_pieces(const GraphView& g, Schedule& s, cudaStream_t st) {
   const uint32_t nrb = s.num_row_blocks;
   const unsigned wblocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div<uint64_t>(nrb, 8), 148ull * 16));
-  k_block_pieces<<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.counts, s.piece_width);
+  HubInit hub{};
+  if (s.eflag && s.hubs) hub = HubInit{s.vinfo, s.save, s.in_cnt, s.eflag, s.eflag_words};
+  k_block_pieces<<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.counts, s.piece_width, hub);
   TB_LAUNCH_CHECK();
   device_scan<uint64_t, OpSum>(s.counts, s.counts, (uint64_t)kPieceLists * nrb + 1, true, OpSum{}, 0ull, s.scan_tmp,
                                st);

@@ -49,7 +49,6 @@ struct Schedule {
   uint32_t* piece_off = nullptr;   // device, kScheduleWords words (see there)
   uint64_t* counts = nullptr;      // device, kPieceLists * nrb + 1: pieces per (list, row block), scanned
   uint64_t* scan_tmp = nullptr;
-  uint32_t* row_scan_tmp = nullptr;
   float* features = nullptr;       // device, nrb x kNumFeatures
   // Hub pass of the merge variant (absent when taken without hubs).
   uint32_t* eflag = nullptr;       // device, bit per CSR position: edge counted by the hub pass
@@ -57,7 +56,8 @@ struct Schedule {
   uint64_t* vinfo = nullptr;       // device, n: (row span in blocks << 32) | bit-row length
   unsigned long long* save = nullptr;  // device, n: blocks a hub walk would save
   uint32_t* in_cnt = nullptr;      // device, n + 1
-  uint32_t* in_off = nullptr;      // device, n + 1: in-list of hub v at [in_off[v], in_off[v+1])
+  uint32_t* in_off = nullptr;      // device, n + 1: in-list of hub v at [in_off[v], in_off[v+1]); then, from
+                                   // n + 1 on, 2(n + 1) piece counts scanned with it (CTA, warp pieces)
   uint64_t* inl = nullptr;         // device: (first block of u's tail << 32) | tail length
   uint64_t inl_cap = 0;            // entries inl (and inrow) hold
   uint32_t* inrow = nullptr;       // device: u of each in-list entry (timing mode only: its own buffer)
@@ -68,7 +68,6 @@ struct Schedule {
   uint32_t* wave_bk = nullptr;     // device: bit-row start of each wave's first row
   uint32_t* wave_cp = nullptr;     // device: CSR position of each wave's first row
   uint32_t* wave_cnt = nullptr;    // device: pieces per (list, wave), scanned to positions
-  uint32_t* hub_pos = nullptr;     // device, 2n + 2: piece counts, scanned to piece positions
   uint32_t* hub_scan_tmp = nullptr;
   bool hubs = true;                // build the hub lists for merge row blocks
   bool hubs_active = false;        // set by build_pieces
