@@ -26,48 +26,138 @@ __device__ __forceinline__ uint32_t graph_of_entry(const uint64_t* eoff, uint32_
   return lo;
 }
 
-// Decodes entry i into global vertex ids. Returns false for an entry naming a
-// vertex outside its graph (flagged) and for a self-loop (silently dropped,
-// as read_mtx does at tribit.cu:261-267).
-__device__ __forceinline__ bool load_entry(const PrepInput& in, uint64_t i, uint32_t& a, uint32_t& b,
-                                           unsigned int* err) {
-  uint64_t e = in.entries[i];
-  uint64_t x = e >> 32, y = e & 0xffffffffull;
-  uint64_t base = 0, lim = in.n;
-  if (in.G) {
-    uint32_t g = graph_of_entry(in.eoff, in.G, i);
-    base = in.voff[g];
-    lim = in.voff[g + 1] - base;
+constexpr uint32_t kNoId = 0xFFFFFFFFu;  // no vertex has this id (n < 2^32)
+
+// Decodes a thread's entries, in increasing order, into global vertex ids. In
+// batch mode the entry's graph is searched for once and then followed (a
+// search an entry: 1,732 us of degrees and 902 of row counts in the 512-graph
+// batch, now 802 and 733).
+struct EntryReader {
+  const PrepInput& in;
+  unsigned int* err;
+  uint64_t base = 0, lim, end = 0;  // the graph's first vertex, its vertices, the end of its entries
+  uint32_t g = 0;
+  __device__ __forceinline__ EntryReader(const PrepInput& in_, unsigned int* err_) : in(in_), err(err_), lim(in_.n) {}
+  // False (ids kNoId) for an entry naming a vertex outside its graph (flagged)
+  // and for a self-loop (silently dropped, as read_mtx does at tribit.cu:261-267).
+  __device__ __forceinline__ bool ids(uint64_t e, uint64_t i, uint32_t& a, uint32_t& b) {
+    if (in.G && i >= end) {
+      for (int t = 0; t < 4 && end && in.eoff[g + 1] <= i; ++t) ++g;
+      if (end == 0 || in.eoff[g + 1] <= i) g = graph_of_entry(in.eoff, in.G, i);
+      end = in.eoff[g + 1];
+      base = in.voff[g];
+      lim = in.voff[g + 1] - base;
+    }
+    const uint64_t x = e >> 32, y = e & 0xffffffffull;
+    a = b = kNoId;
+    if (x >= lim || y >= lim) {
+      atomicOr(err, kErrIdRange);
+      return false;
+    }
+    if (x == y) return false;
+    a = (uint32_t)(x + base);
+    b = (uint32_t)(y + base);
+    return true;
   }
-  if (x >= lim || y >= lim) {
-    atomicOr(err, kErrIdRange);
-    return false;
-  }
-  a = (uint32_t)(x + base);
-  b = (uint32_t)(y + base);
-  return a != b;
+};
+
+// Lanes holding the same key in a row, as a sorted edge list gives them: the
+// run's first lane, its length and whether this lane is the first. One atomic
+// a run takes the place of one a lane (a warp's 32 on one address are served
+// one after another: sorted cliques, degrees 906 us, now 203, row counts 1,006,
+// now 127, row fill 1,226, now 97).
+struct KeyRun {
+  uint32_t first, len;
+  bool head;
+};
+__device__ __forceinline__ KeyRun key_run(uint32_t key) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t prev = __shfl_up_sync(kFull, key, 1);
+  const uint32_t heads = __ballot_sync(kFull, lane == 0 || key != prev);
+  KeyRun r;
+  r.first = 31 - __clz(heads & (kFull >> (31 - lane)));
+  const uint32_t after = lane == 31 ? 0u : heads >> (lane + 1);
+  r.len = (after ? lane + (uint32_t)__ffs(after) : 32u) - r.first;
+  r.head = r.first == lane;
+  return r;
 }
 
-// The degree order only has to be a good order (any total order counts every
-// triangle once): degrees may be counted over every kDegreeSample-th entry
-// (a strided sample, which a sorted input does not bias). Every entry is still
-// checked for range when it is oriented (k_row_count).
-#ifndef TB_DEGREE_SAMPLE
-#define TB_DEGREE_SAMPLE 1
-#endif
-constexpr uint64_t kDegreeSample = TB_DEGREE_SAMPLE;
+// Degrees (with duplicates) over entries [i0, i1), a contiguous share a CTA. A
+// power-law graph's hubs put millions of updates on a few lines of counters,
+// each line served one update at a time (Chung-Lu, 7,115 vertices: 38 us, now 12;
+// RMAT-20, whose updates are spread wider, 612, now 587), so each CTA counts the ids that win a
+// slot of a table in shared memory there: its share is sampled, every sampled
+// id claims its slot and the last one stays, which an id does about as often
+// as it occurs. Ids without a slot are counted in global memory.
+constexpr uint32_t kDegSlots = 8192;
+constexpr uint32_t kDegThreads = 512;
+constexpr uint32_t kDegSample = 4096;  // entries, and the fewest a CTA takes
+constexpr int kDegAhead = 4;           // entries in flight a thread
+__device__ __forceinline__ uint32_t deg_slot(uint32_t id) { return (id ^ (id / kDegSlots)) & (kDegSlots - 1); }
 
-// Degrees (with duplicates) over the sampled entries of [i0, i1).
-__global__ void k_degree(PrepInput in, uint64_t i0, uint64_t i1, uint32_t* __restrict__ deg, unsigned int* err) {
-  const uint64_t first = (i0 + kDegreeSample - 1) / kDegreeSample, last = (i1 + kDegreeSample - 1) / kDegreeSample;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t s = first + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < last; s += stride) {
-    uint32_t a, b;
-    if (load_entry(in, s * kDegreeSample, a, b, err)) {
-      atomicAdd(&deg[a], 1u);
-      atomicAdd(&deg[b], 1u);
+__global__ void __launch_bounds__(kDegThreads) k_degree(PrepInput in, uint64_t i0, uint64_t i1,
+                                                        uint32_t* __restrict__ deg, unsigned int* err) {
+  extern __shared__ uint32_t deg_sm[];
+  uint32_t* tag = deg_sm;
+  uint32_t* cnt = deg_sm + kDegSlots;
+  const uint64_t share = ceil_div<uint64_t>(i1 - i0, gridDim.x);
+  const uint64_t c0 = min(i1, i0 + share * blockIdx.x), c1 = min(i1, c0 + share);
+  for (uint32_t s = threadIdx.x; s < kDegSlots; s += kDegThreads) {
+    tag[s] = kNoId;
+    cnt[s] = 0;
+  }
+  __syncthreads();
+  {
+    EntryReader rd(in, err);
+    const uint64_t step = max((c1 - c0) / kDegSample, (uint64_t)1);
+    for (uint64_t j = threadIdx.x, i = c0 + j * step; j < kDegSample && i < c1; j += kDegThreads, i = c0 + j * step) {
+      uint32_t a, b;
+      if (rd.ids(in.entries[i], i, a, b)) {
+        tag[deg_slot(a)] = a;
+        tag[deg_slot(b)] = b;
+      }
     }
   }
+  __syncthreads();
+  EntryReader rd(in, err);
+  auto count = [&](uint32_t id) {
+    const KeyRun r = key_run(id);
+    if (!r.head || id == kNoId) return;
+    const uint32_t s = deg_slot(id);
+    if (tag[s] == id)
+      atomicAdd(&cnt[s], r.len);
+    else
+      atomicAdd(&deg[id], r.len);
+  };
+  for (uint64_t c = c0; c < c1; c += kDegThreads * kDegAhead) {
+    uint64_t e[kDegAhead];
+#pragma unroll
+    for (int k = 0; k < kDegAhead; ++k) {
+      const uint64_t i = c + k * kDegThreads + threadIdx.x;
+      e[k] = i < c1 ? in.entries[i] : 0ull;  // 0: a self-loop
+    }
+#pragma unroll
+    for (int k = 0; k < kDegAhead; ++k) {
+      const uint64_t i = c + k * kDegThreads + threadIdx.x;
+      uint32_t a = kNoId, b = kNoId;
+      if (i < c1) rd.ids(e[k], i, a, b);
+      __syncwarp();
+      count(a);
+      count(b);
+    }
+  }
+  __syncthreads();
+  for (uint32_t s = threadIdx.x; s < kDegSlots; s += kDegThreads)
+    if (cnt[s]) atomicAdd(&deg[tag[s]], cnt[s]);
+}
+
+void degree_pass(const PrepInput& in, uint64_t i0, uint64_t i1, uint32_t* deg, unsigned int* err, cudaStream_t st) {
+  if (i0 >= i1) return;
+  constexpr int kSmem = 2 * kDegSlots * sizeof(uint32_t);
+  once_per_device<2>([] { TB_CUDA(cudaFuncSetAttribute(k_degree, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem)); });
+  const uint64_t ctas = std::min<uint64_t>(148 * 3, ceil_div<uint64_t>(i1 - i0, kDegSample));
+  k_degree<<<(unsigned)ctas, kDegThreads, kSmem, st>>>(in, i0, i1, deg, err);
+  TB_LAUNCH_CHECK();
 }
 
 __device__ __forceinline__ uint32_t graph_of_vertex(const uint64_t* voff, uint32_t G, uint64_t v) {
@@ -118,42 +208,70 @@ __global__ void k_identity_graph_of(uint64_t n, const uint64_t* voff, uint32_t G
 // pairs gives the CSR and bit-row offsets. The 48-bit global radix sort of
 // (lo, hi) keys that this replaces took six passes over all entries.
 
-// Oriented (lo, hi) of entry i in rank space; false for dropped entries.
-__device__ __forceinline__ bool orient_entry(const PrepInput& in, const uint32_t* __restrict__ rank, uint64_t i,
-                                             uint32_t& lo, uint32_t& hi, unsigned int* err) {
-  uint32_t a, b;
-  if (!load_entry(in, i, a, b, err)) return false;
+// Oriented key (lo << 32) | hi, in rank space, of an entry's ids.
+constexpr uint64_t kDropped = ~0ull;
+__device__ __forceinline__ uint64_t orient(const uint32_t* __restrict__ rank, uint32_t a, uint32_t b) {
   const uint32_t ra = rank ? rank[a] : a, rb = rank ? rank[b] : b;
-  lo = ra < rb ? ra : rb;
-  hi = ra < rb ? rb : ra;
-  return true;
+  return ((uint64_t)min(ra, rb) << 32) | max(ra, rb);
 }
 
 // keys[i] = (lo << 32) | hi of entry i (kDropped for a dropped entry), and
-// cnt[lo] += 1.
-constexpr uint64_t kDropped = ~0ull;
-__global__ void k_row_count(PrepInput in, const uint32_t* __restrict__ rank, uint32_t* __restrict__ cnt,
-                            uint64_t* __restrict__ keys, unsigned int* err) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < in.E; i += stride) {
-    uint32_t lo, hi;
-    uint64_t key = kDropped;
-    if (orient_entry(in, rank, i, lo, hi, err)) {
-      atomicAdd(&cnt[lo], 1u);
-      key = ((uint64_t)lo << 32) | hi;
+// cnt[lo] += 1. A CTA takes tiles of kTile entries, four a thread in flight.
+constexpr int kAhead = 4;
+constexpr uint32_t kTile = kThreads * kAhead;
+__global__ void __launch_bounds__(kThreads) k_row_count(PrepInput in, const uint32_t* __restrict__ rank,
+                                                        uint32_t* __restrict__ cnt, uint64_t* __restrict__ keys,
+                                                        uint32_t tiles, unsigned int* err) {
+  EntryReader rd(in, err);
+  uint64_t c = (uint64_t)blockIdx.x * tiles * kTile;
+  for (uint32_t t = 0; t < tiles && c < in.E; ++t, c += kTile) {
+    uint64_t e[kAhead], key[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint64_t i = c + k * kThreads + threadIdx.x;
+      e[k] = i < in.E ? in.entries[i] : 0ull;
     }
-    keys[i] = key;
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint64_t i = c + k * kThreads + threadIdx.x;
+      uint32_t a, b;
+      key[k] = i < in.E && rd.ids(e[k], i, a, b) ? orient(rank, a, b) : kDropped;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint64_t i = c + k * kThreads + threadIdx.x;
+      const uint32_t lo = (uint32_t)(key[k] >> 32);  // kNoId: dropped
+      const KeyRun r = key_run(lo);
+      if (r.head && lo != kNoId) atomicAdd(&cnt[lo], r.len);
+      if (i < in.E) keys[i] = key[k];
+    }
   }
 }
 
 // nbr[cur[lo]++] = hi (cur starts as the row offsets): the only random
-// accesses are the cursors, which stay in L2.
-__global__ void k_row_fill(const uint64_t* __restrict__ keys, uint64_t E, uint32_t* __restrict__ cur,
-                           uint32_t* __restrict__ nbr) {
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += stride) {
-    const uint64_t key = keys[i];
-    if (key != kDropped) nbr[atomicAdd(&cur[key >> 32], 1u)] = (uint32_t)key;
+// accesses are the cursors, which stay in L2, one update a run of equal lo.
+__global__ void __launch_bounds__(kThreads) k_row_fill(const uint64_t* __restrict__ keys, uint64_t E,
+                                                       uint32_t* __restrict__ cur, uint32_t* __restrict__ nbr) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint64_t c = (uint64_t)blockIdx.x * kTile; c < E; c += (uint64_t)gridDim.x * kTile) {
+    uint64_t key[kAhead];
+    uint32_t at[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint64_t i = c + k * kThreads + threadIdx.x;
+      key[k] = i < E ? keys[i] : kDropped;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint32_t lo = (uint32_t)(key[k] >> 32);
+      const KeyRun r = key_run(lo);
+      uint32_t base = 0;
+      if (r.head && lo != kNoId) base = atomicAdd(&cur[lo], r.len);
+      at[k] = __shfl_sync(kFull, base, r.first) + lane - r.first;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (key[k] != kDropped) nbr[at[k]] = (uint32_t)key[k];
   }
 }
 
@@ -180,14 +298,14 @@ __global__ void __launch_bounds__(kSortThreads) k_row_keys_hist(PrepInput in, co
   h[threadIdx.x] = 0;
   __syncthreads();
   const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
+  EntryReader rd(in, err);
 #pragma unroll 4
   for (int j = 0; j < kSortKeysPerThread; ++j) {
     const uint64_t i = base + (uint64_t)j * kSortThreads + threadIdx.x;
     uint32_t d = 256u;
     if (i < in.E) {
-      uint32_t lo, hi;
-      uint64_t key = kDropped;
-      if (orient_entry(in, rank, i, lo, hi, err)) key = ((uint64_t)lo << 32) | hi;
+      uint32_t a, b;
+      const uint64_t key = rd.ids(in.entries[i], i, a, b) ? orient(rank, a, b) : kDropped;
       keys[i] = key;
       d = (uint32_t)((key >> shift) & 255);
     }
@@ -777,8 +895,7 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
   // row counts 2.9 ms and the histogram 1.0 ms, for 1 GB more of nbr).
   // (Decided from the order, not from deg: the arena's measuring pass hands
   // out null buffers and must plan the same layout.)
-  const bool slots =
-      presort && in.order == TRIBIT_ORDER_DEGREE && kDegreeSample == 1 && 2 * E < 0xFFFFFFFFull;
+  const bool slots = presort && in.order == TRIBIT_ORDER_DEGREE && 2 * E < 0xFFFFFFFFull;
   const uint64_t cap = slots ? 2 * E : E;  // nbr entries
   uint32_t* cnt = ar.take<uint32_t>(n + 1);  // row lengths or slot sizes, then the fill cursors: the row ends
   uint32_t* off = ar.take<uint32_t>(n + 1);  // row starts
@@ -817,7 +934,9 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
   } else {
     TB_CUDA(cudaMemsetAsync(cnt, 0, (n + 1) * sizeof(uint32_t), st));
     if (E > 0) {
-      k_row_count<<<grid_for(E, 8), kThreads, 0, st>>>(in, rank, cnt, keys, &stats->err);
+      const uint64_t per = std::max<uint64_t>(1, E / (148ull * 64 * kTile));  // tiles a CTA
+      k_row_count<<<(unsigned)ceil_div<uint64_t>(E, per * kTile), kThreads, 0, st>>>(in, rank, cnt, keys, (uint32_t)per,
+                                                                                     &stats->err);
       TB_LAUNCH_CHECK();
     }
     device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st);
@@ -831,7 +950,8 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
       fill_keys = radix_sort<uint64_t, NoVal, false>(keys, keys_alt, nullptr, nullptr, E, top + 8, ktmp, st, nullptr,
                                                      top, slots);
     TB_CUDA(cudaMemcpyAsync(cnt, off, (n + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-    k_row_fill<<<grid_for(E, 8), kThreads, 0, st>>>(fill_keys, E, cnt, nbr);
+    k_row_fill<<<(unsigned)std::min<uint64_t>(ceil_div<uint64_t>(E, kTile), 148ull * 64), kThreads, 0, st>>>(
+        fill_keys, E, cnt, nbr);
     TB_LAUNCH_CHECK();
   }
   // Row u: nbr[off[u], cnt[u]) (with no entries every row is empty: 0, 0).
@@ -985,12 +1105,10 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
           TB_CUDA(cudaEventRecord(up.events[k + 1], up.copy_stream));
           TB_CUDA(cudaStreamWaitEvent(st, up.events[k + 1], 0));
           if (i1 == E && up.uploaded) TB_CUDA(cudaEventRecord(up.uploaded, st));
-          k_degree<<<grid_for(i1 - i0, 8), kThreads, 0, st>>>(in, i0, i1, deg, &stats->err);
-          TB_LAUNCH_CHECK();
+          degree_pass(in, i0, i1, deg, &stats->err, st);
         }
-      } else if (E > 0) {
-        k_degree<<<grid_for(E, 8), kThreads, 0, st>>>(in, 0, E, deg, &stats->err);
-        TB_LAUNCH_CHECK();
+      } else {
+        degree_pass(in, 0, E, deg, &stats->err, st);
       }
       int gbits = in.G ? bits_for((uint64_t)in.G) : 0;
       int dbits = bits_for(2 * E + 2);
