@@ -104,7 +104,7 @@ void run_call(tribit_context* c, tb::PrepInput in, const uint64_t* host_entries,
     c->launch = tb::launch_count(c->prep.view, c->sched, c->prep.stats, L.per_graph, cfg, st);
   }
   TB_CUDA(cudaEventRecord(c->ev[3], st));
-  TB_CUDA(cudaMemcpyAsync(c->h_stats, c->prep.stats, sizeof(tb::DeviceStats), cudaMemcpyDeviceToHost, st));
+  tb::read_stats(c, st);
   TB_CUDA(cudaEventRecord(c->ev[4], st));
   TB_CUDA(cudaEventSynchronize(c->ev[4]));
   TB_CUDA(cudaGetLastError());
@@ -150,12 +150,14 @@ void count_device_input(tribit_context* c, const uint64_t* d_entries, uint64_t E
   run_call(c, in, nullptr, nullptr, nullptr, 0, true, res);
 }
 
-void fill_schedule_stats(tribit_context* c, tribit_result* res) {
-  uint32_t words[tb::kScheduleWords];
-  TB_CUDA(cudaMemcpyAsync(words, c->sched.piece_off, sizeof words, cudaMemcpyDeviceToHost, c->st));
-  TB_CUDA(cudaStreamSynchronize(c->st));
-  const uint32_t* lens = words + tb::kOffRowBlocks;
-  res->hub_edges = words[tb::kOffHubEdges];
+void read_stats(tribit_context* c, cudaStream_t st) {
+  TB_CUDA(cudaMemcpyAsync(c->h_stats, c->prep.stats, sizeof(DeviceStats), cudaMemcpyDeviceToHost, st));
+  TB_CUDA(cudaMemcpyAsync(c->h_sched, c->sched.piece_off, kScheduleWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+}
+
+void fill_schedule_stats(const tribit_context* c, tribit_result* res) {
+  const uint32_t* lens = c->h_sched + kOffRowBlocks;
+  res->hub_edges = c->h_sched[kOffHubEdges];
   res->row_blocks = 0;
   for (int v = 0; v < TRIBIT_NUM_VARIANTS; ++v) {
     res->row_blocks_by_variant[v] = lens[v];
@@ -164,8 +166,6 @@ void fill_schedule_stats(tribit_context* c, tribit_result* res) {
 }
 
 }  // namespace tb
-
-using tb::fill_schedule_stats;
 
 extern "C" {
 
@@ -227,7 +227,8 @@ tribit_status tribit_create(const tribit_options* opts, tribit_context** out) {
     TB_CUDA(cudaStreamCreateWithFlags(&c->copy_st, cudaStreamNonBlocking));
     for (auto& e : c->upload_ev) TB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto& e : c->pinned_ev) TB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    TB_CUDA(cudaMallocHost(&c->h_stats, sizeof(tb::DeviceStats)));
+    TB_CUDA(cudaMallocHost(&c->h_stats, sizeof(tb::DeviceStats) + tb::kScheduleWords * sizeof(uint32_t)));
+    c->h_sched = reinterpret_cast<uint32_t*>(c->h_stats + 1);
   });
   if (st != TRIBIT_OK) {
     tribit_destroy(c);
@@ -290,7 +291,7 @@ tribit_status tribit_count_edges(tribit_context* c, const uint64_t* entries, uin
     static const uint64_t dummy = 0;
     run_call(c, in, entries ? entries : &dummy, nullptr, nullptr, 0, true, out);
     if (out) {
-      fill_schedule_stats(c, out);
+      tb::fill_schedule_stats(c, out);
       out->stream_ranges = 1;
       out->stream_tasks = 1;
       out->stream_tier = 0;
@@ -313,7 +314,7 @@ tribit_status tribit_count_edges_device(tribit_context* c, const uint64_t* d_ent
     in.n = num_nodes;
     in.order = c->opts.order;
     run_call(c, in, nullptr, nullptr, nullptr, 0, true, out);
-    if (out) fill_schedule_stats(c, out);
+    if (out) tb::fill_schedule_stats(c, out);
   });
 }
 
@@ -327,7 +328,7 @@ tribit_status tribit_prepare_device(tribit_context* c, const uint64_t* d_entries
     in.n = num_nodes;
     in.order = c->opts.order;
     run_call(c, in, nullptr, nullptr, nullptr, 0, false, out);
-    if (out) fill_schedule_stats(c, out);
+    if (out) tb::fill_schedule_stats(c, out);
   });
 }
 
@@ -496,7 +497,7 @@ tribit_status tribit_read_count(tribit_context* c, tribit_result* out) {
   if (!c || !c->prepared) return TRIBIT_ERR_INVALID_ARGUMENT;
   return guarded(c, [&] {
     DeviceGuard dg(c->device);
-    TB_CUDA(cudaMemcpyAsync(c->h_stats, c->prep.stats, sizeof(tb::DeviceStats), cudaMemcpyDeviceToHost, c->st));
+    tb::read_stats(c, c->st);
     TB_CUDA(cudaStreamSynchronize(c->st));
     TB_CUDA(cudaGetLastError());
     if (c->h_stats->count_err & tb::kErrTimeout) throw StatusError(TRIBIT_ERR_TIMEOUT, "a device-side wait gave up");
@@ -508,7 +509,7 @@ tribit_status tribit_read_count(tribit_context* c, tribit_result* out) {
       out->edges = c->h_stats->edges;
       out->blocks_of_threads = c->launch.ctas;
       out->count_kernels = c->launch.kernels;
-      fill_schedule_stats(c, out);
+      tb::fill_schedule_stats(c, out);
     }
   });
 }
@@ -534,7 +535,7 @@ tribit_status tribit_count_batch(tribit_context* c, const uint64_t* entries, con
     DeviceGuard dg(c->device);
     TB_CUDA(cudaMemcpyAsync(triangles_out, c->per_graph, num_graphs * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->st));
     TB_CUDA(cudaStreamSynchronize(c->st));
-    if (out) fill_schedule_stats(c, out);
+    if (out) tb::fill_schedule_stats(c, out);
   });
 }
 

@@ -172,26 +172,127 @@ __device__ __forceinline__ uint32_t graph_of_vertex(const uint64_t* voff, uint32
   return lo;
 }
 
-// Sort key of vertex v: (graph << dbits) | min(degree, 2^dbits - 1). A stable
-// sort of these keys over ids 0..n-1 gives the (graph, degree, id) order.
+// Vertices are ranked by (graph, degree, id) through a degree key of `bits`
+// bits, two radix passes at 16: degrees below 2^(bits - 1) are exact, larger
+// ones keep their leading bit and the next `mant` ones, so the order is the
+// degrees' but for ties of near-equal hubs (any total order counts each
+// triangle once; this one only bounds the rows' lengths). mant < 0, when many
+// graphs leave few bits: degrees past the range are equal.
+struct DegreeKey {
+  int bits, mant;
+};
+inline DegreeKey degree_key_of(int bits) {
+  if (bits >= 32) return {32, -1};  // exact
+  if (bits < 1) return {0, -1};     // as many graphs as keys: degrees are not told apart
+  int m = bits - 1;                 // (33 - bits) leading bits times 2^m must fit above 2^(bits - 1)
+  while (m >= 0 && ((33ll - bits) << m) > (1ll << (bits - 1))) --m;
+  return {bits, m};
+}
+__device__ __forceinline__ uint32_t degree_key(uint32_t d, DegreeKey k) {
+  if (k.bits >= 32) return d;
+  if (k.bits == 0) return 0;
+  const uint32_t half = 1u << (k.bits - 1);
+  if (d < half) return d;
+  if (k.mant < 0) return min(d, 2 * half - 1);
+  const int e = 31 - __clz(d);  // >= bits - 1 > mant
+  return half + ((uint32_t)(e - (k.bits - 1)) << k.mant) + ((d >> (e - k.mant)) & ((1u << k.mant) - 1u));
+}
+constexpr int kDegreeBits = 16;
+
+// keys[v] = (graph << bits) | degree key. A stable sort of these keys over ids
+// 0..n-1 gives the (graph, degree, id) order.
 __global__ void k_vertex_keys(const uint32_t* __restrict__ deg, uint64_t n, const uint64_t* voff, uint32_t G,
-                              int dbits, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+                              DegreeKey dk, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
   uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n) return;
-  uint32_t cap = dbits >= 32 ? 0xffffffffu : ((1u << dbits) - 1u);
-  uint32_t d = deg[v] < cap ? deg[v] : cap;
-  uint32_t g = G ? graph_of_vertex(voff, G, v) : 0u;
-  keys[v] = dbits >= 32 ? d : ((g << dbits) | d);
+  const uint32_t g = G ? graph_of_vertex(voff, G, v) : 0u;
+  const uint32_t d = degree_key(deg[v], dk);
+  keys[v] = dk.bits >= 32 ? d : ((g << dk.bits) | d);
   vals[v] = (uint32_t)v;
 }
 
+// rank[id] = position, and words of `zero` at 0 (the row counters of the next pass).
 __global__ void k_rank_scatter(const uint32_t* __restrict__ sorted_ids, uint64_t n, uint32_t* __restrict__ rank,
-                               const uint64_t* voff, uint32_t G, uint32_t* __restrict__ graph_of_rank) {
-  uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                               const uint64_t* voff, uint32_t G, uint32_t* __restrict__ graph_of_rank,
+                               uint32_t* __restrict__ zero, uint64_t zero_words) {
+  const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (uint64_t i = r; i < zero_words; i += (uint64_t)gridDim.x * blockDim.x) zero[i] = 0;
   if (r >= n) return;
   uint32_t v = sorted_ids[r];
   rank[v] = (uint32_t)r;
   if (graph_of_rank) graph_of_rank[r] = graph_of_vertex(voff, G, v);
+}
+
+// The same ranks for one graph of at most kRankOneMax vertices, by one CTA:
+// (key << 16) | id words in shared memory, two stable 8-bit passes (a warp a
+// contiguous share, digits ranked by match): one launch in the place of eight.
+constexpr uint32_t kRankOneMax = 16384;
+constexpr uint32_t kRankThreads = 1024;
+constexpr int kRankRounds = kRankOneMax / kRankThreads;
+constexpr size_t kRankSmem = (2 * kRankOneMax + (kRankThreads / 32) * 256) * sizeof(uint32_t);
+__global__ void __launch_bounds__(kRankThreads) k_rank_one(const uint32_t* __restrict__ deg, uint32_t n, DegreeKey dk,
+                                                           uint32_t* __restrict__ rank, uint32_t* __restrict__ zero,
+                                                           uint64_t zero_words) {
+  extern __shared__ uint32_t rank_sm[];
+  __shared__ uint32_t s_sum[8];
+  uint32_t* src = rank_sm;
+  uint32_t* dst = rank_sm + kRankOneMax;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  uint32_t* wcnt = rank_sm + 2 * kRankOneMax;  // [warp][digit]
+  for (uint64_t i = tid; i < zero_words; i += kRankThreads) zero[i] = 0;
+  for (uint32_t i = tid; i < n; i += kRankThreads) src[i] = (degree_key(deg[i], dk) << 16) | i;
+  const uint32_t rounds = (n + kRankThreads - 1) / kRankThreads;  // of 32 a warp
+  for (int shift = 16; shift < 32; shift += 8) {
+    for (uint32_t i = tid; i < (kRankThreads / 32) * 256; i += kRankThreads) wcnt[i] = 0;
+    __syncthreads();
+    uint32_t v[kRankRounds], pos[kRankRounds];
+#pragma unroll
+    for (int r = 0; r < kRankRounds; ++r) {
+      if (r >= (int)rounds) break;
+      const uint32_t i = (w * rounds + r) * 32 + lane;
+      v[r] = i < n ? src[i] : 0u;
+      const uint32_t d = i < n ? (v[r] >> shift) & 255u : 256u;
+      const uint32_t peers = __match_any_sync(kFull, d);
+      const int leader = __ffs(peers) - 1;
+      uint32_t b = 0;
+      if (d < 256 && (int)lane == leader) {
+        b = wcnt[w * 256 + d];
+        wcnt[w * 256 + d] = b + __popc(peers);
+      }
+      pos[r] = __shfl_sync(kFull, b, leader) + __popc(peers & ((1u << lane) - 1u));
+      __syncwarp();
+    }
+    __syncthreads();
+    // Digit d's keys of warp w go after all smaller digits and the digit's of
+    // the warps before.
+    uint32_t tot = 0;
+    if (tid < 256)
+      for (uint32_t q = 0; q < kRankThreads / 32; ++q) {
+        const uint32_t c = wcnt[q * 256 + tid];
+        wcnt[q * 256 + tid] = tot;
+        tot += c;
+      }
+    const uint32_t incl = warp_inclusive_sum(tot);
+    if (tid < 256 && lane == 31) s_sum[w] = incl;
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t before = incl - tot;
+      for (uint32_t q = 0; q < w; ++q) before += s_sum[q];
+      for (uint32_t q = 0; q < kRankThreads / 32; ++q) wcnt[q * 256 + tid] += before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRankRounds; ++r) {
+      if (r >= (int)rounds) break;
+      const uint32_t i = (w * rounds + r) * 32 + lane;
+      if (i < n) dst[wcnt[w * 256 + ((v[r] >> shift) & 255u)] + pos[r]] = v[r];
+    }
+    __syncthreads();
+    uint32_t* t = src;
+    src = dst;
+    dst = t;
+  }
+  for (uint32_t i = tid; i < n; i += kRankThreads) rank[src[i] & 0xFFFFu] = i;
 }
 
 __global__ void k_identity_graph_of(uint64_t n, const uint64_t* voff, uint32_t G, uint32_t* __restrict__ graph_of_rank) {
@@ -714,7 +815,7 @@ __device__ __forceinline__ void emit_span(uint32_t ps, uint32_t pe, uint32_t b, 
 
 // The rows' distinct sorted values (the front of each row's nbr slice, from
 // off[u]) to col, and their bit-row entries (block << 32 | mask) to bent, each
-// written once. Listed CTA rows of more than kWarpSortMax values are emitted
+// written once; their totals to stats (may be null). Listed CTA rows of more than kWarpSortMax values are emitted
 // by a CTA, each warp an eighth of the row from the first block that starts in
 // it. All others are shared out by rows and CSR positions together (`chunk` of
 // them a warp): a warp takes the rows that start in its share, 32 at a time, and
@@ -725,10 +826,14 @@ __device__ __forceinline__ void emit_span(uint32_t ps, uint32_t pe, uint32_t b, 
 __global__ void __launch_bounds__(256) k_emit_rows(const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr,
                                                    const uint64_t* __restrict__ rp, uint32_t n, uint32_t chunk,
                                                    LongRows lng, uint32_t* __restrict__ col,
-                                                   uint64_t* __restrict__ bent) {
+                                                   uint64_t* __restrict__ bent, DeviceStats* stats) {
   __shared__ uint32_t s_delta[8][32];
   __shared__ uint32_t s_head[9], s_cnt[8];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (stats && blockIdx.x == 0 && threadIdx.x == 0) {
+    stats->edges = rp_row(rp[n]);
+    stats->blocks = rp_blk(rp[n]);
+  }
   for (uint32_t bi = blockIdx.x, ncta = lng.count[0]; bi < ncta; bi += gridDim.x) {
     const uint32_t u = lng.rows[ncta - 1 - bi];
     const uint64_t r0 = rp[u], r1 = rp[u + 1];
@@ -820,10 +925,10 @@ unsigned sort_grid(uint64_t n) {
 }
 
 // Row u = nbr[start[u], end[u]) sorted and deduplicated in place for u < n,
-// rows[u] = (distinct << 32) | blocks; E bounds the entries of all rows.
+// rows[u] = (distinct << 32) | blocks; E bounds the entries of all rows. The
+// list lengths in lng start at 0.
 void sort_rows(const uint32_t* start, const uint32_t* end, uint32_t n, uint64_t E, uint32_t* nbr, uint32_t* scratch,
                uint64_t* rows, const LongRows& lng, cudaStream_t st) {
-  TB_CUDA(cudaMemsetAsync(lng.count, 0, 2 * sizeof(uint32_t), st));
   k_sort_rows<<<sort_grid(n), kThreads, 0, st>>>(start, end, n, sort_rows_per_warp(n), nbr, rows, lng);
   TB_LAUNCH_CHECK();
   if (E > kShortRow) {
@@ -885,8 +990,10 @@ __global__ void k_range_carry(uint64_t* __restrict__ rp, uint32_t count, const u
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) rp[k] += c;
 }
 
-void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32_t* deg, cudaStream_t st,
-              Prepared* out, DeviceStats* stats, uint64_t* rp) {
+// cnt (n + 1 words: row lengths or slot sizes, then the fill cursors, which end
+// at the rows' ends) and the two list lengths nbig are 0.
+void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32_t* deg, uint32_t* cnt, uint32_t* nbig,
+              cudaStream_t st, Prepared* out, DeviceStats* stats, uint64_t* rp) {
   const uint64_t E = in.E, n = in.n;
   const bool presort = E >= kPresortMinEntries && n > 256;
   // Slot path: with full degrees, rows take degree-sized slots (2E entries
@@ -897,12 +1004,10 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
   // out null buffers and must plan the same layout.)
   const bool slots = presort && in.order == TRIBIT_ORDER_DEGREE && 2 * E < 0xFFFFFFFFull;
   const uint64_t cap = slots ? 2 * E : E;  // nbr entries
-  uint32_t* cnt = ar.take<uint32_t>(n + 1);  // row lengths or slot sizes, then the fill cursors: the row ends
   uint32_t* off = ar.take<uint32_t>(n + 1);  // row starts
   uint32_t* otmp = take_scan_temp<uint32_t>(ar, n + 1);
   uint64_t* rtmp = take_scan_temp<uint64_t>(ar, n + 1);
   uint32_t* big = ar.take<uint32_t>(n + 1);
-  uint32_t* nbig = ar.take<uint32_t>(2);
   uint32_t* nbr = ar.take<uint32_t>(cap ? cap : 1);
   // The oriented keys (on the slot path both presort buffers), then long
   // rows' sort space (twice nbr).
@@ -926,20 +1031,19 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
   if (slots) {
     k_slot_sizes<<<grid_for(n + 1), kThreads, 0, st>>>(deg, rank, n, cnt);
     TB_LAUNCH_CHECK();
-    device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st);
+    device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st, cnt);
     const uint64_t tiles = ceil_div<uint64_t>(E, kSortTile);
     k_row_keys_hist<<<(unsigned)tiles, kSortThreads, 0, st>>>(in, rank, keys, top, (uint32_t)tiles, ktmp.hist,
                                                                &stats->err);
     TB_LAUNCH_CHECK();
   } else {
-    TB_CUDA(cudaMemsetAsync(cnt, 0, (n + 1) * sizeof(uint32_t), st));
     if (E > 0) {
       const uint64_t per = std::max<uint64_t>(1, E / (148ull * 64 * kTile));  // tiles a CTA
       k_row_count<<<(unsigned)ceil_div<uint64_t>(E, per * kTile), kThreads, 0, st>>>(in, rank, cnt, keys, (uint32_t)per,
                                                                                      &stats->err);
       TB_LAUNCH_CHECK();
     }
-    device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st);
+    device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st, cnt);
   }
   if (E > 0) {
     // One radix pass on the top 8 bits of lo groups the keys into 256 ranges
@@ -949,7 +1053,6 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
     if (presort)
       fill_keys = radix_sort<uint64_t, NoVal, false>(keys, keys_alt, nullptr, nullptr, E, top + 8, ktmp, st, nullptr,
                                                      top, slots);
-    TB_CUDA(cudaMemcpyAsync(cnt, off, (n + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
     k_row_fill<<<(unsigned)std::min<uint64_t>(ceil_div<uint64_t>(E, kTile), 148ull * 64), kThreads, 0, st>>>(
         fill_keys, E, cnt, nbr);
     TB_LAUNCH_CHECK();
@@ -957,9 +1060,7 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
   // Row u: nbr[off[u], cnt[u]) (with no entries every row is empty: 0, 0).
   sort_rows(off, cnt, (uint32_t)n, E, nbr, scratch, rp, lng, st);
   device_scan<uint64_t, OpSum>(rp, rp, n + 1, true, OpSum{}, 0ull, rtmp, st);
-  k_emit_rows<<<emit_grid(E + n), kThreads, 0, st>>>(off, nbr, rp, (uint32_t)n, emit_chunk(E + n), lng, col, bent);
-  TB_LAUNCH_CHECK();
-  k_finalize<<<1, 1, 0, st>>>(rp, n, stats);
+  k_emit_rows<<<emit_grid(E + n), kThreads, 0, st>>>(off, nbr, rp, (uint32_t)n, emit_chunk(E + n), lng, col, bent, stats);
   TB_LAUNCH_CHECK();
 }
 
@@ -998,11 +1099,12 @@ void finish_row_range(const RowRangeBuffers& b, uint32_t s, uint32_t z, uint64_t
   k_range_check<<<grid_for(z), kThreads, 0, st>>>(b.off, b.cursor, z, err);
   TB_LAUNCH_CHECK();
   const LongRows lng{b.big, b.nbig};
+  TB_CUDA(cudaMemsetAsync(b.nbig, 0, 2 * sizeof(uint32_t), st));
   sort_rows(b.off, b.off + 1, z, cnt, b.nbr, b.scratch, rp + s, lng, st);
   device_scan<uint64_t, OpSum>(rp + s, rp + s, (uint64_t)z + 1, true, OpSum{}, 0ull, b.scan_tmp, st);
   k_range_carry<<<grid_for((uint64_t)z + 1), kThreads, 0, st>>>(rp + s, z + 1, b.carry);
   TB_LAUNCH_CHECK();
-  k_emit_rows<<<emit_grid(cnt + z), kThreads, 0, st>>>(b.off, b.nbr, rp + s, z, emit_chunk(cnt + z), lng, col, bent);
+  k_emit_rows<<<emit_grid(cnt + z), kThreads, 0, st>>>(b.off, b.nbr, rp + s, z, emit_chunk(cnt + z), lng, col, bent, nullptr);
   TB_LAUNCH_CHECK();
 }
 
@@ -1032,37 +1134,54 @@ RankBuffers take_rank_buffers(Arena& ar, uint64_t n) {
   return b;
 }
 
-void rank_vertices(const uint32_t* deg, uint64_t n, uint64_t E, const RankBuffers& b, uint32_t* rank, cudaStream_t st) {
-  if (n == 0) return;
-  int dbits = bits_for(2 * E + 2);
-  if (dbits > 32) dbits = 32;
-  k_vertex_keys<<<grid_for(n), kThreads, 0, st>>>(deg, n, nullptr, 0, 32, b.vk, b.vv);
+namespace {
+
+// Ranks of n vertices from their degrees (graphs: the batch's, else G = 0), and
+// `zero_words` of `zero` at 0. The buffers as take_rank_buffers takes them.
+void rank_by_degree(const uint32_t* deg, uint64_t n, const uint64_t* voff, uint32_t G, const RankBuffers& b,
+                    uint32_t* rank, uint32_t* graph_of_rank, uint32_t* zero, uint64_t zero_words, cudaStream_t st) {
+  if (!G && n <= kRankOneMax) {
+    once_per_device<3>(
+        [] { TB_CUDA(cudaFuncSetAttribute(k_rank_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRankSmem)); });
+    k_rank_one<<<1, kRankThreads, kRankSmem, st>>>(deg, (uint32_t)n, degree_key_of(kDegreeBits), rank, zero, zero_words);
+    TB_LAUNCH_CHECK();
+    return;
+  }
+  // Whole radix passes over graph bits and at least 12 degree bits.
+  const int gbits = G ? bits_for((uint64_t)G) : 0;
+  const int total = std::min(32, std::max(kDegreeBits, (gbits + 12 + 7) / 8 * 8));
+  const DegreeKey dk = degree_key_of(total - gbits);
+  k_vertex_keys<<<grid_for(n), kThreads, 0, st>>>(deg, n, voff, G, dk, b.vk, b.vv);
   TB_LAUNCH_CHECK();
   uint32_t* sorted_ids = nullptr;
-  radix_sort<uint32_t, uint32_t, true>(b.vk, b.vk2, b.vv, b.vv2, n, dbits, b.tmp, st, &sorted_ids);
-  k_rank_scatter<<<grid_for(n), kThreads, 0, st>>>(sorted_ids, n, rank, nullptr, 0, nullptr);
+  radix_sort<uint32_t, uint32_t, true>(b.vk, b.vk2, b.vv, b.vv2, n, total, b.tmp, st, &sorted_ids);
+  k_rank_scatter<<<grid_for(n), kThreads, 0, st>>>(sorted_ids, n, rank, voff, G, graph_of_rank, zero, zero_words);
   TB_LAUNCH_CHECK();
+}
+
+}  // namespace
+
+void rank_vertices(const uint32_t* deg, uint64_t n, const RankBuffers& b, uint32_t* rank, cudaStream_t st) {
+  if (n > 0) rank_by_degree(deg, n, nullptr, 0, b, rank, nullptr, nullptr, 0, st);
 }
 
 void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* out) {
   const uint64_t n = in.n, E = in.E;
   if (n > 0xffffffffull || E > 0xfffffffeull)
     throw StatusError(TRIBIT_ERR_TOO_LARGE, "graphs are limited to 2^32-1 vertices and 2^32-2 entries");
+  const bool by_degree = in.order == TRIBIT_ORDER_DEGREE;
   DeviceStats* stats = ar.take<DeviceStats>(1);
+  uint32_t* deg = by_degree ? ar.take<uint32_t>(n ? n : 1) : nullptr;  // right after stats: cleared together
   uint64_t* rp = ar.take<uint64_t>(n + 1);
   uint32_t* rank = nullptr;
   uint32_t* graph_of_rank = in.G ? ar.take<uint32_t>(n ? n : 1) : nullptr;
-  uint32_t *deg = nullptr, *vk = nullptr, *vk2 = nullptr, *vv = nullptr, *vv2 = nullptr;
-  RadixTemp vtmp;
-  const bool by_degree = in.order == TRIBIT_ORDER_DEGREE;
+  // The row counters and, after them, the long rows' list lengths: cleared together.
+  uint32_t* cnt = ar.take<uint32_t>(n + 1);
+  uint32_t* nbig = ar.take<uint32_t>(2);
+  RankBuffers rb;
   if (by_degree) {
     rank = ar.take<uint32_t>(n ? n : 1);
-    deg = ar.take<uint32_t>(n ? n : 1);
-    vk = ar.take<uint32_t>(n ? n : 1);
-    vk2 = ar.take<uint32_t>(n ? n : 1);
-    vv = ar.take<uint32_t>(n ? n : 1);
-    vv2 = ar.take<uint32_t>(n ? n : 1);
-    vtmp = take_radix_temp(ar, n);
+    rb = take_rank_buffers(ar, n);
   }
   out->n = n;
   out->E = E;
@@ -1077,11 +1196,14 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
   // Phase 1 (launch only when not measuring): the upload of host entries,
   // degrees and the rank order.
   if (!ar.measuring()) {
-    TB_CUDA(cudaMemsetAsync(stats, 0, sizeof(DeviceStats), st));
+    const uint64_t zero_words = (uint64_t)(nbig + 2 - cnt);
+    TB_CUDA(cudaMemsetAsync(stats, 0, deg ? (size_t)((char*)(deg + n) - (char*)stats) : sizeof(DeviceStats), st));
+    if (!by_degree || n == 0) TB_CUDA(cudaMemsetAsync(cnt, 0, zero_words * sizeof(uint32_t), st));
     const HostUpload& up = in.upload;
     uint64_t* dst = const_cast<uint64_t*>(in.entries);
     const bool upload = up.host && E > 0;
-    const bool overlap = upload && by_degree && n > 0;
+    const uint64_t pieces = std::min<uint64_t>(kUploadChunks, E / kUploadMinPiece);
+    const bool overlap = upload && by_degree && n > 0 && pieces > 1;
     auto copy = [&](uint64_t* to, const uint64_t* from, uint64_t words, cudaStream_t s) {
       if (up.stage)
         up.stage(up.stage_ctx, to, from, words * sizeof(uint64_t), s);
@@ -1091,14 +1213,13 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
     if (upload && !overlap) copy(dst, up.host, E, st);
     if (upload && !overlap && up.uploaded) TB_CUDA(cudaEventRecord(up.uploaded, st));
     if (by_degree && n > 0) {
-      TB_CUDA(cudaMemsetAsync(deg, 0, n * sizeof(uint32_t), st));
       if (overlap) {
         // The copies wait for the stream's earlier work (which may still read
         // the staging buffer); piece k's degree pass waits for piece k.
         TB_CUDA(cudaEventRecord(up.events[0], st));
         TB_CUDA(cudaStreamWaitEvent(up.copy_stream, up.events[0], 0));
-        const uint64_t piece = ceil_div<uint64_t>(E, kUploadChunks);
-        for (int k = 0; k < kUploadChunks; ++k) {
+        const uint64_t piece = ceil_div<uint64_t>(E, pieces);
+        for (uint64_t k = 0; k < pieces; ++k) {
           const uint64_t i0 = k * piece, i1 = std::min<uint64_t>(E, i0 + piece);
           if (i0 >= i1) break;
           copy(dst + i0, up.host + i0, i1 - i0, up.copy_stream);
@@ -1110,22 +1231,14 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
       } else {
         degree_pass(in, 0, E, deg, &stats->err, st);
       }
-      int gbits = in.G ? bits_for((uint64_t)in.G) : 0;
-      int dbits = bits_for(2 * E + 2);
-      if (dbits > 32 - gbits) dbits = 32 - gbits;
-      k_vertex_keys<<<grid_for(n), kThreads, 0, st>>>(deg, n, in.voff, in.G, in.G ? dbits : 32, vk, vv);
-      TB_LAUNCH_CHECK();
-      uint32_t* sorted_ids = nullptr;
-      radix_sort<uint32_t, uint32_t, true>(vk, vk2, vv, vv2, n, in.G ? gbits + dbits : dbits, vtmp, st, &sorted_ids);
-      k_rank_scatter<<<grid_for(n), kThreads, 0, st>>>(sorted_ids, n, rank, in.voff, in.G, graph_of_rank);
-      TB_LAUNCH_CHECK();
+      rank_by_degree(deg, n, in.voff, in.G, rb, rank, graph_of_rank, cnt, zero_words, st);
     } else if (in.G && n > 0) {
       k_identity_graph_of<<<grid_for(n), kThreads, 0, st>>>(n, in.voff, in.G, graph_of_rank);
       TB_LAUNCH_CHECK();
     }
   }
   // Phase 2: orient, rows, sort + dedup per row, CSR + bit rows.
-  run_rows(ar, in, rank, deg, st, out, stats, rp);
+  run_rows(ar, in, rank, deg, cnt, nbig, st, out, stats, rp);
 }
 
 }  // namespace tb

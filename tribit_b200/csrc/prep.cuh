@@ -47,12 +47,15 @@ struct DeviceStats {
 };
 
 // Upload of host entries overlapped with the degree pass: the entries are
-// copied in kUploadChunks pieces on copy_stream, and each piece's degree pass
+// copied in up to kUploadChunks pieces of at least kUploadMinPiece entries (1
+// MiB; smaller inputs in one copy: a piece's copy, events and launch cost more
+// than 1 MiB's upload) on copy_stream, and each piece's degree pass
 // runs on the preparing stream as soon as the piece has landed. events: at
 // least kUploadChunks + 1 (the first orders the copies after the stream's
 // earlier work); uploaded is recorded on the preparing stream once every
 // piece has landed.
 constexpr int kUploadChunks = 8;
+constexpr uint64_t kUploadMinPiece = 1ull << 17;
 struct HostUpload {
   const uint64_t* host = nullptr;
   cudaStream_t copy_stream = nullptr;
@@ -90,15 +93,15 @@ struct Prepared {
 // preprocessing pipeline on stream st. Stats are zeroed here.
 void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* out);
 
-// The (degree, id) rank order of n vertices from their degrees (E entries
-// counted them, which bounds a degree by 2E): rank[v] = position of v. The
-// buffers come from take_rank_buffers; launches only.
+// The (degree, id) rank order of n vertices from their degrees: rank[v] =
+// position of v, as prepare_graph ranks a single graph. The buffers come from
+// take_rank_buffers; launches only.
 struct RankBuffers {
   uint32_t *vk = nullptr, *vk2 = nullptr, *vv = nullptr, *vv2 = nullptr;
   RadixTemp tmp{};
 };
 RankBuffers take_rank_buffers(Arena& ar, uint64_t n);
-void rank_vertices(const uint32_t* deg, uint64_t n, uint64_t E, const RankBuffers& b, uint32_t* rank, cudaStream_t st);
+void rank_vertices(const uint32_t* deg, uint64_t n, const RankBuffers& b, uint32_t* rank, cudaStream_t st);
 
 // One rank range's rows at a time: the oriented graph's rows [s, s + z) built
 // from that range's keys alone (lo << 32 | hi in rank space, lo in the range,

@@ -85,9 +85,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* in, uint6
   if (threadIdx.x == 0) partial[blockIdx.x] = tot;
 }
 
-// Scans one tile. carry (may be null) holds the exclusive prefix of each tile.
+// Scans one tile. carry (may be null) holds the exclusive prefix of each tile;
+// out2 (may be null) receives the result too.
 template <typename T, typename Op, bool Rev>
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const T* in, T* out, uint64_t n,
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const T* in, T* out, T* out2, uint64_t n,
                                                               const T* __restrict__ carry, Op op, T id,
                                                               bool exclusive) {
   constexpr int kPad = kScanTile + kScanTile / 32;
@@ -121,7 +122,62 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const T* in, T* out
   for (int j = 0; j < kScanItems; ++j) {
     int p = j * kScanThreads + threadIdx.x;
     uint64_t i = base + p;
-    if (i < n) out[scan_index<Rev>(i, n)] = s[p + p / 32];
+    if (i < n) {
+      out[scan_index<Rev>(i, n)] = s[p + p / 32];
+      if (out2) out2[scan_index<Rev>(i, n)] = s[p + p / 32];
+    }
+  }
+}
+
+// A scan of a few tiles by one CTA, tile after tile: one launch in the place
+// of three, whose gaps cost more than the other CTAs save.
+constexpr int kScanOneThreads = 1024;
+constexpr int kScanOneItems = 8;
+constexpr uint64_t kScanOneMax = 4ull * kScanOneThreads * kScanOneItems;
+template <typename T, typename Op, bool Rev>
+__global__ void __launch_bounds__(kScanOneThreads) k_scan_one(const T* in, T* out, T* out2, uint64_t n, Op op, T id,
+                                                              bool exclusive) {
+  __shared__ T warp_tot[kScanOneThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  T carry = id;
+  for (uint64_t base = 0; base < n; base += kScanOneThreads * kScanOneItems) {
+    const uint64_t i0 = base + (uint64_t)threadIdx.x * kScanOneItems;
+    T v[kScanOneItems];
+    T acc = id;
+#pragma unroll
+    for (int k = 0; k < kScanOneItems; ++k) v[k] = i0 + k < n ? in[scan_index<Rev>(i0 + k, n)] : id;
+#pragma unroll
+    for (int k = 0; k < kScanOneItems; ++k) acc = op(acc, v[k]);
+    T inc = acc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const T t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc = op(t, inc);
+    }
+    if (lane == 31) warp_tot[w] = inc;
+    __syncthreads();
+    T x = warp_tot[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const T t = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x = op(t, x);
+    }
+    T pre = carry;
+    const T before = __shfl_sync(0xffffffffu, x, w == 0 ? 0 : w - 1);
+    if (w > 0) pre = op(pre, before);
+    const T ex = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (lane > 0) pre = op(pre, ex);
+    carry = op(carry, __shfl_sync(0xffffffffu, x, 31));
+#pragma unroll
+    for (int k = 0; k < kScanOneItems; ++k) {
+      const T nxt = op(pre, v[k]);
+      if (i0 + k < n) {
+        out[scan_index<Rev>(i0 + k, n)] = exclusive ? pre : nxt;
+        if (out2) out2[scan_index<Rev>(i0 + k, n)] = exclusive ? pre : nxt;
+      }
+      pre = nxt;
+    }
+    __syncthreads();  // warp_tot is rewritten for the next tile
   }
 }
 
@@ -132,13 +188,20 @@ inline uint64_t scan_temp_elems(uint64_t n) {
 }
 
 // out[i] = op-scan of in (exclusive or inclusive); Rev scans from the end.
-// in and out may alias. temp holds scan_temp_elems(n) elements. Launches only.
+// in and out may alias, and so may in and out2 (null, or a second copy of the
+// result). temp holds scan_temp_elems(n) elements. Launches only.
 template <typename T, typename Op, bool Rev = false>
-void device_scan(const T* in, T* out, uint64_t n, bool exclusive, Op op, T id, T* temp, cudaStream_t st) {
+void device_scan(const T* in, T* out, uint64_t n, bool exclusive, Op op, T id, T* temp, cudaStream_t st,
+                 T* out2 = nullptr) {
   if (n == 0) return;
   uint64_t tiles = ceil_div<uint64_t>(n, kScanTile);
   if (tiles == 1) {
-    k_scan_apply<T, Op, Rev><<<1, kScanThreads, 0, st>>>(in, out, n, nullptr, op, id, exclusive);
+    k_scan_apply<T, Op, Rev><<<1, kScanThreads, 0, st>>>(in, out, out2, n, nullptr, op, id, exclusive);
+    TB_LAUNCH_CHECK();
+    return;
+  }
+  if (n <= kScanOneMax) {
+    k_scan_one<T, Op, Rev><<<1, kScanOneThreads, 0, st>>>(in, out, out2, n, op, id, exclusive);
     TB_LAUNCH_CHECK();
     return;
   }
@@ -146,7 +209,7 @@ void device_scan(const T* in, T* out, uint64_t n, bool exclusive, Op op, T id, T
   k_scan_reduce<T, Op, Rev><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, partial, op, id);
   TB_LAUNCH_CHECK();
   device_scan<T, Op, false>(partial, partial, tiles, true, op, id, temp + tiles, st);
-  k_scan_apply<T, Op, Rev><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, partial, op, id, exclusive);
+  k_scan_apply<T, Op, Rev><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, out2, n, partial, op, id, exclusive);
   TB_LAUNCH_CHECK();
 }
 

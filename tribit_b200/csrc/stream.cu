@@ -531,6 +531,7 @@ void count_rows_tier(tribit_context* c, const RowsSource& src, const std::vector
   p.view.rp = L.rp;
   p.view.col = L.col;
   p.view.bent = L.bent;
+  p.view.by_id = c->opts.order == TRIBIT_ORDER_ID;
   p.stats = L.stats;
   p.n = n;
   p.E = E;
@@ -542,7 +543,7 @@ void count_rows_tier(tribit_context* c, const RowsSource& src, const std::vector
   TB_CUDA(cudaEventRecord(c->ev[2], st));
   c->launch = launch_count(p.view, c->sched, p.stats, nullptr, count_config(c), st);
   TB_CUDA(cudaEventRecord(c->ev[3], st));
-  TB_CUDA(cudaMemcpyAsync(c->h_stats, p.stats, sizeof(DeviceStats), cudaMemcpyDeviceToHost, st));
+  read_stats(c, st);
   TB_CUDA(cudaStreamSynchronize(st));
   const DeviceStats& hs = *c->h_stats;
   if (hs.err & (kErrInput | kErrIdRange)) {
@@ -642,7 +643,7 @@ bool count_streamed_if_needed(tribit_context* c, const uint64_t* host, uint64_t 
     TB_LAUNCH_CHECK();
   });
   check_flags(nullptr);
-  rank_vertices(deg, n, E, rb, rank, st);
+  rank_vertices(deg, n, rb, rank, st);
   // Oriented entries per row (with duplicates), their prefix, the longest row.
   TB_CUDA(cudaMemsetAsync(rows, 0, (n + 1) * sizeof(uint32_t), st));
   stream_pass([&](const uint64_t* piece, uint64_t cnt) {
