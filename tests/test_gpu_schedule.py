@@ -1,0 +1,95 @@
+"""Branches of the preprocessing and the schedule at the sizes where they
+change, against the oracle: vertex ranks (one CTA up to 16,384 vertices, radix
+passes beyond; exact degrees up to 32,767), scans (one CTA up to 32,768
+elements), degree counting over sorted and skewed input, heavy and wide rows
+cut into pieces, and groups of short rows. Counts are integers: equality."""
+import numpy as np
+import pytest
+
+import oracle
+import tribit_b200 as tb
+from tests.test_gpu_rows import fans
+
+pytestmark = pytest.mark.gpu
+
+
+def check(e, n, modes=("plain",), orders=("degree", "id")):
+    want, m = oracle.count(e, n)
+    for order in orders:
+        for mode in modes:
+            with tb.Counter(order=order, dispatch=mode) as c:
+                r = c.count_edges(e, n)
+                assert (r.triangles, r.edges) == (want, m), (order, mode)
+
+
+@pytest.mark.parametrize("n", [3, 31, 33, 1023, 1025, 16383, 16384, 16385, 32767, 32768, 32769])
+def test_sizes_around_the_one_cta_kernels(n):
+    check(tb.gen_er(n, 6 * n + 1, seed=n), n)
+
+
+def test_degrees_past_the_exact_keys():
+    # Hubs of 32,767 to 70,000 neighbours: their degree keys keep 11 leading bits.
+    n = 80_000
+    parts = [tb.gen_er(n, 200_000, seed=5)]
+    for hub, k in enumerate((32767, 32768, 33000, 40000, 65535, 65536, 70000)):
+        parts.append((np.uint64(hub) << np.uint64(32)) | (np.uint64(100) + np.arange(k, dtype=np.uint64)))
+    check(np.concatenate(parts), n, orders=("degree",))
+
+
+@pytest.mark.parametrize("kind", ["sorted", "reversed", "one_hub", "self_loops"])
+def test_degree_counting_of_skewed_input(kind):
+    n = 30_000
+    e = np.sort(tb.gen_chung_lu(n, 300_000, 2.0, 3000.0, seed=17))
+    if kind == "reversed":
+        e = (e << np.uint64(32)) | (e >> np.uint64(32))
+    elif kind == "one_hub":  # half of all entries name one vertex
+        e[::2] = (np.uint64(7) << np.uint64(32)) | (e[::2] & np.uint64(0xFFFFFFFF))
+    elif kind == "self_loops":
+        e[1::3] = (e[1::3] >> np.uint64(32)) * np.uint64((1 << 32) + 1)
+    check(e, n)
+
+
+@pytest.mark.parametrize("length, stride", [
+    (257, 32), (512, 32), (513, 33), (1025, 200),  # heavy: masks of up to 7,676 blocks, one and more pieces
+    (900, 1000),                                   # heavy: a hash
+    (1025, 1000), (2049, 500),                     # wide: masks
+    (1100, 1500), (8192, 200),                     # wide: a hash, five pieces
+    (8193, 200), (9000, 190),                      # wide: searched in global memory
+])
+def test_heavy_and_wide_rows(length, stride):
+    n = 2_000_000
+    # The columns' own rows are short; a second fan over the same columns
+    # gives the first one long common neighbourhoods.
+    e = np.concatenate([fans([(length, 64, stride), (length, 64, stride)], n),
+                        np.array([(0 << 32) | 2], dtype=np.uint64)])
+    check(e, n, modes=("plain", "merge", "bitmap"), orders=("id",))
+
+
+def test_long_rows_in_the_hub_builder():
+    # Rows of more than 2,048 neighbours in merge blocks, whose candidates a
+    # CTA lists together; hubs with longer rows than the tails that meet them.
+    check(tb.gen_rmat(15, 24, seed=77), 1 << 15, modes=("merge", "plain"))
+
+
+@pytest.mark.parametrize("size", [2, 17, 32, 33, 34, 70])
+def test_groups_of_short_rows(size):
+    # Cliques: rows of 0 .. size - 1 neighbours, in groups of four up to 32.
+    i, j = np.triu_indices(size, 1)
+    base = (np.arange(101, dtype=np.uint64) * np.uint64(size))[:, None]
+    e = (((base + i.astype(np.uint64)) << np.uint64(32)) | (base + j.astype(np.uint64))).ravel()
+    check(e, 101 * size, modes=("bitmap", "merge"))
+
+
+def test_batch_of_tiny_graphs():
+    # Several graphs in every tile of entries and in every group of rows.
+    rng = np.random.default_rng(4)
+    nodes = rng.integers(1, 40, 3000).astype(np.uint32)
+    sizes = rng.integers(0, 60, 3000)
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.uint64)
+    e = np.concatenate([(rng.integers(0, k, s).astype(np.uint64) << np.uint64(32)) | rng.integers(0, k, s).astype(np.uint64)
+                        for k, s in zip(nodes, sizes)]).astype(np.uint64)
+    want = [oracle.count(e[int(a):int(b)], int(k))[0] if b > a else 0 for a, b, k in zip(off[:-1], off[1:], nodes)]
+    for mode in ("plain", "bitmap", "merge"):
+        with tb.Counter(dispatch=mode) as c:
+            got, r = c.count_batch(e, off, nodes)
+            assert got.tolist() == want and r.triangles == sum(want)

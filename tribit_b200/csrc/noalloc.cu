@@ -98,6 +98,7 @@ extern "C" tribit_status tribit_count_edges_noalloc(const uint64_t* d_entries, u
     in.E = n_entries;
     in.n = num_nodes;
     in.order = TRIBIT_ORDER_DEGREE;
+    in.compact = true;
     // Layout pass: launches nothing. The merge variant's hub lists (and the
     // full features the plain rule needs to choose merge) when they fit the
     // scratch; else bit tiles and the bitmap sweep only. Rejects graphs that

@@ -211,15 +211,25 @@ __global__ void k_vertex_keys(const uint32_t* __restrict__ deg, uint64_t n, cons
   vals[v] = (uint32_t)v;
 }
 
-// rank[id] = position, and words of `zero` at 0 (the row counters of the next pass).
+// The words the row build starts from, set while vertices are ranked: w[r] for
+// rank r (slots: the vertex's degree, its row's slot; else 0), then zeros up to
+// `count` words.
+struct RowWords {
+  uint32_t* w;
+  uint64_t count;
+  bool slots;
+};
+
+// rank[id] = position, and the row words.
 __global__ void k_rank_scatter(const uint32_t* __restrict__ sorted_ids, uint64_t n, uint32_t* __restrict__ rank,
                                const uint64_t* voff, uint32_t G, uint32_t* __restrict__ graph_of_rank,
-                               uint32_t* __restrict__ zero, uint64_t zero_words) {
+                               const uint32_t* __restrict__ deg, RowWords rw) {
   const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (uint64_t i = r; i < zero_words; i += (uint64_t)gridDim.x * blockDim.x) zero[i] = 0;
+  for (uint64_t i = n + r; i < rw.count; i += (uint64_t)gridDim.x * blockDim.x) rw.w[i] = 0;
   if (r >= n) return;
   uint32_t v = sorted_ids[r];
   rank[v] = (uint32_t)r;
+  if (r < rw.count) rw.w[r] = rw.slots ? deg[v] : 0u;
   if (graph_of_rank) graph_of_rank[r] = graph_of_vertex(voff, G, v);
 }
 
@@ -231,15 +241,14 @@ constexpr uint32_t kRankThreads = 1024;
 constexpr int kRankRounds = kRankOneMax / kRankThreads;
 constexpr size_t kRankSmem = (2 * kRankOneMax + (kRankThreads / 32) * 256) * sizeof(uint32_t);
 __global__ void __launch_bounds__(kRankThreads) k_rank_one(const uint32_t* __restrict__ deg, uint32_t n, DegreeKey dk,
-                                                           uint32_t* __restrict__ rank, uint32_t* __restrict__ zero,
-                                                           uint64_t zero_words) {
+                                                           uint32_t* __restrict__ rank, RowWords rw) {
   extern __shared__ uint32_t rank_sm[];
   __shared__ uint32_t s_sum[8];
   uint32_t* src = rank_sm;
   uint32_t* dst = rank_sm + kRankOneMax;
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   uint32_t* wcnt = rank_sm + 2 * kRankOneMax;  // [warp][digit]
-  for (uint64_t i = tid; i < zero_words; i += kRankThreads) zero[i] = 0;
+  for (uint64_t i = n + tid; i < rw.count; i += kRankThreads) rw.w[i] = 0;
   for (uint32_t i = tid; i < n; i += kRankThreads) src[i] = (degree_key(deg[i], dk) << 16) | i;
   const uint32_t rounds = (n + kRankThreads - 1) / kRankThreads;  // of 32 a warp
   for (int shift = 16; shift < 32; shift += 8) {
@@ -292,7 +301,11 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_one(const uint32_t* __res
     src = dst;
     dst = t;
   }
-  for (uint32_t i = tid; i < n; i += kRankThreads) rank[src[i] & 0xFFFFu] = i;
+  for (uint32_t i = tid; i < n; i += kRankThreads) {
+    const uint32_t v = src[i] & 0xFFFFu;
+    rank[v] = i;
+    if (i < rw.count) rw.w[i] = rw.slots ? deg[v] : 0u;
+  }
 }
 
 __global__ void k_identity_graph_of(uint64_t n, const uint64_t* voff, uint32_t G, uint32_t* __restrict__ graph_of_rank) {
@@ -376,15 +389,43 @@ __global__ void __launch_bounds__(kThreads) k_row_fill(const uint64_t* __restric
   }
 }
 
-// Slot path (inputs that take the presort, under degree order): row r is
-// given a slot of deg(v) entries, v the vertex of rank r (every entry oriented
-// from v is one of the deg(v) entries that touch v), so no pass counts the
-// rows: cap[r] = deg(v), cap[n] = 0, scanned to the slot starts.
-__global__ void k_slot_sizes(const uint32_t* __restrict__ deg, const uint32_t* __restrict__ rank, uint64_t n,
-                             uint32_t* __restrict__ cap) {
-  const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < n) cap[rank[v]] = deg[v];
-  if (v == n) cap[n] = 0;
+// Slot path (degree order): row r has a slot of deg(v) entries, v the vertex of
+// rank r (every entry oriented from v is one of the deg(v) entries that touch
+// v), so no pass counts the rows. Without a presort the entries go straight to
+// their rows: no keys are written or read either, one pass in the place of
+// k_row_count and k_row_fill (RMAT-20: 194 + 235 us, now 294).
+__global__ void __launch_bounds__(kThreads) k_row_fill_entries(PrepInput in, const uint32_t* __restrict__ rank,
+                                                               uint32_t* __restrict__ cur, uint32_t* __restrict__ nbr,
+                                                               uint32_t tiles, unsigned int* err) {
+  EntryReader rd(in, err);
+  const uint32_t lane = threadIdx.x & 31;
+  uint64_t c = (uint64_t)blockIdx.x * tiles * kTile;
+  for (uint32_t t = 0; t < tiles && c < in.E; ++t, c += kTile) {
+    uint64_t e[kAhead], key[kAhead];
+    uint32_t at[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint64_t i = c + k * kThreads + threadIdx.x;
+      e[k] = i < in.E ? in.entries[i] : 0ull;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint64_t i = c + k * kThreads + threadIdx.x;
+      uint32_t a, b;
+      key[k] = i < in.E && rd.ids(e[k], i, a, b) ? orient(rank, a, b) : kDropped;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const uint32_t lo = (uint32_t)(key[k] >> 32);
+      const KeyRun r = key_run(lo);
+      uint32_t base = 0;
+      if (r.head && lo != kNoId) base = atomicAdd(&cur[lo], r.len);
+      at[k] = __shfl_sync(kFull, base, r.first) + lane - r.first;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (key[k] != kDropped) nbr[at[k]] = (uint32_t)key[k];
+  }
 }
 
 // Slot path: keys[i] = (lo << 32) | hi of entry i (kDropped for a dropped
@@ -439,8 +480,9 @@ constexpr uint32_t kCtaSortSmem = 8192;  // bitonic rows longer than this are so
 // block left them to a few warps (RMAT-20: the row sort 607 us, the emit 487).
 struct LongRows {
   uint32_t* rows;   // n + 1
-  uint32_t* count;  // [0] CTA rows, [1] warp rows
+  uint32_t* count;  // [0] CTA rows, [1] warp rows, [2] scratch words taken by CTA rows
 };
+constexpr uint64_t kLongWords = 3;
 
 // Bitonic sort of the warp's 32 K values, value r * 32 + lane in x[r] of
 // lane lane, ascending.
@@ -621,8 +663,8 @@ __device__ __forceinline__ uint64_t window_sort(const uint32_t* a, uint32_t L, u
 // a warp per row in registers (bitonic). A CTA row is sorted through column
 // bitmaps when its block span takes at most L / 1024 windows (one window for
 // rows under 2,048), else bitonically, padded to a power of two P, in shared
-// memory (P <= kCtaSortSmem) or in the row's slice [2 s, 2 s + P) of scratch
-// (P <= 2 L; scratch holds twice the entries nbr's row slots hold). Rows are
+// memory (P <= kCtaSortSmem) or in a slice of scratch (P < 2 L; scratch holds two
+// words an entry), as rows of several windows are put together. Rows are
 // taken in strides over the grid (the lists run roughly by rank, so every warp
 // gets the same mix), the longest first.
 __global__ void __launch_bounds__(kLongThreads, 4)
@@ -631,6 +673,14 @@ __global__ void __launch_bounds__(kLongThreads, 4)
   __shared__ uint32_t sm[kBitWords];
   __shared__ uint32_t wsum[2][kLongThreads / 32];
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  __shared__ uint32_t s_at;
+  auto take = [&](uint32_t words) {  // the CTA's next slice of scratch
+    if (tid == 0) s_at = atomicAdd(&lng.count[2], words);
+    __syncthreads();
+    const uint32_t at = s_at;
+    __syncthreads();
+    return at;
+  };
   const uint32_t ncta = lng.count[0], nmid = lng.count[1];
   for (uint32_t bi = blockIdx.x; bi < ncta; bi += gridDim.x) {
     const uint32_t u = lng.rows[ncta - 1 - bi];
@@ -659,7 +709,7 @@ __global__ void __launch_bounds__(kLongThreads, 4)
     if (windows == 1) {  // every entry is read before the first is overwritten
       res = window_sort(nbr + s, L, lo, span, sm, nbr + s, 0);
     } else if ((uint64_t)windows * 1024 <= L) {
-      uint32_t* out = scratch + 2ull * s;
+      uint32_t* out = scratch + take(L);
       for (uint32_t k = 0; k < windows; ++k) {
         const uint32_t w0 = k * kBitWords;
         res += window_sort(nbr + s, L, lo + w0, min(kBitWords, span - w0), sm, out, (uint32_t)(res >> 32));
@@ -668,7 +718,7 @@ __global__ void __launch_bounds__(kLongThreads, 4)
     } else {
       uint32_t P = 1;
       while (P < L) P <<= 1;
-      uint32_t* a = P <= kCtaSortSmem ? sm : scratch + 2ull * s;
+      uint32_t* a = P <= kCtaSortSmem ? sm : scratch + take(P);
       for (uint32_t i = tid; i < P; i += kLongThreads) a[i] = i < L ? nbr[s + i] : kPad;
       __syncthreads();
       for (uint32_t k = 2; k <= P; k <<= 1) {
@@ -990,33 +1040,31 @@ __global__ void k_range_carry(uint64_t* __restrict__ rp, uint32_t count, const u
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) rp[k] += c;
 }
 
-// cnt (n + 1 words: row lengths or slot sizes, then the fill cursors, which end
-// at the rows' ends) and the two list lengths nbig are 0.
-void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32_t* deg, uint32_t* cnt, uint32_t* nbig,
-              cudaStream_t st, Prepared* out, DeviceStats* stats, uint64_t* rp) {
+bool takes_presort(const PrepInput& in) { return in.E >= kPresortMinEntries && in.n > 256; }
+
+// Rows in degree-sized slots (2E entries in all, u32 offsets): no per-row
+// atomics to count them, and, with the presort, its histogram counted while the
+// keys are written (RMAT-24: row counts 2.9 ms and the histogram 1.0 ms, for 4
+// bytes an entry more). Not where the layout has to stay small.
+bool degree_slots(const PrepInput& in) {
+  return in.order == TRIBIT_ORDER_DEGREE && !in.compact && 2 * in.E < 0xFFFFFFFFull;
+}
+
+// cnt: n + 1 words, row counters at 0 or, on the slot path, slot sizes (then the
+// fill cursors, which end at the rows' ends); nbig: kLongWords words at 0.
+void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, uint32_t* cnt, uint32_t* nbig, cudaStream_t st,
+              Prepared* out, DeviceStats* stats, uint64_t* rp) {
   const uint64_t E = in.E, n = in.n;
-  const bool presort = E >= kPresortMinEntries && n > 256;
-  // Slot path: with full degrees, rows take degree-sized slots (2E entries
-  // in all, u32 offsets) and the keys' presort histogram is counted while they
-  // are written: no per-row atomics, no separate histogram pass (RMAT-24:
-  // row counts 2.9 ms and the histogram 1.0 ms, for 1 GB more of nbr).
-  // (Decided from the order, not from deg: the arena's measuring pass hands
-  // out null buffers and must plan the same layout.)
-  const bool slots = presort && in.order == TRIBIT_ORDER_DEGREE && 2 * E < 0xFFFFFFFFull;
+  const bool presort = takes_presort(in), slots = degree_slots(in);
   const uint64_t cap = slots ? 2 * E : E;  // nbr entries
   uint32_t* off = ar.take<uint32_t>(n + 1);  // row starts
   uint32_t* otmp = take_scan_temp<uint32_t>(ar, n + 1);
   uint64_t* rtmp = take_scan_temp<uint64_t>(ar, n + 1);
   uint32_t* big = ar.take<uint32_t>(n + 1);
   uint32_t* nbr = ar.take<uint32_t>(cap ? cap : 1);
-  // The oriented keys (on the slot path both presort buffers), then long
-  // rows' sort space (twice nbr).
-  uint32_t* scratch = ar.take<uint32_t>(2 * cap + 2);
-  uint64_t* keys_alt = nullptr;
-  if (slots)
-    keys_alt = reinterpret_cast<uint64_t*>(scratch + 2 * E + 2);
-  else if (presort)
-    keys_alt = ar.take<uint64_t>(E);
+  // The oriented keys, then long rows' sort space.
+  uint32_t* scratch = ar.take<uint32_t>(2 * E + 2);
+  uint64_t* keys_alt = presort ? ar.take<uint64_t>(E) : nullptr;
   RadixTemp ktmp;
   if (presort) ktmp = take_radix_temp(ar, E);
   uint32_t* col = ar.take<uint32_t>(E + 4);   // + 4: 16-byte quad loads may read three ids past the end
@@ -1028,24 +1076,23 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, const uint32
   const LongRows lng{big, nbig};
   uint64_t* keys = reinterpret_cast<uint64_t*>(scratch);
   const int top = 32 + bits_for(n) - 8;  // the presort digit: the top 8 bits of lo
-  if (slots) {
-    k_slot_sizes<<<grid_for(n + 1), kThreads, 0, st>>>(deg, rank, n, cnt);
+  const uint64_t per = std::max<uint64_t>(1, E / (148ull * 64 * kTile));  // tiles a CTA
+  const unsigned entry_grid = (unsigned)ceil_div<uint64_t>(E, per * kTile);
+  if (!slots && E > 0) {
+    k_row_count<<<entry_grid, kThreads, 0, st>>>(in, rank, cnt, keys, (uint32_t)per, &stats->err);
     TB_LAUNCH_CHECK();
-    device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st, cnt);
+  }
+  device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st, cnt);
+  if (slots && presort) {
     const uint64_t tiles = ceil_div<uint64_t>(E, kSortTile);
     k_row_keys_hist<<<(unsigned)tiles, kSortThreads, 0, st>>>(in, rank, keys, top, (uint32_t)tiles, ktmp.hist,
                                                                &stats->err);
     TB_LAUNCH_CHECK();
-  } else {
-    if (E > 0) {
-      const uint64_t per = std::max<uint64_t>(1, E / (148ull * 64 * kTile));  // tiles a CTA
-      k_row_count<<<(unsigned)ceil_div<uint64_t>(E, per * kTile), kThreads, 0, st>>>(in, rank, cnt, keys, (uint32_t)per,
-                                                                                     &stats->err);
-      TB_LAUNCH_CHECK();
-    }
-    device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st, cnt);
   }
-  if (E > 0) {
+  if (slots && !presort && E > 0) {
+    k_row_fill_entries<<<entry_grid, kThreads, 0, st>>>(in, rank, cnt, nbr, (uint32_t)per, &stats->err);
+    TB_LAUNCH_CHECK();
+  } else if (E > 0) {
     // One radix pass on the top 8 bits of lo groups the keys into 256 ranges
     // of rows, so the fill's cursors and stores at any time stay in one
     // range's few MB of L2 instead of scattering over all rows.
@@ -1074,7 +1121,7 @@ RowRangeBuffers take_row_range_buffers(Arena& ar, uint64_t n, uint64_t cap) {
   b.off = ar.take<uint32_t>(n + 1);
   b.cursor = ar.take<uint32_t>(n + 1);
   b.big = ar.take<uint32_t>(n + 1);
-  b.nbig = ar.take<uint32_t>(2);
+  b.nbig = ar.take<uint32_t>(kLongWords);
   b.carry = ar.take<uint64_t>(1);
   b.scan_tmp = take_scan_temp<uint64_t>(ar, n + 1);
   return b;
@@ -1099,7 +1146,7 @@ void finish_row_range(const RowRangeBuffers& b, uint32_t s, uint32_t z, uint64_t
   k_range_check<<<grid_for(z), kThreads, 0, st>>>(b.off, b.cursor, z, err);
   TB_LAUNCH_CHECK();
   const LongRows lng{b.big, b.nbig};
-  TB_CUDA(cudaMemsetAsync(b.nbig, 0, 2 * sizeof(uint32_t), st));
+  TB_CUDA(cudaMemsetAsync(b.nbig, 0, kLongWords * sizeof(uint32_t), st));
   sort_rows(b.off, b.off + 1, z, cnt, b.nbr, b.scratch, rp + s, lng, st);
   device_scan<uint64_t, OpSum>(rp + s, rp + s, (uint64_t)z + 1, true, OpSum{}, 0ull, b.scan_tmp, st);
   k_range_carry<<<grid_for((uint64_t)z + 1), kThreads, 0, st>>>(rp + s, z + 1, b.carry);
@@ -1137,13 +1184,13 @@ RankBuffers take_rank_buffers(Arena& ar, uint64_t n) {
 namespace {
 
 // Ranks of n vertices from their degrees (graphs: the batch's, else G = 0), and
-// `zero_words` of `zero` at 0. The buffers as take_rank_buffers takes them.
+// the row words. The buffers as take_rank_buffers takes them.
 void rank_by_degree(const uint32_t* deg, uint64_t n, const uint64_t* voff, uint32_t G, const RankBuffers& b,
-                    uint32_t* rank, uint32_t* graph_of_rank, uint32_t* zero, uint64_t zero_words, cudaStream_t st) {
+                    uint32_t* rank, uint32_t* graph_of_rank, const RowWords& rw, cudaStream_t st) {
   if (!G && n <= kRankOneMax) {
     once_per_device<3>(
         [] { TB_CUDA(cudaFuncSetAttribute(k_rank_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRankSmem)); });
-    k_rank_one<<<1, kRankThreads, kRankSmem, st>>>(deg, (uint32_t)n, degree_key_of(kDegreeBits), rank, zero, zero_words);
+    k_rank_one<<<1, kRankThreads, kRankSmem, st>>>(deg, (uint32_t)n, degree_key_of(kDegreeBits), rank, rw);
     TB_LAUNCH_CHECK();
     return;
   }
@@ -1155,14 +1202,14 @@ void rank_by_degree(const uint32_t* deg, uint64_t n, const uint64_t* voff, uint3
   TB_LAUNCH_CHECK();
   uint32_t* sorted_ids = nullptr;
   radix_sort<uint32_t, uint32_t, true>(b.vk, b.vk2, b.vv, b.vv2, n, total, b.tmp, st, &sorted_ids);
-  k_rank_scatter<<<grid_for(n), kThreads, 0, st>>>(sorted_ids, n, rank, voff, G, graph_of_rank, zero, zero_words);
+  k_rank_scatter<<<grid_for(n), kThreads, 0, st>>>(sorted_ids, n, rank, voff, G, graph_of_rank, deg, rw);
   TB_LAUNCH_CHECK();
 }
 
 }  // namespace
 
 void rank_vertices(const uint32_t* deg, uint64_t n, const RankBuffers& b, uint32_t* rank, cudaStream_t st) {
-  if (n > 0) rank_by_degree(deg, n, nullptr, 0, b, rank, nullptr, nullptr, 0, st);
+  if (n > 0) rank_by_degree(deg, n, nullptr, 0, b, rank, nullptr, RowWords{}, st);
 }
 
 void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* out) {
@@ -1175,9 +1222,9 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
   uint64_t* rp = ar.take<uint64_t>(n + 1);
   uint32_t* rank = nullptr;
   uint32_t* graph_of_rank = in.G ? ar.take<uint32_t>(n ? n : 1) : nullptr;
-  // The row counters and, after them, the long rows' list lengths: cleared together.
+  // The row counters and, after them, the long rows' list lengths: set together.
   uint32_t* cnt = ar.take<uint32_t>(n + 1);
-  uint32_t* nbig = ar.take<uint32_t>(2);
+  uint32_t* nbig = ar.take<uint32_t>(kLongWords);
   RankBuffers rb;
   if (by_degree) {
     rank = ar.take<uint32_t>(n ? n : 1);
@@ -1196,9 +1243,9 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
   // Phase 1 (launch only when not measuring): the upload of host entries,
   // degrees and the rank order.
   if (!ar.measuring()) {
-    const uint64_t zero_words = (uint64_t)(nbig + 2 - cnt);
+    const RowWords rw{cnt, (uint64_t)(nbig + kLongWords - cnt), degree_slots(in)};
     TB_CUDA(cudaMemsetAsync(stats, 0, deg ? (size_t)((char*)(deg + n) - (char*)stats) : sizeof(DeviceStats), st));
-    if (!by_degree || n == 0) TB_CUDA(cudaMemsetAsync(cnt, 0, zero_words * sizeof(uint32_t), st));
+    if (!by_degree || n == 0) TB_CUDA(cudaMemsetAsync(cnt, 0, rw.count * sizeof(uint32_t), st));
     const HostUpload& up = in.upload;
     uint64_t* dst = const_cast<uint64_t*>(in.entries);
     const bool upload = up.host && E > 0;
@@ -1231,14 +1278,14 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
       } else {
         degree_pass(in, 0, E, deg, &stats->err, st);
       }
-      rank_by_degree(deg, n, in.voff, in.G, rb, rank, graph_of_rank, cnt, zero_words, st);
+      rank_by_degree(deg, n, in.voff, in.G, rb, rank, graph_of_rank, rw, st);
     } else if (in.G && n > 0) {
       k_identity_graph_of<<<grid_for(n), kThreads, 0, st>>>(n, in.voff, in.G, graph_of_rank);
       TB_LAUNCH_CHECK();
     }
   }
   // Phase 2: orient, rows, sort + dedup per row, CSR + bit rows.
-  run_rows(ar, in, rank, deg, cnt, nbig, st, out, stats, rp);
+  run_rows(ar, in, rank, cnt, nbig, st, out, stats, rp);
 }
 
 }  // namespace tb

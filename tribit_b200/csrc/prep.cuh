@@ -74,6 +74,7 @@ struct PrepInput {
   uint64_t E = 0;
   uint64_t n = 0;                     // vertices (sum over graphs in batch mode)
   int order = TRIBIT_ORDER_DEGREE;
+  bool compact = false;               // rows without degree slots: 4 bytes an entry less, one pass more
   // batch mode (G > 0): graph g owns entries [eoff[g], eoff[g+1]) with local
   // ids in [0, voff[g+1] - voff[g]); its vertices are voff[g] + local id.
   uint32_t G = 0;
@@ -116,7 +117,7 @@ struct RowRangeBuffers {
   uint32_t* off = nullptr;      // n + 1: range-relative row starts
   uint32_t* cursor = nullptr;   // n + 1: fill cursors
   uint32_t* big = nullptr;      // n + 1: the long rows' lists
-  uint32_t* nbig = nullptr;     // 2: their lengths
+  uint32_t* nbig = nullptr;     // their lengths
   uint64_t* carry = nullptr;    // rp of the range's first row before the range is built
   uint64_t* scan_tmp = nullptr;
 };
