@@ -1301,7 +1301,7 @@ constexpr bool kHubPairs = TB_HUB_PAIRS != 0;   // tails read as 16-byte pairs o
 // A hub tail holding at most TB_HUB_COL_RATIO / 100 neighbours a bit block is
 // walked as u's column ids after v (4 bytes a neighbour) instead of its bit-row
 // entries (8 bytes a block); 0 walks every tail as bit rows. Each hub's
-// in-list holds its bit-row tails first (in_cnt[v] of them), then its column
+// in-list holds its bit-row tails first (up to hub.cur[v].x), then its column
 // tails. 1.75 measured best on RMAT-24 and RMAT-22 (1.0 to 3.0 swept).
 #ifndef TB_HUB_COL_RATIO
 #define TB_HUB_COL_RATIO 175
@@ -1536,7 +1536,7 @@ struct HubShared {
 __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t* __restrict__ hub_pieces,
                                              const uint32_t* __restrict__ piece_off,
                                              const uint32_t* __restrict__ in_off,
-                                             const uint32_t* __restrict__ in_bits, const uint64_t* __restrict__ inl,
+                                             HubTable hub, const uint64_t* __restrict__ inl,
                                              const uint32_t* __restrict__ inrow, DeviceStats* stats,
                                              unsigned long long* per_graph, unsigned long long* block_ns,
                                              const HubShared& sh) {
@@ -1614,8 +1614,8 @@ __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t*
     const uint32_t cs = first_at((uint32_t)((uint64_t)tot * w / kHubWarps));
     const uint32_t ce = w + 1 == kHubWarps ? cnt : first_at((uint32_t)((uint64_t)tot * (w + 1) / kHubWarps));
     // Entries before nbits are bit-row tails, the rest column tails.
-    const uint32_t nbits = kHubColRatio ? min(cnt, in_off[v] + in_bits[v] - min(e0, in_off[v] + in_bits[v]))
-                                        : cnt;
+    const uint32_t front = hub.cur[v].x;
+    const uint32_t nbits = kHubColRatio ? min(cnt, front - min(e0, front)) : cnt;
     uint64_t racc = hub_sweep(g, inl + e0, cs, min(ce, nbits), direct, map, bmin, bmax, logb, wruns);
     if (kHubColRatio) racc += hub_sweep_col(g, inl + e0, max(cs, nbits), ce, direct, map, bmin, bmax, logb, wruns);
     if (per_graph) {
@@ -1667,8 +1667,8 @@ __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t*
       table_insert(wtbl, logb, g.bent, bs, be, lane, 32);
     }
     __syncwarp();
-    const uint32_t nbits = kHubColRatio ? min(cnt, in_off[v] + in_bits[v] - min(e0, in_off[v] + in_bits[v]))
-                                        : cnt;
+    const uint32_t front = hub.cur[v].x;
+    const uint32_t nbits = kHubColRatio ? min(cnt, front - min(e0, front)) : cnt;
     uint64_t racc = hub_sweep(g, inl + e0, 0, nbits, direct, wmap, bmin, bmax, logb, wruns);
     if (kHubColRatio) racc += hub_sweep_col(g, inl + e0, nbits, cnt, direct, wmap, bmin, bmax, logb, wruns);
     if (per_graph) {
@@ -1693,7 +1693,7 @@ __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t*
 __global__ void __launch_bounds__(kHubWarps * 32, TB_HUB_MIN_CTAS) k_hub(GraphView g, const uint64_t* __restrict__ hub_pieces,
                                                         const uint32_t* __restrict__ piece_off,
                                                         const uint32_t* __restrict__ in_off,
-                                                        const uint32_t* __restrict__ in_bits,
+                                                        HubTable hub,
                                                         const uint64_t* __restrict__ inl,
                                                         const uint32_t* __restrict__ inrow, DeviceStats* stats,
                                                         unsigned long long* per_graph,
@@ -1704,7 +1704,7 @@ __global__ void __launch_bounds__(kHubWarps * 32, TB_HUB_MIN_CTAS) k_hub(GraphVi
   __shared__ uint32_t s_t;
   __shared__ unsigned long long s_dt;
   const HubShared sh{map, pre, &runs[0][0], 128, &s_t, &s_dt};
-  uint64_t acc = hub_body(g, hub_pieces, piece_off, in_off, in_bits, inl, inrow, stats, per_graph, block_ns, sh);
+  uint64_t acc = hub_body(g, hub_pieces, piece_off, in_off, hub, inl, inrow, stats, per_graph, block_ns, sh);
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(&stats->triangles, (unsigned long long)acc);
 }
@@ -1726,8 +1726,8 @@ static_assert(kHubWarpStride % 4 == 0 && kHubWarpStride * 4 >= kWarpSlots * 8, "
 static_assert(kHubMapWords * 4 >= kWarpsPerCta * kWarpSlots * 8, "the map holds the CTA row table and prefix");
 __global__ void __launch_bounds__(kHubWarps * 32, TB_HUB_MIN_CTAS) k_queue(
     GraphView g, const uint64_t* __restrict__ pieces, const uint32_t* __restrict__ piece_off, DeviceStats* stats,
-    unsigned long long* per_graph, uint32_t width, const uint64_t* __restrict__ hub_pieces, const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ in_bits,
-    const uint64_t* __restrict__ inl) {
+    unsigned long long* per_graph, uint32_t width, const uint64_t* __restrict__ hub_pieces,
+    const uint32_t* __restrict__ in_off, HubTable hub, const uint64_t* __restrict__ inl) {
   __shared__ __align__(16) uint32_t map[kHubMapWords];
   __shared__ uint32_t pre[kHubPiece + 1];
   __shared__ uint32_t runs[kHubWarps][128];
@@ -1743,7 +1743,7 @@ __global__ void __launch_bounds__(kHubWarps * 32, TB_HUB_MIN_CTAS) k_queue(
   acc += pieces_body<TRIBIT_VARIANT_BITMAP>(g, pieces, piece_off, stats, per_graph, nullptr, true, width, ps);
   acc += pieces_body<TRIBIT_VARIANT_MERGE>(g, pieces, piece_off, stats, per_graph, nullptr, false, width, ps);
   __syncthreads();  // the hub's CTA pieces take the whole map
-  acc += hub_body(g, hub_pieces, piece_off, in_off, in_bits, inl, nullptr, stats, per_graph, nullptr, hs);
+  acc += hub_body(g, hub_pieces, piece_off, in_off, hub, inl, nullptr, stats, per_graph, nullptr, hs);
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(&stats->triangles, (unsigned long long)acc);
 }
@@ -2040,19 +2040,17 @@ __device__ uint32_t tile_pieces(const GraphView& g, uint32_t rb, uint32_t* vm) {
 // counts[l * nrb + rb] = pieces, and 1 << 32 for a block with pieces in its
 // variant's list (the scan then counts those blocks too). Bit-tile blocks have
 // tile_pieces, the others one per `width` neighbours of each row. With hub
-// arrays it also starts the hub builder: vinfo[v] = (span << 32) | nb, v's
-// bit-row length and the blocks it spans, and its counters and flags at 0.
+// arrays it also starts the hub builder: every vertex's row words, its counters
+// and the edge flags at 0.
 struct HubInit {
-  uint64_t* vinfo;  // null: no hub pass
-  unsigned long long* save;
-  uint32_t* in_cnt;
+  HubTable hub;
   uint32_t* eflag;
   uint64_t eflag_words;
 };
 __global__ void __launch_bounds__(256) k_block_pieces(GraphView g, uint32_t nrb, const uint8_t* __restrict__ variant_of,
                                                       uint64_t* __restrict__ counts, uint32_t width, HubInit hub) {
   __shared__ uint32_t vm[8][kTileMaxK];
-  if (hub.vinfo)
+  if (hub.hub.info)
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < hub.eflag_words;
          i += (uint64_t)gridDim.x * blockDim.x)
       hub.eflag[i] = 0;
@@ -2064,13 +2062,12 @@ __global__ void __launch_bounds__(256) k_block_pieces(GraphView g, uint32_t nrb,
     const int v = variant_of[rb];
     int list;
     const uint32_t u = rb * 32 + lane;
-    if (hub.vinfo && u < g.n) {
+    if (hub.hub.info && u < g.n) {
       const uint32_t bs = rp_blk(g.rp[u]), be = rp_blk(g.rp[u + 1]);
       uint64_t x = 0;
       if (be > bs) x = ((uint64_t)((uint32_t)(g.bent[be - 1] >> 32) - (uint32_t)(g.bent[bs] >> 32) + 1) << 32) | (be - bs);
-      hub.vinfo[u] = x;
-      hub.save[u] = 0;
-      hub.in_cnt[u] = 0;
+      hub.hub.info[u] = x;
+      hub.hub.cur[u] = make_uint2(0u, 0u);
     }
     const uint32_t np = row_pieces(g, u, v, width, list);
     uint32_t own = __reduce_add_sync(kFull, list == v ? np : 0u), heavy = 0, wide = 0;
@@ -2141,9 +2138,11 @@ __device__ __forceinline__ unsigned long long hub_cost(uint32_t span, uint32_t n
                              : (unsigned long long)kHubHashMul * 3ull * nbv + kHubHashMin;
 }
 
-__device__ __forceinline__ bool hub_candidate(const uint64_t* __restrict__ vinfo, uint32_t v, uint32_t tail,
-                                              uint32_t& nbv, unsigned long long& cost) {
-  const uint64_t vi = vinfo[v];
+constexpr uint32_t kHubMaxCost = kHubMaxSpan / 4 + kHubMaxSpan + kHubHashMul * 3 * kHubMaxHash + kHubHashMin;  // bound
+
+__device__ __forceinline__ bool hub_candidate(const HubTable& hub, uint32_t v, uint32_t tail, uint32_t& nbv,
+                                              unsigned long long& cost) {
+  const uint64_t vi = __ldg(&hub.info[v]);  // not written while edges are walked
   nbv = (uint32_t)vi;
   const uint32_t span = (uint32_t)(vi >> 32);
   cost = hub_cost(span, nbv);
@@ -2152,20 +2151,19 @@ __device__ __forceinline__ bool hub_candidate(const uint64_t* __restrict__ vinfo
 
 // One pass over the edges of the merge row blocks; rows of at most
 // kHubLaneRow neighbours are walked by their own lane, longer rows by the
-// whole warp (mode 1 on a small wave: one warp per row), rows of more than
-// kHubCtaRow, left to the end, by the whole CTA. For the edge at CSR position
-// j, u's tail is u's bit blocks from v's block on. Neighbouring row blocks go to
-// different CTAs, so the top ranks' long rows spread over the chip.
-// Mode 0: counts each hub's candidate in-edges (in_cnt) and adds to save[v]
-// the blocks a hub walk saves (v's row length - tail), but only while save[v]
-// is below the staging cost: the decision save[v] >= cost (k_hub_accept) is
-// then the one the full sum gives, without one atomic per in-edge on the
-// most popular hubs.
-// Mode 1: every candidate edge of an accepted hub (a vertex whose vinfo
+// whole warp, rows of more than kHubCtaRow, left to the end, by the whole CTA.
+// For the edge at CSR position j, u's tail is u's bit blocks from v's block on.
+// Neighbouring rows and row blocks go to different CTAs, so the top ranks' long
+// rows spread over the chip.
+// Mode 0: counts each hub's candidate in-edges and adds up the blocks a hub
+// walk saves (v's row length - tail), in one 64-bit update of v's counters, the
+// savings only while they are below the staging cost: the decision saved >=
+// cost (k_hub_accept) is then the one the full sum gives, and the sum stays in
+// its 32 bits (the updates in flight past the cost add at most kHubMaxSpan each).
+// Mode 1: every candidate edge of an accepted hub (a vertex whose row words
 // k_hub_accept kept) is flagged and appended to the hub's in-list: a bit-row
-// tail (first block, blocks) at the front (in_cnt[v] counts them), a column
-// tail (first CSR position after v, neighbours) at the back (the low word of
-// save[v] counts them). rows (may be null): the pass covers rows
+// tail (first block, blocks) at the front, a column tail (first CSR position
+// after v, neighbours) at the back. rows (may be null): the pass covers rows
 // [rows[0], rows[1]).
 constexpr uint32_t kHubLaneRow = 64;
 constexpr uint32_t kHubCtaRow = 2048;
@@ -2180,10 +2178,8 @@ constexpr uint32_t kHubCtaRows = 256;  // a CTA's list of them; rows past it are
 constexpr uint32_t kHubTop = TB_HUB_TOP;
 
 template <int Mode>
-__global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of, const uint64_t* __restrict__ vinfo,
-                            unsigned long long* __restrict__ save, uint32_t* __restrict__ eflag,
-                            uint32_t* __restrict__ in_cnt, const uint32_t* __restrict__ in_off,
-                            uint64_t* __restrict__ inl, uint32_t* __restrict__ inrow,
+__global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of, HubTable hub,
+                            uint32_t* __restrict__ eflag, uint64_t* __restrict__ inl, uint32_t* __restrict__ inrow,
                             const uint32_t* __restrict__ rows) {
   __shared__ uint32_t s_long[kHubCtaRows], s_nlong, s_heads[8];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -2194,7 +2190,7 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
   // Mode 0: candidate counts and savings of the vertices ranked top_lo and
   // above, per CTA. A CTA adds to a saving only while it is below the cost,
   // as the global sums do, so a CTA's partial sum either is exact or already
-  // reaches the cost by itself: the decision save[v] >= cost is unchanged.
+  // reaches the cost by itself: the decision is unchanged.
   // Bounded: at most blockDim.x adds of at most nbv each past the cost.
   constexpr uint32_t kTop = Mode == 0 ? kHubTop : 0u;
   __shared__ uint32_t s_top[kTop ? 2 * kTop : 1];
@@ -2204,10 +2200,10 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
     __syncthreads();
   }
   // Whether the edge to v (tail blocks) takes part: mode 0, a candidate;
-  // mode 1, a candidate of an accepted hub (k_hub_accept clears the vinfo of
+  // mode 1, a candidate of an accepted hub (k_hub_accept clears the row words of
   // every other vertex, so one read decides).
   auto decide = [&](uint32_t v, uint32_t tail, uint32_t& nbv, unsigned long long& cost) -> bool {
-    return hub_candidate(vinfo, v, tail, nbv, cost);
+    return hub_candidate(hub, v, tail, nbv, cost);
   };
   // Applies mode Mode to the taking-part edge at j (v = col[j]; u's row ends
   // at CSR position re) of row u.
@@ -2220,16 +2216,17 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
         if (*(volatile uint32_t*)(c + 1) < cost) atomicAdd(c + 1, nbv - tail);
         return;
       }
-      atomicAdd(&in_cnt[v], 1u);
-      if (*(volatile const unsigned long long*)&save[v] < cost) atomicAdd(&save[v], (unsigned long long)(nbv - tail));
+      unsigned long long* c = reinterpret_cast<unsigned long long*>(&hub.cur[v]);
+      const bool below = (__ldcg(c) >> 32) < cost;
+      atomicAdd(c, (below ? (unsigned long long)(nbv - tail) << 32 : 0ull) | 1ull);
     } else {
       const uint32_t after = re - j - 1;  // u's neighbours after v
       uint32_t at;
       if (kHubColRatio && (uint64_t)after * 100u <= (uint64_t)tail * kHubColRatio) {
-        at = in_off[v + 1] - 1u - atomicAdd(reinterpret_cast<uint32_t*>(&save[v]), 1u);
+        at = atomicSub(&hub.cur[v].y, 1u) - 1u;
         inl[at] = ((uint64_t)(j + 1) << 32) | after;
       } else {
-        at = in_off[v] + atomicAdd(&in_cnt[v], 1u);
+        at = atomicAdd(&hub.cur[v].x, 1u);
         inl[at] = ((uint64_t)(bs + pos) << 32) | tail;
       }
       if (inrow) inrow[at] = u;  // timing mode only
@@ -2277,65 +2274,65 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
     }
     warp_span(u, rs, re, re, bs, nb, 0, 0xFFFFFFFFu);
   };
-  if (u1 - u0 < (Mode == 1 ? 32u : 8u) * nwarps) {
-    // The in-list fill runs once per row wave; a wave of fewer rows than the
-    // grid has lanes keeps every warp busy with one warp per row. Larger waves
-    // (the first ones: millions of short rows) take the row-block loop below.
-    for (uint32_t u = u0 + warp; u < u1; u += nwarps) {
-      if (variant_of[u >> 5] != TRIBIT_VARIANT_MERGE) continue;
+  // The last rows, one a warp: a whole pass or wave when it has few rows, and
+  // the top ranks' long ones in mode 0 (the first waves of mode 1 hold millions of
+  // short rows); the rest by row blocks, a short row a lane.
+  const uint32_t few = (Mode == 1 ? 32u : 8u) * nwarps;
+  const uint32_t us = u1 - u0 < few ? u0 : Mode == 0 ? max(u0, (u1 - few) & ~31u) : u1;
+  for (uint32_t k = warp; k < u1 - us; k += nwarps) {
+    const uint32_t u = u1 - 1 - k;
+    if (variant_of[u >> 5] != TRIBIT_VARIANT_MERGE) continue;
+    const uint64_t a = g.rp[u], b = g.rp[u + 1];
+    const uint32_t rs = rp_row(a), re = rp_row(b), bs = rp_blk(a);
+    if (re - rs >= 2) warp_row(u, rs, re, bs, rp_blk(b) - bs);
+  }
+  for (uint32_t rb = (u0 >> 5) + warp; rb < ((us + 31) >> 5) && us > u0; rb += nwarps) {
+    if (variant_of[rb] != TRIBIT_VARIANT_MERGE) continue;
+    const uint32_t u = rb * 32 + lane;
+    uint32_t rs = 0, re = 0, bs = 0, nbu = 0;
+    bool mine = u >= u0 && u < us;
+    if (mine) {
       const uint64_t a = g.rp[u], b = g.rp[u + 1];
-      const uint32_t rs = rp_row(a), re = rp_row(b), bs = rp_blk(a);
-      if (re - rs >= 2) warp_row(u, rs, re, bs, rp_blk(b) - bs);
+      rs = rp_row(a);
+      re = rp_row(b);
+      bs = rp_blk(a);
+      nbu = rp_blk(b) - bs;
+      mine = re - rs >= 2;
     }
-  } else {
-    for (uint32_t rb = (u0 >> 5) + warp; rb < ((u1 + 31) >> 5); rb += nwarps) {
-      if (variant_of[rb] != TRIBIT_VARIANT_MERGE) continue;
-      const uint32_t u = rb * 32 + lane;
-      uint32_t rs = 0, re = 0, bs = 0, nbu = 0;
-      bool mine = u >= u0 && u < u1;
-      if (mine) {
-        const uint64_t a = g.rp[u], b = g.rp[u + 1];
-        rs = rp_row(a);
-        re = rp_row(b);
-        bs = rp_blk(a);
-        nbu = rp_blk(b) - bs;
-        mine = re - rs >= 2;
-      }
-      const bool own = mine && re - rs <= kHubLaneRow;
-      if (own) {
-        // Mode 1 gathers the row's flag bits word by word: one atomicOr per
-        // 32 CSR positions (a word may hold the ends of other lanes' rows).
-        uint32_t pos = 0xFFFFFFFFu, prev = 0xFFFFFFFFu, fw = 0xFFFFFFFFu, fb = 0;
-        for (uint32_t j = rs; j < re; ++j) {
-          const uint32_t v = g.col[j];
-          if ((v >> 5) != prev) {
-            ++pos;
-            prev = v >> 5;
-          }
-          const uint32_t tail = nbu - pos;
-          uint32_t nbv = 0;
-          unsigned long long cost = 0;
-          if (!decide(v, tail, nbv, cost)) continue;
-          if (Mode == 1) {
-            if ((j >> 5) != fw) {
-              if (fb) atomicOr(&eflag[fw], fb);
-              fw = j >> 5;
-              fb = 0;
-            }
-            fb |= 1u << (j & 31);
-          }
-          edge(u, bs, j, re, v, pos, tail, nbv, cost);
+    const bool own = mine && re - rs <= kHubLaneRow;
+    if (own) {
+      // Mode 1 gathers the row's flag bits word by word: one atomicOr per
+      // 32 CSR positions (a word may hold the ends of other lanes' rows).
+      uint32_t pos = 0xFFFFFFFFu, prev = 0xFFFFFFFFu, fw = 0xFFFFFFFFu, fb = 0;
+      for (uint32_t j = rs; j < re; ++j) {
+        const uint32_t v = g.col[j];
+        if ((v >> 5) != prev) {
+          ++pos;
+          prev = v >> 5;
         }
-        if (Mode == 1 && fb) atomicOr(&eflag[fw], fb);
+        const uint32_t tail = nbu - pos;
+        uint32_t nbv = 0;
+        unsigned long long cost = 0;
+        if (!decide(v, tail, nbv, cost)) continue;
+        if (Mode == 1) {
+          if ((j >> 5) != fw) {
+            if (fb) atomicOr(&eflag[fw], fb);
+            fw = j >> 5;
+            fb = 0;
+          }
+          fb |= 1u << (j & 31);
+        }
+        edge(u, bs, j, re, v, pos, tail, nbv, cost);
       }
-      // Longer rows: the warp, one row at a time.
-      uint32_t longm = __ballot_sync(kFull, mine && !own);
-      while (longm) {
-        const int r = __ffs(longm) - 1;
-        longm &= longm - 1;
-        warp_row(rb * 32 + r, __shfl_sync(kFull, rs, r), __shfl_sync(kFull, re, r), __shfl_sync(kFull, bs, r),
-                 __shfl_sync(kFull, nbu, r));
-      }
+      if (Mode == 1 && fb) atomicOr(&eflag[fw], fb);
+    }
+    // Longer rows: the warp, one row at a time.
+    uint32_t longm = __ballot_sync(kFull, mine && !own);
+    while (longm) {
+      const int r = __ffs(longm) - 1;
+      longm &= longm - 1;
+      warp_row(rb * 32 + r, __shfl_sync(kFull, rs, r), __shfl_sync(kFull, re, r), __shfl_sync(kFull, bs, r),
+               __shfl_sync(kFull, nbu, r));
     }
   }
   // The CTA's longest rows, an eighth a warp: the block heads of the shares
@@ -2363,31 +2360,29 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
     __syncthreads();
     for (uint32_t t = threadIdx.x; t < kTop && top_lo + t < g.n; t += blockDim.x) {
       const uint32_t c = s_top[2 * t], sv = s_top[2 * t + 1];
-      if (c) atomicAdd(&in_cnt[top_lo + t], c);
-      if (sv) atomicAdd(&save[top_lo + t], (unsigned long long)sv);
+      // Clipped to what decides by itself, so the CTAs' savings stay in 32 bits.
+      if (c)
+        atomicAdd(reinterpret_cast<unsigned long long*>(&hub.cur[top_lo + t]),
+                  ((unsigned long long)min(sv, kHubMaxCost) << 32) | c);
     }
   }
 }
 
 // After mode 0: a hub whose candidates save at least its staging cost keeps
-// its candidate count (the length of its in-list) and is marked in save[v]
-// (1 << 32: the low word then counts its column tails in mode 1); any other
-// vertex gets no in-list, and its vinfo is cleared so that mode 1 takes none
-// of its edges. cnt: the in-list lengths, then the pieces of each hub for a
-// CTA and for a warp, n + 1 of each (0 at the ends), to be scanned as one array.
-__global__ void k_hub_accept(uint64_t* __restrict__ vinfo, uint32_t n, unsigned long long* __restrict__ save,
-                             uint32_t* __restrict__ in_cnt, uint32_t* __restrict__ cnt) {
+// its candidate count (the length of its in-list); any other vertex gets no
+// in-list, and its row words are cleared so that mode 1 takes none of its edges.
+// cnt: the in-list lengths, then the pieces of each hub for a CTA and for a
+// warp, n + 1 of each (0 at the ends), to be scanned as one array.
+__global__ void k_hub_accept(HubTable hub, uint32_t n, uint32_t* __restrict__ cnt) {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v > n) return;
   uint32_t k = 0, c = 0, wc = 0;
   if (v < n) {
-    const uint64_t vi = vinfo[v];
+    const uint64_t vi = hub.info[v];
+    const uint2 c2 = hub.cur[v];
     const uint32_t span = (uint32_t)(vi >> 32), nb = (uint32_t)vi;
-    k = in_cnt[v];
-    in_cnt[v] = 0;
-    if (k > 0 && save[v] < hub_cost(span, nb)) k = 0;
-    if (k == 0) vinfo[v] = 0;  // no candidate in mode 1
-    save[v] = k ? (1ull << 32) : 0ull;
+    k = c2.y >= hub_cost(span, nb) ? c2.x : 0u;
+    if (k == 0) hub.info[v] = 0;  // no candidate in mode 1
     // The warp stages the row when its direct map fits the warp's slice, or,
     // for a row too wide for the CTA's direct map, when its hash does.
     if (span <= kHubWarpSpan || (span > kHubMaxSpan && nb <= kHubWarpHash))
@@ -2400,15 +2395,19 @@ __global__ void k_hub_accept(uint64_t* __restrict__ vinfo, uint32_t n, unsigned 
   cnt[2 * ((uint64_t)n + 1) + v] = wc;
 }
 
-// After the scan: the pieces of every hub and the hub words of piece_off;
-// wave_cnt (2 kHubWaves words, may be null) at 0. Positions count from pos[0],
-// where the in-list entries end.
-__global__ void k_hub_piece_scatter(const uint32_t* __restrict__ pos, uint32_t n, uint64_t* __restrict__ pieces,
-                                    uint32_t* __restrict__ piece_off, uint32_t* __restrict__ wave_cnt) {
+// After the scan: the ends of every hub's empty in-list in its counters, the
+// pieces of every hub and the hub words of piece_off; wave_cnt (2 kHubWaves
+// words, may be null) at 0. in_off: the scanned counts; piece positions count
+// from where the in-list entries end.
+__global__ void k_hub_piece_scatter(const uint32_t* __restrict__ in_off, uint32_t n, HubTable hub,
+                                    uint64_t* __restrict__ pieces, uint32_t* __restrict__ piece_off,
+                                    uint32_t* __restrict__ wave_cnt) {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t* pos = in_off + (uint64_t)n + 1;
   const uint32_t* wpos = pos + (uint64_t)n + 1;
   const uint32_t base = pos[0];
   if (v < n) {
+    hub.cur[v] = make_uint2(in_off[v], in_off[v + 1]);
     for (uint32_t k = 0, at = pos[v] - base, np = pos[v + 1] - pos[v]; k < np; ++k)
       pieces[at + k] = ((uint64_t)v << 32) | (k * kHubPiece);
     for (uint32_t k = 0, at = wpos[v] - base, np = wpos[v + 1] - wpos[v]; k < np; ++k)
@@ -2460,39 +2459,92 @@ __device__ __forceinline__ uint32_t wave_of_block(const uint32_t* __restrict__ w
 }
 
 // Counting sort of the hub pieces by the wave of their first tail, within
-// each list (CTA pieces [0, Pc), warp pieces [Pc, P)). cnt: 2 kHubWaves.
-__global__ void k_piece_waves(const uint64_t* __restrict__ pieces, const uint32_t* __restrict__ piece_off,
-                              const uint32_t* __restrict__ in_off, const uint32_t* __restrict__ in_bits,
-                              const uint64_t* __restrict__ inl, const uint32_t* __restrict__ wave_bk,
-                              const uint32_t* __restrict__ wave_cp, uint32_t* __restrict__ cnt,
-                              uint8_t* __restrict__ wave) {
-  const uint32_t pc_n = piece_off[kOffHubCta], all = piece_off[kOffHubAll];
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < all; p += gridDim.x * blockDim.x) {
-    const uint64_t pc = pieces[p];
-    const uint32_t v = (uint32_t)(pc >> 32), k = (uint32_t)pc;  // the piece's first entry: k of v's list
-    const bool bits = !kHubColRatio || k < in_bits[v];
-    const uint32_t w = wave_of_block(bits ? wave_bk : wave_cp, (uint32_t)(inl[in_off[v] + k] >> 32));
-    wave[p] = (uint8_t)w;
-    atomicAdd(&cnt[(p < pc_n ? 0 : kHubWaves) + w], 1u);
-  }
+// each list (CTA pieces [0, Pc), warp pieces [Pc, P)): the digit of a piece is
+// its list's wave. Each CTA counts its contiguous share in shared memory, one
+// atomic per warp and digit, and later takes one range per digit for it: with an
+// atomic per piece on the 64 counters the two passes were bound by them
+// (RMAT-20: 58 + 57 us; a count 3,990 us, now 3,896).
+struct PieceShare {
+  uint32_t begin, end, ctas;  // this CTA's pieces; the CTA pieces of all
+};
+__device__ __forceinline__ PieceShare piece_share(const uint32_t* __restrict__ piece_off) {
+  const uint32_t all = piece_off[kOffHubAll];
+  const uint32_t per = (all + gridDim.x - 1) / gridDim.x;
+  const uint64_t b = (uint64_t)per * blockIdx.x;
+  return {(uint32_t)min(b, (uint64_t)all), (uint32_t)min(b + per, (uint64_t)all), piece_off[kOffHubCta]};
 }
 
+__device__ __forceinline__ void count_digit(uint32_t* h, uint32_t digit, bool in) {
+  const uint32_t peers = __match_any_sync(kFull, in ? digit : 2 * kHubWaves);
+  if (in && (threadIdx.x & 31) == (uint32_t)__ffs(peers) - 1u) atomicAdd(&h[digit], (uint32_t)__popc(peers));
+}
+
+__global__ void __launch_bounds__(256) k_piece_waves(const uint64_t* __restrict__ pieces,
+                                                     const uint32_t* __restrict__ piece_off,
+                                                     const uint32_t* __restrict__ in_off,
+                                                     HubTable hub,
+                                                     const uint64_t* __restrict__ inl,
+                                                     const uint32_t* __restrict__ wave_bk,
+                                                     const uint32_t* __restrict__ wave_cp, uint32_t* __restrict__ cnt,
+                                                     uint8_t* __restrict__ wave) {
+  __shared__ uint32_t h[2 * kHubWaves];
+  for (uint32_t i = threadIdx.x; i < 2 * kHubWaves; i += 256) h[i] = 0;
+  __syncthreads();
+  const PieceShare sh = piece_share(piece_off);
+  for (uint32_t c = sh.begin; c < sh.end; c += 256) {
+    const uint32_t p = c + threadIdx.x;
+    const bool in = p < sh.end;
+    uint32_t digit = 0;
+    if (in) {
+      const uint64_t pc = pieces[p];
+      const uint32_t v = (uint32_t)(pc >> 32), at = in_off[v] + (uint32_t)pc;  // the piece's first entry
+      const bool bits = !kHubColRatio || at < hub.cur[v].x;
+      digit = (p < sh.ctas ? 0 : kHubWaves) + wave_of_block(bits ? wave_bk : wave_cp, (uint32_t)(inl[at] >> 32));
+      wave[p] = (uint8_t)digit;
+    }
+    count_digit(h, digit, in);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < 2 * kHubWaves; i += 256)
+    if (h[i]) atomicAdd(&cnt[i], h[i]);
+}
+
+static_assert(kHubWaves == 32, "a lane scans one wave of each list");
 __global__ void k_wave_scan(uint32_t* __restrict__ cnt, const uint32_t* __restrict__ piece_off) {
-  uint32_t run = 0;
-  for (uint32_t i = 0; i < 2 * kHubWaves; ++i) {
-    if (i == kHubWaves) run = piece_off[kOffHubCta];  // warp pieces follow the CTA pieces
-    const uint32_t c = cnt[i];
-    cnt[i] = run;
-    run += c;
-  }
+  const uint32_t lane = threadIdx.x;
+  const uint32_t c = cnt[lane], w = cnt[kHubWaves + lane];
+  cnt[lane] = warp_inclusive_sum(c) - c;
+  cnt[kHubWaves + lane] = piece_off[kOffHubCta] + warp_inclusive_sum(w) - w;  // warp pieces follow the CTA pieces
 }
 
-__global__ void k_piece_wave_scatter(const uint64_t* __restrict__ pieces, const uint32_t* __restrict__ piece_off,
-                                     const uint8_t* __restrict__ wave, uint32_t* __restrict__ pos,
-                                     uint64_t* __restrict__ out) {
-  const uint32_t pc_n = piece_off[kOffHubCta], all = piece_off[kOffHubAll];
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < all; p += gridDim.x * blockDim.x)
-    out[atomicAdd(&pos[(p < pc_n ? 0 : kHubWaves) + wave[p]], 1u)] = pieces[p];
+__global__ void __launch_bounds__(256) k_piece_wave_scatter(const uint64_t* __restrict__ pieces,
+                                                            const uint32_t* __restrict__ piece_off,
+                                                            const uint8_t* __restrict__ wave,
+                                                            uint32_t* __restrict__ pos, uint64_t* __restrict__ out) {
+  __shared__ uint32_t h[2 * kHubWaves];
+  for (uint32_t i = threadIdx.x; i < 2 * kHubWaves; i += 256) h[i] = 0;
+  __syncthreads();
+  const PieceShare sh = piece_share(piece_off);
+  for (uint32_t c = sh.begin; c < sh.end; c += 256) {
+    const uint32_t p = c + threadIdx.x;
+    count_digit(h, p < sh.end ? wave[p] : 0u, p < sh.end);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < 2 * kHubWaves; i += 256)
+    if (h[i]) h[i] = atomicAdd(&pos[i], h[i]);
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t c = sh.begin; c < sh.end; c += 256) {
+    const uint32_t p = c + threadIdx.x;
+    const bool in = p < sh.end;
+    const uint32_t digit = in ? wave[p] : 2 * kHubWaves;
+    const uint32_t peers = __match_any_sync(kFull, digit);
+    const uint32_t leader = (uint32_t)__ffs(peers) - 1u;
+    uint32_t at = 0;
+    if (in && lane == leader) at = atomicAdd(&h[digit], (uint32_t)__popc(peers));
+    at = __shfl_sync(kFull, at, leader) + __popc(peers & ((1u << lane) - 1u));
+    if (in) out[at] = pieces[p];
+  }
 }
 
 }  // namespace
@@ -2511,9 +2563,8 @@ Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, bool hubs) {
   if (hubs) {
     s.eflag_words = E / 32 + 2;
     s.eflag = ar.take<uint32_t>(s.eflag_words);
-    s.vinfo = ar.take<uint64_t>(n + 1);
-    s.save = ar.take<unsigned long long>(n + 1);
-    s.in_cnt = ar.take<uint32_t>(n + 1);
+    s.hub.info = ar.take<uint64_t>(n + 1);
+    s.hub.cur = ar.take<uint2>(n + 1);
     s.in_off = ar.take<uint32_t>(3 * (n + 1));
     s.inl_cap = E + 1;
     s.inl = ar.take<uint64_t>(s.inl_cap);
@@ -2541,31 +2592,30 @@ static void build_hubs(const GraphView& g, Schedule& s, cudaStream_t st) {
   // Candidates counted and savings summed in one pass (k_block_pieces zeroed
   // the counters); each hub accepted or not as a whole; its in-list sized by
   // its candidates, then filled.
-  k_hub_edges<0><<<eblocks, 256, 0, st>>>(g, s.variant_of, s.vinfo, s.save, s.eflag, s.in_cnt, s.in_off, s.inl,
-                                           nullptr, nullptr);
+  k_hub_edges<0><<<eblocks, 256, 0, st>>>(g, s.variant_of, s.hub, s.eflag, s.inl, nullptr, nullptr);
   TB_LAUNCH_CHECK();
-  k_hub_accept<<<vblocks, 256, 0, st>>>(s.vinfo, (uint32_t)n, s.save, s.in_cnt, s.in_off);
+  k_hub_accept<<<vblocks, 256, 0, st>>>(s.hub, (uint32_t)n, s.in_off);
   TB_LAUNCH_CHECK();
   device_scan<uint32_t, OpSum>(s.in_off, s.in_off, 3 * (n + 1), true, OpSum{}, 0u, s.hub_scan_tmp, st);
   const uint32_t waves = hub_waves(s.inl_cap - 1);
   uint64_t* pieces = waves == 1 ? s.hub_pieces : s.hub_pieces2;
+  k_hub_piece_scatter<<<vblocks, 256, 0, st>>>(s.in_off, (uint32_t)n, s.hub, pieces, s.piece_off,
+                                               waves == 1 ? nullptr : s.wave_cnt);
+  TB_LAUNCH_CHECK();
   if (waves > 1) {
     k_wave_bounds<<<1, kHubWaves + 1, 0, st>>>(g, waves, s.wave_lo, s.wave_bk, s.wave_cp);
     TB_LAUNCH_CHECK();
   }
   for (uint32_t w = 0; w < waves; ++w) {  // in-lists filled wave by wave: ordered by wave
-    k_hub_edges<1><<<eblocks, 256, 0, st>>>(g, s.variant_of, s.vinfo, s.save, s.eflag, s.in_cnt, s.in_off, s.inl,
-                                             s.hub_rows ? s.inrow : nullptr, waves == 1 ? nullptr : s.wave_lo + w);
+    k_hub_edges<1><<<eblocks, 256, 0, st>>>(g, s.variant_of, s.hub, s.eflag, s.inl, s.hub_rows ? s.inrow : nullptr,
+                                             waves == 1 ? nullptr : s.wave_lo + w);
     TB_LAUNCH_CHECK();
   }
-  k_hub_piece_scatter<<<std::max(vblocks, 1u), 256, 0, st>>>(s.in_off + n + 1, (uint32_t)n, pieces, s.piece_off,
-                                                             waves == 1 ? nullptr : s.wave_cnt);
-  TB_LAUNCH_CHECK();
   if (waves > 1) {
-    k_piece_waves<<<148 * 8, 256, 0, st>>>(s.hub_pieces2, s.piece_off, s.in_off, s.in_cnt, s.inl, s.wave_bk,
-                                            s.wave_cp, s.wave_cnt, s.piece_wave);
+    k_piece_waves<<<148 * 8, 256, 0, st>>>(s.hub_pieces2, s.piece_off, s.in_off, s.hub, s.inl, s.wave_bk, s.wave_cp,
+                                            s.wave_cnt, s.piece_wave);
     TB_LAUNCH_CHECK();
-    k_wave_scan<<<1, 1, 0, st>>>(s.wave_cnt, s.piece_off);
+    k_wave_scan<<<1, 32, 0, st>>>(s.wave_cnt, s.piece_off);
     TB_LAUNCH_CHECK();
     k_piece_wave_scatter<<<148 * 8, 256, 0, st>>>(s.hub_pieces2, s.piece_off, s.piece_wave, s.wave_cnt, s.hub_pieces);
     TB_LAUNCH_CHECK();
@@ -2577,7 +2627,7 @@ void build_pieces(const GraphView& g, Schedule& s, cudaStream_t st) {
   const uint32_t nrb = s.num_row_blocks;
   const unsigned wblocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div<uint64_t>(nrb, 8), 148ull * 16));
   HubInit hub{};
-  if (s.eflag && s.hubs) hub = HubInit{s.vinfo, s.save, s.in_cnt, s.eflag, s.eflag_words};
+  if (s.eflag && s.hubs) hub = HubInit{s.hub, s.eflag, s.eflag_words};
   k_block_pieces<<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.counts, s.piece_width, hub);
   TB_LAUNCH_CHECK();
   device_scan<uint64_t, OpSum>(s.counts, s.counts, (uint64_t)kPieceLists * nrb + 1, true, OpSum{}, 0ull, s.scan_tmp,
@@ -2651,7 +2701,7 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
     // One persistent kernel for the row pieces and the hub pass; the tiles and
     // the fallback rows (whose list k_queue fills) after it.
     k_queue<<<(unsigned)(sms * kHubCtasPerSm), kHubWarps * 32, 0, st>>>(
-        g, s.pieces, s.piece_off, stats, per_graph, s.piece_width, s.hub_pieces, s.in_off, s.in_cnt, s.inl);
+        g, s.pieces, s.piece_off, stats, per_graph, s.piece_width, s.hub_pieces, s.in_off, s.hub, s.inl);
     TB_LAUNCH_CHECK();
     if (s.tile_engine == TRIBIT_TILES_TCGEN05)
       k_tiles_tc<<<(unsigned)(sms * kTcCtasPerSm), kTcThreads, sizeof(TcSmem), st>>>(
@@ -2682,7 +2732,7 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
       g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, false, s.piece_width);
   TB_LAUNCH_CHECK();
   rows_wide();
-  k_hub<<<(unsigned)(sms * kHubCtasPerSm), kHubWarps * 32, 0, st>>>(g, s.hub_pieces, s.piece_off, s.in_off, s.in_cnt,
+  k_hub<<<(unsigned)(sms * kHubCtasPerSm), kHubWarps * 32, 0, st>>>(g, s.hub_pieces, s.piece_off, s.in_off, s.hub,
                                                                      s.inl, s.inrow, stats, per_graph, cfg.block_ns);
   TB_LAUNCH_CHECK();
   if (cfg.variant_stop) TB_CUDA(cudaEventRecord(cfg.variant_stop, st));

@@ -41,6 +41,17 @@ enum { kListHeavy = TRIBIT_NUM_VARIANTS, kListWide, kPieceLists };
 // pieces of each variant.
 enum { kOffHubCta = kPieceLists + 1, kOffHubAll, kOffHubEdges, kOffRowBlocks, kScheduleWords = kOffRowBlocks + TRIBIT_NUM_VARIANTS };
 
+// What the hub builder keeps of a vertex: its bit row, (blocks it spans << 32) |
+// length, 0 for a vertex that is no hub; and, apart from it (the row words are
+// only read while edges are walked, and stay in the L1), a pair of counters:
+// while candidates are counted, their number and the blocks their walks would
+// save; then the next place in its in-list for a bit-row tail (from the front)
+// and the last one taken for a column tail (from the back).
+struct HubTable {
+  uint64_t* info = nullptr;  // n + 1; null: no hub pass
+  uint2* cur = nullptr;      // n + 1
+};
+
 struct Schedule {
   uint32_t num_row_blocks = 0;
   uint8_t* variant_of = nullptr;   // device, per row block
@@ -53,9 +64,7 @@ struct Schedule {
   // Hub pass of the merge variant (absent when taken without hubs).
   uint32_t* eflag = nullptr;       // device, bit per CSR position: edge counted by the hub pass
   uint64_t eflag_words = 0;
-  uint64_t* vinfo = nullptr;       // device, n: (row span in blocks << 32) | bit-row length
-  unsigned long long* save = nullptr;  // device, n: blocks a hub walk would save
-  uint32_t* in_cnt = nullptr;      // device, n + 1
+  HubTable hub;                    // device
   uint32_t* in_off = nullptr;      // device, n + 1: in-list of hub v at [in_off[v], in_off[v+1]); then, from
                                    // n + 1 on, 2(n + 1) piece counts scanned with it (CTA, warp pieces)
   uint64_t* inl = nullptr;         // device: (first block of u's tail << 32) | tail length
@@ -63,7 +72,7 @@ struct Schedule {
   uint32_t* inrow = nullptr;       // device: u of each in-list entry (timing mode only: its own buffer)
   uint64_t* hub_pieces = nullptr;  // device: (v << 32) | first in-list entry; CTA pieces, then warp pieces
   uint64_t* hub_pieces2 = nullptr; // device: the pieces in hub order, before the wave sort
-  uint8_t* piece_wave = nullptr;   // device: wave of each piece's first tail
+  uint8_t* piece_wave = nullptr;   // device: digit of each piece (its list and the wave of its first tail)
   uint32_t* wave_lo = nullptr;     // device: first row of each wave, then n
   uint32_t* wave_bk = nullptr;     // device: bit-row start of each wave's first row
   uint32_t* wave_cp = nullptr;     // device: CSR position of each wave's first row
