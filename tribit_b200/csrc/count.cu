@@ -919,6 +919,7 @@ __global__ void __launch_bounds__(kTcThreads) k_tiles_tc(GraphView g, const uint
   TcSmem& sm = *reinterpret_cast<TcSmem*>(tc_raw);
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const uint32_t p0 = piece_off[TRIBIT_VARIANT_MMA], len = piece_off[TRIBIT_VARIANT_MMA + 1] - p0;
+  if (blockIdx.x >= len) return;  // a CTA a piece is enough, and most graphs have few
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&sm.mbar)), "r"(1u) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1844,14 +1845,16 @@ __global__ void __launch_bounds__(256) k_wide_work(GraphView g, uint32_t nrb, fl
 // loads in flight a lane, and a wide block's by all warps of the CTA: walked
 // row by row on one warp, the top ranks' blocks (32 long rows each) ran long
 // after the rest (RMAT-20: 341 us, now 192; RMAT-17 by id: 1,459, now 206).
-__global__ void __launch_bounds__(256) k_features(GraphView g, uint32_t nrb, int mode, float* __restrict__ feat,
+__global__ void __launch_bounds__(256, 5) k_features(GraphView g, uint32_t nrb, int mode, float* __restrict__ feat,
                                                   uint8_t* __restrict__ variant_of, int full, float tile_min_nnz,
                                                   float merge_ratio) {
   __shared__ uint64_t s_wb[8], s_wm[8];
   __shared__ uint32_t s_vmax[8], s_top[8], s_wide[8];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (uint32_t rb0 = blockIdx.x * 8; rb0 < nrb; rb0 += gridDim.x * 8) {
-    const uint32_t rb = rb0 + w;
+  // Warp k's block of a turn: neighbouring (and so similarly wide) blocks lie in different CTAs.
+  for (uint32_t turn = 0; (uint64_t)turn * gridDim.x * 8 < nrb; ++turn) {
+    auto block_of = [&](uint32_t k) { return (turn * 8 + k) * gridDim.x + blockIdx.x; };
+    const uint32_t rb = block_of(w);
     const uint32_t u = rb * 32 + lane;
     uint32_t d = 0, nbu = 0, lo = 0xFFFFFFFFu, hi = 0, start = 0;
     if (rb < nrb && u < g.n) {
@@ -1883,7 +1886,7 @@ __global__ void __launch_bounds__(256) k_features(GraphView g, uint32_t nrb, int
         for (uint32_t k = 0; k < 8; ++k) wides |= s_wide[k] << k;
         for (uint32_t k = 0; k < 8; ++k) {
           if (!((wides >> k) & 1u)) continue;
-          const uint32_t uk = (rb0 + k) * 32 + lane;
+          const uint32_t uk = block_of(k) * 32 + lane;
           uint32_t sk = 0, dk = 0;
           if (uk < g.n) {
             sk = rp_row(g.rp[uk]);
@@ -2020,13 +2023,21 @@ __device__ uint32_t tile_pieces(const GraphView& g, uint32_t rb, uint32_t* vm) {
   if (hi - lo + 1 > (uint32_t)kTileMaxK) return 1u;
   for (uint32_t i = lane; i < (uint32_t)kTileMaxK; i += 32) vm[i] = 0u;
   __syncwarp();
-  for (uint32_t r = 0; r < 32; ++r) {
-    if (!((amask >> r) & 1u)) continue;
-    const uint32_t rbs = __shfl_sync(kFull, bs, r), rbe = __shfl_sync(kFull, be, r);
-    for (uint32_t k = rbs + lane; k < rbe; k += 32) {
+  // The active rows' entries, which lie together but for rows of one neighbour
+  // and heavy ones: walked flat between the inactive rows.
+  const uint32_t gaps = __ballot_sync(kFull, !active && be > bs);
+  for (uint32_t r = 0; r < 32;) {
+    const uint32_t on = amask >> r;
+    if (!on) break;
+    r += (uint32_t)__ffs(on) - 1u;                                     // the run's first row
+    const uint32_t stop = gaps >> r, n = stop ? (uint32_t)__ffs(stop) - 1u : 32u - r;  // rows up to the next gap
+    const uint32_t lastr = 31u - (uint32_t)__clz(amask & (r + n == 32 ? kFull : (1u << (r + n)) - 1u));
+    const uint32_t k0 = __shfl_sync(kFull, bs, r), k1 = __shfl_sync(kFull, be, lastr);
+    for (uint32_t k = k0 + lane; k < k1; k += 32) {
       const uint64_t e = g.bent[k];
       atomicOr(&vm[(uint32_t)(e >> 32) - lo], (uint32_t)e);
     }
+    r += n;
   }
   __syncwarp();
   uint32_t c = 0;

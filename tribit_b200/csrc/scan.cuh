@@ -129,55 +129,60 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const T* in, T* out
   }
 }
 
-// A scan of a few tiles by one CTA, tile after tile: one launch in the place
-// of three, whose gaps cost more than the other CTAs save.
+// A scan of up to kScanOneMax bytes by one CTA: one launch in the place of three,
+// whose gaps cost more than the other CTAs save. A warp takes a contiguous 32nd,
+// all of its loads in flight at once.
 constexpr int kScanOneThreads = 1024;
-constexpr int kScanOneItems = 8;
-constexpr uint64_t kScanOneMax = 4ull * kScanOneThreads * kScanOneItems;
+constexpr uint64_t kScanOneMax = 128 * 1024;  // bytes: 32 words of 4 bytes a thread, 16 of 8
 template <typename T, typename Op, bool Rev>
 __global__ void __launch_bounds__(kScanOneThreads) k_scan_one(const T* in, T* out, T* out2, uint64_t n, Op op, T id,
                                                               bool exclusive) {
+  constexpr int kItems = kScanOneMax / sizeof(T) / kScanOneThreads;
   __shared__ T warp_tot[kScanOneThreads / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  T carry = id;
-  for (uint64_t base = 0; base < n; base += kScanOneThreads * kScanOneItems) {
-    const uint64_t i0 = base + (uint64_t)threadIdx.x * kScanOneItems;
-    T v[kScanOneItems];
-    T acc = id;
+  const int items = (int)((n + kScanOneThreads - 1) / kScanOneThreads);  // a warp's rounds of 32
+  const uint64_t base = (uint64_t)w * items * 32 + lane;
+  T v[kItems];
+  T run = id;  // the warp's elements of the rounds before
 #pragma unroll
-    for (int k = 0; k < kScanOneItems; ++k) v[k] = i0 + k < n ? in[scan_index<Rev>(i0 + k, n)] : id;
+  for (int k = 0; k < kItems; ++k) {
+    const uint64_t i = base + k * 32;
+    v[k] = k < items && i < n ? in[scan_index<Rev>(i, n)] : id;
+  }
 #pragma unroll
-    for (int k = 0; k < kScanOneItems; ++k) acc = op(acc, v[k]);
-    T inc = acc;
+  for (int k = 0; k < kItems; ++k) {
+    if (k >= items) break;
+    T inc = v[k];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const T t = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= o) inc = op(t, inc);
     }
-    if (lane == 31) warp_tot[w] = inc;
-    __syncthreads();
-    T x = warp_tot[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const T t = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x = op(t, x);
+    const T tot = __shfl_sync(0xffffffffu, inc, 31);
+    if (exclusive) {
+      inc = __shfl_up_sync(0xffffffffu, inc, 1);
+      if (lane == 0) inc = id;
     }
-    T pre = carry;
-    const T before = __shfl_sync(0xffffffffu, x, w == 0 ? 0 : w - 1);
-    if (w > 0) pre = op(pre, before);
-    const T ex = __shfl_up_sync(0xffffffffu, inc, 1);
-    if (lane > 0) pre = op(pre, ex);
-    carry = op(carry, __shfl_sync(0xffffffffu, x, 31));
+    v[k] = op(run, inc);
+    run = op(run, tot);
+  }
+  if (lane == 0) warp_tot[w] = run;
+  __syncthreads();
+  T x = warp_tot[lane];
 #pragma unroll
-    for (int k = 0; k < kScanOneItems; ++k) {
-      const T nxt = op(pre, v[k]);
-      if (i0 + k < n) {
-        out[scan_index<Rev>(i0 + k, n)] = exclusive ? pre : nxt;
-        if (out2) out2[scan_index<Rev>(i0 + k, n)] = exclusive ? pre : nxt;
-      }
-      pre = nxt;
+  for (int o = 1; o < 32; o <<= 1) {
+    const T t = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x = op(t, x);
+  }
+  const T before = __shfl_sync(0xffffffffu, x, w == 0 ? 0 : w - 1);
+#pragma unroll
+  for (int k = 0; k < kItems; ++k) {
+    const uint64_t i = base + k * 32;
+    if (k < items && i < n) {
+      const T y = w > 0 ? op(before, v[k]) : v[k];
+      out[scan_index<Rev>(i, n)] = y;
+      if (out2) out2[scan_index<Rev>(i, n)] = y;
     }
-    __syncthreads();  // warp_tot is rewritten for the next tile
   }
 }
 
@@ -200,7 +205,7 @@ void device_scan(const T* in, T* out, uint64_t n, bool exclusive, Op op, T id, T
     TB_LAUNCH_CHECK();
     return;
   }
-  if (n <= kScanOneMax) {
+  if (n * sizeof(T) <= kScanOneMax) {
     k_scan_one<T, Op, Rev><<<1, kScanOneThreads, 0, st>>>(in, out, out2, n, op, id, exclusive);
     TB_LAUNCH_CHECK();
     return;
