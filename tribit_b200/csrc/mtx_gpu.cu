@@ -25,6 +25,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstring>
 #include <thread>
@@ -240,21 +241,34 @@ struct FileMap {
   }
 };
 
-// Reads [off, off + len) of the file into dst with up to kReadThreads threads.
-bool read_piece(int fd, char* dst, uint64_t off, size_t len) {
+// Reads [off, off + len) of the file into dst with up to kReadThreads threads,
+// each its share in chunks of kReadChunk, and calls done(chunk's offset, bytes)
+// on the reading thread as each chunk lands. False when a read fails or done
+// returns false.
+constexpr size_t kReadChunk = 512u << 10;
+template <class Done>
+bool read_piece(int fd, char* dst, uint64_t off, size_t len, const Done& done) {
   const int nt = (int)std::max<size_t>(1, std::min<size_t>(kReadThreads, len >> 20));
   std::vector<std::thread> th;
   std::vector<char> ok(nt, 1);
   const size_t share = (len + nt - 1) / nt;
   auto work = [&](int k) {
-    size_t a = k * share, b = std::min(len, a + share);
-    while (a < b) {
-      const ssize_t r = pread(fd, dst + a, b - a, (off_t)(off + a));
-      if (r <= 0) {
+    const size_t b = std::min(len, (k + 1) * share);
+    for (size_t a = std::min(len, k * share); a < b;) {
+      const size_t e = std::min(b, a + kReadChunk);
+      for (size_t at = a; at < e;) {
+        const ssize_t r = pread(fd, dst + at, e - at, (off_t)(off + at));
+        if (r <= 0) {
+          ok[k] = 0;
+          return;
+        }
+        at += (size_t)r;
+      }
+      if (!done(a, e - a)) {
         ok[k] = 0;
         return;
       }
-      a += (size_t)r;
+      a = e;
     }
   };
   for (int k = 1; k < nt; ++k) th.emplace_back(work, k);
@@ -335,23 +349,32 @@ tribit_status tribit_load_mtx(tribit_context* c, const char* path, uint64_t* num
     TB_CUDA(cudaMemsetAsync(text + B, '\n', text_bytes - B, s));
     if (!c->pinned[0])
       for (auto& p : c->pinned) TB_CUDA(cudaMallocHost(&p, tb::kPinnedPiece));
-    // Pieces of the body: read into pinned buffer k & 1 while the previous
-    // piece's copy runs; a buffer is refilled once its copy has finished.
+    // Pieces of the body: read into pinned buffer k & 1, each chunk copied to the
+    // device by the thread that read it (so that reading and copying overlap within
+    // a piece: a 13 MB file 2,040 -> 1,693 us a call); a buffer is refilled once
+    // its copies have finished.
     TB_CUDA(cudaEventRecord(c->upload_ev[0], s));
     TB_CUDA(cudaStreamWaitEvent(c->copy_st, c->upload_ev[0], 0));
     bool io_ok = true;
+    std::atomic<cudaError_t> copy_err{cudaSuccess};
     uint64_t k = 0;
     for (uint64_t at = 0; at < B; at += tb::kPinnedPiece, ++k) {
       const size_t len = (size_t)std::min<uint64_t>(tb::kPinnedPiece, B - at);
       const int b = (int)(k & 1);
       char* buf = static_cast<char*>(c->pinned[b]);
       tb::pinned_wait(c, b);
-      if (!tb::read_piece(f.fd, buf, off0 + at, len)) {
+      const bool read = tb::read_piece(f.fd, buf, off0 + at, len, [&](size_t o, size_t bytes) {
+        cudaError_t e = cudaSetDevice(c->device);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(text + at + o, buf + o, bytes, cudaMemcpyHostToDevice, c->copy_st);
+        if (e != cudaSuccess) copy_err = e;
+        return e == cudaSuccess;
+      });
+      tb::pinned_used(c, b, c->copy_st);  // also after a failure: some copies may be queued
+      TB_CUDA(copy_err.load());
+      if (!read) {
         io_ok = false;
         break;
       }
-      TB_CUDA(cudaMemcpyAsync(text + at, buf, len, cudaMemcpyHostToDevice, c->copy_st));
-      tb::pinned_used(c, b, c->copy_st);
     }
     TB_CUDA(cudaEventRecord(c->upload_ev[3], c->copy_st));
     TB_CUDA(cudaStreamWaitEvent(s, c->upload_ev[3], 0));
