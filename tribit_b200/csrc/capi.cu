@@ -50,7 +50,7 @@ void layout(tribit_context* c, bool measure, const tb::PrepInput& in, bool stage
   // Measuring: walk the same takes prepare_graph / take_schedule will do.
   tb::Prepared tmp;
   tb::prepare_graph(ar, pin, c->st, &tmp);
-  (void)tb::take_schedule(ar, in.n, in.E);
+  (void)tb::take_schedule(ar, in.n, in.E, nullptr);
 }
 
 // Runs preprocessing + schedule (+ counting when count == true) for one input.
@@ -93,7 +93,7 @@ void run_call(tribit_context* c, tb::PrepInput in, const uint64_t* host_entries,
   }
   tb::drop_graph(c);
   tb::prepare_graph(c->arena, pin, st, &c->prep);
-  c->sched = tb::take_schedule(c->arena, in.n, in.E);
+  c->sched = tb::take_schedule(c->arena, in.n, in.E, c->prep.stats);
   tb::apply_dispatch(c, st);
   c->per_graph = L.per_graph;
   c->num_graphs = G;
@@ -152,12 +152,11 @@ void count_device_input(tribit_context* c, const uint64_t* d_entries, uint64_t E
 
 void read_stats(tribit_context* c, cudaStream_t st) {
   TB_CUDA(cudaMemcpyAsync(c->h_stats, c->prep.stats, sizeof(DeviceStats), cudaMemcpyDeviceToHost, st));
-  TB_CUDA(cudaMemcpyAsync(c->h_sched, c->sched.piece_off, kScheduleWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
 }
 
 void fill_schedule_stats(const tribit_context* c, tribit_result* res) {
-  const uint32_t* lens = c->h_sched + kOffRowBlocks;
-  res->hub_edges = c->h_sched[kOffHubEdges];
+  const uint32_t* lens = c->h_stats->sched + kOffRowBlocks;
+  res->hub_edges = c->h_stats->sched[kOffHubEdges];
   res->row_blocks = 0;
   for (int v = 0; v < TRIBIT_NUM_VARIANTS; ++v) {
     res->row_blocks_by_variant[v] = lens[v];
@@ -227,8 +226,7 @@ tribit_status tribit_create(const tribit_options* opts, tribit_context** out) {
     TB_CUDA(cudaStreamCreateWithFlags(&c->copy_st, cudaStreamNonBlocking));
     for (auto& e : c->upload_ev) TB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto& e : c->pinned_ev) TB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    TB_CUDA(cudaMallocHost(&c->h_stats, sizeof(tb::DeviceStats) + tb::kScheduleWords * sizeof(uint32_t)));
-    c->h_sched = reinterpret_cast<uint32_t*>(c->h_stats + 1);
+    TB_CUDA(cudaMallocHost(&c->h_stats, sizeof(tb::DeviceStats)));
   });
   if (st != TRIBIT_OK) {
     tribit_destroy(c);

@@ -28,7 +28,6 @@ struct tribit_context {
   cudaStream_t copy_st = nullptr;                       // host uploads (overlapped with the degree pass)
   cudaEvent_t upload_ev[tb::kUploadChunks + 1] = {};
   tb::DeviceStats* h_stats = nullptr;  // pinned
-  uint32_t* h_sched = nullptr;         // pinned, after h_stats: the schedule's kScheduleWords
   // Tuned launch parameters (tribit_set_tuning / tribit_autotune).
   int ctas_per_sm = 0;
   uint32_t piece_width = 64;
@@ -112,8 +111,7 @@ size_t call_bytes(tribit_context* c, uint64_t E, uint64_t n, int order, bool sta
 // dispatcher (tribit_count_edges_device with an explicit order).
 void count_device_input(tribit_context* c, const uint64_t* d_entries, uint64_t E, uint64_t n, int order,
                         tribit_result* res);
-// Queues the copy of the device's counters and schedule words to h_stats and
-// h_sched; once it is done, fill_schedule_stats gives result.row_blocks,
+// Queues the copy of the device's counters to h_stats; once it is done, fill_schedule_stats gives result.row_blocks,
 // row_blocks_by_variant and hub_edges.
 void read_stats(tribit_context* c, cudaStream_t st);
 void fill_schedule_stats(const tribit_context* c, tribit_result* res);

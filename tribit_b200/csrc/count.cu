@@ -403,6 +403,16 @@ struct PiecesShared {
   uint32_t* s_row;
 };
 
+// A worker's next pieces of a list of len, `grab` at a time: of a list that one
+// turn of all `workers` covers, a fixed share (no worker waits for a cursor that
+// thousands of others update; a graph of 1,000 vertices spent a third of its
+// count there), else from the cursor. One thread calls it; `turn` counts calls.
+__device__ __forceinline__ uint32_t next_pieces(unsigned int* cursor, uint32_t len, uint32_t worker, uint32_t workers,
+                                                uint32_t grab, uint32_t turn) {
+  if (len <= (uint64_t)workers * grab) return turn == 0 ? worker * grab : len;
+  return atomicAdd(cursor, grab);
+}
+
 // The row-piece variant V over its pieces (and, with `heavy`, first the heavy
 // pieces, one CTA per piece); returns this thread's partial count.
 template <int V>
@@ -425,8 +435,8 @@ __device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64
     uint64_t* ctbl = sh.smem;
     uint32_t* pre = reinterpret_cast<uint32_t*>(sh.smem) + kHeavyMaxSpan;
     const uint32_t h0 = piece_off[kListHeavy], hlen = piece_off[kListHeavy + 1] - h0;
-    for (;;) {
-      if (threadIdx.x == 0) s_row = atomicAdd(&stats->cursor[kCurHeavy], 1u);
+    for (uint32_t turn = 0;; ++turn) {
+      if (threadIdx.x == 0) s_row = next_pieces(&stats->cursor[kCurHeavy], hlen, blockIdx.x, gridDim.x, 1, turn);
       __syncthreads();
       const uint32_t t = s_row;
       if (t >= hlen) break;
@@ -518,9 +528,11 @@ __device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64
   int logb = 0;
   uint32_t bmin = 0, bmax = 0, d = 0;
   uint32_t* wmap = reinterpret_cast<uint32_t*>(tbl);  // the slice as a direct-mapped row
-  for (;;) {
+  for (uint32_t turn = 0;; ++turn) {
     uint32_t t0 = 0;
-    if (lane == 0) t0 = atomicAdd(&stats->cursor[kCurVariant0 + V], kGrab);
+    if (lane == 0)
+      t0 = next_pieces(&stats->cursor[kCurVariant0 + V], len, w * gridDim.x + blockIdx.x, kWarpsPerCta * gridDim.x,
+                       kGrab, turn);
     t0 = __shfl_sync(kFull, t0, 0);
     if (t0 >= len) break;
     const uint32_t t1 = min(t0 + kGrab, len);
@@ -1549,8 +1561,8 @@ __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t*
   const uint32_t wlen = piece_off[kOffHubAll] - len;
   uint64_t acc = 0;
   // Phase 1: hubs with wide rows, one CTA per piece.
-  for (;;) {
-    if (threadIdx.x == 0) s_t = atomicAdd(&stats->cursor[kCurHub], 1u);
+  for (uint32_t turn = 0;; ++turn) {
+    if (threadIdx.x == 0) s_t = next_pieces(&stats->cursor[kCurHub], len, blockIdx.x, gridDim.x, 1, turn);
     __syncthreads();
     const uint32_t t = s_t;
     if (t >= len) break;
@@ -1636,9 +1648,12 @@ __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t*
   // Phase 2: hubs whose row fits a warp's slice of the map, one warp per
   // piece, in wave order.
   uint32_t* wmap = map + w * kHubWarpStride;
-  for (;;) {
+  for (uint32_t turn = 0;; ++turn) {
     uint32_t t0 = 0;
-    if (lane == 0) t0 = atomicAdd(&stats->cursor[kCurHubWarp], 1u);
+    // (From the last CTA on: the first ones have the CTA pieces of a small graph.)
+    if (lane == 0)
+      t0 = next_pieces(&stats->cursor[kCurHubWarp], wlen, w * gridDim.x + gridDim.x - 1 - blockIdx.x,
+                       kHubWarps * gridDim.x, 1, turn);
     const uint32_t t = __shfl_sync(kFull, t0, 0);
     if (t >= wlen) break;
     const unsigned long long t_start = block_ns ? cycles() : 0ull;
@@ -2091,13 +2106,38 @@ __global__ void __launch_bounds__(256) k_block_pieces(GraphView g, uint32_t nrb,
   }
 }
 
-// After the scan of counts: every list's pieces, in (list, row) order, and
-// piece_off. The hub words of piece_off start at 0.
+// Up to this many counts every CTA of k_piece_scatter scans them itself (10 a
+// thread), a launch less.
+constexpr uint32_t kScatterScan = 2560;
+
+// After the scan of counts (Scan: doing it): every list's pieces, in (list,
+// row) order, and piece_off. The hub words of piece_off start at 0.
+template <bool Scan>
 __global__ void __launch_bounds__(256) k_piece_scatter(GraphView g, uint32_t nrb,
                                                        const uint8_t* __restrict__ variant_of,
-                                                       const uint64_t* __restrict__ counts,
+                                                       const uint64_t* __restrict__ counts_in,
                                                        uint32_t* __restrict__ piece_off, uint64_t* __restrict__ pieces,
                                                        uint32_t width) {
+  __shared__ uint64_t s_counts[Scan ? kScatterScan + 1 : 1];
+  const uint64_t* counts = counts_in;
+  if constexpr (Scan) {
+    constexpr uint32_t kItems = kScatterScan / 256;
+    const uint32_t n = kPieceLists * nrb;
+    for (uint32_t i = threadIdx.x; i < kScatterScan; i += 256) s_counts[i] = i < n ? counts_in[i] : 0ull;
+    __syncthreads();
+    uint64_t v[kItems], sum = 0, tot;
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; ++k) sum += v[k] = s_counts[threadIdx.x * kItems + k];
+    uint64_t pre = block_exclusive_scan<uint64_t>(sum, OpSum{}, 0ull, &tot);
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; ++k) {
+      s_counts[threadIdx.x * kItems + k] = pre;
+      pre += v[k];
+    }
+    if (threadIdx.x == 0) s_counts[kScatterScan] = tot;
+    __syncthreads();
+    counts = s_counts;  // from the last count on, every entry is the total
+  }
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -2382,26 +2422,85 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
 // in-list, and its row words are cleared so that mode 1 takes none of its edges.
 // cnt: the in-list lengths, then the pieces of each hub for a CTA and for a
 // warp, n + 1 of each (0 at the ends), to be scanned as one array.
+__device__ __forceinline__ void hub_accept(const HubTable& hub, uint32_t v, uint32_t& k, uint32_t& c, uint32_t& wc) {
+  const uint64_t vi = hub.info[v];
+  const uint2 c2 = hub.cur[v];
+  const uint32_t span = (uint32_t)(vi >> 32), nb = (uint32_t)vi;
+  k = c2.y >= hub_cost(span, nb) ? c2.x : 0u;
+  // The warp stages the row when its direct map fits the warp's slice, or,
+  // for a row too wide for the CTA's direct map, when its hash does.
+  const bool warp = span <= kHubWarpSpan || (span > kHubMaxSpan && nb <= kHubWarpHash);
+  wc = warp ? (k + kHubWarpPiece - 1) / kHubWarpPiece : 0u;
+  c = warp ? 0u : (k + kHubPiece - 1) / kHubPiece;
+}
+
 __global__ void k_hub_accept(HubTable hub, uint32_t n, uint32_t* __restrict__ cnt) {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v > n) return;
   uint32_t k = 0, c = 0, wc = 0;
   if (v < n) {
-    const uint64_t vi = hub.info[v];
-    const uint2 c2 = hub.cur[v];
-    const uint32_t span = (uint32_t)(vi >> 32), nb = (uint32_t)vi;
-    k = c2.y >= hub_cost(span, nb) ? c2.x : 0u;
+    hub_accept(hub, v, k, c, wc);
     if (k == 0) hub.info[v] = 0;  // no candidate in mode 1
-    // The warp stages the row when its direct map fits the warp's slice, or,
-    // for a row too wide for the CTA's direct map, when its hash does.
-    if (span <= kHubWarpSpan || (span > kHubMaxSpan && nb <= kHubWarpHash))
-      wc = (k + kHubWarpPiece - 1) / kHubWarpPiece;
-    else
-      c = (k + kHubPiece - 1) / kHubPiece;
   }
   cnt[v] = k;
   cnt[(uint64_t)n + 1 + v] = c;
   cnt[2 * ((uint64_t)n + 1) + v] = wc;
+}
+
+// k_hub_accept, the scan and k_hub_piece_scatter for a graph of few vertices, in
+// one CTA: a warp takes a contiguous 32nd, sums it, then places it.
+constexpr uint32_t kHubOneMax = 16384;
+__global__ void __launch_bounds__(1024) k_hub_accept_one(HubTable hub, uint32_t n, uint32_t* __restrict__ in_off,
+                                                         uint64_t* __restrict__ pieces,
+                                                         uint32_t* __restrict__ piece_off) {
+  __shared__ uint32_t s_k[32], s_c[32], s_w[32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t rounds = (n + 1023) / 1024, v0 = w * rounds * 32;
+  uint32_t sk = 0, sc = 0, sw = 0;
+  for (uint32_t r = 0; r < rounds; ++r) {
+    const uint32_t v = v0 + r * 32 + lane;
+    uint32_t k = 0, c = 0, wc = 0;
+    if (v < n) hub_accept(hub, v, k, c, wc);
+    sk += k;
+    sc += c;
+    sw += wc;
+  }
+  sk = __reduce_add_sync(kFull, sk);
+  sc = __reduce_add_sync(kFull, sc);
+  sw = __reduce_add_sync(kFull, sw);
+  if (lane == 0) {
+    s_k[w] = sk;
+    s_c[w] = sc;
+    s_w[w] = sw;
+  }
+  __syncthreads();
+  const uint32_t ik = warp_inclusive_sum(s_k[lane]), ic = warp_inclusive_sum(s_c[lane]),
+                 iw = warp_inclusive_sum(s_w[lane]);
+  const uint32_t tk = __shfl_sync(kFull, ik, 31), tc = __shfl_sync(kFull, ic, 31), tw = __shfl_sync(kFull, iw, 31);
+  uint32_t ak = __shfl_sync(kFull, ik, w) - sk, ac = __shfl_sync(kFull, ic, w) - sc,
+           aw = tc + __shfl_sync(kFull, iw, w) - sw;  // warp pieces follow the CTA pieces
+  if (threadIdx.x == 0) {
+    in_off[n] = tk;
+    piece_off[kOffHubCta] = tc;
+    piece_off[kOffHubAll] = tc + tw;
+    piece_off[kOffHubEdges] = tk;
+  }
+  for (uint32_t r = 0; r < rounds; ++r) {
+    const uint32_t v = v0 + r * 32 + lane;
+    uint32_t k = 0, c = 0, wc = 0;
+    if (v < n) hub_accept(hub, v, k, c, wc);
+    const uint32_t jk = warp_inclusive_sum(k), jc = warp_inclusive_sum(c), jw = warp_inclusive_sum(wc);
+    if (v < n) {
+      if (k == 0) hub.info[v] = 0;
+      in_off[v] = ak + jk - k;
+      hub.cur[v] = make_uint2(ak + jk - k, ak + jk);
+      for (uint32_t q = 0; q < c; ++q) pieces[ac + jc - c + q] = ((uint64_t)v << 32) | (q * kHubPiece);
+      for (uint32_t q = 0; q < wc; ++q) pieces[aw + jw - wc + q] = ((uint64_t)v << 32) | (q * kHubWarpPiece);
+    }
+    ak += __shfl_sync(kFull, jk, 31);
+    ac += __shfl_sync(kFull, jc, 31);
+    aw += __shfl_sync(kFull, jw, 31);
+  }
 }
 
 // After the scan: the ends of every hub's empty in-list in its counters, the
@@ -2558,14 +2657,14 @@ __global__ void __launch_bounds__(256) k_piece_wave_scatter(const uint64_t* __re
 
 }  // namespace
 
-Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, bool hubs) {
+Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, DeviceStats* stats, bool hubs) {
   Schedule s;
   const uint32_t nrb = (uint32_t)ceil_div<uint64_t>(n, 32);
   s.num_row_blocks = nrb;
   s.variant_of = ar.take<uint8_t>(nrb + 1);
   s.piece_cap = 2 * n + E / kMinPieceWidth + 64;  // row pieces, plus up to 16 per bit-tile block
   s.pieces = ar.take<uint64_t>(s.piece_cap);
-  s.piece_off = ar.take<uint32_t>(kScheduleWords);
+  s.piece_off = stats ? stats->sched : nullptr;
   s.counts = ar.take<uint64_t>((uint64_t)kPieceLists * nrb + 1);
   s.scan_tmp = take_scan_temp<uint64_t>(ar, (uint64_t)kPieceLists * nrb + 1);
   s.features = ar.take<float>((uint64_t)nrb * kNumFeatures + 1);
@@ -2603,14 +2702,18 @@ static void build_hubs(const GraphView& g, Schedule& s, cudaStream_t st) {
   // its candidates, then filled.
   k_hub_edges<0><<<eblocks, 256, 0, st>>>(g, s.variant_of, s.hub, s.eflag, s.inl, nullptr, nullptr);
   TB_LAUNCH_CHECK();
-  k_hub_accept<<<vblocks, 256, 0, st>>>(s.hub, (uint32_t)n, s.in_off);
-  TB_LAUNCH_CHECK();
-  device_scan<uint32_t, OpSum>(s.in_off, s.in_off, 3 * (n + 1), true, OpSum{}, 0u, s.hub_scan_tmp, st);
   const uint32_t waves = hub_waves(s.inl_cap - 1);
-  uint64_t* pieces = waves == 1 ? s.hub_pieces : s.hub_pieces2;
-  k_hub_piece_scatter<<<vblocks, 256, 0, st>>>(s.in_off, (uint32_t)n, s.hub, pieces, s.piece_off,
-                                               waves == 1 ? nullptr : s.wave_cnt);
-  TB_LAUNCH_CHECK();
+  if (waves == 1 && n <= kHubOneMax) {
+    k_hub_accept_one<<<1, 1024, 0, st>>>(s.hub, (uint32_t)n, s.in_off, s.hub_pieces, s.piece_off);
+    TB_LAUNCH_CHECK();
+  } else {
+    k_hub_accept<<<vblocks, 256, 0, st>>>(s.hub, (uint32_t)n, s.in_off);
+    TB_LAUNCH_CHECK();
+    device_scan<uint32_t, OpSum>(s.in_off, s.in_off, 3 * (n + 1), true, OpSum{}, 0u, s.hub_scan_tmp, st);
+    k_hub_piece_scatter<<<vblocks, 256, 0, st>>>(s.in_off, (uint32_t)n, s.hub, waves == 1 ? s.hub_pieces : s.hub_pieces2,
+                                                 s.piece_off, waves == 1 ? nullptr : s.wave_cnt);
+    TB_LAUNCH_CHECK();
+  }
   if (waves > 1) {
     k_wave_bounds<<<1, kHubWaves + 1, 0, st>>>(g, waves, s.wave_lo, s.wave_bk, s.wave_cp);
     TB_LAUNCH_CHECK();
@@ -2639,9 +2742,14 @@ void build_pieces(const GraphView& g, Schedule& s, cudaStream_t st) {
   if (s.eflag && s.hubs) hub = HubInit{s.hub, s.eflag, s.eflag_words};
   k_block_pieces<<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.counts, s.piece_width, hub);
   TB_LAUNCH_CHECK();
-  device_scan<uint64_t, OpSum>(s.counts, s.counts, (uint64_t)kPieceLists * nrb + 1, true, OpSum{}, 0ull, s.scan_tmp,
-                               st);
-  k_piece_scatter<<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.counts, s.piece_off, s.pieces, s.piece_width);
+  if ((uint64_t)kPieceLists * nrb <= kScatterScan) {
+    k_piece_scatter<true><<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.counts, s.piece_off, s.pieces, s.piece_width);
+  } else {
+    device_scan<uint64_t, OpSum>(s.counts, s.counts, (uint64_t)kPieceLists * nrb + 1, true, OpSum{}, 0ull, s.scan_tmp,
+                                 st);
+    k_piece_scatter<false><<<wblocks, 256, 0, st>>>(g, nrb, s.variant_of, s.counts, s.piece_off, s.pieces,
+                                                    s.piece_width);
+  }
   TB_LAUNCH_CHECK();
   build_hubs(g, s, st);
 }

@@ -39,7 +39,8 @@ enum { kListHeavy = TRIBIT_NUM_VARIANTS, kListWide, kPieceLists };
 // piece_off: where each list starts in `pieces` (and where the last ends), the
 // hub pass's CTA pieces, all its pieces and its edges, then the row blocks with
 // pieces of each variant.
-enum { kOffHubCta = kPieceLists + 1, kOffHubAll, kOffHubEdges, kOffRowBlocks, kScheduleWords = kOffRowBlocks + TRIBIT_NUM_VARIANTS };
+enum { kOffHubCta = kPieceLists + 1, kOffHubAll, kOffHubEdges, kOffRowBlocks };
+static_assert(kOffRowBlocks + TRIBIT_NUM_VARIANTS == kScheduleWords, "piece_off's words in DeviceStats");
 
 // What the hub builder keeps of a vertex: its bit row, (blocks it spans << 32) |
 // length, 0 for a vertex that is no hub; and, apart from it (the row words are
@@ -57,7 +58,7 @@ struct Schedule {
   uint8_t* variant_of = nullptr;   // device, per row block
   uint64_t* pieces = nullptr;      // device, (row << 32) | first neighbour, one segment per piece list
   uint64_t piece_cap = 0;
-  uint32_t* piece_off = nullptr;   // device, kScheduleWords words (see there)
+  uint32_t* piece_off = nullptr;   // device, kScheduleWords words in DeviceStats (see kOff*)
   uint64_t* counts = nullptr;      // device, kPieceLists * nrb + 1: pieces per (list, row block), scanned
   uint64_t* scan_tmp = nullptr;
   float* features = nullptr;       // device, nrb x kNumFeatures
@@ -106,8 +107,9 @@ struct CountConfig {
 // 3-5% slower (5 CTAs an SM for the row pieces instead of 6-7).
 constexpr uint64_t kQueueMaxEntries = 1ull << 24;
 
-// hubs: also take the hub-pass arrays (about 13 bytes per entry).
-Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, bool hubs = true);
+// hubs: also take the hub-pass arrays (about 13 bytes per entry). stats: the
+// prepared graph's, which holds the schedule's words (null when measuring).
+Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, DeviceStats* stats, bool hubs = true);
 
 // Computes row-block features, the per-block variant (mode: TRIBIT_DISPATCH_*),
 // and the per-variant piece lists. full_features adds the neighbour-side

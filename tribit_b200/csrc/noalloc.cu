@@ -108,7 +108,7 @@ extern "C" tribit_status tribit_count_edges_noalloc(const uint64_t* d_entries, u
       ar.begin(true);
       tb::Prepared probe;
       tb::prepare_graph(ar, in, st, &probe);
-      (void)tb::take_schedule(ar, num_nodes, n_entries, hubs);
+      (void)tb::take_schedule(ar, num_nodes, n_entries, nullptr, hubs);
       if (!hubs || ar.used() <= kNoAllocScratchBytes) break;
       hubs = false;
     }
@@ -116,7 +116,7 @@ extern "C" tribit_status tribit_count_edges_noalloc(const uint64_t* d_entries, u
     ar.begin(false);
     tb::Prepared prep;
     tb::prepare_graph(ar, in, st, &prep);
-    tb::Schedule sched = tb::take_schedule(ar, num_nodes, n_entries, hubs);
+    tb::Schedule sched = tb::take_schedule(ar, num_nodes, n_entries, prep.stats, hubs);
     tb::build_schedule(prep.view, sched, TRIBIT_DISPATCH_PLAIN, hubs, st);
     tb::CountConfig cfg;
     cfg.num_sms = sms;

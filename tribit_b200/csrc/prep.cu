@@ -224,6 +224,7 @@ struct RowWords {
   uint32_t* w;
   uint64_t count;
   bool slots;
+  uint32_t* off;  // slots, up to kRankOneMax vertices: the slots' starts, also to w (else null)
 };
 
 // rank[id] = position, and the row words.
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_one(const uint32_t* __res
   uint32_t* dst = rank_sm + kRankOneMax;
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   uint32_t* wcnt = rank_sm + 2 * kRankOneMax;  // [warp][digit]
-  for (uint64_t i = n + tid; i < rw.count; i += kRankThreads) rw.w[i] = 0;
+  for (uint64_t i = n + (rw.off ? 1 : 0) + tid; i < rw.count; i += kRankThreads) rw.w[i] = 0;
   for (uint32_t i = tid; i < n; i += kRankThreads) src[i] = (degree_key(deg[i], dk) << 16) | i;
   const uint32_t rounds = (n + kRankThreads - 1) / kRankThreads;  // of 32 a warp
   for (int shift = 16; shift < 32; shift += 8) {
@@ -307,11 +308,42 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_one(const uint32_t* __res
     src = dst;
     dst = t;
   }
-  for (uint32_t i = tid; i < n; i += kRankThreads) {
-    const uint32_t v = src[i] & 0xFFFFu;
-    rank[v] = i;
-    if (i < rw.count) rw.w[i] = rw.slots ? deg[v] : 0u;
+  if (!rw.off) {
+    for (uint32_t i = tid; i < n; i += kRankThreads) {
+      const uint32_t v = src[i] & 0xFFFFu;
+      rank[v] = i;
+      if (i < rw.count) rw.w[i] = rw.slots ? deg[v] : 0u;
+    }
+    return;
   }
+  // Ranks, and the scan of the degrees in rank order.
+  uint32_t d[kRankRounds], sum = 0;
+#pragma unroll
+  for (int r = 0; r < kRankRounds; ++r) {
+    const uint32_t i = (w * rounds + r) * 32 + lane;
+    d[r] = 0;
+    if (r < (int)rounds && i < n) {
+      const uint32_t v = src[i] & 0xFFFFu;
+      rank[v] = i;
+      d[r] = deg[v];
+    }
+    sum += d[r];
+  }
+  sum = __reduce_add_sync(kFull, sum);
+  if (lane == 0) wcnt[w] = sum;
+  __syncthreads();
+  const uint32_t tot = wcnt[lane], incl = warp_inclusive_sum(tot);
+  uint32_t at = __shfl_sync(kFull, incl, w) - sum;
+#pragma unroll
+  for (int r = 0; r < kRankRounds; ++r) {
+    if (r >= (int)rounds) break;
+    const uint32_t i = (w * rounds + r) * 32 + lane;
+    const uint32_t id = warp_inclusive_sum(d[r]);
+    if (i < n) rw.off[i] = rw.w[i] = at + id - d[r];
+    at += __shfl_sync(kFull, id, 31);
+  }
+  const uint32_t all = __shfl_sync(kFull, incl, 31);
+  if (tid == 0) rw.off[n] = rw.w[n] = all;
 }
 
 __global__ void k_identity_graph_of(uint64_t n, const uint64_t* voff, uint32_t G, uint32_t* __restrict__ graph_of_rank) {
@@ -1092,14 +1124,17 @@ bool degree_slots(const PrepInput& in) {
   return in.order == TRIBIT_ORDER_DEGREE && !in.compact && 2 * in.E < 0xFFFFFFFFull;
 }
 
+// The one-CTA ranking scans the slot sizes too.
+bool rank_scans(const PrepInput& in) { return degree_slots(in) && !in.G && in.n > 0 && in.n <= kRankOneMax; }
+
 // cnt: n + 1 words, row counters at 0 or, on the slot path, slot sizes (then the
 // fill cursors, which end at the rows' ends); nbig: kLongWords words at 0.
-void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, uint32_t* cnt, uint32_t* nbig, cudaStream_t st,
-              Prepared* out, DeviceStats* stats, uint64_t* rp) {
+// off: n + 1 words, the row starts (set already where rank_scans(in)).
+void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, uint32_t* cnt, uint32_t* off, uint32_t* nbig,
+              cudaStream_t st, Prepared* out, DeviceStats* stats, uint64_t* rp) {
   const uint64_t E = in.E, n = in.n;
   const bool presort = takes_presort(in), slots = degree_slots(in);
   const uint64_t cap = slots ? 2 * E : E;  // nbr entries
-  uint32_t* off = ar.take<uint32_t>(n + 1);  // row starts
   uint32_t* otmp = take_scan_temp<uint32_t>(ar, n + 1);
   uint64_t* rtmp = take_scan_temp<uint64_t>(ar, n + 1);
   uint32_t* big = ar.take<uint32_t>(n + 1);
@@ -1124,7 +1159,7 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, uint32_t* cn
     k_row_count<<<entry_grid, kThreads, 0, st>>>(in, rank, cnt, keys, (uint32_t)per, &stats->err);
     TB_LAUNCH_CHECK();
   }
-  device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st, cnt);
+  if (!rank_scans(in)) device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st, cnt);
   if (slots && presort) {
     const uint64_t tiles = ceil_div<uint64_t>(E, kSortTile);
     k_row_keys_hist<<<(unsigned)tiles, kSortThreads, 0, st>>>(in, rank, keys, top, (uint32_t)tiles, ktmp.hist,
@@ -1267,6 +1302,7 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
   // The row counters and, after them, the long rows' list lengths: set together.
   uint32_t* cnt = ar.take<uint32_t>(n + 1);
   uint32_t* nbig = ar.take<uint32_t>(kLongWords);
+  uint32_t* off = ar.take<uint32_t>(n + 1);
   RankBuffers rb;
   if (by_degree) {
     rank = ar.take<uint32_t>(n ? n : 1);
@@ -1285,7 +1321,7 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
   // Phase 1 (launch only when not measuring): the upload of host entries,
   // degrees and the rank order.
   if (!ar.measuring()) {
-    const RowWords rw{cnt, (uint64_t)(nbig + kLongWords - cnt), degree_slots(in)};
+    const RowWords rw{cnt, (uint64_t)(nbig + kLongWords - cnt), degree_slots(in), rank_scans(in) ? off : nullptr};
     TB_CUDA(cudaMemsetAsync(stats, 0, deg ? (size_t)((char*)(deg + n) - (char*)stats) : sizeof(DeviceStats), st));
     if (!by_degree || n == 0) TB_CUDA(cudaMemsetAsync(cnt, 0, rw.count * sizeof(uint32_t), st));
     const HostUpload& up = in.upload;
@@ -1327,7 +1363,7 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
     }
   }
   // Phase 2: orient, rows, sort + dedup per row, CSR + bit rows.
-  run_rows(ar, in, rank, cnt, nbig, st, out, stats, rp);
+  run_rows(ar, in, rank, cnt, off, nbig, st, out, stats, rp);
 }
 
 }  // namespace tb

@@ -35,10 +35,12 @@ __device__ __forceinline__ uint32_t rp_row(uint64_t w) { return (uint32_t)(w >> 
 __device__ __forceinline__ uint32_t rp_blk(uint64_t w) { return (uint32_t)w; }
 
 // Counters the device writes and the host reads back once per call.
+constexpr int kScheduleWords = 12;
 struct DeviceStats {
   unsigned long long edges;        // undirected edges after dedup (m)
   unsigned long long blocks;       // bit-row entries (nb)
   unsigned int err;                // kErr* flags of the preprocessing
+  unsigned int sched[kScheduleWords];  // the schedule's list ends and totals (Schedule::piece_off)
   unsigned int pad;
   // From here on cleared by each counting launch.
   unsigned long long triangles;

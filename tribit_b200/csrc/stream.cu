@@ -392,7 +392,7 @@ size_t rows_layout(Arena& ar, bool measure, uint64_t n, uint64_t kept, uint64_t 
   L->build = take_row_range_buffers(ar, n, cap);
   const size_t build_end = ar.used();
   ar.rewind(rows_end);
-  L->sched = take_schedule(ar, n, kept, hubs);
+  L->sched = take_schedule(ar, n, kept, L->stats, hubs);
   return std::max(build_end, ar.used());
 }
 
