@@ -93,3 +93,38 @@ def test_batch_of_tiny_graphs():
         with tb.Counter(dispatch=mode) as c:
             got, r = c.count_batch(e, off, nodes)
             assert got.tolist() == want and r.triangles == sum(want)
+
+
+def test_batch_in_chunks():
+    # 17 million entries: four chunks of whole graphs, ranked and built one after
+    # the other; graphs without entries or vertices at their borders, a graph
+    # longer than a chunk, and a last chunk without entries.
+    parts, nodes = [], []
+    for i in range(40):
+        n = 500 + 37 * i
+        nodes += [n, 0, 3]
+        parts += [tb.gen_er(n, 100_000 + 997 * i, seed=i), [], []]
+    nodes += [40_000, 1, 0, 5] + [2_000] * 3 + [7, 0]
+    parts += [tb.gen_rmat(15, 280, seed=9), [], [], []] + [tb.gen_er(2_000, 1_000_000, seed=s) for s in (1, 2, 3)] + [[], []]
+    parts = [np.asarray(p, dtype=np.uint64) for p in parts]
+    off = np.concatenate([[0], np.cumsum([p.size for p in parts])]).astype(np.uint64)
+    assert off[-1] > 4 << 22
+    want = [oracle.count(p, k)[0] if p.size else 0 for p, k in zip(parts, nodes)]
+    for mode in ("plain", "merge"):
+        with tb.Counter(dispatch=mode) as c:
+            for _ in range(2):
+                got, r = c.count_batch(np.concatenate(parts), off, nodes)
+                assert got.tolist() == want and r.triangles == sum(want)
+
+
+@pytest.mark.parametrize("length", [3, 4, 5, 31, 32, 33, 64, 65, 255, 256])
+def test_merge_with_long_neighbour_rows(length):
+    # A row of `length` blocks over neighbours whose rows are a few times longer
+    # than its tail: searched in either direction.
+    n = 200_000
+    cols = np.uint64(40) + np.uint64(32) * np.arange(length, dtype=np.uint64)
+    e = [(np.uint64(1) << np.uint64(32)) | cols]
+    for i, c in enumerate(cols):  # every neighbour's row: the tail and up to 8 times as many others
+        far = np.uint64(40 + 32 * length) + np.uint64(64) * np.arange((i % 9) * (length - i), dtype=np.uint64)
+        e += [(c << np.uint64(32)) | cols[i + 1:], (c << np.uint64(32)) | far[far < n]]
+    check(np.concatenate(e), n, modes=("merge", "bitmap"), orders=("id",))

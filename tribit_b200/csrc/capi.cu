@@ -90,6 +90,8 @@ void run_call(tribit_context* c, tb::PrepInput in, const uint64_t* host_entries,
   if (G) {
     pin.eoff = L.eoff;
     pin.voff = L.voff;
+    pin.host_eoff = host_eoff;
+    pin.host_voff = host_voff;
   }
   tb::drop_graph(c);
   tb::prepare_graph(c->arena, pin, st, &c->prep);
