@@ -22,6 +22,8 @@ namespace {
 constexpr uint32_t kFull = 0xffffffffu;
 constexpr int kWarpsPerCta = 8;
 constexpr int kWarpSlots = 512;                      // 8-byte words of shared memory per warp
+constexpr int kWarpSlotShift = 32 - 9;                // a 32-bit hash's leading bits: the slot
+static_assert(kWarpSlots == 1 << (32 - kWarpSlotShift), "slots");
 constexpr uint32_t kWarpMaxBlocks = kWarpSlots / 2;  // bitmap rows up to this many bit blocks
 constexpr int kCtaThreads = 512;
 constexpr int kCtaLogSlots = 14;                     // 16384 slots = 128 KiB
@@ -104,6 +106,46 @@ struct BitmapProbe {
     return (table_find(t, logb, blk) >> (w & 31)) & k & 1u;
   }
 };
+
+// ---- rows of at most 32 blocks ----------------------------------------------
+// One block a lane, hashed into the warp's kWarpSlots slots, one block a slot: a
+// lookup is one 8-byte read and one compare, without a loop. Two blocks that
+// meet on a slot: one of them, `xb`, is compared apart; more than that, and
+// another multiplier is taken. The table is left as it was found, empty: each
+// lane takes its block out again, so that a row clears nothing.
+struct SmallProbe {
+  const uint64_t* t;
+  uint32_t mult, xb, xm;
+  __device__ __forceinline__ uint32_t operator()(uint64_t e) const {
+    const uint32_t blk = (uint32_t)(e >> 32);
+    const uint64_t s = t[blk * mult >> kWarpSlotShift];
+    uint32_t m = (uint32_t)(s >> 32) == blk ? (uint32_t)s : 0u;
+    if (blk == xb) m = xm;
+    return (uint32_t)__popc((uint32_t)e & m);
+  }
+};
+
+// Stages e, the lane's block (lanes >= nb: none), in the warp's empty table;
+// mine: the lane's slot. False: no multiplier tried does, the table is empty.
+__device__ __forceinline__ bool small_insert(uint64_t* t, uint64_t e, uint32_t nb, SmallProbe& p, uint32_t& mine) {
+  const uint32_t lane = threadIdx.x & 31;
+  p.t = t;
+  p.mult = 0x9E3779B1u;
+  for (int tries = 0; tries < 8; ++tries, p.mult = p.mult * 0x85EBCA6Bu) {
+    mine = (uint32_t)(e >> 32) * p.mult >> kWarpSlotShift;
+    if (lane < nb) t[mine] = e;
+    __syncwarp();
+    const uint32_t lost = __ballot_sync(kFull, lane < nb && t[mine] != e);
+    const int s = lost ? __ffs(lost) - 1 : 0;
+    p.xb = __shfl_sync(kFull, (uint32_t)(e >> 32), s);
+    p.xm = __shfl_sync(kFull, (uint32_t)e, s);
+    if (!lost) p.xb = kFull;  // no row has this block
+    if (!(lost & (lost - 1))) return true;
+    if (lane < nb) t[mine] = kEmptySlot;
+    __syncwarp();
+  }
+  return false;
+}
 
 // ---- the neighbour sweep ---------------------------------------------------
 // Visits every item of the lists of slots [cs, ce), in chunks of 32 slots
@@ -263,9 +305,6 @@ __device__ __forceinline__ uint64_t sweep(const GraphView& g, uint32_t cs, uint3
       item);
 }
 
-// Bit-row sweep: every bit block of v = col[j], j in the slots, scored by
-// probe (a hash or direct-map lookup in u's staged row), flattened with
-// kBitsDepth blocks in flight per lane (sweep_runs; wsm: the warp's 64 words).
 #ifndef TB_BITS_DEPTH
 #define TB_BITS_DEPTH 4
 #endif
@@ -276,106 +315,115 @@ __device__ __forceinline__ uint64_t col_entry(uint32_t w, bool keep) {
   return ((uint64_t)(w >> 5) << 32) | (keep ? 1u << (w & 31) : 0u);
 }
 
+// The bit row of the neighbour at CSR position j, empty where the hub pass counts the edge.
+__device__ __forceinline__ void neighbour_blocks(const GraphView& g, uint32_t j, uint32_t& ib, uint32_t& il) {
+  if (edge_to_hub(g, j)) return;
+  const uint32_t v = g.col[j];
+  const uint32_t* low = reinterpret_cast<const uint32_t*>(g.rp);  // the low word of rp[v] is its bit row's start
+  ib = low[2ull * v];
+  il = low[2ull * v + 2] - ib;
+}
+
+// Items of the slots of a chunk, concatenated (excl, il: this lane's slot): bit
+// l set iff a slot's items start at item b + l.
+__device__ __forceinline__ uint32_t starts_in(uint32_t excl, uint32_t il, uint32_t b) {
+  return __reduce_or_sync(kFull, il && excl - b < 32u ? 1u << (excl - b) : 0u);
+}
+
+// Scores the items of 32 lists, lane l's at [ib, ib + il). The lists are
+// concatenated and lane l takes items base + l + 32 r, r < Depth, of the
+// concatenation, issuing all loads before it uses any, so a warp keeps
+// 32 * Depth loads in flight however short the lists are. load(k) reads item k,
+// probe(x) scores it; a 0 must score 0. An item's owner: in short lists, one OR
+// across the warp of where the lists start gives the owners of 32 items as a
+// population count (a binary search by five shuffles an item; with the small rows' table below, planted
+// partition of 2 million vertices 4,249 us, now 3,407);
+// from kWalkItems items on (Walks), each lane finds the owner of its first
+// item by binary search and then only advances it (a lane's items only grow), one
+// compare an item. wsm: 64 words of the warp. Must be called by all 32 lanes.
+#ifndef TB_WALK_ITEMS
+#define TB_WALK_ITEMS 1024
+#endif
+constexpr uint32_t kWalkItems = TB_WALK_ITEMS;
+template <int Depth, bool Walks, class Load, class Probe>
+__device__ __forceinline__ uint32_t run_items(uint32_t ib, uint32_t il, const Load& load, const Probe& probe,
+                                              uint32_t* wsm) {
+  const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u, le = kFull >> (31 - lane);
+  const uint32_t incl = warp_inclusive_sum(il), excl = incl - il, total = __shfl_sync(kFull, incl, 31);
+  if (Walks && total >= kWalkItems) {
+    __syncwarp();
+    wsm[lane] = incl;
+    wsm[32 + lane] = ib - excl;  // item t of the chunk, owned by slot s, is item off_s + t
+    __syncwarp();
+    uint32_t s = 0, racc = 0;
+#pragma unroll
+    for (uint32_t st = 16; st >= 1; st >>= 1)
+      if (wsm[s + st - 1] <= lane) s += st;
+    uint32_t lim = wsm[s], off = wsm[32 + s];
+    for (uint32_t base = 0; base < total; base += 32 * Depth) {
+      uint64_t x[Depth];
+#pragma unroll
+      for (int r = 0; r < Depth; ++r) {
+        const uint32_t t = base + 32 * r + lane;
+        while (t >= lim && s < 31) {
+          ++s;
+          lim = wsm[s];
+          off = wsm[32 + s];
+        }
+        x[r] = t < total ? load(off + t) : 0ull;
+      }
+#pragma unroll
+      for (int r = 0; r < Depth; ++r) racc += probe(x[r]);
+    }
+    return racc;
+  }
+  const uint32_t some = __ballot_sync(kFull, il > 0);
+  __syncwarp();
+  if (il) wsm[__popc(some & lt)] = ib - excl;  // item t of the chunk, owned by slot s, is item off_s + t
+  __syncwarp();
+  uint32_t racc = 0, slot = kFull;
+  for (uint32_t base = 0; base < total; base += 32 * Depth) {
+    uint64_t x[Depth];
+#pragma unroll
+    for (int r = 0; r < Depth; ++r) {
+      const uint32_t at = base + 32 * r;
+      x[r] = 0;
+      if (r == 0 || at < total) {  // the whole warp
+        const uint32_t m = starts_in(excl, il, at), s = slot + __popc(m & le);
+        slot += __popc(m);
+        if (at + lane < total) x[r] = load(wsm[s] + at + lane);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < Depth; ++r)
+      if (r == 0 || base + 32 * r < total) racc += probe(x[r]);
+  }
+  return racc;
+}
+
+template <class Probe>
+__device__ __forceinline__ uint64_t sweep_bits(const GraphView& g, uint32_t ib, uint32_t il, uint32_t cs, uint32_t ce,
+                                               uint32_t step, const Probe& probe, uint32_t* wsm) {
+  uint64_t acc = 0;
+  for (uint32_t c = cs;;) {
+    acc += run_items<kBitsDepth, true>(ib, il, [&](uint32_t k) -> uint64_t { return g.bent[k]; }, probe, wsm);
+    c += step * 32;
+    if (c >= ce) break;
+    ib = il = 0;
+    const uint32_t j = c + (threadIdx.x & 31);
+    if (j < ce) neighbour_blocks(g, j, ib, il);
+  }
+  __syncwarp();
+  return acc;
+}
+
+// The same with the owners of sweep_runs: rows whose neighbours' lists are long.
 template <class Probe>
 __device__ __forceinline__ uint64_t sweep_bits(const GraphView& g, uint32_t cs, uint32_t ce, uint32_t chunk0,
                                                uint32_t step, const Probe& probe, uint32_t* wsm) {
   return sweep_runs<kBitsDepth, 32>(
-      cs, ce, chunk0, step,
-      [&](uint32_t j, uint32_t& ib, uint32_t& il) {
-        if (edge_to_hub(g, j)) return;
-        const uint32_t v = g.col[j];
-        const uint64_t a = g.rp[v], b = g.rp[v + 1];
-        ib = rp_blk(a);
-        il = rp_blk(b) - ib;
-      },
+      cs, ce, chunk0, step, [&](uint32_t j, uint32_t& ib, uint32_t& il) { neighbour_blocks(g, j, ib, il); },
       [&](uint32_t k) -> uint64_t { return g.bent[k]; }, probe, wsm);
-}
-
-// Mask of block x in the sorted bit row r[lo, end), or 0.
-__device__ __forceinline__ uint32_t search_mask(const uint64_t* r, uint32_t lo, uint32_t end, uint32_t x) {
-  uint32_t hi = end;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if ((uint32_t)(r[mid] >> 32) < x)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  if (lo < end) {
-    const uint64_t e = r[lo];
-    if ((uint32_t)(e >> 32) == x) return (uint32_t)e;
-  }
-  return 0u;
-}
-
-// Sorted-list intersection of bit rows (the merge variant). u's bit row is in
-// shared memory (urow, nbu entries, ascending block). For each neighbour v of
-// the chunk, the shorter of u's tail -- u's entries from v's block on, the
-// only ones that can meet N+(v) -- and v's bit row is walked, and every block
-// of it is binary-searched in the other list. Edges given to the hub pass,
-// where u's tail was the shorter list, are skipped. Must be called by all 32
-// lanes.
-__device__ __forceinline__ uint64_t sweep_merge(const GraphView& g, const uint64_t* urow, uint32_t nbu, uint32_t cs,
-                                                uint32_t ce) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint64_t acc = 0;
-  auto item = [&](uint32_t k, bool walk_u, uint32_t ob, uint32_t oe) -> uint32_t {
-    const uint64_t e = walk_u ? urow[k] : g.bent[k];
-    const uint32_t m = walk_u ? search_mask(g.bent, ob, oe, (uint32_t)(e >> 32))
-                              : search_mask(urow, ob, oe, (uint32_t)(e >> 32));
-    return (uint32_t)__popc((uint32_t)e & m);
-  };
-  for (uint32_t c = cs; c < ce; c += 32) {
-    const uint32_t j = c + lane;
-    uint32_t ab = 0, len = 0, ob = 0, oe = 0, walk_u = 0;
-    if (j < ce && !edge_to_hub(g, j)) {
-      const uint32_t v = g.col[j];
-      const uint64_t va = g.rp[v], vb = g.rp[v + 1];
-      const uint32_t vbs = rp_blk(va), vbe = rp_blk(vb);
-      uint32_t lo = 0, hi = nbu;  // position of v's block in u's row
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if ((uint32_t)(urow[mid] >> 32) < (v >> 5))
-          lo = mid + 1;
-        else
-          hi = mid;
-      }
-      const uint32_t ta = nbu - lo, tb = vbe - vbs;
-      walk_u = ta <= tb ? 1u : 0u;
-      if (walk_u) {
-        ab = lo, len = ta, ob = vbs, oe = vbe;
-      } else {
-        ab = vbs, len = tb, ob = lo, oe = nbu;
-      }
-    }
-    uint32_t longm = __ballot_sync(kFull, len >= kLong);
-    while (longm) {
-      const int s = __ffs(longm) - 1;
-      longm &= longm - 1;
-      const uint32_t sab = __shfl_sync(kFull, ab, s), slen = __shfl_sync(kFull, len, s);
-      const uint32_t sob = __shfl_sync(kFull, ob, s), soe = __shfl_sync(kFull, oe, s);
-      const bool sw = __shfl_sync(kFull, walk_u, s) != 0;
-      for (uint32_t k = lane; k < slen; k += 32) acc += item(sab + k, sw, sob, soe);
-    }
-    const uint32_t sl = len >= kLong ? 0u : len;
-    const uint32_t incl = warp_inclusive_sum(sl);
-    const uint32_t total = __shfl_sync(kFull, incl, 31);
-    const uint32_t excl = incl - sl;
-    for (uint32_t base = 0; base < total; base += 32) {
-      const uint32_t t = base + lane;
-      uint32_t s = 0;
-#pragma unroll
-      for (uint32_t st = 16; st >= 1; st >>= 1) {
-        const uint32_t x = __shfl_sync(kFull, incl, s + st - 1);
-        if (x <= t) s += st;
-      }
-      const uint32_t sab = __shfl_sync(kFull, ab, s), sex = __shfl_sync(kFull, excl, s);
-      const uint32_t sob = __shfl_sync(kFull, ob, s), soe = __shfl_sync(kFull, oe, s);
-      const bool sw = __shfl_sync(kFull, walk_u, s) != 0;
-      if (t < total) acc += item(sab + (t - sex), sw, sob, soe);
-    }
-  }
-  return acc;
 }
 
 // SM cycle counter; a piece runs on one SM, so differences are meaningful.
@@ -383,17 +431,9 @@ __device__ __forceinline__ unsigned long long cycles() { return (unsigned long l
 
 // ---- warp-per-piece kernels (bitmap and merge variants) --------------------
 
-// Merge row blocks' edges left to the row sweep (not taken by the hub pass)
-// are walked by sorted-list merge with binary searches (0), or, like the
-// bitmap variant's, as v's bit blocks probed in u's direct-mapped or hashed
-// row (1). Build-time switch for measurement.
-#ifndef TB_MERGE_BITS
-#define TB_MERGE_BITS 0
-#endif
-
 // Shared memory of the row-piece bodies: the CTA's flat table (at least
 // kWarpsPerCta * kWarpSlots words of 8 bytes, the warps' slices at `stride`
-// words apart), the warps' run buffers (`run_stride` words apart, >= 64) and
+// words apart), the warps' run buffers (`run_stride` words apart, >= 96) and
 // a CTA word.
 struct PiecesShared {
   uint64_t* smem;
@@ -403,215 +443,278 @@ struct PiecesShared {
   uint32_t* s_row;
 };
 
-// A worker's next pieces of a list of len, `grab` at a time: of a list that one
-// turn of all `workers` covers, a fixed share (no worker waits for a cursor that
-// thousands of others update; a graph of 1,000 vertices spent a third of its
-// count there), else from the cursor. One thread calls it; `turn` counts calls.
-__device__ __forceinline__ uint32_t next_pieces(unsigned int* cursor, uint32_t len, uint32_t worker, uint32_t workers,
-                                                uint32_t grab, uint32_t turn) {
-  if (len <= (uint64_t)workers * grab) return turn == 0 ? worker * grab : len;
-  return atomicAdd(cursor, grab);
+// A list of len pieces that one turn of all workers covers, `grab` each, is
+// shared out by worker number instead of through a cursor that thousands of
+// warps update (a third of the count of a graph of 1,000 vertices).
+__device__ __forceinline__ bool one_turn(uint32_t len, uint32_t workers, uint32_t grab) {
+  return len <= (uint64_t)workers * grab;
 }
 
-// The row-piece variant V over its pieces (and, with `heavy`, first the heavy
-// pieces, one CTA per piece); returns this thread's partial count.
-template <int V>
-__device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64_t* __restrict__ pieces,
-                                                const uint32_t* __restrict__ piece_off, DeviceStats* stats,
-                                                unsigned long long* per_graph, unsigned long long* block_ns, bool heavy,
-                                                uint32_t width, const PiecesShared& sh) {
-  constexpr bool kSorted = V == TRIBIT_VARIANT_MERGE && !TB_MERGE_BITS;  // u staged as a sorted row
+// The heavy list's pieces: neighbours of the rows too wide for a warp's slice,
+// one piece at a time per CTA, with a CTA-shared table in the same shared
+// memory and all warps sweeping the piece's neighbour chunks. Returns this
+// thread's partial count.
+__device__ __forceinline__ uint64_t heavy_body(const GraphView& g, const uint64_t* __restrict__ pieces,
+                                               const uint32_t* __restrict__ piece_off, DeviceStats* stats,
+                                               unsigned long long* per_graph, unsigned long long* block_ns,
+                                               const PiecesShared& sh) {
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint64_t* tbl = sh.smem + w * sh.stride;
   uint32_t* wruns = sh.runs + w * sh.run_stride;
   uint32_t& s_row = *sh.s_row;
-
-  const uint32_t p0 = piece_off[V], len = piece_off[V + 1] - p0;
   uint64_t acc = 0;
-  // Phase 1 (first kernel only): pieces of the rows too wide for a warp's
-  // slice, one at a time per CTA, with a CTA-shared table in the same shared
-  // memory and all warps sweeping the piece's neighbour chunks.
-  if (heavy) {
-    uint64_t* ctbl = sh.smem;
-    uint32_t* pre = reinterpret_cast<uint32_t*>(sh.smem) + kHeavyMaxSpan;
-    const uint32_t h0 = piece_off[kListHeavy], hlen = piece_off[kListHeavy + 1] - h0;
-    for (uint32_t turn = 0;; ++turn) {
-      if (threadIdx.x == 0) s_row = next_pieces(&stats->cursor[kCurHeavy], hlen, blockIdx.x, gridDim.x, 1, turn);
-      __syncthreads();
-      const uint32_t t = s_row;
-      if (t >= hlen) break;
-      const uint64_t pc = pieces[h0 + (hlen - 1 - t)];
-      const uint32_t u = (uint32_t)(pc >> 32);
-      const unsigned long long h_start = (block_ns && threadIdx.x == 0) ? cycles() : 0ull;
-      const uint64_t a = g.rp[u], b = g.rp[u + 1];
-      const uint32_t rs = rp_row(a) + (uint32_t)pc, bs = rp_blk(a), be = rp_blk(b);
-      const uint32_t d = min(rp_row(b) - rs, kHeavyPiece);
-      // u's row: a direct-mapped mask array over its block span when that
-      // fits, else the bucketed hash.
-      const uint32_t bmin = (uint32_t)(g.bent[bs] >> 32), bmax = (uint32_t)(g.bent[be - 1] >> 32);
-      const uint32_t span = bmax - bmin + 1;
-      const bool direct = span <= kHeavyMaxSpan;
-      uint32_t* cmap = reinterpret_cast<uint32_t*>(ctbl);
-      const int logb = table_logb(be - bs);
-      if (direct) {
-        for (uint32_t i = threadIdx.x; i < span; i += blockDim.x) cmap[i] = 0u;
-      } else {
-        table_clear(ctbl, logb, threadIdx.x, blockDim.x);
-      }
-      // Item prefix: pre[j] = bit blocks of the neighbours before j, pre[d] = all.
-      for (uint32_t j = threadIdx.x; j < d; j += blockDim.x) {
-        const uint32_t v = g.col[rs + j];
-        pre[j] = edge_to_hub(g, rs + j) ? 0u : rp_blk(g.rp[v + 1]) - rp_blk(g.rp[v]);
-      }
-      __syncthreads();
-      if (direct) {
-        for (uint32_t k = bs + threadIdx.x; k < be; k += blockDim.x) {
-          const uint64_t e = g.bent[k];
-          cmap[(uint32_t)(e >> 32) - bmin] = (uint32_t)e;
-        }
-      } else {
-        table_insert(ctbl, logb, g.bent, bs, be, threadIdx.x, blockDim.x);
-      }
-      {
-        const uint32_t per = (d + blockDim.x - 1) / blockDim.x, j0 = threadIdx.x * per;
-        uint32_t lsum = 0;
-        for (uint32_t k = 0; k < per && j0 + k < d; ++k) lsum += pre[j0 + k];
-        uint32_t tot;
-        uint32_t ex = block_exclusive_scan<uint32_t>(lsum, OpSum{}, 0u, &tot);
-        for (uint32_t k = 0; k < per && j0 + k < d; ++k) {
-          const uint32_t x = pre[j0 + k];
-          pre[j0 + k] = ex;
-          ex += x;
-        }
-        if (threadIdx.x == 0) pre[d] = tot;
-      }
-      __syncthreads();
-      // Warp w takes the neighbours whose first item falls in the w-th equal
-      // share of the piece's items, so the warps finish together.
-      const uint32_t tot = pre[d];
-      auto first_at = [&](uint32_t x) -> uint32_t {  // first j with pre[j] >= x
-        uint32_t lo = 0, hi = d;
-        while (lo < hi) {
-          const uint32_t mid = (lo + hi) >> 1;
-          if (pre[mid] < x)
-            lo = mid + 1;
-          else
-            hi = mid;
-        }
-        return lo;
-      };
-      const uint32_t cs = first_at((uint32_t)((uint64_t)tot * w / kWarpsPerCta));
-      const uint32_t ce = w + 1 == kWarpsPerCta ? d : first_at((uint32_t)((uint64_t)tot * (w + 1) / kWarpsPerCta));
-      uint64_t racc;
-      if (direct) {
-        racc = sweep_bits(g, rs + cs, rs + ce, 0, 1, [&](uint64_t e) -> uint32_t {
-          const uint32_t o = (uint32_t)(e >> 32) - bmin;
-          return o < span ? (uint32_t)__popc((uint32_t)e & cmap[o]) : 0u;
-        }, wruns);
-      } else {
-        const BitmapProbe probe{ctbl, logb, bmin, bmax};
-        racc = sweep_bits(g, rs + cs, rs + ce, 0, 1, probe, wruns);
-      }
-      if (per_graph) {
-        const uint64_t s = warp_sum(racc);
-        if (lane == 0 && s) atomicAdd(&per_graph[g.graph_of_rank[u]], (unsigned long long)s);
-      }
-      acc += racc;
-      __syncthreads();  // the table and s_row are rewritten for the next piece
-      // Timing: the piece's CTA cycles in warp-cycles, like the warp pieces'.
-      if (block_ns && threadIdx.x == 0) atomicAdd(&block_ns[u >> 5], (cycles() - h_start) * kWarpsPerCta);
+  uint64_t* ctbl = sh.smem;
+  uint32_t* pre = reinterpret_cast<uint32_t*>(sh.smem) + kHeavyMaxSpan;
+  const uint32_t h0 = piece_off[kListHeavy], hlen = piece_off[kListHeavy + 1] - h0;
+  const bool fixed = one_turn(hlen, gridDim.x, 1);
+  do {
+    if (threadIdx.x == 0) s_row = fixed ? blockIdx.x : atomicAdd(&stats->cursor[kCurHeavy], 1u);
+    __syncthreads();
+    const uint32_t t = s_row;
+    if (t >= hlen) break;
+    const uint64_t pc = pieces[h0 + (hlen - 1 - t)];
+    const uint32_t u = (uint32_t)(pc >> 32);
+    const unsigned long long h_start = (block_ns && threadIdx.x == 0) ? cycles() : 0ull;
+    const uint64_t a = g.rp[u], b = g.rp[u + 1];
+    const uint32_t rs = rp_row(a) + (uint32_t)pc, bs = rp_blk(a), be = rp_blk(b);
+    const uint32_t d = min(rp_row(b) - rs, kHeavyPiece);
+    // u's row: a direct-mapped mask array over its block span when that
+    // fits, else the bucketed hash.
+    const uint32_t bmin = (uint32_t)(g.bent[bs] >> 32), bmax = (uint32_t)(g.bent[be - 1] >> 32);
+    const uint32_t span = bmax - bmin + 1;
+    const bool direct = span <= kHeavyMaxSpan;
+    uint32_t* cmap = reinterpret_cast<uint32_t*>(ctbl);
+    const int logb = table_logb(be - bs);
+    if (direct) {
+      for (uint32_t i = threadIdx.x; i < span; i += blockDim.x) cmap[i] = 0u;
+    } else {
+      table_clear(ctbl, logb, threadIdx.x, blockDim.x);
+    }
+    // Item prefix: pre[j] = bit blocks of the neighbours before j, pre[d] = all.
+    for (uint32_t j = threadIdx.x; j < d; j += blockDim.x) {
+      const uint32_t v = g.col[rs + j];
+      pre[j] = edge_to_hub(g, rs + j) ? 0u : rp_blk(g.rp[v + 1]) - rp_blk(g.rp[v]);
     }
     __syncthreads();
-  }
-  uint32_t cur = 0xFFFFFFFFu;  // row whose structure is loaded
-  bool cur_direct = false;
-  int logb = 0;
-  uint32_t bmin = 0, bmax = 0, d = 0;
-  uint32_t* wmap = reinterpret_cast<uint32_t*>(tbl);  // the slice as a direct-mapped row
-  for (uint32_t turn = 0;; ++turn) {
-    uint32_t t0 = 0;
-    if (lane == 0)
-      t0 = next_pieces(&stats->cursor[kCurVariant0 + V], len, w * gridDim.x + blockIdx.x, kWarpsPerCta * gridDim.x,
-                       kGrab, turn);
-    t0 = __shfl_sync(kFull, t0, 0);
-    if (t0 >= len) break;
-    const uint32_t t1 = min(t0 + kGrab, len);
-    for (uint32_t t = t0; t < t1; ++t) {
-      const uint64_t pc = pieces[p0 + (len - 1 - t)];
-      const uint32_t u = (uint32_t)(pc >> 32), first = (uint32_t)pc;
-      const uint64_t a = g.rp[u], b = g.rp[u + 1];
-      const uint32_t rs = rp_row(a), re = rp_row(b);
-      unsigned long long t_start = 0;
-      if (block_ns && lane == 0) t_start = cycles();
-      if (u != cur) {
-        __syncwarp();
-        cur = u;
-        if (kSorted) {
-          const uint32_t bs = rp_blk(a), be = rp_blk(b);
-          d = be - bs;  // u's bit-row length, at most kWarpMaxBlocks
-          for (uint32_t k = lane; k < d; k += 32) tbl[k] = g.bent[bs + k];
-        } else {
-          const uint32_t bs = rp_blk(a), be = rp_blk(b);
-          bmin = (uint32_t)(g.bent[bs] >> 32);
-          bmax = (uint32_t)(g.bent[be - 1] >> 32);
-          // A row whose blocks span at most the slice's 1,024 words is
-          // direct-mapped (one load per probe); others are hashed.
-          cur_direct = bmax - bmin < kWarpSlots * 2;
-          if (cur_direct) {
-            for (uint32_t i = lane; i <= bmax - bmin; i += 32) wmap[i] = 0u;
-            __syncwarp();
-            for (uint32_t k = bs + lane; k < be; k += 32) {
-              const uint64_t e = g.bent[k];
-              wmap[(uint32_t)(e >> 32) - bmin] = (uint32_t)e;
-            }
-          } else {
-            logb = table_logb(be - bs);
-            table_clear(tbl, logb, lane, 32);
-            __syncwarp();
-            table_insert(tbl, logb, g.bent, bs, be, lane, 32);
-          }
-        }
-        __syncwarp();
+    if (direct) {
+      for (uint32_t k = bs + threadIdx.x; k < be; k += blockDim.x) {
+        const uint64_t e = g.bent[k];
+        cmap[(uint32_t)(e >> 32) - bmin] = (uint32_t)e;
       }
-      const uint32_t cs = rs + first, ce = min(cs + width, re);
-      uint64_t racc;
-      if (kSorted) {
-        racc = sweep_merge(g, tbl, d, cs, ce);
-      } else if (cur_direct) {
-        const uint32_t span = bmax - bmin + 1;
-        racc = sweep_bits(g, cs, ce, 0, 1, [&](uint64_t e) -> uint32_t {
-          const uint32_t o = (uint32_t)(e >> 32) - bmin;
-          return o < span ? (uint32_t)__popc((uint32_t)e & wmap[o]) : 0u;
-        }, wruns);
-      } else {
-        const BitmapProbe probe{tbl, logb, bmin, bmax};
-        racc = sweep_bits(g, cs, ce, 0, 1, probe, wruns);
-      }
-      if (per_graph) {
-        const uint64_t s = warp_sum(racc);
-        if (lane == 0 && s) atomicAdd(&per_graph[g.graph_of_rank[u]], (unsigned long long)s);
-      }
-      if (block_ns) {
-        __syncwarp();
-        if (lane == 0) atomicAdd(&block_ns[u >> 5], cycles() - t_start);
-      }
-      acc += racc;
+    } else {
+      table_insert(ctbl, logb, g.bent, bs, be, threadIdx.x, blockDim.x);
     }
-  }
+    {
+      const uint32_t per = (d + blockDim.x - 1) / blockDim.x, j0 = threadIdx.x * per;
+      uint32_t lsum = 0;
+      for (uint32_t k = 0; k < per && j0 + k < d; ++k) lsum += pre[j0 + k];
+      uint32_t tot;
+      uint32_t ex = block_exclusive_scan<uint32_t>(lsum, OpSum{}, 0u, &tot);
+      for (uint32_t k = 0; k < per && j0 + k < d; ++k) {
+        const uint32_t x = pre[j0 + k];
+        pre[j0 + k] = ex;
+        ex += x;
+      }
+      if (threadIdx.x == 0) pre[d] = tot;
+    }
+    __syncthreads();
+    // Warp w takes the neighbours whose first item falls in the w-th equal
+    // share of the piece's items, so the warps finish together.
+    const uint32_t tot = pre[d];
+    auto first_at = [&](uint32_t x) -> uint32_t {  // first j with pre[j] >= x
+      uint32_t lo = 0, hi = d;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (pre[mid] < x)
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      return lo;
+    };
+    const uint32_t cs = first_at((uint32_t)((uint64_t)tot * w / kWarpsPerCta));
+    const uint32_t ce = w + 1 == kWarpsPerCta ? d : first_at((uint32_t)((uint64_t)tot * (w + 1) / kWarpsPerCta));
+    uint64_t racc;
+    if (direct) {
+      racc = sweep_bits(g, rs + cs, rs + ce, 0, 1, [&](uint64_t e) -> uint32_t {
+        const uint32_t o = (uint32_t)(e >> 32) - bmin;
+        return o < span ? (uint32_t)__popc((uint32_t)e & cmap[o]) : 0u;
+      }, wruns);
+    } else {
+      const BitmapProbe probe{ctbl, logb, bmin, bmax};
+      racc = sweep_bits(g, rs + cs, rs + ce, 0, 1, probe, wruns);
+    }
+    if (per_graph) {
+      const uint64_t s = warp_sum(racc);
+      if (lane == 0 && s) atomicAdd(&per_graph[g.graph_of_rank[u]], (unsigned long long)s);
+    }
+    acc += racc;
+    __syncthreads();  // the table and s_row are rewritten for the next piece
+    // Timing: the piece's CTA cycles in warp-cycles, like the warp pieces'.
+    if (block_ns && threadIdx.x == 0) atomicAdd(&block_ns[u >> 5], (cycles() - h_start) * kWarpsPerCta);
+  } while (!fixed);
+  __syncthreads();
   return acc;
 }
 
+// The row-piece variant V over its pieces; returns this thread's partial count.
 template <int V>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) k_pieces_warp(GraphView g, const uint64_t* __restrict__ pieces,
+__device__ __forceinline__ uint64_t pieces_body(const GraphView& g, const uint64_t* __restrict__ pieces,
+                                                const uint32_t* __restrict__ piece_off, DeviceStats* stats,
+                                                unsigned long long* per_graph, unsigned long long* block_ns,
+                                                uint32_t width, const PiecesShared& sh) {
+  constexpr bool kMerge = V == TRIBIT_VARIANT_MERGE;
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint64_t* tbl = sh.smem + w * sh.stride;
+  uint32_t* wruns = sh.runs + w * sh.run_stride;
+  const uint32_t p0 = piece_off[V], len = piece_off[V + 1] - p0;
+  uint64_t acc = 0;
+  uint32_t cur = 0xFFFFFFFFu;  // row whose structure is loaded
+  // How it is loaded: in the slots of SmallProbe (mult, xb, xm), direct-mapped
+  // (bmin, span), or hashed (logb, bmin, bmax).
+  enum { kSmall, kDirect, kHashed } kind = kHashed;
+  uint32_t q0 = 0, q1 = 0, q2 = 0;
+  uint32_t* mine = wruns + 64 + lane;  // this lane's slot of a small row, or kFull
+  uint32_t* wmap = reinterpret_cast<uint32_t*>(tbl);  // the slice as a direct-mapped row
+  auto count_piece = [&](uint64_t pc) {
+    const uint32_t u = (uint32_t)(pc >> 32), first = (uint32_t)pc;
+    const uint64_t a = g.rp[u], b = g.rp[u + 1];
+    const uint32_t rs = rp_row(a), re = rp_row(b);
+    unsigned long long t_start = 0;
+    if (block_ns && lane == 0) t_start = cycles();
+    const uint32_t cs = rs + first, ce = min(cs + width, re);
+    // The first 32 neighbours' rows are looked up while u's row is staged (one after
+    // the other, a short row was a chain of nine dependent reads).
+    uint32_t ib = 0, il = 0;
+    if (cs + lane < ce) neighbour_blocks(g, cs + lane, ib, il);
+    if (u != cur) {
+      __syncwarp();
+      cur = u;
+      const uint32_t bs = rp_blk(a), nb = rp_blk(b) - bs;
+      const uint64_t e = lane < nb ? g.bent[bs + lane] : 0ull;
+      const bool empty = kind == kSmall;  // the slice holds nothing but that row
+      if (empty && *mine != kFull) tbl[*mine] = kEmptySlot;
+      const uint32_t bmin = __shfl_sync(kFull, (uint32_t)(e >> 32), 0);
+      uint32_t bmax = __shfl_sync(kFull, (uint32_t)(e >> 32), (nb - 1) & 31);
+      if (nb > 32) bmax = (uint32_t)(g.bent[bs + nb - 1] >> 32);
+      kind = kHashed;
+      if (bmax - bmin < kWarpSlots * 2) {
+        // A row whose blocks span at most the slice's 1,024 words is direct-mapped:
+        // one 4-byte read a probe, and neighbouring blocks on neighbouring banks.
+        kind = kDirect;
+        q0 = bmin;
+        q1 = bmax - bmin + 1;
+        __syncwarp();
+        for (uint32_t i = lane; i < q1; i += 32) wmap[i] = 0u;
+        __syncwarp();
+        if (lane < nb) wmap[(uint32_t)(e >> 32) - bmin] = (uint32_t)e;
+        for (uint32_t k = lane + 32; k < nb; k += 32) {
+          const uint64_t x = g.bent[bs + k];
+          wmap[(uint32_t)(x >> 32) - bmin] = (uint32_t)x;
+        }
+      } else if (nb <= 32) {
+        if (!empty)
+          for (uint32_t i = lane; i < kWarpSlots; i += 32) tbl[i] = kEmptySlot;
+        __syncwarp();
+        SmallProbe sp;
+        uint32_t slot;
+        if (small_insert(tbl, e, nb, sp, slot)) {
+          kind = kSmall;
+          *mine = lane < nb ? slot : kFull;
+          q0 = sp.mult;
+          q1 = sp.xb;
+          q2 = sp.xm;
+        }
+      }
+      if (kind == kHashed) {
+        const int logb = table_logb(nb);
+        q0 = (uint32_t)logb;
+        q1 = bmin;
+        q2 = bmax;
+        __syncwarp();
+        table_clear(tbl, logb, lane, 32);
+        __syncwarp();
+        table_insert(tbl, logb, g.bent, bs, bs + nb, lane, 32);
+      }
+      __syncwarp();
+    }
+    uint64_t racc;
+    if (kind == kSmall) {
+      racc = sweep_bits(g, ib, il, cs, ce, 1, SmallProbe{tbl, q0, q1, q2}, wruns);
+    } else if (kind == kDirect) {
+      racc = sweep_bits(g, ib, il, cs, ce, 1, [&](uint64_t e) -> uint32_t {
+        const uint32_t o = (uint32_t)(e >> 32) - q0;
+        return o < q1 ? (uint32_t)__popc((uint32_t)e & wmap[o]) : 0u;
+      }, wruns);
+    } else {
+      racc = sweep_bits(g, ib, il, cs, ce, 1, BitmapProbe{tbl, (int)q0, q1, q2}, wruns);
+    }
+    if (per_graph) {
+      const uint64_t s = warp_sum(racc);
+      if (lane == 0 && s) atomicAdd(&per_graph[g.graph_of_rank[u]], (unsigned long long)s);
+    }
+    if (block_ns) {
+      __syncwarp();
+      if (lane == 0) atomicAdd(&block_ns[u >> 5], cycles() - t_start);
+    }
+    acc += racc;
+  };
+  // The merge pieces of rows whose edges all went to the hub pass (most rows of
+  // a power-law graph) are dropped 32 at a time by the flag words alone. What is
+  // left has v's row the shorter list on nearly every edge, so it is probed like
+  // the bitmap pieces (searching either list in the other: RMAT-22 count alone
+  // 7,031 us, now 6,372; searching u's tail where v's row is 8 times as long:
+  // the pieces 1.77 ms, then 1.89).
+  const uint32_t grab = kMerge && len >= 64u * 32u * gridDim.x ? 32u : kGrab;
+  const bool fixed = one_turn(len, kWarpsPerCta * gridDim.x, grab);
+  do {
+    uint32_t t0 = 0;
+    if (lane == 0)
+      t0 = fixed ? (w * gridDim.x + blockIdx.x) * grab : atomicAdd(&stats->cursor[kCurVariant0 + V], grab);
+    t0 = __shfl_sync(kFull, t0, 0);
+    if (t0 >= len) break;
+    if constexpr (kMerge) {
+      // Lane i: piece t0 + i and whether it has edges to count.
+      uint64_t my_pc = 0;
+      bool live = lane < min(grab, len - t0);
+      if (live) {
+        my_pc = pieces[p0 + (len - 1 - t0 - lane)];
+        if (g.eflag) {
+          const uint32_t s = rp_row(g.rp[my_pc >> 32]) + (uint32_t)my_pc;
+          const uint32_t e = min(s + width, rp_row(g.rp[(my_pc >> 32) + 1]));
+          uint32_t left = 0;  // flags not set in [s, e)
+          for (uint32_t k = s >> 5; k <= (e - 1) >> 5; ++k) {
+            uint32_t f = ~g.eflag[k];
+            if (k == s >> 5) f &= kFull << (s & 31);
+            if (k == (e - 1) >> 5) f &= kFull >> (31 - ((e - 1) & 31));
+            left |= f;
+          }
+          live = left != 0;
+        }
+      }
+      for (uint32_t todo = __ballot_sync(kFull, live); todo; todo &= todo - 1)
+        count_piece(__shfl_sync(kFull, my_pc, __ffs(todo) - 1));
+    } else {
+      const uint32_t t1 = min(t0 + grab, len);
+      for (uint32_t t = t0; t < t1; ++t) count_piece(pieces[p0 + (len - 1 - t)]);
+    }
+  } while (!fixed);
+  return acc;
+}
+
+// Five CTAs an SM, 48 registers: six at 40 spill into the sweeps (planted partition,
+// bitmap pieces: 1.46 ms, then 1.92).
+template <int V>
+__global__ void __launch_bounds__(kWarpsPerCta * 32, 5) k_pieces_warp(GraphView g, const uint64_t* __restrict__ pieces,
                                                                     const uint32_t* __restrict__ piece_off,
                                                                     DeviceStats* stats, unsigned long long* per_graph,
-                                                                    unsigned long long* block_ns, bool heavy,
-                                                                    uint32_t width) {
+                                                                    unsigned long long* block_ns, uint32_t width) {
   __shared__ __align__(16) uint64_t smem[kWarpsPerCta][kWarpSlots];
-  __shared__ uint32_t runs[kWarpsPerCta][64];
+  __shared__ uint32_t runs[kWarpsPerCta][96];
   __shared__ uint32_t s_row;
-  const PiecesShared sh{&smem[0][0], kWarpSlots, &runs[0][0], 64, &s_row};
-  uint64_t acc = pieces_body<V>(g, pieces, piece_off, stats, per_graph, block_ns, heavy, width, sh);
+  const PiecesShared sh{&smem[0][0], kWarpSlots, &runs[0][0], 96, &s_row};
+  uint64_t acc = 0;
+  if (V == TRIBIT_VARIANT_BITMAP) acc = heavy_body(g, pieces, piece_off, stats, per_graph, block_ns, sh);
+  acc += pieces_body<V>(g, pieces, piece_off, stats, per_graph, block_ns, width, sh);
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0 && acc) atomicAdd(&stats->triangles, (unsigned long long)acc);
 }
@@ -1561,8 +1664,9 @@ __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t*
   const uint32_t wlen = piece_off[kOffHubAll] - len;
   uint64_t acc = 0;
   // Phase 1: hubs with wide rows, one CTA per piece.
-  for (uint32_t turn = 0;; ++turn) {
-    if (threadIdx.x == 0) s_t = next_pieces(&stats->cursor[kCurHub], len, blockIdx.x, gridDim.x, 1, turn);
+  const bool fixed = one_turn(len, gridDim.x, 1);
+  do {
+    if (threadIdx.x == 0) s_t = fixed ? blockIdx.x : atomicAdd(&stats->cursor[kCurHub], 1u);
     __syncthreads();
     const uint32_t t = s_t;
     if (t >= len) break;
@@ -1644,16 +1748,16 @@ __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t*
         atomicAdd(&block_ns[inrow[e0 + i] >> 5], (unsigned long long)(per_block * (pre[i + 1] - pre[i]) + 0.5));
       __syncthreads();
     }
-  }
+  } while (!fixed);
   // Phase 2: hubs whose row fits a warp's slice of the map, one warp per
   // piece, in wave order.
   uint32_t* wmap = map + w * kHubWarpStride;
-  for (uint32_t turn = 0;; ++turn) {
+  const bool wfixed = one_turn(wlen, kHubWarps * gridDim.x, 1);
+  do {
     uint32_t t0 = 0;
     // (From the last CTA on: the first ones have the CTA pieces of a small graph.)
     if (lane == 0)
-      t0 = next_pieces(&stats->cursor[kCurHubWarp], wlen, w * gridDim.x + gridDim.x - 1 - blockIdx.x,
-                       kHubWarps * gridDim.x, 1, turn);
+      t0 = wfixed ? w * gridDim.x + gridDim.x - 1 - blockIdx.x : atomicAdd(&stats->cursor[kCurHubWarp], 1u);
     const uint32_t t = __shfl_sync(kFull, t0, 0);
     if (t >= wlen) break;
     const unsigned long long t_start = block_ns ? cycles() : 0ull;
@@ -1700,7 +1804,7 @@ __device__ __forceinline__ uint64_t hub_body(const GraphView& g, const uint64_t*
         atomicAdd(&block_ns[inrow[e0 + i] >> 5], (unsigned long long)(per_block * (uint32_t)inl[e0 + i] + 0.5));
     }
     __syncwarp();  // the slice is rewritten for the next piece
-  }
+  } while (!wfixed);
   return acc;
 }
 
@@ -1754,8 +1858,9 @@ __global__ void __launch_bounds__(kHubWarps * 32, TB_HUB_MIN_CTAS) k_queue(
   // (warps), then, once the CTA's warps meet, the hub's CTA pieces and its
   // warp pieces. (Hub CTA pieces right after the heavy rows, before the warp
   // pieces, measured 0.5-3% slower on RMAT-18 to 24.)
-  acc += pieces_body<TRIBIT_VARIANT_BITMAP>(g, pieces, piece_off, stats, per_graph, nullptr, true, width, ps);
-  acc += pieces_body<TRIBIT_VARIANT_MERGE>(g, pieces, piece_off, stats, per_graph, nullptr, false, width, ps);
+  acc += heavy_body(g, pieces, piece_off, stats, per_graph, nullptr, ps);
+  acc += pieces_body<TRIBIT_VARIANT_BITMAP>(g, pieces, piece_off, stats, per_graph, nullptr, width, ps);
+  acc += pieces_body<TRIBIT_VARIANT_MERGE>(g, pieces, piece_off, stats, per_graph, nullptr, width, ps);
   __syncthreads();  // the hub's CTA pieces take the whole map
   acc += hub_body(g, hub_pieces, piece_off, in_off, hub, inl, nullptr, stats, per_graph, nullptr, hs);
   acc = warp_sum(acc);
@@ -2836,7 +2941,7 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
   // heavy row, tile block and hub piece adds its warp-cycles to its row block.
   if (cfg.variant_start) TB_CUDA(cudaEventRecord(cfg.variant_start, st));
   k_pieces_warp<TRIBIT_VARIANT_BITMAP><<<warp_grid, kWarpsPerCta * 32, 0, st>>>(
-      g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, true, s.piece_width);
+      g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, s.piece_width);
   TB_LAUNCH_CHECK();
   if (s.tile_engine == TRIBIT_TILES_TCGEN05)
     k_tiles_tc<<<(unsigned)(sms * kTcCtasPerSm), kTcThreads, sizeof(TcSmem), st>>>(
@@ -2846,16 +2951,16 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
         g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns);
   TB_LAUNCH_CHECK();
   k_pieces_warp<TRIBIT_VARIANT_MERGE><<<warp_grid, kWarpsPerCta * 32, 0, st>>>(
-      g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, false, s.piece_width);
+      g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, s.piece_width);
   TB_LAUNCH_CHECK();
   rows_wide();
   k_hub<<<(unsigned)(sms * kHubCtasPerSm), kHubWarps * 32, 0, st>>>(g, s.hub_pieces, s.piece_off, s.in_off, s.hub,
                                                                      s.inl, s.inrow, stats, per_graph, cfg.block_ns);
   TB_LAUNCH_CHECK();
   if (cfg.variant_stop) TB_CUDA(cudaEventRecord(cfg.variant_stop, st));
-  info.ctas += 2ull * warp_grid +
+  info.ctas += 2ull * warp_grid + 6ull * sms +
                ((s.tile_engine == TRIBIT_TILES_TCGEN05 ? (uint64_t)kTcCtasPerSm : 5ull) + kHubCtasPerSm) * sms;
-  info.kernels += 4;
+  info.kernels += 5;
   return info;
 }
 
