@@ -128,3 +128,45 @@ def test_merge_with_long_neighbour_rows(length):
         far = np.uint64(40 + 32 * length) + np.uint64(64) * np.arange((i % 9) * (length - i), dtype=np.uint64)
         e += [(c << np.uint64(32)) | cols[i + 1:], (c << np.uint64(32)) | far[far < n]]
     check(np.concatenate(e), n, modes=("merge", "bitmap"), orders=("id",))
+
+
+@pytest.mark.parametrize("model", ["kernels", "queue"])
+@pytest.mark.parametrize("engine", ["tcgen05", "mma_sync"])
+@pytest.mark.parametrize("n", [10_000, 300_000])  # from 245,633 vertices on: the wide rows' kernel too
+def test_launch_counts_are_the_launches(model, engine, n):
+    # The counting launch captured into a graph: its kernel nodes and their grids.
+    import ctypes
+
+    import torch
+    cu = ctypes.CDLL("libcuda.so.1")
+    e = tb.gen_er(n, 3 * n, seed=n)
+    d = torch.from_numpy(e.view(np.int64)).cuda()
+    side = torch.cuda.Stream()
+    with tb.Counter() as c:
+        c.set_stream(side.cuda_stream)
+        c.set_tuning(launch_model=model)
+        c.set_tile_engine(engine)
+        c.prepare_device(d.data_ptr(), d.numel(), n)
+        c.launch_count()
+        side.synchronize()
+        stream, graph, num = ctypes.c_void_p(side.cuda_stream), ctypes.c_void_p(), ctypes.c_size_t()
+        assert cu.cuStreamBeginCapture_v2(stream, 1) == 0
+        c.launch_count()
+        assert cu.cuStreamEndCapture(stream, ctypes.byref(graph)) == 0
+        assert cu.cuGraphGetNodes(graph, None, ctypes.byref(num)) == 0
+        nodes = (ctypes.c_void_p * num.value)()
+        assert cu.cuGraphGetNodes(graph, nodes, ctypes.byref(num)) == 0
+        kernels = ctas = 0
+        for node in nodes:
+            kind, params = ctypes.c_int(), (ctypes.c_uint32 * 32)()
+            assert cu.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+            if kind.value != 0:  # CU_GRAPH_NODE_TYPE_KERNEL
+                continue
+            assert cu.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(node), params) == 0
+            kernels += 1
+            ctas += params[2] * params[3] * params[4]  # the grid follows the function's pointer
+        assert cu.cuGraphDestroy(graph) == 0
+        r = c.read_count()
+        assert (r.count_kernels, r.blocks_of_threads) == (kernels, ctas)
+        assert kernels == {"kernels": 4, "queue": 2}[model] + (n > 245_632)
+        c.set_stream(0)

@@ -2909,31 +2909,37 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
   const unsigned warp_grid = (unsigned)(sms * per_sm);
   LaunchInfo info;
   TB_CUDA(cudaMemsetAsync(&stats->triangles, 0, sizeof(DeviceStats) - offsetof(DeviceStats, triangles), st));
-  // Wide rows span more blocks than the heavy phase's masks, so smaller graphs have none.
-  const bool wide = ceil_div<uint64_t>(g.n, 32) > kHeavyMaxSpan;
-  auto rows_wide = [&] {
-    if (!wide) return;
-    k_rows_wide<<<(unsigned)sms, kCtaThreads, sizeof(uint64_t) << kCtaLogSlots, st>>>(g, s.pieces, s.piece_off, stats,
-                                                                                      per_graph, cfg.block_ns);
+  auto launched = [&](uint64_t ctas) {  // after every launch: checks it and counts it
     TB_LAUNCH_CHECK();
-    info.ctas += sms;
+    info.ctas += ctas;
     ++info.kernels;
   };
+  auto tiles = [&] {
+    const bool tc = s.tile_engine == TRIBIT_TILES_TCGEN05;
+    const unsigned grid = (unsigned)(sms * (tc ? kTcCtasPerSm : 5));
+    if (tc)
+      k_tiles_tc<<<grid, kTcThreads, sizeof(TcSmem), st>>>(g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns,
+                                                           cfg.tile_wait_polls, cfg.tile_test_no_commit);
+    else
+      k_tiles_mma<<<grid, kTileWarps * 32, kTileWarps * sizeof(TileSmem), st>>>(g, s.pieces, s.piece_off, stats,
+                                                                                per_graph, cfg.block_ns);
+    launched(grid);
+  };
+  // Wide rows span more blocks than the heavy phase's masks, so smaller graphs have none.
+  auto rows_wide = [&] {
+    if (ceil_div<uint64_t>(g.n, 32) <= kHeavyMaxSpan) return;
+    k_rows_wide<<<(unsigned)sms, kCtaThreads, sizeof(uint64_t) << kCtaLogSlots, st>>>(g, s.pieces, s.piece_off, stats,
+                                                                                      per_graph, cfg.block_ns);
+    launched(sms);
+  };
+  const unsigned hub_grid = (unsigned)(sms * kHubCtasPerSm);
   if (cfg.queue && !cfg.block_ns && !cfg.variant_start) {
     // One persistent kernel for the row pieces and the hub pass; the tiles and
-    // the fallback rows (whose list k_queue fills) after it.
-    k_queue<<<(unsigned)(sms * kHubCtasPerSm), kHubWarps * 32, 0, st>>>(
-        g, s.pieces, s.piece_off, stats, per_graph, s.piece_width, s.hub_pieces, s.in_off, s.hub, s.inl);
-    TB_LAUNCH_CHECK();
-    if (s.tile_engine == TRIBIT_TILES_TCGEN05)
-      k_tiles_tc<<<(unsigned)(sms * kTcCtasPerSm), kTcThreads, sizeof(TcSmem), st>>>(
-          g, s.pieces, s.piece_off, stats, per_graph, nullptr, cfg.tile_wait_polls, cfg.tile_test_no_commit);
-    else
-      k_tiles_mma<<<(unsigned)(sms * 5), kTileWarps * 32, kTileWarps * sizeof(TileSmem), st>>>(
-          g, s.pieces, s.piece_off, stats, per_graph, nullptr);
-    TB_LAUNCH_CHECK();
-    info.ctas = (uint64_t)(kHubCtasPerSm + (s.tile_engine == TRIBIT_TILES_TCGEN05 ? kTcCtasPerSm : 5)) * sms;
-    info.kernels = 2;
+    // the wide rows after it.
+    k_queue<<<hub_grid, kHubWarps * 32, 0, st>>>(g, s.pieces, s.piece_off, stats, per_graph, s.piece_width,
+                                                 s.hub_pieces, s.in_off, s.hub, s.inl);
+    launched(hub_grid);
+    tiles();
     rows_wide();
     return info;
   }
@@ -2942,25 +2948,16 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
   if (cfg.variant_start) TB_CUDA(cudaEventRecord(cfg.variant_start, st));
   k_pieces_warp<TRIBIT_VARIANT_BITMAP><<<warp_grid, kWarpsPerCta * 32, 0, st>>>(
       g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, s.piece_width);
-  TB_LAUNCH_CHECK();
-  if (s.tile_engine == TRIBIT_TILES_TCGEN05)
-    k_tiles_tc<<<(unsigned)(sms * kTcCtasPerSm), kTcThreads, sizeof(TcSmem), st>>>(
-        g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, cfg.tile_wait_polls, cfg.tile_test_no_commit);
-  else
-    k_tiles_mma<<<(unsigned)(sms * 5), kTileWarps * 32, kTileWarps * sizeof(TileSmem), st>>>(
-        g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns);
-  TB_LAUNCH_CHECK();
+  launched(warp_grid);
+  tiles();
   k_pieces_warp<TRIBIT_VARIANT_MERGE><<<warp_grid, kWarpsPerCta * 32, 0, st>>>(
       g, s.pieces, s.piece_off, stats, per_graph, cfg.block_ns, s.piece_width);
-  TB_LAUNCH_CHECK();
+  launched(warp_grid);
   rows_wide();
-  k_hub<<<(unsigned)(sms * kHubCtasPerSm), kHubWarps * 32, 0, st>>>(g, s.hub_pieces, s.piece_off, s.in_off, s.hub,
-                                                                     s.inl, s.inrow, stats, per_graph, cfg.block_ns);
-  TB_LAUNCH_CHECK();
+  k_hub<<<hub_grid, kHubWarps * 32, 0, st>>>(g, s.hub_pieces, s.piece_off, s.in_off, s.hub, s.inl, s.inrow, stats,
+                                             per_graph, cfg.block_ns);
+  launched(hub_grid);
   if (cfg.variant_stop) TB_CUDA(cudaEventRecord(cfg.variant_stop, st));
-  info.ctas += 2ull * warp_grid + 6ull * sms +
-               ((s.tile_engine == TRIBIT_TILES_TCGEN05 ? (uint64_t)kTcCtasPerSm : 5ull) + kHubCtasPerSm) * sms;
-  info.kernels += 5;
   return info;
 }
 
