@@ -525,9 +525,10 @@ constexpr uint32_t kCtaSortSmem = 8192;  // bitonic rows longer than this are so
 // block left them to a few warps (RMAT-20: the row sort 607 us, the emit 487).
 struct LongRows {
   uint32_t* rows;   // n + 1
-  uint32_t* count;  // [0] CTA rows, [1] warp rows, [2] scratch words taken by CTA rows
+  uint32_t* count;  // kLongWords words, 8-byte aligned: CTA rows, warp rows, a SortSpace of scratch words taken by CTA rows
+  __device__ __forceinline__ SortSpace* taken() const { return reinterpret_cast<SortSpace*>(count + 2); }
 };
-constexpr uint64_t kLongWords = 3;
+constexpr uint64_t kLongWords = 2 + sizeof(SortSpace) / sizeof(uint32_t);
 
 // Bitonic sort of the warp's 32 K values, value r * 32 + lane in x[r] of
 // lane lane, ascending.
@@ -751,11 +752,11 @@ __global__ void __launch_bounds__(kLongThreads, 4)
   __shared__ uint32_t sm[kBitWords];
   __shared__ uint32_t wsum[2][kLongThreads / 32];
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  __shared__ uint32_t s_at;
+  __shared__ SortSpace s_at;
   auto take = [&](uint32_t words) {  // the CTA's next slice of scratch
-    if (tid == 0) s_at = atomicAdd(&lng.count[2], words);
+    if (tid == 0) s_at = atomicAdd(lng.taken(), (SortSpace)words);
     __syncthreads();
-    const uint32_t at = s_at;
+    const SortSpace at = s_at;
     __syncthreads();
     return at;
   };
@@ -1411,7 +1412,7 @@ void rank_vertices(const uint32_t* deg, uint64_t n, const RankBuffers& b, uint32
 
 void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* out) {
   const uint64_t n = in.n, E = in.E;
-  if (n > 0xffffffffull || E > 0xfffffffeull)
+  if (n > 0xffffffffull || E > kMaxEntries)
     throw StatusError(TRIBIT_ERR_TOO_LARGE, "graphs are limited to 2^32-1 vertices and 2^32-2 entries");
   const bool by_degree = in.order == TRIBIT_ORDER_DEGREE;
   DeviceStats* stats = ar.take<DeviceStats>(1);

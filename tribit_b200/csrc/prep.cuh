@@ -34,6 +34,13 @@ struct GraphView {
 __device__ __forceinline__ uint32_t rp_row(uint64_t w) { return (uint32_t)(w >> 32); }
 __device__ __forceinline__ uint32_t rp_blk(uint64_t w) { return (uint32_t)w; }
 
+constexpr uint64_t kMaxEntries = 0xfffffffeull;  // of one graph or batch
+
+// Words of sort space handed out to the long rows of one build: up to two an
+// entry, which passes 32 bits from 2^31 entries on.
+using SortSpace = unsigned long long;
+static_assert(2 * kMaxEntries <= (SortSpace)-1, "every long row's slice lies after the one before");
+
 // Counters the device writes and the host reads back once per call.
 constexpr int kScheduleWords = 12;
 struct DeviceStats {
