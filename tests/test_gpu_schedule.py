@@ -1,6 +1,6 @@
 """Branches of the preprocessing and the schedule at the sizes where they
 change, against the oracle: vertex ranks (one CTA up to 16,384 vertices, radix
-passes beyond; exact degrees up to 32,767), scans (one CTA up to 32,768
+passes beyond; hubs of 32,768 and more placed by their full degrees), scans (one CTA up to 32,768
 elements), degree counting over sorted and skewed input, heavy and wide rows
 cut into pieces, and groups of short rows. Counts are integers: equality."""
 import numpy as np
@@ -8,6 +8,7 @@ import pytest
 
 import oracle
 import tribit_b200 as tb
+from tests.graphs import zip_pairs
 from tests.test_gpu_rows import fans
 
 pytestmark = pytest.mark.gpu
@@ -28,12 +29,67 @@ def test_sizes_around_the_one_cta_kernels(n):
 
 
 def test_degrees_past_the_exact_keys():
-    # Hubs of 32,767 to 70,000 neighbours: their degree keys keep 11 leading bits.
+    # Hubs of 32,767 to 70,000 neighbours: keys of 11 leading bits, then their full degrees.
     n = 80_000
     parts = [tb.gen_er(n, 200_000, seed=5)]
     for hub, k in enumerate((32767, 32768, 33000, 40000, 65535, 65536, 70000)):
         parts.append((np.uint64(hub) << np.uint64(32)) | (np.uint64(100) + np.arange(k, dtype=np.uint64)))
     check(np.concatenate(parts), n, orders=("degree",))
+
+
+def hubs_of_near_equal_degree(n, hubs, times):
+    """`hubs` vertices of 32,768 and more entries, one entry less an id, the first five joined to all hubs; the rest
+    of their entries name the other vertices, each about `times` times."""
+    i, j = np.triu_indices(hubs, 1)
+    i, j = i[i < 5], j[i < 5]
+    parts = [zip_pairs(np.stack([i, j], 1))]
+    joined = np.bincount(i, minlength=hubs) + np.bincount(j, minlength=hubs)
+    others = hubs + np.arange(-(-(32_768 + hubs) // times), dtype=np.uint64)
+    assert others[-1] < n
+    for h in range(hubs):
+        parts.append((np.uint64(h) << np.uint64(32)) | np.resize(others, 32_768 + hubs - 1 - h - joined[h]))
+    return np.random.default_rng(n).permutation(np.concatenate(parts))
+
+
+def rows_in_degree_order(e, n):
+    """(neighbours, longest row) of every 32-row block under (degree, id) order, degrees counted with duplicates."""
+    a, b = (e >> np.uint64(32)).astype(np.int64), (e & np.uint64(0xFFFFFFFF)).astype(np.int64)
+    a, b = a[a != b], b[a != b]
+    rank = np.empty(n, dtype=np.int64)
+    rank[np.argsort(np.bincount(a, minlength=n) + np.bincount(b, minlength=n), kind="stable")] = np.arange(n)
+    lo, hi = np.minimum(rank[a], rank[b]), np.maximum(rank[a], rank[b])
+    rows = np.bincount(np.unique(lo * n + hi) // n, minlength=-(-n // 32) * 32).reshape(-1, 32)
+    return rows.sum(1), rows.max(1)
+
+
+@pytest.mark.parametrize("n, hubs, times", [(11_101, 45, 3), (16_001, 40, 4), (16_545, 45, 2), (90_001, 60, 1)])
+@pytest.mark.parametrize("call", ["device", "host", "batch", "budget"])
+def test_hubs_of_near_equal_degree_are_ranked_by_degree(n, hubs, times, call):
+    # Degrees that share their leading 11 bits, falling with the id, over a row-block
+    # border: ranked by id, every hub's row would hold the wrong hubs. The features
+    # give a block's neighbours and its longest row, log2(1 + x) in fp32.
+    import torch
+    e = hubs_of_near_equal_degree(n, hubs, times)
+    with tb.Counter() as c:
+        base = 0
+        if call == "device":
+            d = torch.from_numpy(e.view(np.int64)).cuda()
+            c.prepare_device(d.data_ptr(), d.numel(), n)
+        elif call == "host":
+            c.count_edges(e, n)
+        elif call == "batch":  # after two small graphs of 32 and 64 vertices
+            small = [tb.gen_er(32, 100, seed=1), tb.gen_er(64, 100, seed=2)]
+            c.count_batch(np.concatenate(small + [e]), np.array([0, 100, 200, 200 + e.size], dtype=np.uint64),
+                          np.array([32, 64, n], dtype=np.uint32))
+            base = 3
+        else:
+            c.set_stream_options("rows")
+            c.set_device_budget(c.device_bytes(e.size, n) * 3 // 4)
+            assert c.count_edges(e, n).stream_tier == 1
+        f = c.block_features().astype(np.float64)[base:]
+    nnz, longest = rows_in_degree_order(e, n)
+    np.testing.assert_allclose(np.exp2(f[:, 1]) - 1, nnz, rtol=1e-5, atol=1e-5)
+    np.testing.assert_allclose(np.exp2(f[:, 5]) - 1, longest, rtol=1e-5, atol=1e-5)
 
 
 @pytest.mark.parametrize("kind", ["sorted", "reversed", "one_hub", "self_loops"])

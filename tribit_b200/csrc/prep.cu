@@ -182,18 +182,20 @@ __device__ __forceinline__ uint32_t graph_of_vertex(const uint64_t* voff, uint32
 
 // Vertices are ranked by (graph, degree, id) through a degree key of `bits`
 // bits, two radix passes at 16: degrees below 2^(bits - 1) are exact, larger
-// ones keep their leading bit and the next `mant` ones, so the order is the
-// degrees' but for ties of near-equal hubs (any total order counts each
-// triangle once; this one only bounds the rows' lengths). mant < 0, when many
-// graphs leave few bits: degrees past the range are equal.
+// ones (hubs, at most 2E >> (bits - 1) of them) keep their leading bit and the
+// next `mant` ones. Hubs that share a key lie side by side after the sort and
+// are then placed by their degrees (hub_place), so the order is the full
+// degrees' in half the passes. mant < 0, when many graphs leave fewer than
+// kDegreeBits: degrees are capped at 2^bits - 1.
 struct DegreeKey {
   int bits, mant;
 };
+constexpr int kDegreeBits = 16;
 inline DegreeKey degree_key_of(int bits) {
-  if (bits >= 32) return {32, -1};  // exact
-  if (bits < 1) return {0, -1};     // as many graphs as keys: degrees are not told apart
-  int m = bits - 1;                 // (33 - bits) leading bits times 2^m must fit above 2^(bits - 1)
-  while (m >= 0 && ((33ll - bits) << m) > (1ll << (bits - 1))) --m;
+  if (bits >= 32) return {32, -1};           // exact
+  if (bits < kDegreeBits) return {bits, -1};  // at 0, degrees are not told apart
+  int m = bits - 1;                          // (33 - bits) leading bits times 2^m must fit above 2^(bits - 1)
+  while (((33ll - bits) << m) > (1ll << (bits - 1))) --m;
   return {bits, m};
 }
 __device__ __forceinline__ uint32_t degree_key(uint32_t d, DegreeKey k) {
@@ -205,7 +207,20 @@ __device__ __forceinline__ uint32_t degree_key(uint32_t d, DegreeKey k) {
   const int e = 31 - __clz(d);  // >= bits - 1 > mant
   return half + ((uint32_t)(e - (k.bits - 1)) << k.mant) + ((d >> (e - k.mant)) & ((1u << k.mant) - 1u));
 }
-constexpr int kDegreeBits = 16;
+// Whether vertices of other degrees may share the key (graph bits above it, if any).
+__device__ __forceinline__ bool hub_key(uint32_t key, DegreeKey k) {
+  return k.mant >= 0 && ((key >> (k.bits - 1)) & 1u);
+}
+// Place in (key, degree, id) order of the vertex at place r of the stable (key,
+// id) order of n vertices, its key a hub key. key_at(p), degree_at(p): of the vertex at place p.
+template <class KeyAt, class DegreeAt>
+__device__ __forceinline__ uint64_t hub_place(uint64_t r, uint64_t n, const KeyAt& key_at, const DegreeAt& degree_at) {
+  const uint32_t key = key_at(r), d = degree_at(r);
+  uint64_t at = r;
+  for (uint64_t p = r; p > 0 && key_at(p - 1) == key; --p) at -= degree_at(p - 1) > d;
+  for (uint64_t p = r + 1; p < n && key_at(p) == key; ++p) at += degree_at(p) < d;
+  return at;
+}
 
 // keys[v] = (graph << bits) | degree key. A stable sort of these keys over ids
 // 0..n-1 gives the (graph, degree, id) order.
@@ -232,17 +247,20 @@ struct RowWords {
 };
 
 // rank[id] = v0 + position, and the row words (from the first rank's on).
-__global__ void k_rank_scatter(const uint32_t* __restrict__ sorted_ids, uint64_t v0, uint64_t n,
-                               uint32_t* __restrict__ rank,
+__global__ void k_rank_scatter(const uint32_t* __restrict__ sorted_keys, const uint32_t* __restrict__ sorted_ids,
+                               uint64_t v0, uint64_t n, DegreeKey dk, uint32_t* __restrict__ rank,
                                const uint64_t* voff, uint32_t G, uint32_t* __restrict__ graph_of_rank,
                                const uint32_t* __restrict__ deg, RowWords rw) {
   const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (uint64_t i = n + r; i < rw.count; i += (uint64_t)gridDim.x * blockDim.x) rw.w[i] = 0;
   if (r >= n) return;
-  uint32_t v = sorted_ids[r];
-  rank[v] = (uint32_t)(v0 + r);
-  if (r < rw.count) rw.w[r] = rw.slots ? deg[v] : 0u;
-  if (graph_of_rank) graph_of_rank[v0 + r] = graph_of_vertex(voff, G, v);
+  const uint32_t v = sorted_ids[r];
+  uint64_t at = r;
+  if (hub_key(sorted_keys[r], dk))
+    at = hub_place(r, n, [&](uint64_t p) { return sorted_keys[p]; }, [&](uint64_t p) { return deg[sorted_ids[p]]; });
+  rank[v] = (uint32_t)(v0 + at);
+  if (at < rw.count) rw.w[at] = rw.slots ? deg[v] : 0u;
+  if (graph_of_rank) graph_of_rank[v0 + at] = graph_of_vertex(voff, G, v);
 }
 
 // The same ranks for one graph of at most kRankOneMax vertices, by one CTA:
@@ -307,6 +325,21 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_one(const uint32_t* __res
       if (r >= (int)rounds) break;
       const uint32_t i = (w * rounds + r) * 32 + lane;
       if (i < n) dst[wcnt[w * 256 + ((v[r] >> shift) & 255u)] + pos[r]] = v[r];
+    }
+    __syncthreads();
+    uint32_t* t = src;
+    src = dst;
+    dst = t;
+  }
+  bool hubs = false;
+  for (uint32_t i = tid; i < n; i += kRankThreads) hubs |= hub_key(src[i] >> 16, dk);
+  if (__syncthreads_or(hubs ? 1 : 0)) {
+    for (uint32_t i = tid; i < n; i += kRankThreads) {
+      uint32_t at = i;
+      if (hub_key(src[i] >> 16, dk))
+        at = (uint32_t)hub_place(i, n, [&](uint64_t p) { return src[p] >> 16; },
+                                 [&](uint64_t p) { return deg[src[p] & 0xFFFFu]; });
+      dst[at] = src[i];
     }
     __syncthreads();
     uint32_t* t = src;
@@ -1310,15 +1343,17 @@ void rank_by_degree(const uint32_t* deg, uint64_t v0, uint64_t n, const uint64_t
     TB_LAUNCH_CHECK();
     return;
   }
-  // Whole radix passes over graph bits and at least 12 degree bits.
+  // Whole radix passes over the graph bits and, where 32 bits leave as many, kDegreeBits of degree.
   const int gbits = G ? bits_for((uint64_t)(g1 - g0)) : 0;
-  const int total = std::min(32, std::max(kDegreeBits, (gbits + 12 + 7) / 8 * 8));
+  const int total = std::min(32, (gbits + kDegreeBits + 7) / 8 * 8);
   const DegreeKey dk = degree_key_of(total - gbits);
   k_vertex_keys<<<grid_for(n), kThreads, 0, st>>>(deg, v0, n, voff, G, g0, dk, b.vk, b.vv);
   TB_LAUNCH_CHECK();
   uint32_t* sorted_ids = nullptr;
-  radix_sort<uint32_t, uint32_t, true>(b.vk, b.vk2, b.vv, b.vv2, n, total, b.tmp, st, &sorted_ids);
-  k_rank_scatter<<<grid_for(n), kThreads, 0, st>>>(sorted_ids, v0, n, rank, voff, G, graph_of_rank, deg, rw);
+  const uint32_t* sorted_keys =
+      radix_sort<uint32_t, uint32_t, true>(b.vk, b.vk2, b.vv, b.vv2, n, total, b.tmp, st, &sorted_ids);
+  k_rank_scatter<<<grid_for(n), kThreads, 0, st>>>(sorted_keys, sorted_ids, v0, n, dk, rank, voff, G, graph_of_rank, deg,
+                                                   rw);
   TB_LAUNCH_CHECK();
 }
 
