@@ -208,3 +208,68 @@ def test_streamed_rows_tier_on_a_million_vertices(pinned):
             assert _schedule(r)[:2] == _schedule(want)[:2]
             c.set_device_budget(0)
             c.set_stream_options("auto", 0)
+
+
+def test_one_piece_count_in_the_least_memory():
+    # Rows without degree-sized slots, 4 bytes an entry less: 8 bytes staged, 4
+    # of rows, 8 of scratch, 4 + 8 of CSR and bit rows, 8 of hub in-lists, and
+    # less than 1 of pieces and flags.
+    n, E = 60_000, 1_000_000
+    e = tb.gen_chung_lu(n, E, 2.1, 3000.0, seed=6)
+    want = oracle.count(e, n)
+    with tb.Counter() as c:
+        need = c.device_bytes(E, n)
+        assert (c.device_bytes(2 * E, n) - need) / E < 41
+        for budget in (need, need + 2 * E, need + 4 * E, 0):
+            c.set_device_budget(budget)
+            r = c.count_edges(e, n)
+            assert (r.triangles, r.edges, r.stream_ranges) == (*want, 1), budget
+        c.set_device_budget(need - 4096)
+        r = c.count_edges(e, n)
+        assert (r.triangles, r.edges) == want and r.stream_tier in (ROWS, PAIRS)
+
+
+@pytest.mark.parametrize("call", ["device", "prepare", "batch"])
+def test_calls_that_only_compact_rows_leave_room_for(call):
+    # All but a little more than the compact layout's device memory (33 bytes an
+    # entry and 8 staged, see above) is taken by another allocation, so the
+    # arena with degree-sized slots (4 bytes an entry more) cannot be had.
+    import torch
+    n, E = 1 << 20, 50_000_000
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randint(0, n, (2, E), generator=g, device="cuda", dtype=torch.int64)
+    d = (x[0] << 32) | x[1]
+    host = d.cpu().numpy().view(np.uint64) if call == "batch" else None
+    off, nodes = np.array([0, E], dtype=np.uint64), np.array([n], dtype=np.uint32)
+
+    def count(c):
+        if call == "batch":
+            per_graph, r = c.count_batch(host, off, nodes)
+            return int(per_graph[0]), r.edges
+        if call == "device":
+            r = c.count_edges_device(d.data_ptr(), E, n)
+        else:
+            m = c.prepare_device(d.data_ptr(), E, n).edges
+            c.launch_count()
+            r = c.read_count()
+            assert r.edges == m
+        return r.triangles, r.edges
+
+    with tb.Counter() as c:
+        want = count(c)
+        room = c.device_bytes(0, n) + (42 if call == "batch" else 34) * E
+    del x
+    with tb.Counter() as c:
+        c.count_edges(tb.gen_er(100, 300, seed=1), 100)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        other = torch.empty(free - room, dtype=torch.uint8, device="cuda")
+        try:
+            assert torch.cuda.mem_get_info()[0] < room + E
+            assert count(c) == want
+            left = torch.cuda.mem_get_info()[0]
+            assert count(c) == want and torch.cuda.mem_get_info()[0] == left  # the arena is kept
+        finally:
+            del other
+            torch.cuda.empty_cache()

@@ -53,15 +53,35 @@ void layout(tribit_context* c, bool measure, const tb::PrepInput& in, bool stage
   (void)tb::take_schedule(ar, in.n, in.E, nullptr);
 }
 
+// The arena of one call: rows in degree-sized slots where their 4 bytes an
+// entry more can be had, else compact rows. (An arena that would have to grow
+// past the free memory is not given up for the attempt.)
+void reserve_layout(tribit_context* c, tb::PrepInput& in, bool stage, uint32_t G, CallLayout* L) {
+  layout(c, true, in, stage, G, L);
+  size_t fr = 0, tot = 0;
+  if (!in.compact && c->arena.used() > c->arena.capacity()) {
+    TB_CUDA(cudaMemGetInfo(&fr, &tot));
+    in.compact = c->arena.used() > fr + c->arena.capacity();
+    if (in.compact) layout(c, true, in, stage, G, L);
+  }
+  try {
+    c->arena.reserve(c->arena.used(), c->device_budget == 0);
+  } catch (const StatusError& e) {
+    if (e.status != TRIBIT_ERR_OUT_OF_MEMORY || in.compact) throw;
+    in.compact = true;
+    layout(c, true, in, stage, G, L);
+    c->arena.reserve(c->arena.used(), c->device_budget == 0);
+  }
+  layout(c, false, in, stage, G, L);
+}
+
 // Runs preprocessing + schedule (+ counting when count == true) for one input.
 void run_call(tribit_context* c, tb::PrepInput in, const uint64_t* host_entries, const uint64_t* host_eoff,
               const uint64_t* host_voff, uint32_t G, bool count, tribit_result* res) {
   DeviceGuard dg(c->device);
   const bool stage = host_entries != nullptr;
   CallLayout L;
-  layout(c, true, in, stage, G, &L);
-  c->arena.reserve(c->arena.used(), c->device_budget == 0);
-  layout(c, false, in, stage, G, &L);
+  reserve_layout(c, in, stage, G, &L);
   cudaStream_t st = c->st;
   TB_CUDA(cudaEventRecord(c->ev[0], st));
   if (G) {
@@ -132,11 +152,12 @@ void run_call(tribit_context* c, tb::PrepInput in, const uint64_t* host_entries,
 
 namespace tb {
 
-size_t call_bytes(tribit_context* c, uint64_t E, uint64_t n, int order, bool stage) {
+size_t call_bytes(tribit_context* c, uint64_t E, uint64_t n, int order, bool stage, bool compact) {
   tb::PrepInput in;
   in.E = E;
   in.n = n;
   in.order = order;
+  in.compact = compact;
   CallLayout L;
   layout(c, true, in, stage, 0, &L);
   return c->arena.used();
@@ -283,8 +304,8 @@ tribit_status tribit_count_edges(tribit_context* c, const uint64_t* entries, uin
                                  tribit_result* out) {
   if (!c || (!entries && n_entries)) return TRIBIT_ERR_INVALID_ARGUMENT;
   return guarded(c, [&] {
-    if (entries && tb::count_streamed_if_needed(c, entries, n_entries, num_nodes, out)) return;
     tb::PrepInput in;
+    if (entries && tb::count_streamed_if_needed(c, entries, n_entries, num_nodes, &in.compact, out)) return;
     in.E = n_entries;
     in.n = num_nodes;
     in.order = c->opts.order;
@@ -301,7 +322,7 @@ tribit_status tribit_count_edges(tribit_context* c, const uint64_t* entries, uin
 
 tribit_status tribit_device_bytes(tribit_context* c, uint64_t n_entries, uint64_t num_nodes, uint64_t* bytes) {
   if (!c || !bytes) return TRIBIT_ERR_INVALID_ARGUMENT;
-  return guarded(c, [&] { *bytes = tb::call_bytes(c, n_entries, num_nodes, c->opts.order, true); });
+  return guarded(c, [&] { *bytes = tb::call_bytes(c, n_entries, num_nodes, c->opts.order, true, true); });
 }
 
 tribit_status tribit_count_edges_device(tribit_context* c, const uint64_t* d_entries, uint64_t n_entries,

@@ -105,8 +105,9 @@ tribit_status guarded(tribit_context* ctx, F&& body) {
 void apply_dispatch(tribit_context* c, cudaStream_t st);
 
 // Device bytes of the context's arena for one count of E entries on n
-// vertices in `order` (stage: host input staged on the device).
-size_t call_bytes(tribit_context* c, uint64_t E, uint64_t n, int order, bool stage);
+// vertices in `order` (stage: host input staged on the device; compact:
+// PrepInput::compact, the least a count takes).
+size_t call_bytes(tribit_context* c, uint64_t E, uint64_t n, int order, bool stage, bool compact);
 // One count of E device entries on n vertices in `order` with the context's
 // dispatcher (tribit_count_edges_device with an explicit order).
 void count_device_input(tribit_context* c, const uint64_t* d_entries, uint64_t E, uint64_t n, int order,
@@ -116,8 +117,10 @@ void count_device_input(tribit_context* c, const uint64_t* d_entries, uint64_t E
 void read_stats(tribit_context* c, cudaStream_t st);
 void fill_schedule_stats(const tribit_context* c, tribit_result* res);
 // Counts host entries in rank ranges when their buffers exceed the device
-// budget (stream.cu). Returns false, doing nothing, when they fit.
-bool count_streamed_if_needed(tribit_context* c, const uint64_t* host, uint64_t E, uint64_t n, tribit_result* res);
+// budget (stream.cu). Returns false, doing nothing, when they fit; *compact:
+// whether only with compact rows.
+bool count_streamed_if_needed(tribit_context* c, const uint64_t* host, uint64_t E, uint64_t n, bool* compact,
+                              tribit_result* res);
 // Copies bytes of host memory to device memory through the context's two
 // pinned buffers (host threads fill one while the other's copy runs).
 void upload_via_pinned(tribit_context* c, const void* src, size_t bytes, void* dst);

@@ -568,11 +568,15 @@ void count_rows_tier(tribit_context* c, const RowsSource& src, const std::vector
   res->stream_tier = TRIBIT_STREAM_ROWS;
 }
 
-bool count_streamed_if_needed(tribit_context* c, const uint64_t* host, uint64_t E, uint64_t n, tribit_result* res) {
+bool count_streamed_if_needed(tribit_context* c, const uint64_t* host, uint64_t E, uint64_t n, bool* compact,
+                              tribit_result* res) {
   DeviceGuard dg(c->device);
+  *compact = false;
   if (n == 0 || E == 0) return false;
   const uint64_t budget = budget_bytes(c);
-  if (call_bytes(c, E, n, c->opts.order, true) <= budget) return false;
+  if (call_bytes(c, E, n, c->opts.order, true, false) <= budget) return false;
+  *compact = true;
+  if (call_bytes(c, E, n, c->opts.order, true, true) <= budget) return false;
   if (n > 0x7fffffffull)
     throw StatusError(TRIBIT_ERR_TOO_LARGE, "counting in rank ranges takes fewer than 2^31 vertices");
   const auto t0 = std::chrono::steady_clock::now();
@@ -676,10 +680,10 @@ bool count_streamed_if_needed(tribit_context* c, const uint64_t* host, uint64_t 
     cap = plan.cap;
   } else {
     const uint64_t n2 = 2 * n;
-    const uint64_t fixed = call_bytes(c, 0, n2, TRIBIT_ORDER_ID, false);
+    const uint64_t fixed = call_bytes(c, 0, n2, TRIBIT_ORDER_ID, false, true);
     const uint64_t probe = 1ull << 20;
     const uint64_t per_entry =
-        (call_bytes(c, probe, n2, TRIBIT_ORDER_ID, false) - fixed) / probe + 1 + sizeof(uint64_t);
+        (call_bytes(c, probe, n2, TRIBIT_ORDER_ID, false, true) - fixed) / probe + 1 + sizeof(uint64_t);
     if (budget <= fixed)
       throw StatusError(TRIBIT_ERR_OUT_OF_MEMORY, "the device budget is below a range task's per-vertex buffers");
     cap = std::min<uint64_t>((budget - fixed) / per_entry / 3, 0xfffffffeull / 3);
