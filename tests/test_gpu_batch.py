@@ -92,3 +92,56 @@ def test_queue_kernel_matches_oracle(dispatch):
             for _ in range(2):
                 c.launch_count()
                 assert c.read_count().triangles == want[0]
+
+
+def _device_work(call):
+    """Names of the copies and kernels that call() puts on the device."""
+    from torch.profiler import ProfilerActivity, profile
+    torch.zeros(1, device="cuda")
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    return [e.name for e in prof.events()]
+
+
+@pytest.mark.parametrize("before, after, E", [(0, 0, 1 << 20), (0, 0, 3_000_017), (3, 40, 9_000_017), (40, 0, 9_000_001)])
+def test_batch_that_one_graph_dominates(before, after, E):
+    # The large graph is copied in pieces, its degrees counted as they land.
+    rng = np.random.default_rng(E + before)
+    nodes = [int(k) for k in rng.integers(2, 60, before)] + [50_000] + [int(k) for k in rng.integers(2, 60, after)]
+    parts = [tb.gen_er(k, 100, seed=i) if k < 60 else tb.gen_er(k, E, seed=i) for i, k in enumerate(nodes)]
+    off = np.concatenate([[0], np.cumsum([p.size for p in parts])]).astype(np.uint64)
+    e = torch.from_numpy(np.concatenate(parts).view(np.int64)).pin_memory().numpy().view(np.uint64)
+    want = [oracle.count(p, k)[0] for p, k in zip(parts, nodes)]
+    with tb.Counter() as c:
+        for _ in range(2):
+            got, r = c.count_batch(e, off, np.asarray(nodes, dtype=np.uint32))
+            assert got.tolist() == want and r.triangles == sum(want)
+        work = _device_work(lambda: c.count_batch(e, off, np.asarray(nodes, dtype=np.uint32)))
+        pieces = max(1, min(8, e.size >> 20))
+        assert sum("k_degree" in w for w in work) >= pieces
+        assert sum("Memcpy HtoD" in w for w in work) >= pieces + 2  # and the offsets
+        e[-1 if not after else int(off[before + 1]) - 1] = (1 << 32) | 50_000  # in its last piece
+        with pytest.raises(tb.TribitError) as ex:
+            c.count_batch(e, off, np.asarray(nodes, dtype=np.uint32))
+        assert ex.value.status == 5
+
+
+def test_batch_with_a_graph_that_presorts():
+    # 2^27 entries: 128 copies of a graph's, each in another order, before and after small graphs.
+    base = tb.gen_rmat(15, 32, seed=3)
+    rng = np.random.default_rng(2)
+    big = np.concatenate([np.roll(base, int(rng.integers(base.size))) for _ in range((1 << 27) // base.size)])
+    small = [tb.gen_er(500, 3_000, seed=i) for i in range(6)]
+    parts, nodes = small[:3] + [big] + small[3:], [500] * 3 + [1 << 15] + [500] * 3
+    assert big.size == 1 << 27
+    off = np.concatenate([[0], np.cumsum([p.size for p in parts])]).astype(np.uint64)
+    want = [oracle.count(base if p is big else p, k) for p, k in zip(parts, nodes)]
+    e = np.concatenate(parts)
+    nodes, got = np.asarray(nodes, dtype=np.uint32), []
+    with tb.Counter() as c:
+        for _ in range(2):
+            work = _device_work(lambda: got.append(c.count_batch(e, off, nodes)))
+            assert any("k_row_keys_hist" in w for w in work)
+        for counts, r in got:
+            assert counts.tolist() == [t for t, _ in want] and r.edges == sum(m for _, m in want)

@@ -76,8 +76,8 @@ void reserve_layout(tribit_context* c, tb::PrepInput& in, bool stage, uint32_t G
 }
 
 // Runs preprocessing + schedule (+ counting when count == true) for one input.
-void run_call(tribit_context* c, tb::PrepInput in, const uint64_t* host_entries, const uint64_t* host_eoff,
-              const uint64_t* host_voff, uint32_t G, bool count, tribit_result* res) {
+void run_call(tribit_context* c, tb::PrepInput in, const uint64_t* host_entries, uint32_t G, bool count,
+              tribit_result* res) {
   DeviceGuard dg(c->device);
   const bool stage = host_entries != nullptr;
   CallLayout L;
@@ -85,8 +85,8 @@ void run_call(tribit_context* c, tb::PrepInput in, const uint64_t* host_entries,
   cudaStream_t st = c->st;
   TB_CUDA(cudaEventRecord(c->ev[0], st));
   if (G) {
-    TB_CUDA(cudaMemcpyAsync(L.eoff, host_eoff, (G + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    TB_CUDA(cudaMemcpyAsync(L.voff, host_voff, (G + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+    TB_CUDA(cudaMemcpyAsync(L.eoff, in.host_eoff, (G + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+    TB_CUDA(cudaMemcpyAsync(L.voff, in.host_voff, (G + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     TB_CUDA(cudaMemsetAsync(L.per_graph, 0, G * sizeof(unsigned long long), st));
   }
   tb::PrepInput pin = in;
@@ -110,8 +110,6 @@ void run_call(tribit_context* c, tb::PrepInput in, const uint64_t* host_entries,
   if (G) {
     pin.eoff = L.eoff;
     pin.voff = L.voff;
-    pin.host_eoff = host_eoff;
-    pin.host_voff = host_voff;
   }
   tb::drop_graph(c);
   tb::prepare_graph(c->arena, pin, st, &c->prep);
@@ -170,7 +168,7 @@ void count_device_input(tribit_context* c, const uint64_t* d_entries, uint64_t E
   in.E = E;
   in.n = n;
   in.order = order;
-  run_call(c, in, nullptr, nullptr, nullptr, 0, true, res);
+  run_call(c, in, nullptr, 0, true, res);
 }
 
 void read_stats(tribit_context* c, cudaStream_t st) {
@@ -310,7 +308,7 @@ tribit_status tribit_count_edges(tribit_context* c, const uint64_t* entries, uin
     in.n = num_nodes;
     in.order = c->opts.order;
     static const uint64_t dummy = 0;
-    run_call(c, in, entries ? entries : &dummy, nullptr, nullptr, 0, true, out);
+    run_call(c, in, entries ? entries : &dummy, 0, true, out);
     if (out) {
       tb::fill_schedule_stats(c, out);
       out->stream_ranges = 1;
@@ -334,7 +332,7 @@ tribit_status tribit_count_edges_device(tribit_context* c, const uint64_t* d_ent
     in.E = n_entries;
     in.n = num_nodes;
     in.order = c->opts.order;
-    run_call(c, in, nullptr, nullptr, nullptr, 0, true, out);
+    run_call(c, in, nullptr, 0, true, out);
     if (out) tb::fill_schedule_stats(c, out);
   });
 }
@@ -348,7 +346,7 @@ tribit_status tribit_prepare_device(tribit_context* c, const uint64_t* d_entries
     in.E = n_entries;
     in.n = num_nodes;
     in.order = c->opts.order;
-    run_call(c, in, nullptr, nullptr, nullptr, 0, false, out);
+    run_call(c, in, nullptr, 0, false, out);
     if (out) tb::fill_schedule_stats(c, out);
   });
 }
@@ -551,8 +549,10 @@ tribit_status tribit_count_batch(tribit_context* c, const uint64_t* entries, con
     in.n = voff[num_graphs];
     in.order = c->opts.order;
     in.G = num_graphs;
+    in.host_eoff = entry_offsets;
+    in.host_voff = voff.data();
     static const uint64_t dummy = 0;
-    run_call(c, in, entries ? entries : &dummy, entry_offsets, voff.data(), num_graphs, true, out);
+    run_call(c, in, entries ? entries : &dummy, num_graphs, true, out);
     DeviceGuard dg(c->device);
     TB_CUDA(cudaMemcpyAsync(triangles_out, c->per_graph, num_graphs * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->st));
     TB_CUDA(cudaStreamSynchronize(c->st));

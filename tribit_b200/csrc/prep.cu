@@ -1,5 +1,6 @@
 // GPU preprocessing pipeline; see prep.cuh.
 #include <algorithm>
+#include <vector>
 
 #include "prep.cuh"
 #include "scan.cuh"
@@ -506,27 +507,28 @@ __global__ void __launch_bounds__(kThreads) k_row_fill_entries(PrepInput in, uin
   }
 }
 
-// Slot path: keys[i] = (lo << 32) | hi of entry i (kDropped for a dropped
-// entry), over the presort's radix tiles, each tile also counting its keys'
+// Slot path: keys[i - i0] = (lo - r0) << 32 | hi of entry i of [i0, i1) (kDropped for a
+// dropped entry; r0: at most every lo), over the presort's radix tiles, each tile also counting its keys'
 // presort digits (key >> shift) & 255 into hist (digit-major, as k_radix_hist
 // leaves them): the keys and the presort's histogram in one pass.
-__global__ void __launch_bounds__(kSortThreads) k_row_keys_hist(PrepInput in, const uint32_t* __restrict__ rank,
+__global__ void __launch_bounds__(kSortThreads) k_row_keys_hist(PrepInput in, uint64_t i0, uint64_t i1,
+                                                                 const uint32_t* __restrict__ rank, uint32_t r0,
                                                                  uint64_t* __restrict__ keys, int shift,
                                                                  uint32_t tiles, uint32_t* __restrict__ hist,
                                                                  unsigned int* err) {
   __shared__ uint32_t h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
-  const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
+  const uint64_t base = i0 + (uint64_t)blockIdx.x * kSortTile;
   EntryReader rd(in, err);
 #pragma unroll 4
   for (int j = 0; j < kSortKeysPerThread; ++j) {
     const uint64_t i = base + (uint64_t)j * kSortThreads + threadIdx.x;
     uint32_t d = 256u;
-    if (i < in.E) {
+    if (i < i1) {
       uint32_t a, b;
-      const uint64_t key = rd.ids(in.entries[i], i, a, b) ? orient(rank, a, b) : kDropped;
-      keys[i] = key;
+      const uint64_t key = rd.ids(in.entries[i], i, a, b) ? orient(rank, a, b) - ((uint64_t)r0 << 32) : kDropped;
+      keys[i - i0] = key;
       d = (uint32_t)((key >> shift) & 255);
     }
     const uint32_t peers = __match_any_sync(kFull, d);
@@ -1166,6 +1168,11 @@ bool takes_presort(const PrepInput& in) {
 
 uint64_t entry_tiles(uint64_t E) { return std::max<uint64_t>(1, E / (148ull * 64 * kTile)); }  // a CTA's
 
+// Pieces a host input of E entries is copied in, of at least `least` entries each.
+uint64_t upload_pieces(uint64_t E, uint64_t least) {
+  return std::max<uint64_t>(1, std::min<uint64_t>(kUploadChunks, E / least));
+}
+
 // Queues the copy of host entries [i0, i1).
 void upload_entries(const PrepInput& in, uint64_t i0, uint64_t i1, cudaStream_t st) {
   const HostUpload& up = in.upload;
@@ -1178,6 +1185,17 @@ void upload_entries(const PrepInput& in, uint64_t i0, uint64_t i1, cudaStream_t 
     TB_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, st));
 }
 
+// Inputs that presort group their keys by one radix pass on the top 8 bits of
+// lo into 256 ranges of rows, so the fill's cursors and stores at any time stay
+// in one range's few MB of L2 instead of scattering over all rows.
+int presort_digit(uint64_t rows) { return 32 + bits_for(rows) - 8; }
+
+void fill_keys(const uint64_t* keys, uint64_t E, uint32_t* cur, uint32_t* nbr, cudaStream_t st) {
+  k_row_fill<<<(unsigned)std::min<uint64_t>(ceil_div<uint64_t>(E, kTile), 148ull * 64), kThreads, 0, st>>>(keys, E, cur,
+                                                                                                         nbr);
+  TB_LAUNCH_CHECK();
+}
+
 void fill_entries(const PrepInput& in, uint64_t i0, uint64_t i1, const uint32_t* rank, uint32_t* cur, uint32_t* nbr,
                   unsigned int* err, cudaStream_t st) {
   if (i0 >= i1) return;
@@ -1185,6 +1203,21 @@ void fill_entries(const PrepInput& in, uint64_t i0, uint64_t i1, const uint32_t*
   k_row_fill_entries<<<(unsigned)ceil_div<uint64_t>(i1 - i0, per * kTile), kThreads, 0, st>>>(in, i0, i1, rank, cur, nbr,
                                                                                              (uint32_t)per, err);
   TB_LAUNCH_CHECK();
+}
+
+// The keys of entries [i0, i1), presorted, into the rows from rank r0 on, z of them, in slots. The buffers hold i1 - i0
+// keys.
+void fill_presorted(const PrepInput& in, uint64_t i0, uint64_t i1, const uint32_t* rank, uint64_t r0, uint64_t z,
+                    uint64_t* keys, uint64_t* keys_alt, const RadixTemp& tmp, uint32_t* cur, uint32_t* nbr,
+                    unsigned int* err, cudaStream_t st) {
+  const uint64_t E = i1 - i0, tiles = ceil_div<uint64_t>(E, kSortTile);
+  const int top = presort_digit(z);
+  k_row_keys_hist<<<(unsigned)tiles, kSortThreads, 0, st>>>(in, i0, i1, rank, (uint32_t)r0, keys, top, (uint32_t)tiles,
+                                                             tmp.hist, err);
+  TB_LAUNCH_CHECK();
+  const uint64_t* sorted =
+      radix_sort<uint64_t, NoVal, false>(keys, keys_alt, nullptr, nullptr, E, top + 8, tmp, st, nullptr, top, true);
+  fill_keys(sorted, E, cur + r0, nbr, st);
 }
 
 // Rows in degree-sized slots (2E entries in all, u32 offsets): no per-row
@@ -1223,7 +1256,6 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, uint32_t* cn
 
   const LongRows lng{big, nbig};
   uint64_t* keys = reinterpret_cast<uint64_t*>(scratch);
-  const int top = 32 + bits_for(n) - 8;  // the presort digit: the top 8 bits of lo
   const uint64_t per = entry_tiles(E);
   const unsigned entry_grid = (unsigned)ceil_div<uint64_t>(E, per * kTile);
   if (!slots && E > 0) {
@@ -1232,24 +1264,15 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, uint32_t* cn
   }
   if (!rank_scans(in)) device_scan<uint32_t, OpSum>(cnt, off, n + 1, true, OpSum{}, 0u, otmp, st, cnt);
   if (slots && presort) {
-    const uint64_t tiles = ceil_div<uint64_t>(E, kSortTile);
-    k_row_keys_hist<<<(unsigned)tiles, kSortThreads, 0, st>>>(in, rank, keys, top, (uint32_t)tiles, ktmp.hist,
-                                                               &stats->err);
-    TB_LAUNCH_CHECK();
-  }
-  if (slots && !presort && E > 0) {
+    fill_presorted(in, 0, E, rank, 0, n, keys, keys_alt, ktmp, cnt, nbr, &stats->err, st);
+  } else if (slots) {
     fill_entries(in, 0, E, rank, cnt, nbr, &stats->err, st);
   } else if (E > 0) {
-    // One radix pass on the top 8 bits of lo groups the keys into 256 ranges
-    // of rows, so the fill's cursors and stores at any time stay in one
-    // range's few MB of L2 instead of scattering over all rows.
-    const uint64_t* fill_keys = keys;
+    const int top = presort_digit(n);
+    const uint64_t* sorted = keys;
     if (presort)
-      fill_keys = radix_sort<uint64_t, NoVal, false>(keys, keys_alt, nullptr, nullptr, E, top + 8, ktmp, st, nullptr,
-                                                     top, slots);
-    k_row_fill<<<(unsigned)std::min<uint64_t>(ceil_div<uint64_t>(E, kTile), 148ull * 64), kThreads, 0, st>>>(
-        fill_keys, E, cnt, nbr);
-    TB_LAUNCH_CHECK();
+      sorted = radix_sort<uint64_t, NoVal, false>(keys, keys_alt, nullptr, nullptr, E, top + 8, ktmp, st, nullptr, top);
+    fill_keys(sorted, E, cnt, nbr, st);
   }
   // Row u: nbr[off[u], cnt[u]) (with no entries every row is empty: 0, 0).
   sort_rows(off, cnt, (uint32_t)n, E, nbr, scratch, rp, lng, st);
@@ -1367,14 +1390,54 @@ namespace {
 // consecutive: a chunk of graphs is ranked and its rows built as soon as its
 // entries have landed, while the next chunk is copied. (All graphs built after
 // the last entry had landed: 512 graphs, 87.5 million entries, 21.4 ms, now 19.1.)
+// A chunk that one graph dominates is copied, and its degrees counted, in pieces
+// as a single graph's are, and a graph of kPresortMinEntries or more has its
+// chunk's keys presorted. (Chunks of smaller graphs need no presort: a graph's
+// entries, and so its cursors, are together.)
 constexpr uint64_t kBatchChunk = 1ull << 22;  // entries, at least; at most kUploadChunks chunks
+// A piece's least entries: a batch's degree pass searches for its graphs, so a
+// piece gains less than a single graph's (100 graphs, 2^20 entries: 620 us in
+// pieces of 2^17, 594 in one; one graph of 2^22: 1,512 and 1,503 in pieces of 2^17 and 2^20, 1,538 in one).
+constexpr uint64_t kBatchPiece = 1ull << 20;
+
+struct BatchChunk {
+  uint64_t g0, g1;  // its graphs
+  bool presort;
+};
+std::vector<BatchChunk> batch_plan(const PrepInput& in) {
+  const uint64_t chunks = std::max<uint64_t>(1, std::min<uint64_t>(kUploadChunks, in.E / kBatchChunk));
+  std::vector<BatchChunk> plan;
+  for (uint64_t k = 0, g0 = 0; k < chunks; ++k) {
+    // The graphs whose entries end in the k-th share, or all that are left.
+    const uint64_t g1 = k + 1 == chunks ? in.G
+                                        : (uint64_t)(std::upper_bound(in.host_eoff + g0 + 1, in.host_eoff + in.G + 1,
+                                                                      in.E * (k + 1) / chunks) -
+                                                     in.host_eoff - 1);
+    BatchChunk c{g0, g1, false};
+    for (uint64_t g = g0; g < g1; ++g)
+      c.presort |= in.host_eoff[g + 1] - in.host_eoff[g] >= kPresortMinEntries &&
+                   in.host_voff[g + 1] - in.host_voff[g] > 256;
+    if (g1 > g0) plan.push_back(c);
+    g0 = g1;
+  }
+  return plan;
+}
 
 struct BatchBuffers {
   uint32_t *otmp = nullptr, *big = nullptr, *nbr = nullptr, *scratch = nullptr, *col = nullptr;
-  uint64_t *rtmp = nullptr, *bent = nullptr, *carry = nullptr;
+  uint64_t *rtmp = nullptr, *bent = nullptr, *carry = nullptr, *keys_alt = nullptr;
+  RadixTemp ktmp;
 };
-BatchBuffers take_batch_buffers(Arena& ar, uint64_t n, uint64_t E) {
+BatchBuffers take_batch_buffers(Arena& ar, const PrepInput& in, const std::vector<BatchChunk>& plan) {
+  const uint64_t n = in.n, E = in.E;
   BatchBuffers b;
+  uint64_t keys = 0;  // the most that a chunk presorts; they lie in scratch
+  for (const BatchChunk& c : plan)
+    if (c.presort) keys = std::max(keys, in.host_eoff[c.g1] - in.host_eoff[c.g0]);
+  if (keys) {
+    b.keys_alt = ar.take<uint64_t>(keys);
+    b.ktmp = take_radix_temp(ar, keys);
+  }
   b.otmp = take_scan_temp<uint32_t>(ar, n + 1);
   b.rtmp = take_scan_temp<uint64_t>(ar, n + 1);
   b.carry = ar.take<uint64_t>(1);
@@ -1386,42 +1449,46 @@ BatchBuffers take_batch_buffers(Arena& ar, uint64_t n, uint64_t E) {
   return b;
 }
 
-void build_batch(const PrepInput& in, const BatchBuffers& b, uint32_t* deg, const RankBuffers& rb, uint32_t* rank,
-                 uint32_t* graph_of_rank, uint32_t* cnt, uint32_t* off, uint32_t* nbig, cudaStream_t st,
-                 DeviceStats* stats, uint64_t* rp) {
+void build_batch(const PrepInput& in, const std::vector<BatchChunk>& plan, const BatchBuffers& b, uint32_t* deg,
+                 const RankBuffers& rb, uint32_t* rank, uint32_t* graph_of_rank, uint32_t* cnt, uint32_t* off,
+                 uint32_t* nbig, cudaStream_t st, DeviceStats* stats, uint64_t* rp) {
   const uint64_t n = in.n, E = in.E;
   const HostUpload& up = in.upload;
-  const uint64_t chunks = std::max<uint64_t>(1, std::min<uint64_t>(kUploadChunks, E / kBatchChunk));
-  const bool upload = up.host && E > 0, overlap = upload && chunks > 1;
+  const uint64_t pieces = upload_pieces(E, kBatchPiece), piece = ceil_div<uint64_t>(E, pieces);
+  const bool upload = up.host && E > 0, overlap = upload && pieces > 1;
   TB_CUDA(cudaMemsetAsync(stats, 0, (size_t)((char*)(deg + n) - (char*)stats), st));
   TB_CUDA(cudaMemsetAsync(rp, 0, sizeof(uint64_t), st));
   if (overlap) {  // the copies wait for the stream's earlier work, which may still read the staging buffer
     TB_CUDA(cudaEventRecord(up.events[0], st));
     TB_CUDA(cudaStreamWaitEvent(up.copy_stream, up.events[0], 0));
   }
-  for (uint64_t k = 0, g0 = 0; k < chunks; ++k) {
-    // Graphs [g0, g1): those whose entries end in the k-th share, or all that are left.
-    const uint64_t g1 = k + 1 == chunks ? in.G
-                                        : (uint64_t)(std::upper_bound(in.host_eoff + g0 + 1, in.host_eoff + in.G + 1,
-                                                                      E * (k + 1) / chunks) -
-                                                     in.host_eoff - 1);
-    const uint64_t e0 = in.host_eoff[g0], e1 = in.host_eoff[g1], v0 = in.host_voff[g0], v1 = in.host_voff[g1];
+  for (const BatchChunk& c : plan) {
+    const uint64_t e0 = in.host_eoff[c.g0], e1 = in.host_eoff[c.g1], v0 = in.host_voff[c.g0], v1 = in.host_voff[c.g1];
     const uint64_t z = v1 - v0;
-    if (upload && e1 > e0) {
-      upload_entries(in, e0, e1, overlap ? up.copy_stream : st);
-      if (overlap) {
-        TB_CUDA(cudaEventRecord(up.events[k + 1], up.copy_stream));
-        TB_CUDA(cudaStreamWaitEvent(st, up.events[k + 1], 0));
+    // The chunk in the pieces nearest in size to a single graph's.
+    const uint64_t parts = std::max<uint64_t>(1, (e1 - e0 + piece / 2) / std::max<uint64_t>(1, piece));
+    for (uint64_t k = 0; k < parts; ++k) {
+      const uint64_t i0 = e0 + (e1 - e0) * k / parts, i1 = e0 + (e1 - e0) * (k + 1) / parts;
+      if (upload && i1 > i0) {
+        upload_entries(in, i0, i1, overlap ? up.copy_stream : st);
+        if (overlap) {  // a wait keeps the record it was queued after, so one event serves all pieces
+          TB_CUDA(cudaEventRecord(up.events[1], up.copy_stream));
+          TB_CUDA(cudaStreamWaitEvent(st, up.events[1], 0));
+        }
       }
+      if (upload && i1 > i0 && i1 == E && up.uploaded) TB_CUDA(cudaEventRecord(up.uploaded, st));
+      degree_pass(in, i0, i1, deg, &stats->err, st);
     }
-    if (upload && k + 1 == chunks && up.uploaded) TB_CUDA(cudaEventRecord(up.uploaded, st));
-    if (e1 > e0) degree_pass(in, e0, e1, deg, &stats->err, st);
     if (z > 0) {
       // Everything of the chunk from its first rank on; slots from 2 e0 on, offsets within the chunk.
-      rank_by_degree(deg, v0, z, in.voff, in.G, (uint32_t)g0, (uint32_t)g1, rb, rank, graph_of_rank,
+      rank_by_degree(deg, v0, z, in.voff, in.G, (uint32_t)c.g0, (uint32_t)c.g1, rb, rank, graph_of_rank,
                      RowWords{cnt + v0, z + 1, true, nullptr}, st);
       device_scan<uint32_t, OpSum>(cnt + v0, off + v0, z + 1, true, OpSum{}, 0u, b.otmp, st, cnt + v0);
-      fill_entries(in, e0, e1, rank, cnt, b.nbr + 2 * e0, &stats->err, st);
+      if (c.presort)
+        fill_presorted(in, e0, e1, rank, v0, z, reinterpret_cast<uint64_t*>(b.scratch), b.keys_alt, b.ktmp, cnt,
+                       b.nbr + 2 * e0, &stats->err, st);
+      else
+        fill_entries(in, e0, e1, rank, cnt, b.nbr + 2 * e0, &stats->err, st);
       TB_CUDA(cudaMemsetAsync(nbig, 0, kLongWords * sizeof(uint32_t), st));
       TB_CUDA(cudaMemcpyAsync(b.carry, rp + v0, sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
       const LongRows lng{b.big, nbig};
@@ -1433,7 +1500,6 @@ void build_batch(const PrepInput& in, const BatchBuffers& b, uint32_t* deg, cons
                                                                emit_chunk(e1 - e0 + z), lng, b.col, b.bent, nullptr);
       TB_LAUNCH_CHECK();
     }
-    g0 = g1;
   }
   k_finalize<<<1, 1, 0, st>>>(rp, n, stats);
   TB_LAUNCH_CHECK();
@@ -1475,10 +1541,11 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
   out->view.by_id = !by_degree;
 
   if (batch_chunks(in)) {
-    const BatchBuffers b = take_batch_buffers(ar, n, E);
+    const std::vector<BatchChunk> plan = batch_plan(in);
+    const BatchBuffers b = take_batch_buffers(ar, in, plan);
     out->view.col = b.col;
     out->view.bent = b.bent;
-    if (!ar.measuring()) build_batch(in, b, deg, rb, rank, graph_of_rank, cnt, off, nbig, st, stats, rp);
+    if (!ar.measuring()) build_batch(in, plan, b, deg, rb, rank, graph_of_rank, cnt, off, nbig, st, stats, rp);
     return;
   }
   // Phase 1 (launch only when not measuring): the upload of host entries,
@@ -1489,7 +1556,7 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
     if (!by_degree || n == 0) TB_CUDA(cudaMemsetAsync(cnt, 0, rw.count * sizeof(uint32_t), st));
     const HostUpload& up = in.upload;
     const bool upload = up.host && E > 0;
-    const uint64_t pieces = std::min<uint64_t>(kUploadChunks, E / kUploadMinPiece);
+    const uint64_t pieces = upload_pieces(E, kUploadMinPiece);
     const bool overlap = upload && by_degree && n > 0 && pieces > 1;
     if (upload && !overlap) upload_entries(in, 0, E, st);
     if (upload && !overlap && up.uploaded) TB_CUDA(cudaEventRecord(up.uploaded, st));

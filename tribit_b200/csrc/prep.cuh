@@ -89,7 +89,7 @@ struct PrepInput {
   uint32_t G = 0;
   const uint64_t* eoff = nullptr;  // device, G + 1
   const uint64_t* voff = nullptr;  // device, G + 1
-  const uint64_t* host_eoff = nullptr;  // the same on the host
+  const uint64_t* host_eoff = nullptr;  // the same on the host, also while measuring
   const uint64_t* host_voff = nullptr;
 };
 
