@@ -63,7 +63,7 @@ def rows_in_degree_order(e, n):
 
 
 @pytest.mark.parametrize("n, hubs, times", [(11_101, 45, 3), (16_001, 40, 4), (16_545, 45, 2), (90_001, 60, 1)])
-@pytest.mark.parametrize("call", ["device", "host", "batch", "budget"])
+@pytest.mark.parametrize("call", ["device", "host", "batch", "batch16", "budget"])
 def test_hubs_of_near_equal_degree_are_ranked_by_degree(n, hubs, times, call):
     # Degrees that share their leading 11 bits, falling with the id, over a row-block
     # border: ranked by id, every hub's row would hold the wrong hubs. The features
@@ -77,11 +77,11 @@ def test_hubs_of_near_equal_degree_are_ranked_by_degree(n, hubs, times, call):
             c.prepare_device(d.data_ptr(), d.numel(), n)
         elif call == "host":
             c.count_edges(e, n)
-        elif call == "batch":  # after two small graphs of 32 and 64 vertices
-            small = [tb.gen_er(32, 100, seed=1), tb.gen_er(64, 100, seed=2)]
-            c.count_batch(np.concatenate(small + [e]), np.array([0, 100, 200, 200 + e.size], dtype=np.uint64),
-                          np.array([32, 64, n], dtype=np.uint32))
-            base = 3
+        elif call.startswith("batch"):  # after small graphs of 32 vertices: 14 and 12 bits of degree in the keys
+            base = 15 if call == "batch16" else 2
+            small = [tb.gen_er(32, 100, seed=i) for i in range(base)]
+            off = np.append(100 * np.arange(base + 1), 100 * base + e.size).astype(np.uint64)
+            c.count_batch(np.concatenate(small + [e]), off, np.array([32] * base + [n], dtype=np.uint32))
         else:
             c.set_stream_options("rows")
             c.set_device_budget(c.device_bytes(e.size, n) * 3 // 4)

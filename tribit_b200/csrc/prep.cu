@@ -186,15 +186,20 @@ __device__ __forceinline__ uint32_t graph_of_vertex(const uint64_t* voff, uint32
 // ones (hubs, at most 2E >> (bits - 1) of them) keep their leading bit and the
 // next `mant` ones. Hubs that share a key lie side by side after the sort and
 // are then placed by their degrees (hub_place), so the order is the full
-// degrees' in half the passes. mant < 0, when many graphs leave fewer than
-// kDegreeBits: degrees are capped at 2^bits - 1.
+// degrees' in half the passes. That compares hubs of one key pairwise: from
+// kDegreeBits on there are few, with kLeastDegreeBits where 2E >> (bits - 1) is at
+// most kHubGroup. mant < 0, when many graphs leave fewer bits: degrees are capped at 2^bits - 1.
 struct DegreeKey {
   int bits, mant;
 };
-constexpr int kDegreeBits = 16;
-inline DegreeKey degree_key_of(int bits) {
-  if (bits >= 32) return {32, -1};           // exact
-  if (bits < kDegreeBits) return {bits, -1};  // at 0, degrees are not told apart
+constexpr int kDegreeBits = 16, kLeastDegreeBits = 12;
+constexpr uint64_t kHubGroup = 8192;
+inline bool told_apart(int bits, uint64_t E) {
+  return bits >= kDegreeBits || (bits >= kLeastDegreeBits && (2 * E) >> (bits - 1) <= kHubGroup);
+}
+inline DegreeKey degree_key_of(int bits, uint64_t E) {
+  if (bits >= 32) return {32, -1};              // exact
+  if (!told_apart(bits, E)) return {bits, -1};  // at 0, degrees are not told apart
   int m = bits - 1;                          // (33 - bits) leading bits times 2^m must fit above 2^(bits - 1)
   while (((33ll - bits) << m) > (1ll << (bits - 1))) --m;
   return {bits, m};
@@ -1354,22 +1359,23 @@ RankBuffers take_rank_buffers(Arena& ar, uint64_t n) {
 namespace {
 
 // Ranks of n vertices from v0 on, graphs [g0, g1) of a batch (a single graph: G
-// = 0), from their degrees, and the row words. The buffers as take_rank_buffers
+// = 0), from their degrees over E entries, and the row words. The buffers as take_rank_buffers
 // takes them.
-void rank_by_degree(const uint32_t* deg, uint64_t v0, uint64_t n, const uint64_t* voff, uint32_t G, uint32_t g0,
-                    uint32_t g1, const RankBuffers& b, uint32_t* rank, uint32_t* graph_of_rank, const RowWords& rw,
+void rank_by_degree(const uint32_t* deg, uint64_t E, uint64_t v0, uint64_t n, const uint64_t* voff, uint32_t G,
+                    uint32_t g0, uint32_t g1, const RankBuffers& b, uint32_t* rank, uint32_t* graph_of_rank, const RowWords& rw,
                     cudaStream_t st) {
   if (!G && n <= kRankOneMax) {
     once_per_device<3>(
         [] { TB_CUDA(cudaFuncSetAttribute(k_rank_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRankSmem)); });
-    k_rank_one<<<1, kRankThreads, kRankSmem, st>>>(deg, (uint32_t)n, degree_key_of(kDegreeBits), rank, rw);
+    k_rank_one<<<1, kRankThreads, kRankSmem, st>>>(deg, (uint32_t)n, degree_key_of(kDegreeBits, E), rank, rw);
     TB_LAUNCH_CHECK();
     return;
   }
-  // Whole radix passes over the graph bits and, where 32 bits leave as many, kDegreeBits of degree.
+  // Whole radix passes over the graph bits and as many degree bits as tell all degrees apart (or as there are).
   const int gbits = G ? bits_for((uint64_t)(g1 - g0)) : 0;
-  const int total = std::min(32, (gbits + kDegreeBits + 7) / 8 * 8);
-  const DegreeKey dk = degree_key_of(total - gbits);
+  int total = 16;
+  while (total < 32 && !told_apart(total - gbits, E)) total += 8;
+  const DegreeKey dk = degree_key_of(total - gbits, E);
   k_vertex_keys<<<grid_for(n), kThreads, 0, st>>>(deg, v0, n, voff, G, g0, dk, b.vk, b.vv);
   TB_LAUNCH_CHECK();
   uint32_t* sorted_ids = nullptr;
@@ -1481,7 +1487,7 @@ void build_batch(const PrepInput& in, const std::vector<BatchChunk>& plan, const
     }
     if (z > 0) {
       // Everything of the chunk from its first rank on; slots from 2 e0 on, offsets within the chunk.
-      rank_by_degree(deg, v0, z, in.voff, in.G, (uint32_t)c.g0, (uint32_t)c.g1, rb, rank, graph_of_rank,
+      rank_by_degree(deg, e1 - e0, v0, z, in.voff, in.G, (uint32_t)c.g0, (uint32_t)c.g1, rb, rank, graph_of_rank,
                      RowWords{cnt + v0, z + 1, true, nullptr}, st);
       device_scan<uint32_t, OpSum>(cnt + v0, off + v0, z + 1, true, OpSum{}, 0u, b.otmp, st, cnt + v0);
       if (c.presort)
@@ -1507,8 +1513,8 @@ void build_batch(const PrepInput& in, const std::vector<BatchChunk>& plan, const
 
 }  // namespace
 
-void rank_vertices(const uint32_t* deg, uint64_t n, const RankBuffers& b, uint32_t* rank, cudaStream_t st) {
-  if (n > 0) rank_by_degree(deg, 0, n, nullptr, 0, 0, 0, b, rank, nullptr, RowWords{}, st);
+void rank_vertices(const uint32_t* deg, uint64_t n, uint64_t E, const RankBuffers& b, uint32_t* rank, cudaStream_t st) {
+  if (n > 0) rank_by_degree(deg, E, 0, n, nullptr, 0, 0, 0, b, rank, nullptr, RowWords{}, st);
 }
 
 void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* out) {
@@ -1579,7 +1585,7 @@ void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* ou
       } else {
         degree_pass(in, 0, E, deg, &stats->err, st);
       }
-      rank_by_degree(deg, 0, n, in.voff, in.G, 0, in.G, rb, rank, graph_of_rank, rw, st);
+      rank_by_degree(deg, E, 0, n, in.voff, in.G, 0, in.G, rb, rank, graph_of_rank, rw, st);
     } else if (in.G && n > 0) {
       k_identity_graph_of<<<grid_for(n), kThreads, 0, st>>>(n, in.voff, in.G, graph_of_rank);
       TB_LAUNCH_CHECK();

@@ -105,7 +105,7 @@ struct Prepared {
 // preprocessing pipeline on stream st. Stats are zeroed here.
 void prepare_graph(Arena& ar, const PrepInput& in, cudaStream_t st, Prepared* out);
 
-// The (degree, id) rank order of n vertices from their degrees: rank[v] =
+// The (degree, id) rank order of n vertices from their degrees over E entries: rank[v] =
 // position of v, as prepare_graph ranks a single graph. The buffers come from
 // take_rank_buffers; launches only.
 struct RankBuffers {
@@ -113,7 +113,7 @@ struct RankBuffers {
   RadixTemp tmp{};
 };
 RankBuffers take_rank_buffers(Arena& ar, uint64_t n);
-void rank_vertices(const uint32_t* deg, uint64_t n, const RankBuffers& b, uint32_t* rank, cudaStream_t st);
+void rank_vertices(const uint32_t* deg, uint64_t n, uint64_t E, const RankBuffers& b, uint32_t* rank, cudaStream_t st);
 
 // One rank range's rows at a time: the oriented graph's rows [s, s + z) built
 // from that range's keys alone (lo << 32 | hi in rank space, lo in the range,

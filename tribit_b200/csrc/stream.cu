@@ -647,7 +647,7 @@ bool count_streamed_if_needed(tribit_context* c, const uint64_t* host, uint64_t 
     TB_LAUNCH_CHECK();
   });
   check_flags(nullptr);
-  rank_vertices(deg, n, rb, rank, st);
+  rank_vertices(deg, n, E, rb, rank, st);
   // Oriented entries per row (with duplicates), their prefix, the longest row.
   TB_CUDA(cudaMemsetAsync(rows, 0, (n + 1) * sizeof(uint32_t), st));
   stream_pass([&](const uint64_t* piece, uint64_t cnt) {
