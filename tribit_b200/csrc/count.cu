@@ -288,9 +288,8 @@ __device__ __forceinline__ bool edge_to_hub(const GraphView& g, uint32_t j) {
   return g.eflag && ((g.eflag[j >> 5] >> (j & 31)) & 1u);
 }
 
-// The neighbour sweep: slots are CSR positions j, each the list of v = col[j]:
-// its bit blocks (Blocks) or its neighbour ids.
-template <bool Blocks, class Item>
+// The neighbour sweep: slots are CSR positions j, each the list of v = col[j]'s neighbour ids.
+template <class Item>
 __device__ __forceinline__ uint64_t sweep(const GraphView& g, uint32_t cs, uint32_t ce, uint32_t chunk0,
                                           uint32_t step, const Item& item) {
   return sweep_lists(
@@ -298,9 +297,8 @@ __device__ __forceinline__ uint64_t sweep(const GraphView& g, uint32_t cs, uint3
       [&](uint32_t j, uint32_t& ib, uint32_t& il) {
         if (edge_to_hub(g, j)) return;
         const uint32_t v = g.col[j];
-        const uint64_t a = g.rp[v], b = g.rp[v + 1];
-        ib = Blocks ? rp_blk(a) : rp_row(a);
-        il = (Blocks ? rp_blk(b) : rp_row(b)) - ib;
+        ib = rp_row(g.rp[v]);
+        il = rp_row(g.rp[v + 1]) - ib;
       },
       item);
 }
@@ -309,11 +307,8 @@ __device__ __forceinline__ uint64_t sweep(const GraphView& g, uint32_t cs, uint3
 #define TB_BITS_DEPTH 4
 #endif
 constexpr int kBitsDepth = TB_BITS_DEPTH;
-// Column id w as a one-bit entry of its block; `keep` false: the block alone
-// (matches nothing).
-__device__ __forceinline__ uint64_t col_entry(uint32_t w, bool keep) {
-  return ((uint64_t)(w >> 5) << 32) | (keep ? 1u << (w & 31) : 0u);
-}
+// Column id w as a one-bit entry of its block.
+__device__ __forceinline__ uint64_t col_entry(uint32_t w) { return ((uint64_t)(w >> 5) << 32) | (1u << (w & 31)); }
 
 // The bit row of the neighbour at CSR position j, empty where the hub pass counts the edge.
 __device__ __forceinline__ void neighbour_blocks(const GraphView& g, uint32_t j, uint32_t& ib, uint32_t& il) {
@@ -338,19 +333,19 @@ __device__ __forceinline__ uint32_t starts_in(uint32_t excl, uint32_t il, uint32
 // across the warp of where the lists start gives the owners of 32 items as a
 // population count (a binary search by five shuffles an item; with the small rows' table below, planted
 // partition of 2 million vertices 4,249 us, now 3,407);
-// from kWalkItems items on (Walks), each lane finds the owner of its first
+// from kWalkItems items on, each lane finds the owner of its first
 // item by binary search and then only advances it (a lane's items only grow), one
 // compare an item. wsm: 64 words of the warp. Must be called by all 32 lanes.
 #ifndef TB_WALK_ITEMS
 #define TB_WALK_ITEMS 1024
 #endif
 constexpr uint32_t kWalkItems = TB_WALK_ITEMS;
-template <int Depth, bool Walks, class Load, class Probe>
+template <int Depth, class Load, class Probe>
 __device__ __forceinline__ uint32_t run_items(uint32_t ib, uint32_t il, const Load& load, const Probe& probe,
                                               uint32_t* wsm) {
   const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u, le = kFull >> (31 - lane);
   const uint32_t incl = warp_inclusive_sum(il), excl = incl - il, total = __shfl_sync(kFull, incl, 31);
-  if (Walks && total >= kWalkItems) {
+  if (total >= kWalkItems) {
     __syncwarp();
     wsm[lane] = incl;
     wsm[32 + lane] = ib - excl;  // item t of the chunk, owned by slot s, is item off_s + t
@@ -406,7 +401,7 @@ __device__ __forceinline__ uint64_t sweep_bits(const GraphView& g, uint32_t ib, 
                                                uint32_t step, const Probe& probe, uint32_t* wsm) {
   uint64_t acc = 0;
   for (uint32_t c = cs;;) {
-    acc += run_items<kBitsDepth, true>(ib, il, [&](uint32_t k) -> uint64_t { return g.bent[k]; }, probe, wsm);
+    acc += run_items<kBitsDepth>(ib, il, [&](uint32_t k) -> uint64_t { return g.bent[k]; }, probe, wsm);
     c += step * 32;
     if (c >= ce) break;
     ib = il = 0;
@@ -1311,7 +1306,7 @@ __global__ void __launch_bounds__(kCtaThreads) k_rows_wide(GraphView g, const ui
       racc = sweep_bits(g, cs, ce, w, nw, probe, runs[w]);
     } else {
       const uint32_t last = g.col[re - 1];
-      racc = sweep<false>(g, cs, ce, w, nw, [&](uint32_t k, uint32_t c) -> uint32_t {
+      racc = sweep(g, cs, ce, w, nw, [&](uint32_t k, uint32_t c) -> uint32_t {
         const uint32_t x = g.col[k];
         if (x > last) return 0u;
         uint32_t lo = c + 1, hi = re;
@@ -1391,10 +1386,7 @@ constexpr uint32_t kHubWarpPiece = TB_HUB_WARP_PIECE;  // in-edges per warp piec
 #ifndef TB_HUB_WAVE_SHIFT
 #define TB_HUB_WAVE_SHIFT 22
 #endif
-#ifndef TB_HUB_WAVES
-#define TB_HUB_WAVES 32
-#endif
-constexpr uint32_t kHubWaves = TB_HUB_WAVES;    // row ranges the hub pieces are ordered by (power of 2)
+constexpr uint32_t kHubWaves = 32;  // row ranges the hub pieces are ordered by, at most: a lane scans one (k_wave_scan)
 // Waves of a graph of E entries: one up to 2^23 (bit rows of at most 64 MiB, which
 // the L2 holds whatever the order), then one per 2^22 entries: each wave is a
 // launch with a tail of its own (one per 2^21: RMAT-20 0.4%, cliques 2% slower; 2^20: 2%).
@@ -1532,7 +1524,7 @@ __device__ __forceinline__ uint64_t sweep_col_quads(const GraphView& g, const ui
             b = (uint32_t)(x >> 32);
             l = (uint32_t)x;
           },
-          [&](uint32_t k) -> uint64_t { return col_entry(g.col[k], true); }, probe, wsm);
+          [&](uint32_t k) -> uint64_t { return col_entry(g.col[k]); }, probe, wsm);
       continue;
     }
     const uint32_t ie = ib + il;
@@ -2314,8 +2306,8 @@ __device__ __forceinline__ bool hub_candidate(const HubTable& hub, uint32_t v, u
 // savings only while they are below the staging cost: the decision saved >=
 // cost (k_hub_accept) is then the one the full sum gives, and the sum stays in
 // its 32 bits (the updates in flight past the cost add at most kHubMaxSpan each).
-// Mode 1: every candidate edge of an accepted hub (a vertex whose row words
-// k_hub_accept kept) is flagged and appended to the hub's in-list: a bit-row
+// Mode 1: every candidate edge of an accepted hub (k_hub_accept cleared the row
+// words of every other vertex, so one read decides) is flagged and appended to the hub's in-list: a bit-row
 // tail (first block, blocks) at the front, a column tail (first CSR position
 // after v, neighbours) at the back. rows (may be null): the pass covers rows
 // [rows[0], rows[1]).
@@ -2353,12 +2345,6 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
     for (uint32_t t = threadIdx.x; t < 2 * kTop; t += blockDim.x) s_top[t] = 0;
     __syncthreads();
   }
-  // Whether the edge to v (tail blocks) takes part: mode 0, a candidate;
-  // mode 1, a candidate of an accepted hub (k_hub_accept clears the row words of
-  // every other vertex, so one read decides).
-  auto decide = [&](uint32_t v, uint32_t tail, uint32_t& nbv, unsigned long long& cost) -> bool {
-    return hub_candidate(hub, v, tail, nbv, cost);
-  };
   // Applies mode Mode to the taking-part edge at j (v = col[j]; u's row ends
   // at CSR position re) of row u.
   auto edge = [&](uint32_t u, uint32_t bs, uint32_t j, uint32_t re, uint32_t v, uint32_t pos, uint32_t tail,
@@ -2404,16 +2390,16 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
       const uint32_t tail = nb - pos;
       uint32_t nbv = 0;
       unsigned long long cost = 0;
-      const bool hub = in && decide(v, tail, nbv, cost);
+      const bool taken = in && hub_candidate(hub, v, tail, nbv, cost);
       if (Mode == 1) {
-        const uint32_t bits = __ballot_sync(kFull, hub);
+        const uint32_t bits = __ballot_sync(kFull, taken);
         if (lane == 0 && bits) {
           const uint32_t sh = c & 31;
           atomicOr(&eflag[c >> 5], bits << sh);
           if (sh && (bits >> (32 - sh))) atomicOr(&eflag[(c >> 5) + 1], bits >> (32 - sh));
         }
       }
-      if (hub) edge(u, bs, j, re, v, pos, tail, nbv, cost);
+      if (taken) edge(u, bs, j, re, v, pos, tail, nbv, cost);
     }
   };
   auto warp_row = [&](uint32_t u, uint32_t rs, uint32_t re, uint32_t bs, uint32_t nb) {
@@ -2467,7 +2453,7 @@ __global__ void k_hub_edges(GraphView g, const uint8_t* __restrict__ variant_of,
         const uint32_t tail = nbu - pos;
         uint32_t nbv = 0;
         unsigned long long cost = 0;
-        if (!decide(v, tail, nbv, cost)) continue;
+        if (!hub_candidate(hub, v, tail, nbv, cost)) continue;
         if (Mode == 1) {
           if ((j >> 5) != fw) {
             if (fb) atomicOr(&eflag[fw], fb);
@@ -2722,7 +2708,6 @@ __global__ void __launch_bounds__(256) k_piece_waves(const uint64_t* __restrict_
     if (h[i]) atomicAdd(&cnt[i], h[i]);
 }
 
-static_assert(kHubWaves == 32, "a lane scans one wave of each list");
 __global__ void k_wave_scan(uint32_t* __restrict__ cnt, const uint32_t* __restrict__ piece_off) {
   const uint32_t lane = threadIdx.x;
   const uint32_t c = cnt[lane], w = cnt[kHubWaves + lane];
