@@ -147,8 +147,9 @@ const char* tribit_version(void);
 tribit_status tribit_count_edges(tribit_context* ctx, const uint64_t* entries, uint64_t n_entries, uint64_t num_nodes,
                                  tribit_result* out);
 /* Device memory (bytes) a one-piece tribit_count_edges of n_entries entries on
- * num_nodes vertices needs in this context (its arena, staged input included;
- * it takes 4 bytes an entry more where they can be had). */
+ * num_nodes vertices takes in this context (its arena, staged input included).
+ * Below 2^27 entries it also takes 4 bytes an entry more where they can be
+ * had; from there on it can do with 4 bytes an entry less. */
 tribit_status tribit_device_bytes(tribit_context* ctx, uint64_t n_entries, uint64_t num_nodes, uint64_t* bytes);
 /* Caps the device memory later tribit_count_edges calls of this context may
  * use (bytes; 0 = what the device has free at the call). */

@@ -273,3 +273,12 @@ def test_calls_that_only_compact_rows_leave_room_for(call):
         finally:
             del other
             torch.cuda.empty_cache()
+
+
+def test_device_bytes_from_the_presort_size_on():
+    # 2^27 entries and more: 8 bytes staged, 8 of rows in degree-sized slots, 16
+    # of keys in the presort's two buffers, 4 + 8 of CSR and bit rows, 8 of hub
+    # in-lists, and less than 1 of pieces, flags and digit counts.
+    with tb.Counter() as c:
+        per_entry = (c.device_bytes(1 << 28, 1 << 20) - c.device_bytes(1 << 27, 1 << 20)) / (1 << 27)
+        assert 52 < per_entry < 53

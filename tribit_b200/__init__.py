@@ -344,7 +344,7 @@ class Counter:
         _check(lib.tribit_set_stream_options(self._h, STREAM_TIERS[tier], int(range_entries)), self._h)
 
     def device_bytes(self, n_entries: int, num_nodes: int) -> int:
-        """Device memory a one-piece count_edges of this size needs."""
+        """Device memory a one-piece count_edges of this size takes (see tribit_device_bytes)."""
         b = _u64()
         _check(lib.tribit_device_bytes(self._h, int(n_entries), int(num_nodes), ctypes.byref(b)), self._h)
         return b.value

@@ -320,7 +320,9 @@ tribit_status tribit_count_edges(tribit_context* c, const uint64_t* entries, uin
 
 tribit_status tribit_device_bytes(tribit_context* c, uint64_t n_entries, uint64_t num_nodes, uint64_t* bytes) {
   if (!c || !bytes) return TRIBIT_ERR_INVALID_ARGUMENT;
-  return guarded(c, [&] { *bytes = tb::call_bytes(c, n_entries, num_nodes, c->opts.order, true, true); });
+  return guarded(c, [&] {
+    *bytes = tb::call_bytes(c, n_entries, num_nodes, c->opts.order, true, n_entries < tb::kPresortMinEntries);
+  });
 }
 
 tribit_status tribit_count_edges_device(tribit_context* c, const uint64_t* d_entries, uint64_t n_entries,

@@ -543,13 +543,6 @@ __global__ void __launch_bounds__(kSortThreads) k_row_keys_hist(PrepInput in, ui
   hist[(uint64_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
 
-#ifndef TB_PRESORT_MIN
-#define TB_PRESORT_MIN (1ull << 27)
-#endif
-// Smaller inputs fill straight from the keys: their rows (under 512 MB) keep
-// enough of the fill in L2 that the extra pass costs more than it saves
-// (measured: RMAT-22 13.3 ms without, 13.6-14.1 with; RMAT-24 50.8 -> 48.6).
-constexpr uint64_t kPresortMinEntries = TB_PRESORT_MIN;
 constexpr uint32_t kPad = 0xFFFFFFFFu;  // sorts last; no vertex has this rank (n < 2^32)
 constexpr uint32_t kShortRow = 32;       // longer rows go to the lists of k_sort_long
 constexpr uint32_t kWarpSortMax = 1024;  // longer rows are sorted by a CTA
