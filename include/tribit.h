@@ -61,7 +61,7 @@ enum {
 enum {
   TRIBIT_DISPATCH_PLAIN = 0,   /* fixed thresholds on row-block features */
   TRIBIT_DISPATCH_LEARNED = 1, /* MLP over row-block features (tribit_model_*) */
-  TRIBIT_DISPATCH_MERGE = 2,   /* force sorted-list merge everywhere */
+  TRIBIT_DISPATCH_MERGE = 2,   /* force merge (row pieces and the hub pass) everywhere */
   TRIBIT_DISPATCH_BITMAP = 3,  /* force LOP3 + popc on bit-packed rows everywhere */
   TRIBIT_DISPATCH_MMA = 4      /* force b1 AND+POPC tensor-core tiles everywhere */
 };
@@ -173,19 +173,19 @@ tribit_status tribit_read_count(tribit_context* ctx, tribit_result* out);
 
 /* ---- launch tuning and CUDA-graph replay (no counterpart in the reference) - */
 typedef struct tribit_tuning {
-  int ctas_per_sm;      /* CTAs per SM of the warp-per-piece kernels; 0 = default (6) */
+  int ctas_per_sm;      /* CTAs per SM of the warp-per-piece kernels, which run five at a time; 0 = default (6) */
   uint32_t piece_width; /* neighbours per work piece: a multiple of 32, >= 32 (default 64) */
   float tile_min_nnz;   /* plain dispatch: fewest edges of a row block sent to the bit tiles, which
                            also need 1/8 of the tile's cells set (default 64; 1e30 = off) */
   float count_ms;       /* tribit_autotune: measured counting time of this setting */
-  float merge_ratio;    /* plain dispatch: a row block not sent to the tiles goes to the sorted-list
+  float merge_ratio;    /* plain dispatch: a row block not sent to the tiles goes to
                            merge when its neighbours' bit rows average at least merge_ratio times
                            its own rows' length, else to the bitmap sweep (default 0.75; 1e30 = never) */
   uint32_t launch_model; /* TRIBIT_LAUNCH_KERNELS: one persistent kernel per variant;
                             TRIBIT_LAUNCH_QUEUE: the row-piece and hub work in one persistent
                             kernel whose CTAs take heavy rows, hub CTA pieces, then per warp
                             bitmap, merge and hub pieces from the device cursors (the bit tiles
-                            and the fallback rows keep their kernels; ctas_per_sm unused);
+                            and the wide rows keep their kernels; ctas_per_sm unused);
                             TRIBIT_LAUNCH_AUTO (default): the queue up to 2^24 entries, where
                             kernel boundaries weigh most, else the kernels */
 } tribit_tuning;

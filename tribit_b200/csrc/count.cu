@@ -1,16 +1,16 @@
 // Counting kernels; see count.cuh.
 //
-// A piece is (row u, neighbours [s, min(s + 64, d+(u)))). A warp that takes a
-// piece of u loads u's row into a per-warp shared-memory structure -- a
-// bucketed hash of u's 32-column bit blocks (bitmap variant) or u's sorted
-// neighbour list (merge variant) -- reusing it when its next piece is of the
-// same row, then visits every item of every neighbour v of the piece: v's bit
-// blocks (bitmap) or v's neighbours (merge), each looked up in u's structure.
-// Neighbours with long lists are swept by all 32 lanes; short lists are
-// flattened across lanes. Rows whose structure does not fit a warp's slice are
-// cut into pieces of their own for a CTA each (heavy), and rows too large for
-// that for a CTA with a larger table or a search in global memory (wide), so
-// every piece of every list is counted exactly once.
+// A piece is (row u, neighbours [s, min(s + width, d+(u)))). A warp that takes a
+// piece of u stages u's 32-column bit blocks in its slice of shared memory --
+// direct-mapped masks where their span is short, one block a slot for up to 32
+// blocks, else a bucketed hash -- reusing them when its next piece is of the same
+// row, then looks up every bit block of every neighbour v of the piece there.
+// The merge variant's pieces are counted in the same way; what sets it apart is
+// the hub pass, which takes the edges whose tail of u is shorter than v's row.
+// The neighbours' lists are flattened across lanes. Rows of more blocks than a
+// warp's slice holds are cut into pieces of their own for a CTA each (heavy), and
+// rows too large for that for a CTA with a larger table or a search in global
+// memory (wide), so every piece of every list is counted exactly once.
 #include <cstddef>
 
 #include "count.cuh"
@@ -1333,9 +1333,9 @@ __global__ void __launch_bounds__(kCtaThreads) k_rows_wide(GraphView g, const ui
 }
 
 // ---- hub pass: the merge variant's walks of u's tail ------------------------
-// For an edge (u, v) of a merge row block, the sorted-list intersection walks
-// the shorter of u's tail (u's bit blocks from v's block on: the only ones
-// that can meet N+(v)) and v's bit row. Where the tail is shorter and v's row
+// For an edge (u, v) of a merge row block, the matches lie in u's tail (u's bit
+// blocks from v's block on: the only ones that can meet N+(v)) and in v's bit
+// row; u's own pieces look up all of v's row. Where the tail is shorter and v's row
 // spans at most kHubMaxSpan blocks, the schedule groups the edge under v (the
 // hub) and flags it so the row sweeps skip it. A CTA then stages v's bit row
 // once as a direct-mapped array of masks over its block span, and its warps
@@ -1826,7 +1826,7 @@ __global__ void __launch_bounds__(kHubWarps * 32, TB_HUB_MIN_CTAS) k_hub(GraphVi
 // then each warp bitmap and merge pieces, then the CTA hub CTA pieces and each
 // warp hub warp pieces, so no CTA waits at a kernel boundary for another
 // kernel's tail. The
-// bit tiles (128-thread CTAs with tensor memory) and the fallback rows (128
+// bit tiles (128-thread CTAs with tensor memory) and the wide rows (128
 // KiB tables), which need other CTA shapes, keep their own kernels. Shared
 // memory: warp w's slice at w * kHubWarpStride words serves both bodies (a
 // row-piece table needs kWarpSlots 8-byte words), and the CTA phases use the
@@ -2062,12 +2062,12 @@ __global__ void __launch_bounds__(256, 5) k_features(GraphView g, uint32_t nrb, 
       // share one narrow column range and are dense in it (at least 1/8 of
       // the 32 x 32 * span cells set, and tile_min_nnz edges): on disjoint
       // cliques tiles beat the sweeps, on sparse small graphs (1-2 % dense)
-      // they lose. Otherwise the sorted-list merge where the neighbours' bit
-      // rows average at least merge_ratio times the block's own (wb / nnz
-      // against nb / rows; needs the neighbour-side pass): the power-law
-      // case, where the merge's hub pass walks u's short tail against a long,
-      // staged row of v instead of probing every block of v. The bitmap sweep
-      // everywhere else (rows and neighbours of similar length).
+      // they lose. Otherwise merge where the neighbours' bit rows average at
+      // least merge_ratio times the block's own (wb / nnz against nb / rows;
+      // needs the neighbour-side pass): the power-law case, where the hub pass
+      // walks u's short tail against a long, staged row of v instead of probing
+      // every block of v. The bitmap sweep everywhere else (rows and
+      // neighbours of similar length).
       uint8_t var = TRIBIT_VARIANT_BITMAP;
       if (span > 0.f && span <= (float)kTileMaxK && nnz >= tile_min_nnz && nnz >= span * (1024.f / kTileMinDensityInv))
         var = TRIBIT_VARIANT_MMA;
@@ -2890,6 +2890,8 @@ LaunchInfo launch_count(const GraphView& graph, const Schedule& s, DeviceStats* 
     TB_CUDA(cudaFuncSetAttribute(k_tiles_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem)));
   });
   const int sms = cfg.num_sms > 0 ? cfg.num_sms : 148;
+  // Unset: six a multiprocessor, of which the row pieces' registers let five run
+  // at a time; five, six and seven count the same from RMAT-19 to RMAT-24, four 8% slower.
   const int per_sm = cfg.ctas_per_sm > 0 ? cfg.ctas_per_sm : 6;
   const unsigned warp_grid = (unsigned)(sms * per_sm);
   LaunchInfo info;

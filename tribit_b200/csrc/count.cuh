@@ -101,21 +101,24 @@ struct CountConfig {
   bool queue = false;                      // TRIBIT_LAUNCH_QUEUE (not in the timing mode)
 };
 
-// TRIBIT_LAUNCH_AUTO takes the queue kernel up to this many entries: on one
-// B200 it counted Chung-Lu n = 7,115 in 0.051 ms instead of 0.085, RMAT-16
-// 32% and RMAT-18 12% faster, RMAT-20 (2^24 entries) even, and RMAT-21 to 24
-// 3-5% slower (5 CTAs an SM for the row pieces instead of 6-7).
+// TRIBIT_LAUNCH_AUTO takes the queue kernel up to this many entries, where the
+// boundaries between kernels weigh most (plain dispatch, queue and kernels:
+// RMAT-16 90 and 154 us, RMAT-18 234 and 293, RMAT-20, 2^24 entries, 1,170 and
+// 1,237). Beyond, it depends on the graph: RMAT-22 6.31 and 6.64 ms, RMAT-24 37.35
+// and 37.22, but planted partition of 2 million vertices 1.88 and 1.58, Erdos-Renyi
+// of 2^25 entries 2.17 and 2.11.
 constexpr uint64_t kQueueMaxEntries = 1ull << 24;
 
-// hubs: also take the hub-pass arrays (about 13 bytes per entry). stats: the
+// hubs: also take the hub-pass arrays (about 8 bytes per entry and 36 per vertex). stats: the
 // prepared graph's, which holds the schedule's words (null when measuring).
 Schedule take_schedule(Arena& ar, uint64_t n, uint64_t E, DeviceStats* stats, bool hubs = true);
+
+// Sends the row blocks dispatched to the merge variant to the bitmap sweep.
+void merge_blocks_to_bitmap(Schedule& s, cudaStream_t st);
 
 // Computes row-block features, the per-block variant (mode: TRIBIT_DISPATCH_*),
 // and the per-variant piece lists. full_features adds the neighbour-side
 // features (one extra pass over the edges) the learned dispatcher needs.
-// Sends the row blocks dispatched to the merge variant to the bitmap sweep.
-void merge_blocks_to_bitmap(Schedule& s, cudaStream_t st);
 void build_schedule(const GraphView& g, Schedule& s, int mode, bool full_features, cudaStream_t st);
 
 // Row-block features (full adds the neighbour-side ones) and the plain or

@@ -498,7 +498,7 @@ void apply_dispatch(tribit_context* c, cudaStream_t st) {
   }
   // Both rules choose merge for the hub pass; a schedule taken without hub
   // lists (the rows tier under a small device budget) sweeps those blocks as
-  // bitmaps instead (RMAT-24: 132 ms all-bitmap against 168 ms merge without
+  // bitmaps instead (RMAT-24: 122 ms all-bitmap against 130 ms merge without
   // the hub pass).
   if (!c->sched.eflag && (mode == TRIBIT_DISPATCH_LEARNED || mode == TRIBIT_DISPATCH_PLAIN))
     merge_blocks_to_bitmap(c->sched, st);

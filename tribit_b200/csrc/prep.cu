@@ -399,7 +399,7 @@ __global__ void k_identity_graph_of(uint64_t n, const uint64_t* voff, uint32_t G
 // Every entry is oriented from its lower-ranked endpoint lo to the higher hi.
 // A counting sort by lo (the histogram is the oriented out-degree) places the
 // hi's of each row together; each row is then sorted and deduplicated on its
-// own (rows are short: with degree order no row exceeds sqrt(2m) entries), and
+// own (rows are short: with degree order none has more than sqrt(2E) neighbours), and
 // one scan of the per-row (distinct neighbours, distinct 32-column blocks)
 // pairs gives the CSR and bit-row offsets. The 48-bit global radix sort of
 // (lo, hi) keys that this replaces took six passes over all entries.
