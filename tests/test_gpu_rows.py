@@ -103,3 +103,20 @@ def test_rows_between_long_runs_of_empty_rows():
         with tb.Counter(order=order) as c:
             r = c.count_edges(noisy(e, seed=3, copies=2), n)
             assert (r.triangles, r.edges) == (want, m)
+
+
+def test_presorted_fill_keeps_its_ctas_together():
+    # 2^27 entries presort their keys; the fill's CTAs then take them in launch
+    # order, a few tiles of 1,024 each, instead of all striding through all of them.
+    import torch
+
+    from tests.test_gpu_batch import _device_work
+    n, E = 1 << 20, 1 << 27
+    base = tb.gen_rmat(16, 16, seed=8)
+    want = oracle.count(base, 1 << 16)
+    d = torch.from_numpy(base.view(np.int64)).cuda().repeat(E // base.size)
+    with tb.Counter() as c:
+        r = c.count_edges_device(d.data_ptr(), E, n)
+        assert (r.triangles, r.edges) == want
+        assert _device_work(lambda: c.count_edges_device(d.data_ptr(), E, n),
+                            lambda work: any("k_row_fill(" in w and 8 * 1024 * g[0] >= E for w, g in work)) is not False
