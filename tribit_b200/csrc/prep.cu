@@ -285,7 +285,12 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_one(const uint32_t* __res
   const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   uint32_t* wcnt = rank_sm + 2 * kRankOneMax;  // [warp][digit]
   for (uint64_t i = n + (rw.off ? 1 : 0) + tid; i < rw.count; i += kRankThreads) rw.w[i] = 0;
-  for (uint32_t i = tid; i < n; i += kRankThreads) src[i] = (degree_key(deg[i], dk) << 16) | i;
+  bool hubs = false;  // whether a key of this thread's, then any thread's, is a hub's
+  for (uint32_t i = tid; i < n; i += kRankThreads) {
+    const uint32_t key = degree_key(deg[i], dk);
+    hubs |= hub_key(key, dk);
+    src[i] = (key << 16) | i;
+  }
   const uint32_t rounds = (n + kRankThreads - 1) / kRankThreads;  // of 32 a warp
   for (int shift = 16; shift < 32; shift += 8) {
     for (uint32_t i = tid; i < (kRankThreads / 32) * 256; i += kRankThreads) wcnt[i] = 0;
@@ -332,14 +337,12 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_one(const uint32_t* __res
       const uint32_t i = (w * rounds + r) * 32 + lane;
       if (i < n) dst[wcnt[w * 256 + ((v[r] >> shift) & 255u)] + pos[r]] = v[r];
     }
-    __syncthreads();
+    hubs = __syncthreads_or(hubs ? 1 : 0) != 0;
     uint32_t* t = src;
     src = dst;
     dst = t;
   }
-  bool hubs = false;
-  for (uint32_t i = tid; i < n; i += kRankThreads) hubs |= hub_key(src[i] >> 16, dk);
-  if (__syncthreads_or(hubs ? 1 : 0)) {
+  if (hubs) {
     for (uint32_t i = tid; i < n; i += kRankThreads) {
       uint32_t at = i;
       if (hub_key(src[i] >> 16, dk))
