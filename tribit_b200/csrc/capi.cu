@@ -54,12 +54,12 @@ void layout(tribit_context* c, bool measure, const tb::PrepInput& in, bool stage
 }
 
 // The arena of one call: rows in degree-sized slots where their 4 bytes an
-// entry more can be had, else compact rows. (An arena that would have to grow
-// past the free memory is not given up for the attempt.)
+// entry more can be had, else compact rows. (Once an arena of a size could not be
+// had, a held one is not given up again for the attempt unless the memory is free.)
 void reserve_layout(tribit_context* c, tb::PrepInput& in, bool stage, uint32_t G, CallLayout* L) {
   layout(c, true, in, stage, G, L);
-  size_t fr = 0, tot = 0;
-  if (!in.compact && c->arena.used() > c->arena.capacity()) {
+  if (!in.compact && c->arena.used() > c->arena.capacity() && c->arena.used() >= c->refused_bytes) {
+    size_t fr = 0, tot = 0;
     TB_CUDA(cudaMemGetInfo(&fr, &tot));
     in.compact = c->arena.used() > fr + c->arena.capacity();
     if (in.compact) layout(c, true, in, stage, G, L);
@@ -68,6 +68,7 @@ void reserve_layout(tribit_context* c, tb::PrepInput& in, bool stage, uint32_t G
     c->arena.reserve(c->arena.used(), c->device_budget == 0);
   } catch (const StatusError& e) {
     if (e.status != TRIBIT_ERR_OUT_OF_MEMORY || in.compact) throw;
+    c->refused_bytes = c->arena.used();
     in.compact = true;
     layout(c, true, in, stage, G, L);
     c->arena.reserve(c->arena.used(), c->device_budget == 0);

@@ -54,6 +54,7 @@ struct tribit_context {
   // Device memory the context may use (tribit_set_device_budget; 0: what the
   // device has free); graphs needing more are counted in rank ranges.
   uint64_t device_budget = 0;
+  uint64_t refused_bytes = ~0ull;      // the last arena size that could not be had
   uint32_t launch_model = TRIBIT_LAUNCH_AUTO;  // tribit_tuning.launch_model
   int stream_tier = 0;                 // TRIBIT_STREAM_* (tribit_set_stream_options)
   uint64_t stream_range_entries = 0;   // bound on a rank range's entries (0: the budget's)
