@@ -88,6 +88,40 @@ def test_training_reduces_loss_and_save_load_roundtrip(tmp_path):
         np.testing.assert_array_equal(c2.model_predict(x[:100]), pred)
 
 
+@pytest.mark.parametrize("rows", [2, 15, 16, 17, 24, 25, 511, 512, 513, 2048, 2049])
+def test_passes_where_rows_a_warp_and_split_change(rows):
+    # One row a warp and 8-row sums up to 512 rows, two rows a warp up to 2,048;
+    # tolerances as above.
+    x, y = _data(max(rows, 4), seed=rows)
+    norm = _norm(x, y)
+    x, y = x[:rows], y[:rows]
+    with tb.Counter() as c:
+        c.model_init(norm, seed=17)
+        p = c.model_params()
+        eff = c.model_params(effective=True)
+        g, loss = c.model_gradients(x, y)
+        train_loss = c.model_train(x, y, epochs=1, batch=rows, lr=1e-3, seed=1)
+        got = c.model_params()
+    _, want_loss, want = mlp.forward_backward(eff, norm, x, y)
+    assert abs(loss - want_loss) <= 1e-4 * want_loss and abs(train_loss - want_loss) <= 1e-4 * want_loss
+    assert np.abs(g - want).max() <= 1e-4 * np.abs(want).max()
+    # The first Adam step moves a parameter by lr g / (|g| + 1e-8): by lr where |g| is
+    # 1e-5 and more, and a parameter of up to 0.5 rounds that by 2^-25, 3e-5 of it.
+    big = np.abs(want) > max(1e-2 * np.abs(want).max(), 1e-5)
+    np.testing.assert_allclose((got - p)[big], -1e-3 * np.sign(want)[big], rtol=2e-3)
+
+
+def test_small_training_batches_are_spread_over_ctas():
+    from tests.test_gpu_batch import _device_work
+    x, y = _data(320, seed=4)
+    with tb.Counter() as c:
+        c.model_init(_norm(x, y), seed=3)
+        assert _device_work(lambda: c.model_train(x, y, epochs=1, batch=32),
+                            lambda work: any("k_fwd_bwd" in w and g[0] >= 4 for w, g in work) and
+                            any("k_wgrad(" in w and g[0] >= 4 for w, g in work) and
+                            not any("k_wgrad_sum" in w for w, _ in work)) is not False
+
+
 def _epoch_order(rows, seed):
     """Rows in the order an epoch takes them: a shuffle driven by tb_rand (csrc/gen.h)."""
     u = np.uint64

@@ -12,7 +12,7 @@ int main() {
   uint32_t most = 0;
   for (uint32_t b = 1; b <= 60000; ++b) {
     const uint32_t ctas = tb::wgrad_ctas(b), rows = tb::wgrad_rows(b);
-    if (rows % tb::kGradTile || (uint64_t)ctas * rows < b || ctas > tb::kGradCtas) return std::printf("split %u\n", b), 1;
+    if (rows % tb::wgrad_unit(b) || (uint64_t)ctas * rows < b || ctas > tb::kGradCtas) return std::printf("split %u\n", b), 1;
     most = std::max(most, ctas);  // the most CTAs a batch of up to b rows takes
     if (tb::wgrad_parts(b) < most) return std::printf("%u rows: %u parts, %u CTAs\n", b, tb::wgrad_parts(b), most), 1;
   }

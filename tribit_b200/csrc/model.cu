@@ -27,9 +27,12 @@ __host__ __device__ __forceinline__ bool is_weight(int p) {
 // then serves kRows rows, and a unit's activations are read back four at a time
 // as one broadcast. One row a warp, its activations passed by shuffles, was
 // bound by the shuffles and weight reads: 65,521 rows predicted in 110 us, now
-// 36; forward and backward 161, now 71.
+// 36; forward and backward 161, now 71. A batch that leaves the chip idle is
+// better spread (forward_backward): a training step of 32 rows takes 22.9 us with
+// a row a warp and 29 with eight, of 512 25.4 and 33, of 1,024 30 with two and 36
+// with eight, of 4,096 60 either way, of 8,192 98 with one and 95 with eight.
 constexpr int kRows = 8;
-static_assert(kRows * kIn == 4 * 32, "a warp loads kRows rows of features as one float4 a lane");
+static_assert(kRows * kIn <= 4 * 32, "a warp loads its rows of features as one float4 a lane");
 constexpr int kW2tStride = kH1 + 1;  // padded: transposing W2 writes 32 different banks
 
 // Shared-memory image of a model: parameters, normalisation and, for the
@@ -64,20 +67,20 @@ struct Acts {  // per-row activations kept for the weight gradients
 
 // a[r], b[r] += sum over the K inputs of row r (at h + r * K, ascending) times
 // columns lane and lane + 32 of w (rows of `stride` floats).
-template <int K>
+template <int K, int R>
 __device__ __forceinline__ void dense(const float* __restrict__ w, int stride, const float* __restrict__ h,
-                                      float (&a)[kRows], float (&b)[kRows]) {
+                                      float (&a)[R], float (&b)[R]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll 4
   for (int k = 0; k < K; k += 4) {
-    float4 x[kRows];
+    float4 x[R];
 #pragma unroll
-    for (int r = 0; r < kRows; ++r) x[r] = *reinterpret_cast<const float4*>(h + r * K + k);
+    for (int r = 0; r < R; ++r) x[r] = *reinterpret_cast<const float4*>(h + r * K + k);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float wa = w[(k + q) * stride + lane], wb = w[(k + q) * stride + lane + 32];
 #pragma unroll
-      for (int r = 0; r < kRows; ++r) {
+      for (int r = 0; r < R; ++r) {
         const float v = q == 0 ? x[r].x : q == 1 ? x[r].y : q == 2 ? x[r].z : x[r].w;
         a[r] = fmaf(v, wa, a[r]);
         b[r] = fmaf(v, wb, b[r]);
@@ -87,46 +90,47 @@ __device__ __forceinline__ void dense(const float* __restrict__ w, int stride, c
 }
 
 // Lane l's two units of every row into the warp's activations.
-__device__ __forceinline__ void put_units(float* act, const float (&a)[kRows], const float (&b)[kRows]) {
+template <int R>
+__device__ __forceinline__ void put_units(float* act, const float (&a)[R], const float (&b)[R]) {
   const int lane = threadIdx.x & 31;
   __syncwarp();
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) {
+  for (int r = 0; r < R; ++r) {
     act[r * kH1 + lane] = a[r];
     act[r * kH1 + lane + 32] = b[r];
   }
   __syncwarp();
 }
 
-// kRows rows a warp; lane l owns hidden units l and l + 32 of both layers.
+// R rows a warp; lane l owns hidden units l and l + 32 of both layers.
 // Computes the normalised predictions of the rows x(r), r < rows (the others
 // repeat row 0 and are not stored); with Train also the backward pass for the
 // MSE loss on normalised targets y(r) (scaled by inv_count), storing what the
 // weight-gradient kernel needs in slots slot .. slot + rows and returning the
 // rows' summed squared error.
-template <bool Train, class RowOf>
+template <bool Train, int R, class RowOf>
 __device__ __forceinline__ float rows_pass(const SmemModel& s, const float* w2t, float* act, const float* __restrict__ X,
                                            const float* __restrict__ Y, const RowOf& row_of, int rows, float inv_count,
-                                           float (&out)[kRows][kOut], const Acts* acts, uint32_t slot) {
+                                           float (&out)[R][kOut], const Acts* acts, uint32_t slot) {
   const int lane = threadIdx.x & 31;
-  {
+  __syncwarp();
+  if (lane < R * kIn / 4) {
     const int r = lane / (kIn / 4), q = (lane % (kIn / 4)) * 4;
     const float4 x = *reinterpret_cast<const float4*>(X + (size_t)row_of(r < rows ? r : 0) * kIn + q);
     const float4 v = make_float4((x.x - s.norm[q]) / s.norm[kIn + q], (x.y - s.norm[q + 1]) / s.norm[kIn + q + 1],
                                  (x.z - s.norm[q + 2]) / s.norm[kIn + q + 2],
                                  (x.w - s.norm[q + 3]) / s.norm[kIn + q + 3]);
-    __syncwarp();
     *reinterpret_cast<float4*>(act + r * kIn + q) = v;
     if (Train && r < rows) *reinterpret_cast<float4*>(acts->xn + (size_t)(slot + r) * kIn + q) = v;
-    __syncwarp();
   }
-  float a[kRows], b[kRows];  // the layer's pre-activations
+  __syncwarp();
+  float a[R], b[R];  // the layer's pre-activations
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) a[r] = s.p[kB1 + lane], b[r] = s.p[kB1 + lane + 32];
-  dense<kIn>(s.p + kW1, kH1, act, a, b);
+  for (int r = 0; r < R; ++r) a[r] = s.p[kB1 + lane], b[r] = s.p[kB1 + lane + 32];
+  dense<kIn, R>(s.p + kW1, kH1, act, a, b);
   uint32_t on1 = 0;  // bits 2r, 2r + 1: row r's two units are active
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) {
+  for (int r = 0; r < R; ++r) {
     if (Train) on1 |= (a[r] > 0.f ? 1u << (2 * r) : 0u) | (b[r] > 0.f ? 2u << (2 * r) : 0u);
     a[r] = fmaxf(a[r], 0.f), b[r] = fmaxf(b[r], 0.f);
     if (Train && r < rows) {
@@ -134,13 +138,13 @@ __device__ __forceinline__ float rows_pass(const SmemModel& s, const float* w2t,
       acts->h1[(size_t)(slot + r) * kH1 + lane + 32] = b[r];
     }
   }
-  put_units(act, a, b);
+  put_units<R>(act, a, b);
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) a[r] = s.p[kB2 + lane], b[r] = s.p[kB2 + lane + 32];
-  dense<kH1>(s.p + kW2, kH2, act, a, b);
+  for (int r = 0; r < R; ++r) a[r] = s.p[kB2 + lane], b[r] = s.p[kB2 + lane + 32];
+  dense<kH1, R>(s.p + kW2, kH2, act, a, b);
   uint32_t on2 = 0;
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) {
+  for (int r = 0; r < R; ++r) {
     if (Train) on2 |= (a[r] > 0.f ? 1u << (2 * r) : 0u) | (b[r] > 0.f ? 2u << (2 * r) : 0u);
     const float h2a = fmaxf(a[r], 0.f), h2b = fmaxf(b[r], 0.f);
 #pragma unroll
@@ -154,7 +158,7 @@ __device__ __forceinline__ float rows_pass(const SmemModel& s, const float* w2t,
   if constexpr (!Train) return 0.f;
   float sq = 0.f;
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) {
+  for (int r = 0; r < R; ++r) {
     float dh2a = 0.f, dh2b = 0.f;
     const size_t yr = (size_t)row_of(r < rows ? r : 0) * kOut;
 #pragma unroll
@@ -176,12 +180,12 @@ __device__ __forceinline__ float rows_pass(const SmemModel& s, const float* w2t,
       acts->dz2[(size_t)(slot + r) * kH2 + lane + 32] = b[r];
     }
   }
-  put_units(act, a, b);
+  put_units<R>(act, a, b);
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) a[r] = 0.f, b[r] = 0.f;
-  dense<kH2>(w2t, kW2tStride, act, a, b);
+  for (int r = 0; r < R; ++r) a[r] = 0.f, b[r] = 0.f;
+  dense<kH2, R>(w2t, kW2tStride, act, a, b);
 #pragma unroll
-  for (int r = 0; r < kRows; ++r)
+  for (int r = 0; r < R; ++r)
     if (r < rows) {
       acts->dz1[(size_t)(slot + r) * kH1 + lane] = (on1 >> (2 * r)) & 1u ? a[r] : 0.f;
       acts->dz1[(size_t)(slot + r) * kH1 + lane + 32] = (on1 >> (2 * r)) & 2u ? b[r] : 0.f;
@@ -189,7 +193,8 @@ __device__ __forceinline__ float rows_pass(const SmemModel& s, const float* w2t,
   return sq;
 }
 
-// Forward + backward over rows idx[r0 .. r0 + B) (idx null: identity).
+// Forward + backward over rows idx[r0 .. r0 + B) (idx null: identity), R a warp.
+template <int R>
 __global__ void __launch_bounds__(kModelThreads) k_fwd_bwd(const float* __restrict__ X, const float* __restrict__ Y,
                                                             const uint32_t* __restrict__ idx, uint32_t r0, uint32_t B,
                                                             const float* __restrict__ eff,
@@ -202,19 +207,19 @@ __global__ void __launch_bounds__(kModelThreads) k_fwd_bwd(const float* __restri
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   float* act = st.m.act[threadIdx.x >> 5];
   float sq = 0.f;
-  for (uint64_t i = (uint64_t)warp * kRows; i < B; i += (uint64_t)nw * kRows) {
+  for (uint64_t i = (uint64_t)warp * R; i < B; i += (uint64_t)nw * R) {
     const uint32_t base = r0 + (uint32_t)i;
-    float out[kRows][kOut];
-    sq += rows_pass<true>(st.m, st.w2t, act, X, Y, [&](int r) { return idx ? idx[base + r] : base + r; },
-                          (int)min((uint64_t)kRows, B - i), inv_count, out, &acts, (uint32_t)i);
+    float out[R][kOut];
+    sq += rows_pass<true, R>(st.m, st.w2t, act, X, Y, [&](int r) { return idx ? idx[base + r] : base + r; },
+                             (int)min((uint64_t)R, B - i), inv_count, out, &acts, (uint32_t)i);
   }
   if ((threadIdx.x & 31) == 0 && sq != 0.f) atomicAdd(loss, sq);
 }
 
 // The weight gradients in two steps: CTA c sums rows [c R, c R + R) of the
 // batch into part[c] (every parameter's sum in registers, rows staged kGradTile
-// at a time), and k_wgrad_sum adds the CTAs' sums in order, so the result depends on the
-// batch size alone. The 64 x 64 block is 4 x 4 sums a thread (two 16-byte
+// at a time), and k_wgrad_sum, or the step that uses them (k_adam), adds the CTAs' sums in
+// order, so the result depends on the batch size alone. The 64 x 64 block is 4 x 4 sums a thread (two 16-byte
 // shared reads for 16 products). One thread a parameter walking all rows left
 // all but 22 CTAs of the chip idle, each step a pair of dependent L2 reads:
 // 65,521 rows in 4,656 us, now 99. Sizes: wgrad_rows, wgrad_ctas.
@@ -282,13 +287,15 @@ __global__ void __launch_bounds__(256) k_wgrad(Acts a, uint32_t B, float* __rest
 static_assert(kIn == 16 && kH1 == 64 && kH2 == 64 && kH2 * kOut <= 256 && kH1 + kH2 + kOut <= 256,
               "k_wgrad's thread layout");
 
-__global__ void k_wgrad_sum(const float* __restrict__ part, uint32_t ctas, float* __restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kNumParams) return;
+__device__ __forceinline__ float sum_parts(const float* __restrict__ part, uint32_t parts, int p) {
   float g = 0.f;
 #pragma unroll 8
-  for (uint32_t c = 0; c < ctas; ++c) g += part[(size_t)c * kNumParams + p];
-  grad[p] = g;
+  for (uint32_t c = 0; c < parts; ++c) g += part[(size_t)c * kNumParams + p];
+  return g;
+}
+__global__ void k_wgrad_sum(const float* __restrict__ part, uint32_t parts, float* __restrict__ grad) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < kNumParams) grad[p] = sum_parts(part, parts, p);
 }
 
 __device__ __forceinline__ float to_eff(int p, float w) {
@@ -296,10 +303,11 @@ __device__ __forceinline__ float to_eff(int p, float w) {
 }
 
 __global__ void k_adam(float* __restrict__ master, float* __restrict__ eff, float* __restrict__ m, float* __restrict__ v,
-                       const float* __restrict__ grad, float lr, float b1, float b2, float eps, float c1, float c2) {
+                       const float* __restrict__ part, uint32_t parts, float lr, float b1, float b2, float eps, float c1,
+                       float c2) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kNumParams) return;
-  const float g = grad[p];
+  const float g = sum_parts(part, parts, p);
   const float mm = b1 * m[p] + (1.f - b1) * g;
   const float vv = b2 * v[p] + (1.f - b2) * g * g;
   m[p] = mm;
@@ -327,7 +335,7 @@ __global__ void __launch_bounds__(kModelThreads) k_predict(const float* __restri
   for (uint64_t i = (uint64_t)warp * kRows; i < rows; i += (uint64_t)nw * kRows) {
     const uint32_t base = (uint32_t)i, n = (uint32_t)min((uint64_t)kRows, rows - i);
     float out[kRows][kOut];
-    rows_pass<false>(s, nullptr, s.act[threadIdx.x >> 5], X, nullptr, [&](int r) { return base + r; }, (int)n, 0.f, out,
+    rows_pass<false, kRows>(s, nullptr, s.act[threadIdx.x >> 5], X, nullptr, [&](int r) { return base + r; }, (int)n, 0.f, out,
                      nullptr, 0);
     float v = 0.f;  // lane r * kOut + o: output o of row r
 #pragma unroll
@@ -353,7 +361,7 @@ __global__ void __launch_bounds__(kModelThreads) k_dispatch(const float* __restr
   for (uint64_t i = (uint64_t)warp * kRows; i < nrb; i += (uint64_t)nw * kRows) {
     const uint32_t base = (uint32_t)i, n = (uint32_t)min((uint64_t)kRows, nrb - i);
     float out[kRows][kOut];
-    rows_pass<false>(s, nullptr, s.act[threadIdx.x >> 5], feat, nullptr, [&](int r) { return base + r; }, (int)n, 0.f,
+    rows_pass<false, kRows>(s, nullptr, s.act[threadIdx.x >> 5], feat, nullptr, [&](int r) { return base + r; }, (int)n, 0.f,
                      out, nullptr, 0);
     float y[kOut] = {};  // lane r: the outputs of row r
 #pragma unroll
@@ -382,15 +390,17 @@ __global__ void __launch_bounds__(kModelThreads) k_dispatch(const float* __restr
 
 void set_smem_attrs() {
   once_per_device<1>([] {
-    TB_CUDA(cudaFuncSetAttribute(k_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemTrain)));
+    TB_CUDA(cudaFuncSetAttribute(k_fwd_bwd<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemTrain)));
+    TB_CUDA(cudaFuncSetAttribute(k_fwd_bwd<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemTrain)));
+    TB_CUDA(cudaFuncSetAttribute(k_fwd_bwd<kRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemTrain)));
     TB_CUDA(cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemModel)));
     TB_CUDA(cudaFuncSetAttribute(k_dispatch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemModel)));
   });
 }
 
-// CTAs for `rows` rows, kRows a warp at a time.
-unsigned grid_warps(uint64_t rows) {
-  const uint64_t g = ceil_div<uint64_t>(rows, kModelThreads / 32 * kRows);
+// CTAs for `rows` rows, `per` a warp at a time.
+unsigned grid_warps(uint64_t rows, int per = kRows) {
+  const uint64_t g = ceil_div<uint64_t>(rows, kModelThreads / 32 * (uint64_t)per);
   return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(g, 148ull * 3));
 }
 
@@ -431,14 +441,31 @@ TrainBuffers stage_training(tribit_context* c, const float* X, const float* Y, u
   return t;
 }
 
+// Forward and backward of the batch's B rows, from row (of idx) r0 on, into t.acts.
+void forward_backward(const TrainBuffers& t, const uint32_t* idx, uint32_t r0, uint32_t B, const DeviceModel& m,
+                      cudaStream_t st) {
+  const float inv = 1.f / (float)(kOut * B);
+  auto launch = [&](auto kernel, int per) {
+    kernel<<<grid_warps(B, per), kModelThreads, sizeof(SmemTrain), st>>>(t.X, t.Y, idx, r0, B, m.eff, m.norm, inv, t.acts,
+                                                                         t.loss);
+    TB_LAUNCH_CHECK();
+  };
+  if (B <= kSmallBatch)
+    launch(k_fwd_bwd<1>, 1);
+  else if (B <= 4 * kSmallBatch)
+    launch(k_fwd_bwd<2>, 2);
+  else
+    launch(k_fwd_bwd<kRows>, kRows);
+}
+
 // The gradient of the batch of B rows in t.acts (B at most the batch t was laid out for: an epoch's last batch is
 // often shorter).
-void weight_gradients(const TrainBuffers& t, uint32_t B, float* grad, cudaStream_t st) {
+// In t.part, as the sums of so many parts (the result), to be added in order.
+uint32_t weight_gradients(const TrainBuffers& t, uint32_t B, cudaStream_t st) {
   const uint32_t ctas = wgrad_ctas(B);
   k_wgrad<<<ctas, 256, 0, st>>>(t.acts, B, t.part);
   TB_LAUNCH_CHECK();
-  k_wgrad_sum<<<(kNumParams + 63) / 64, 64, 0, st>>>(t.part, ctas, grad);
-  TB_LAUNCH_CHECK();
+  return ctas;
 }
 
 void require_model(tribit_context* c) {
@@ -585,13 +612,16 @@ tribit_status tribit_model_gradients(tribit_context* c, const float* x, const fl
     tb::set_smem_attrs();
     tb::TrainBuffers t = tb::stage_training(c, x, y, rows, (uint32_t)rows);
     TB_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(float), c->st));
-    const float inv = 1.f / (float)(tb::kOut * rows);
-    tb::k_fwd_bwd<<<tb::grid_warps(rows), tb::kModelThreads, sizeof(tb::SmemTrain), c->st>>>(
-        t.X, t.Y, nullptr, 0, (uint32_t)rows, c->model.eff, c->model.norm, inv, t.acts, t.loss);
-    TB_LAUNCH_CHECK();
-    tb::weight_gradients(t, (uint32_t)rows, c->model.grad, c->st);
+    tb::forward_backward(t, nullptr, 0, (uint32_t)rows, c->model, c->st);
+    const uint32_t parts = tb::weight_gradients(t, (uint32_t)rows, c->st);
+    const float* sum = t.part;
+    if (parts > 1) {
+      tb::k_wgrad_sum<<<(tb::kNumParams + 63) / 64, 64, 0, c->st>>>(t.part, parts, c->model.grad);
+      TB_LAUNCH_CHECK();
+      sum = c->model.grad;
+    }
     float loss = 0.f;
-    TB_CUDA(cudaMemcpyAsync(grad, c->model.grad, tb::kNumParams * sizeof(float), cudaMemcpyDeviceToHost, c->st));
+    TB_CUDA(cudaMemcpyAsync(grad, sum, tb::kNumParams * sizeof(float), cudaMemcpyDeviceToHost, c->st));
     TB_CUDA(cudaMemcpyAsync(&loss, t.loss, sizeof(float), cudaMemcpyDeviceToHost, c->st));
     TB_CUDA(cudaStreamSynchronize(c->st));
     if (loss_out) *loss_out = loss / (float)(tb::kOut * rows);
@@ -617,14 +647,11 @@ tribit_status tribit_model_train(tribit_context* c, const float* x, const float*
       TB_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(float), c->st));
       for (uint64_t r0 = 0; r0 < rows; r0 += B) {
         const uint32_t nb = (uint32_t)std::min<uint64_t>(B, rows - r0);
-        const float inv = 1.f / (float)(tb::kOut * nb);
-        tb::k_fwd_bwd<<<tb::grid_warps(nb), tb::kModelThreads, sizeof(tb::SmemTrain), c->st>>>(
-            t.X, t.Y, t.idx, (uint32_t)r0, nb, c->model.eff, c->model.norm, inv, t.acts, t.loss);
-        TB_LAUNCH_CHECK();
-        tb::weight_gradients(t, nb, c->model.grad, c->st);
+        tb::forward_backward(t, t.idx, (uint32_t)r0, nb, c->model, c->st);
+        const uint32_t parts = tb::weight_gradients(t, nb, c->st);
         const int step = ++c->model.steps;
-        tb::k_adam<<<(tb::kNumParams + 255) / 256, 256, 0, c->st>>>(
-            c->model.master, c->model.eff, c->model.m, c->model.v, c->model.grad, lr, b1, b2, eps,
+        tb::k_adam<<<(tb::kNumParams + 63) / 64, 64, 0, c->st>>>(
+            c->model.master, c->model.eff, c->model.m, c->model.v, t.part, parts, lr, b1, b2, eps,
             1.f - std::pow(b1, (float)step), 1.f - std::pow(b2, (float)step));
         TB_LAUNCH_CHECK();
       }
