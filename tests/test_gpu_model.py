@@ -111,6 +111,21 @@ def test_passes_where_rows_a_warp_and_split_change(rows):
     np.testing.assert_allclose((got - p)[big], -1e-3 * np.sign(want)[big], rtol=2e-3)
 
 
+@pytest.mark.parametrize("seed", [0, 1, 2])
+def test_loss_of_many_rows_keeps_its_digits(seed):
+    # Thousands of warps add their sums of squares: in double. What is left is the
+    # result's own rounding (2^-24) and the mean of the rows' fp32 errors, whose
+    # signs vary (each at most about 64 * 2^-24 of the row, over 65,521 rows).
+    x, y = _data(65521, seed=seed)
+    norm = _norm(x, y)
+    with tb.Counter() as c:
+        c.model_init(norm, seed=seed)
+        p = c.model_params(effective=True)
+        losses = [c.model_gradients(x, y)[1] for _ in range(5)]
+    want = mlp.forward_backward(p, norm, x, y)[1]
+    assert max(abs(loss - want) for loss in losses) <= 3e-7 * want, [loss / want - 1 for loss in losses]
+
+
 def test_small_training_batches_are_spread_over_ctas():
     from tests.test_gpu_batch import _device_work
     x, y = _data(320, seed=4)

@@ -199,21 +199,23 @@ __global__ void __launch_bounds__(kModelThreads) k_fwd_bwd(const float* __restri
                                                             const uint32_t* __restrict__ idx, uint32_t r0, uint32_t B,
                                                             const float* __restrict__ eff,
                                                             const float* __restrict__ norm, float inv_count, Acts acts,
-                                                            float* loss) {
+                                                            double* loss) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmemTrain& st = *reinterpret_cast<SmemTrain*>(smem_raw);
   load_model(st.m, eff, norm, st.w2t);
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   float* act = st.m.act[threadIdx.x >> 5];
-  float sq = 0.f;
+  // The warps' sums are added as they finish, in double: in float, the order of arrival
+  // left up to 3e-6 of the loss.
+  double sq = 0.0;
   for (uint64_t i = (uint64_t)warp * R; i < B; i += (uint64_t)nw * R) {
     const uint32_t base = r0 + (uint32_t)i;
     float out[R][kOut];
     sq += rows_pass<true, R>(st.m, st.w2t, act, X, Y, [&](int r) { return idx ? idx[base + r] : base + r; },
                              (int)min((uint64_t)R, B - i), inv_count, out, &acts, (uint32_t)i);
   }
-  if ((threadIdx.x & 31) == 0 && sq != 0.f) atomicAdd(loss, sq);
+  if ((threadIdx.x & 31) == 0 && sq != 0.0) atomicAdd(loss, sq);
 }
 
 // The weight gradients in two steps: CTA c sums rows [c R, c R + R) of the
@@ -408,7 +410,7 @@ struct TrainBuffers {
   float* X = nullptr;
   float* Y = nullptr;
   uint32_t* idx = nullptr;
-  float* loss = nullptr;
+  double* loss = nullptr;
   float* part = nullptr;  // wgrad_parts(B) x kNumParams: the gradient's partial sums
   Acts acts{};
 };
@@ -418,7 +420,7 @@ TrainBuffers layout_train(Arena& ar, uint64_t rows, uint32_t B) {
   t.X = ar.take<float>(rows * kIn + 1);
   t.Y = ar.take<float>(rows * kOut + 1);
   t.idx = ar.take<uint32_t>(rows + 1);
-  t.loss = ar.take<float>(1);
+  t.loss = ar.take<double>(1);
   t.acts.xn = ar.take<float>((uint64_t)B * kIn);
   t.acts.h1 = ar.take<float>((uint64_t)B * kH1);
   t.acts.dz1 = ar.take<float>((uint64_t)B * kH1);
@@ -611,7 +613,7 @@ tribit_status tribit_model_gradients(tribit_context* c, const float* x, const fl
     DeviceGuard dg(c->device);
     tb::set_smem_attrs();
     tb::TrainBuffers t = tb::stage_training(c, x, y, rows, (uint32_t)rows);
-    TB_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(float), c->st));
+    TB_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(double), c->st));
     tb::forward_backward(t, nullptr, 0, (uint32_t)rows, c->model, c->st);
     const uint32_t parts = tb::weight_gradients(t, (uint32_t)rows, c->st);
     const float* sum = t.part;
@@ -620,11 +622,11 @@ tribit_status tribit_model_gradients(tribit_context* c, const float* x, const fl
       TB_LAUNCH_CHECK();
       sum = c->model.grad;
     }
-    float loss = 0.f;
+    double loss = 0.0;
     TB_CUDA(cudaMemcpyAsync(grad, sum, tb::kNumParams * sizeof(float), cudaMemcpyDeviceToHost, c->st));
-    TB_CUDA(cudaMemcpyAsync(&loss, t.loss, sizeof(float), cudaMemcpyDeviceToHost, c->st));
+    TB_CUDA(cudaMemcpyAsync(&loss, t.loss, sizeof(double), cudaMemcpyDeviceToHost, c->st));
     TB_CUDA(cudaStreamSynchronize(c->st));
-    if (loss_out) *loss_out = loss / (float)(tb::kOut * rows);
+    if (loss_out) *loss_out = (float)(loss / (double)(tb::kOut * rows));
   });
 }
 
@@ -639,12 +641,12 @@ tribit_status tribit_model_train(tribit_context* c, const float* x, const float*
     tb::TrainBuffers t = tb::stage_training(c, x, y, rows, B);
     std::vector<uint32_t> order(rows);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    float last = 0.f;
+    double last = 0.0;
     for (uint32_t ep = 0; ep < epochs; ++ep) {
       for (uint64_t i = 0; i < rows; ++i) order[i] = (uint32_t)i;
       for (uint64_t i = rows - 1; i > 0; --i) std::swap(order[i], order[tb_rand(seed + ep, i) % (i + 1)]);
       TB_CUDA(cudaMemcpyAsync(t.idx, order.data(), rows * sizeof(uint32_t), cudaMemcpyHostToDevice, c->st));
-      TB_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(float), c->st));
+      TB_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(double), c->st));
       for (uint64_t r0 = 0; r0 < rows; r0 += B) {
         const uint32_t nb = (uint32_t)std::min<uint64_t>(B, rows - r0);
         tb::forward_backward(t, t.idx, (uint32_t)r0, nb, c->model, c->st);
@@ -655,10 +657,10 @@ tribit_status tribit_model_train(tribit_context* c, const float* x, const float*
             1.f - std::pow(b1, (float)step), 1.f - std::pow(b2, (float)step));
         TB_LAUNCH_CHECK();
       }
-      TB_CUDA(cudaMemcpyAsync(&last, t.loss, sizeof(float), cudaMemcpyDeviceToHost, c->st));
+      TB_CUDA(cudaMemcpyAsync(&last, t.loss, sizeof(double), cudaMemcpyDeviceToHost, c->st));
       TB_CUDA(cudaStreamSynchronize(c->st));
     }
-    if (loss_out) *loss_out = last / (float)(tb::kOut * rows);
+    if (loss_out) *loss_out = (float)(last / (double)(tb::kOut * rows));
   });
 }
 
