@@ -127,14 +127,13 @@ def test_loss_of_many_rows_keeps_its_digits(seed):
 
 
 def test_small_training_batches_are_spread_over_ctas():
-    from tests.test_gpu_batch import _device_work
+    from tests.test_gpu_batch import _launches
     x, y = _data(320, seed=4)
     with tb.Counter() as c:
         c.model_init(_norm(x, y), seed=3)
-        assert _device_work(lambda: c.model_train(x, y, epochs=1, batch=32),
-                            lambda work: any("k_fwd_bwd" in w and g[0] >= 4 for w, g in work) and
-                            any("k_wgrad(" in w and g[0] >= 4 for w, g in work) and
-                            not any("k_wgrad_sum" in w for w, _ in work)) is not False
+        for kernel in ("k_fwd_bwd", "k_wgrad"):  # 32 rows: a row a warp of 8, 8-row sums, added by the step
+            grids = _launches(lambda: c.model_train(x, y, epochs=1, batch=32), kernel)
+            assert all(g == 4 for g in grids), (kernel, grids)
 
 
 def _epoch_order(rows, seed):

@@ -105,18 +105,20 @@ def test_rows_between_long_runs_of_empty_rows():
             assert (r.triangles, r.edges) == (want, m)
 
 
-def test_presorted_fill_keeps_its_ctas_together():
-    # 2^27 entries presort their keys; the fill's CTAs then take them in launch
-    # order, a few tiles of 1,024 each, instead of all striding through all of them.
+@pytest.mark.parametrize("log_n", [20, 23])
+def test_presorted_fill_keeps_its_ctas_together_on_sparse_rows(log_n):
+    # 2^27 entries presort their keys. With fewer than 32 entries a row the fill's
+    # CTAs take them in launch order, a few tiles of 1,024 each; with more they all
+    # stride through all of them.
     import torch
 
-    from tests.test_gpu_batch import _device_work
-    n, E = 1 << 20, 1 << 27
+    from tests.test_gpu_batch import _launches
+    n, E = 1 << log_n, 1 << 27
     base = tb.gen_rmat(16, 16, seed=8)
     want = oracle.count(base, 1 << 16)
     d = torch.from_numpy(base.view(np.int64)).cuda().repeat(E // base.size)
     with tb.Counter() as c:
         r = c.count_edges_device(d.data_ptr(), E, n)
         assert (r.triangles, r.edges) == want
-        assert _device_work(lambda: c.count_edges_device(d.data_ptr(), E, n),
-                            lambda work: any("k_row_fill(" in w and 8 * 1024 * g[0] >= E for w, g in work)) is not False
+        grids = _launches(lambda: c.count_edges_device(d.data_ptr(), E, n), "k_row_fill(")
+        assert all((8 * 1024 * g >= E) == (E < 32 * n) for g in grids), grids

@@ -449,16 +449,14 @@ __global__ void __launch_bounds__(kThreads) k_row_count(PrepInput in, const uint
 
 // nbr[cur[lo]++] = hi (cur starts as the row offsets): the only random
 // accesses are the cursors, which stay in L2, one update a run of equal lo. A
-// CTA takes kFillTiles tiles in a row, so that the CTAs at work are together in
-// the presorted keys and their stores in a few ranges of rows (RMAT-24, all CTAs
-// striding through all keys: 4.9 ms, now 3.9; RMAT-23 preprocessing 14.0, now 14.1; 16 tiles
-// and more lose both).
-constexpr uint64_t kFillTiles = 4;
-__global__ void __launch_bounds__(kThreads) k_row_fill(const uint64_t* __restrict__ keys, uint64_t E,
+// CTA takes `tiles` tiles in a row, then on by the grid (fill_keys).
+__global__ void __launch_bounds__(kThreads) k_row_fill(const uint64_t* __restrict__ keys, uint64_t E, uint32_t tiles,
                                                        uint32_t* __restrict__ cur, uint32_t* __restrict__ nbr) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint64_t c0 = blockIdx.x * kFillTiles * kTile, c1 = min(E, c0 + kFillTiles * kTile);
-  for (uint64_t c = c0; c < c1; c += kTile) {
+  const uint64_t ahead = ((uint64_t)(gridDim.x - 1) * tiles + 1) * kTile;  // from the last of its tiles to the next first
+  uint32_t t = 1;
+  for (uint64_t c = (uint64_t)blockIdx.x * tiles * kTile; c < E; c += t == 1 ? ahead : kTile) {
+    t = t == tiles ? 1 : t + 1;
     uint64_t key[kAhead];
     uint32_t at[kAhead];
 #pragma unroll
@@ -1197,8 +1195,19 @@ void upload_entries(const PrepInput& in, uint64_t i0, uint64_t i1, cudaStream_t 
 // in one range's few MB of L2 instead of scattering over all rows.
 int presort_digit(uint64_t rows) { return 32 + bits_for(rows) - 8; }
 
-void fill_keys(const uint64_t* keys, uint64_t E, uint32_t* cur, uint32_t* nbr, cudaStream_t st) {
-  k_row_fill<<<(unsigned)ceil_div<uint64_t>(E, kFillTiles * kTile), kThreads, 0, st>>>(keys, E, cur, nbr);
+// Presorted keys of sparse rows are taken in launch order, four tiles a CTA, so
+// that the CTAs at work stay together in the keys and their stores in a few ranges
+// of rows (RMAT-24, 16 entries a vertex, 4.9 ms striding, now 3.8; RMAT-23
+// preprocessing 13.7 and 13.8, Erdos-Renyi of 2^27 entries on 2^23 vertices 10.0 and
+// 9.8). With more entries a row the CTAs would meet on its cursor and stride through
+// all keys instead (preprocessing striding and together: RMAT-22 of 32 entries a vertex
+// 12.0 and 12.2, RMAT-20 of 128 10.8 and 12.0, RMAT-16 of 2,048 8.1 and 16.3).
+void fill_keys(const uint64_t* keys, uint64_t E, uint64_t rows, bool presorted, uint32_t* cur, uint32_t* nbr,
+               cudaStream_t st) {
+  const bool together = presorted && E < 32 * rows;
+  const uint64_t tiles = together ? 4 : 1, most = together ? ~0ull : 148ull * 64;
+  k_row_fill<<<(unsigned)std::min<uint64_t>(ceil_div<uint64_t>(E, tiles * kTile), most), kThreads, 0, st>>>(
+      keys, E, (uint32_t)tiles, cur, nbr);
   TB_LAUNCH_CHECK();
 }
 
@@ -1223,7 +1232,7 @@ void fill_presorted(const PrepInput& in, uint64_t i0, uint64_t i1, const uint32_
   TB_LAUNCH_CHECK();
   const uint64_t* sorted =
       radix_sort<uint64_t, NoVal, false>(keys, keys_alt, nullptr, nullptr, E, top + 8, tmp, st, nullptr, top, true);
-  fill_keys(sorted, E, cur + r0, nbr, st);
+  fill_keys(sorted, E, z, true, cur + r0, nbr, st);
 }
 
 // Rows in degree-sized slots (2E entries in all, u32 offsets): no per-row
@@ -1278,7 +1287,7 @@ void run_rows(Arena& ar, const PrepInput& in, const uint32_t* rank, uint32_t* cn
     const uint64_t* sorted = keys;
     if (presort)
       sorted = radix_sort<uint64_t, NoVal, false>(keys, keys_alt, nullptr, nullptr, E, top + 8, ktmp, st, nullptr, top);
-    fill_keys(sorted, E, cnt, nbr, st);
+    fill_keys(sorted, E, n, presort && slots, cnt, nbr, st);
   }
   // Row u: nbr[off[u], cnt[u]) (with no entries every row is empty: 0, 0).
   sort_rows(off, cnt, (uint32_t)n, E, nbr, scratch, rp, lng, st);
